@@ -1,85 +1,198 @@
-// y = x W^T in true fp32 (no tensor-core mode has a 24-bit significand): 64 x 64 tiles, 4 x 4 outputs per thread,
-// operands through shared memory 16 k at a time.  Same three forms as the grouped tcgen05 kernel: plain, one weight
-// per head (column blocks of x and y), one weight per expert (row tiles of 128).  GLU: gate rows and, n rows further, up rows
-// side by side.  This serves the fp32 mode of the models that have one, where exactness matters more than speed.
+// y = x W^T in true fp32 (no tensor-core mode has a 24-bit significand), for the fp32 mode of the models that have one.  Same
+// three forms as the grouped tcgen05 kernel: plain, one weight per head (column blocks of x and y), one weight per expert (row
+// tiles of 128).  GLU: half of a tile's weight rows are gate rows, the other half the up rows n further.
+//
+// Bound by the FMA units: 8 x 8 outputs per thread in packed pairs.  A pair holds the sums over even and over odd k, so that both
+// operands are pairs as they lie in memory (k contiguous): no transposing, no duplicating, 16-byte cp.async into a ring and
+// 16-byte reads out of it, 128 packed FMAs for 16 reads.  Rows of a stage are 36 floats long: the eight lanes that read eight
+// neighbouring rows meet eight different groups of banks.  The KS groups of a CTA take 32 k each of a stage and add their sums up
+// in shared memory in a fixed order: a tile of 64 x 64 then has 256 threads, and 500 rows x 1024 columns already give 128 CTAs.
 #include "mdb_common.cuh"
 
 namespace mdb {
 
-constexpr int kF32Tile = 64, kF32K = 16;
+constexpr int kF32K = 32, kF32Ld = kF32K + 4;      // k of a group's stage; floats between rows
 
-template <bool GLU>
-__global__ void __launch_bounds__(256) gemm_f32_kernel(const mdb_gemm_args a) {
+template <int BM, int BN, int TM, int TN, int KS, int STAGES>
+struct F32Plan {
+  static constexpr int TX = BN / TN, TY = BM / TM, kGroup = TX * TY, kThreads = kGroup * KS;
+  static constexpr int kRows = BM + BN, kStage = KS * kRows * kF32Ld;                       // floats
+  static constexpr int kSmemBytes = STAGES * kStage * 4;
+  static_assert(TX % 8 == 0 && (KS == 1 || TM % KS == 0), "eight lanes share a row of x; the last sums are dealt out by rows");
+  static_assert(KS * BM * BN <= STAGES * kStage, "the groups' sums fit where the operands were");
+};
+
+__device__ __forceinline__ unsigned long long f32_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+template <int BM, int BN, int TM, int TN, int KS, int STAGES, bool GLU>
+__global__ void __launch_bounds__(F32Plan<BM, BN, TM, TN, KS, STAGES>::kThreads, 1) gemm_f32_kernel(const mdb_gemm_args a) {
+  using P = F32Plan<BM, BN, TM, TN, KS, STAGES>;
+  extern __shared__ __align__(16) float f32_smem[];
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ float xs[kF32K][kF32Tile + 4], ws[kF32K][kF32Tile + 4], us[GLU ? kF32K : 1][kF32Tile + 4];
-  int64_t row0 = static_cast<int64_t>(blockIdx.y) * kF32Tile, w_row0 = 0;
+  constexpr int kCols = GLU ? BN / 2 : BN;                 // output columns of a tile
+  const int64_t row0 = static_cast<int64_t>(blockIdx.y) * BM;
+  int64_t w_row0 = 0;
   int x_col = 0, y_col = 0;
   if (a.form == MDB_GEMM_HEADS) {
-    x_col = y_col = blockIdx.z;
     w_row0 = static_cast<int64_t>(blockIdx.z) * a.n;
-    x_col *= a.k;
-    y_col *= a.n;
+    x_col = blockIdx.z * a.k;
+    y_col = blockIdx.z * a.n;
   } else if (a.form == MDB_GEMM_EXPERTS) {
     const int tile = static_cast<int>(row0 / kMoeTileRows);
     if (tile >= *a.num_tiles) return;
     w_row0 = static_cast<int64_t>(a.tile_expert[tile]) * a.n;
   }
-  const float* x = static_cast<const float*>(a.x);
+  const float* x = static_cast<const float*>(a.x) + x_col;
   const float* w = static_cast<const float*>(a.w);
-  const int n0 = blockIdx.x * kF32Tile;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int lr = threadIdx.x >> 2, lk = (threadIdx.x & 3) * 4;      // loader: row of the tile, first of four k
-  float acc[4][4] = {}, up[4][4] = {};
-  for (int k0 = 0; k0 < a.k; k0 += kF32K) {
-    float4 xv = make_float4(0.f, 0.f, 0.f, 0.f), wv = xv, uv = xv;
-    if (row0 + lr < a.m) xv = *reinterpret_cast<const float4*>(x + (row0 + lr) * a.ldx + x_col + k0 + lk);
-    if (n0 + lr < a.n) wv = *reinterpret_cast<const float4*>(w + (w_row0 + n0 + lr) * a.k + k0 + lk);
-    if (GLU && n0 + lr < a.n) uv = *reinterpret_cast<const float4*>(w + (w_row0 + a.n + n0 + lr) * a.k + k0 + lk);
-    __syncthreads();
-    xs[lk][lr] = xv.x; xs[lk + 1][lr] = xv.y; xs[lk + 2][lr] = xv.z; xs[lk + 3][lr] = xv.w;
-    ws[lk][lr] = wv.x; ws[lk + 1][lr] = wv.y; ws[lk + 2][lr] = wv.z; ws[lk + 3][lr] = wv.w;
-    if (GLU) { us[GLU ? lk : 0][lr] = uv.x; us[GLU ? lk + 1 : 0][lr] = uv.y; us[GLU ? lk + 2 : 0][lr] = uv.z; us[GLU ? lk + 3 : 0][lr] = uv.w; }
-    __syncthreads();
+  const int n0 = blockIdx.x * kCols;
+  const uint32_t smem = smem_u32(f32_smem);
+
+  // 16-byte pieces of a stage: [group][x rows, then weight rows][eight of four k]; what lies outside arrives as zeros
+  auto fill = [&](int step) {
+    const uint32_t st = smem + (step % STAGES) * P::kStage * 4;
+    const int k_step = step * KS * kF32K;
+    for (int i = threadIdx.x; i < KS * P::kRows * (kF32K / 4); i += P::kThreads) {
+      const int c = i % (kF32K / 4), r = i / (kF32K / 4) % P::kRows, g = i / (kF32K / 4) / P::kRows;
+      const int k = k_step + g * kF32K + c * 4;
+      const float* src = x;
+      bool in = k < a.k;
+      if (r < BM) {
+        in = in && row0 + r < a.m;
+        src = x + (row0 + r) * a.ldx + k;
+      } else {
+        const int rw = r - BM, up = GLU && rw >= kCols ? 1 : 0, col = n0 + rw - up * kCols;
+        in = in && col < a.n;
+        src = w + (w_row0 + col + (up ? a.n : 0)) * a.k + k;
+      }
+      const uint32_t bytes = in ? 16u : 0u;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(st + ((g * P::kRows + r) * kF32Ld + c * 4) * 4),
+                   "l"(in ? src : static_cast<const float*>(a.w)), "r"(bytes) : "memory");
+    }
+  };
+
+  const int group = threadIdx.x / P::kGroup, lid = threadIdx.x % P::kGroup, tx = lid % P::TX, ty = lid / P::TX;
+  unsigned long long acc[TM][TN];
 #pragma unroll
-    for (int k = 0; k < kF32K; ++k) {
-      float xr[4], wr[4];
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) { xr[i] = xs[k][ty * 4 + i]; wr[i] = ws[k][tx * 4 + i]; }
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
+  const int steps = (a.k + KS * kF32K - 1) / (KS * kF32K);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+  for (int s = 0; s < STAGES - 1; ++s) {
+    if (s < steps) fill(s);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  for (int s = 0; s < steps; ++s) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+    __syncthreads();                                       // stage s is there for everyone, and stage s - 1 has been read
+    if (s + STAGES - 1 < steps) fill(s + STAGES - 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const float* st = f32_smem + (s % STAGES) * P::kStage + group * P::kRows * kF32Ld;
+    const float* xs = st + ty * kF32Ld;
+    const float* ws = st + (BM + tx) * kF32Ld;
+#pragma unroll 2
+    for (int k = 0; k < kF32K; k += 4) {
+      ulonglong2 xr[TM];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          acc[i][j] = fmaf(xr[i], wr[j], acc[i][j]);
-          if (GLU) up[i][j] = fmaf(xr[i], us[GLU ? k : 0][tx * 4 + j], up[i][j]);
-        }
+      for (int i = 0; i < TM; ++i) xr[i] = *reinterpret_cast<const ulonglong2*>(xs + i * P::TY * kF32Ld + k);
+#pragma unroll
+      for (int j = 0; j < TN; ++j) {
+        const ulonglong2 wr = *reinterpret_cast<const ulonglong2*>(ws + j * P::TX * kF32Ld + k);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) acc[i][j] = f32_fma2(xr[i].x, wr.x, acc[i][j]);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) acc[i][j] = f32_fma2(xr[i].y, wr.y, acc[i][j]);
+      }
     }
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
   float* y = static_cast<float*>(a.y);
+  auto leave = [&](int i, const float (&v)[TN]) {          // row i of the thread's outputs
+    const int64_t row = row0 + i * P::TY + ty;
+    if (row >= a.m) return;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int64_t row = row0 + ty * 4 + i;
-    if (row >= a.m) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int col = n0 + tx * 4 + j;
+    for (int j = 0; j < (GLU ? TN / 2 : TN); ++j) {
+      const int col = n0 + j * P::TX + tx;
       if (col >= a.n) continue;
-      float v = acc[i][j];
-      if (a.act == MDB_ACT_RELU2) { v = fmaxf(v, 0.f); v *= v; }
-      if (a.act == MDB_ACT_SILU && col >= a.act_from) v /= 1.0f + expf(-v);
-      if (GLU) v = fmaxf(v, 0.f) * up[i][j];
-      y[row * a.ldy + y_col + col] = v;
+      float z = v[j];
+      if (a.act == MDB_ACT_RELU2) { z = fmaxf(z, 0.f); z *= z; }
+      if (a.act == MDB_ACT_SILU && col >= a.act_from) z /= 1.0f + expf(-z);
+      if (GLU) z = fmaxf(z, 0.f) * v[GLU ? j + TN / 2 : 0];
+      y[row * a.ldy + y_col + col] = z;
     }
+  };
+  auto sum = [](unsigned long long p) { return __uint_as_float(static_cast<uint32_t>(p)) + __uint_as_float(static_cast<uint32_t>(p >> 32)); };
+  if (KS == 1) {
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+      float v[TN];
+#pragma unroll
+      for (int j = 0; j < TN; ++j) v[j] = sum(acc[i][j]);
+      leave(i, v);
+    }
+    return;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) f32_smem[((group * TM + i) * TN + j) * P::kGroup + lid] = sum(acc[i][j]);
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < (KS == 1 ? 1 : TM / KS); ++r) {
+    const int i = group * (TM / KS) + r;
+    float v[TN];
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      v[j] = 0.f;
+#pragma unroll
+      for (int g = 0; g < KS; ++g) v[j] += f32_smem[((g * TM + i) * TN + j) * P::kGroup + lid];
+    }
+    leave(i, v);
   }
 }
 
+template <int BM, int BN, int TM, int TN, int KS, int STAGES, bool GLU>
+static int gemm_f32_run(const mdb_gemm_args& a, cudaStream_t st) {
+  using P = F32Plan<BM, BN, TM, TN, KS, STAGES>;
+  auto kernel = gemm_f32_kernel<BM, BN, TM, TN, KS, STAGES, GLU>;
+  static PerDeviceOnce attr_once;
+  const int dev = attr_once.slot();
+  if (dev < 0) return MDB_ERR_CUDA;
+  if (!attr_once.done[dev]) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P::kSmemBytes) != cudaSuccess) return MDB_ERR_CUDA;
+    attr_once.done[dev] = true;
+  }
+  const int cols = GLU ? BN / 2 : BN;
+  const int64_t row_tiles = (static_cast<int64_t>(a.m) + BM - 1) / BM;
+  const dim3 grid((a.n + cols - 1) / cols, static_cast<int>(row_tiles), a.form == MDB_GEMM_HEADS ? a.heads : 1);
+  return mdb_launch(kernel, grid, dim3(P::kThreads), P::kSmemBytes, st, a);
+}
+
+// Rounds of 148 tiles times the FMA time of a tile per k: 128 cycles for 128 x 128 (a tenth less, it reads half as much through
+// L2), 32 for 64 x 64, and 8 for 16 x 32, whose 4 x 4 outputs per thread are bound by shared memory at half the FMA rate.
+template <bool GLU>
+static int gemm_f32_dispatch(const mdb_gemm_args& a, cudaStream_t st) {
+  const int64_t z = a.form == MDB_GEMM_HEADS ? a.heads : 1, n = GLU ? 2LL * a.n : a.n;
+  auto rounds = [&](int bm, int bn) {
+    return (((static_cast<int64_t>(a.m) + bm - 1) / bm) * ((n + bn - 1) / bn) * z + 147) / 148;
+  };
+  const int64_t wide = rounds(128, 128) * 115, mid = rounds(64, 64) * 32, narrow = rounds(16, 32) * 8;
+  // grids reach 65535 row tiles: as many rows as tiles of 64 allowed
+  if (narrow < mid && narrow < wide && a.m <= 16 * 65535) return gemm_f32_run<16, 32, 4, 4, 4, 4, GLU>(a, st);
+  if (mid < wide) return gemm_f32_run<64, 64, 8, 8, 4, 3, GLU>(a, st);
+  return gemm_f32_run<128, 128, 8, 8, 1, 4, GLU>(a, st);
+}
+
 static int gemm_f32_launch(const mdb_gemm_args& a, cudaStream_t st) {
-  if (a.k % kF32K != 0) return MDB_ERR_UNSUPPORTED;
-  const int64_t row_tiles = (static_cast<int64_t>(a.m) + kF32Tile - 1) / kF32Tile;
-  if (row_tiles > 65535 || a.heads > 65535) return MDB_ERR_UNSUPPORTED;
-  const dim3 grid((a.n + kF32Tile - 1) / kF32Tile, static_cast<int>(row_tiles), a.form == MDB_GEMM_HEADS ? a.heads : 1);
-  if (a.act == MDB_ACT_RELU_GLU) return mdb_launch(gemm_f32_kernel<true>, grid, dim3(256), 0, st, a);
-  return mdb_launch(gemm_f32_kernel<false>, grid, dim3(256), 0, st, a);
+  if (a.k % 16 != 0) return MDB_ERR_UNSUPPORTED;
+  if ((static_cast<int64_t>(a.m) + 63) / 64 > 65535 || a.heads > 65535) return MDB_ERR_UNSUPPORTED;
+  return a.act == MDB_ACT_RELU_GLU ? gemm_f32_dispatch<true>(a, st) : gemm_f32_dispatch<false>(a, st);
 }
 
 }  // namespace mdb

@@ -1,0 +1,133 @@
+"""The fp32 products and the scans in blocks of 16 tokens at the edges of their tiles, blocks and dispatch rules."""
+import importlib
+
+import pytest
+import torch
+
+from oracle import hybrid_oracle as orc
+
+pkg = importlib.import_module("mineru-diffusion_b200")
+ops = pkg.ops
+pytestmark = pytest.mark.gpu
+DEV, F32, F64 = "cuda", torch.float32, torch.float64
+
+
+def gen(seed):
+    return torch.Generator().manual_seed(seed)
+
+
+def rel(got, ref):
+    got, ref = got.double().cpu(), ref.double().cpu()
+    return float((got - ref).norm() / ref.norm().clamp_min(1e-30))
+
+
+# tiles of 16 x 32, 64 x 64 and 128 x 128, with rows, columns and k that fill none of them.  An fp32 sum of k products is off by
+# at most k * 2^-24 and, with errors of either sign, by about sqrt(k) * 2^-24 = 2.7e-6 at k = 2000.
+@pytest.mark.parametrize("m,n,k", [(1, 4, 16), (15, 36, 48), (17, 132, 144), (63, 1028, 272), (65, 1000, 528), (129, 4100, 80), (500, 1024, 2000),
+                                   (1030, 2300, 112), (2050, 2052, 176)])
+@pytest.mark.parametrize("act", [ops.ACT_NONE, ops.ACT_RELU2, ops.ACT_RELU_GLU, ops.ACT_SILU])
+def test_fp32_product_tiles(m, n, k, act):
+    x, w = torch.randn(m, k + 8, generator=gen(1)), torch.randn(2 * n if act == ops.ACT_RELU_GLU else n, k, generator=gen(2)) * k ** -0.5
+    y = torch.full((m + 1, n + 4), 7.0, device=DEV)
+    ops.gemm(x.to(DEV)[:, :k], w.to(DEV), y[:m, :n], act=act, act_from=4 if act == ops.ACT_SILU else 0)
+    z = x[:, :k].to(DEV, F64) @ w.to(DEV, F64).T
+    if act == ops.ACT_RELU2:
+        z = torch.relu(z) ** 2
+    elif act == ops.ACT_RELU_GLU:
+        z = torch.relu(z[:, :n]) * z[:, n:]
+    elif act == ops.ACT_SILU:
+        z[:, 4:] = torch.nn.functional.silu(z[:, 4:])
+    assert rel(y[:m, :n], z) < 3e-6
+    assert float((y[:m, n:] - 7).abs().max()) == 0 and float((y[m] - 7).abs().max()) == 0
+    assert pkg._lib.device_status() == 0
+
+
+def _portions(counts, starts, slots):
+    cu = torch.tensor([0] + list(counts)).cumsum(0)
+    row_seq = torch.cat([torch.full((n,), i) for i, n in enumerate(counts)])
+    return tuple(torch.as_tensor(x).to(torch.int32).to(DEV) for x in (row_seq, cu, starts, slots))
+
+
+def mlstm_parts(q, k, v, li, lf):
+    S, n, m = torch.zeros(q.shape[1], q.shape[2], v.shape[2], dtype=F64), torch.zeros(q.shape[1:], dtype=F64), torch.zeros(q.shape[1], dtype=F64)
+    num, den = [], []
+    for t in range(len(q)):
+        new = torch.maximum(lf[t] + m, li[t])
+        a, b, m = torch.exp(lf[t] + m - new), torch.exp(li[t] - new), new
+        S = a[:, None, None] * S + b[:, None, None] * k[t][:, :, None] * v[t][:, None]
+        n = a[:, None] * n + b[:, None] * k[t]
+        num.append(torch.einsum("hdv,hd->hv", S, q[t]))
+        den.append(torch.maximum((n * q[t]).sum(-1).abs(), torch.exp(-m)) + 1e-6)
+    return torch.stack(num), torch.stack(den)
+
+
+# token counts around a block, two portions one behind the other, a padding entry; columns that fill 16, 32 and 64 wide CTAs or
+# do not; one and several heads per key head; enough heads for the wide CTAs.  2e-6: thrice what the token by token form shows.
+@pytest.mark.parametrize("mode", [ops.SCAN_DELTA, ops.SCAN_MLSTM, ops.SCAN_DECAY])
+@pytest.mark.parametrize("H,KH,D,DV,bs", [(2, 1, 64, 24, 3), (3, 3, 128, 33, 3), (8, 4, 128, 80, 3), (20, 20, 128, 128, 3), (40, 40, 64, 70, 3)])
+def test_scan_in_blocks(mode, H, KH, D, DV, bs):
+    if mode == ops.SCAN_MLSTM:
+        KH = H
+    first, second, slots = [47, 16, 1], [17, 33, 31], [2, 0, 3]
+    rep, cols, nb = H // KH, DV + (mode == ops.SCAN_MLSTM), ops.scan_blocks(DV)
+    state = torch.full((5, H, cols, D), 5.0, device=DEV)            # a slot is never cleared
+    mst = torch.full((5, H, nb), 5.0, device=DEV)
+    total = [a + b for a, b in zip(first, second)]
+    g = gen(H + D)
+    k = torch.nn.functional.normalize(torch.randn(sum(total), KH, D, generator=g), dim=-1)
+    q = torch.randn(sum(total), KH, D, generator=g) * D ** -0.5
+    v = torch.randn(sum(total), H, DV, generator=g)
+    decay = torch.exp(-torch.exp(torch.randn(sum(total), H, D, generator=g) - 1))
+    decay[::7, :, ::5] = 0.0                                        # a decay may forget everything
+    beta = torch.rand(sum(total), H, generator=g)
+    li, lf = torch.randn(sum(total), H, generator=g) * 4, torch.nn.functional.logsigmoid(torch.randn(sum(total), H, generator=g) * 3 + 1)
+    skip = torch.randn(H, generator=g)
+    base = [0] + torch.tensor(total).cumsum(0).tolist()
+    got_o, got_d = torch.zeros(sum(total), H, DV), torch.ones(sum(total), H)
+    for part, counts in enumerate((first, second)):
+        rows = torch.cat([torch.arange(base[i] + (first[i] if part else 0), base[i] + (first[i] if part else 0) + n) for i, n in enumerate(counts)])
+        pad = torch.cat([rows, rows[:20]])                           # a padding entry of 20 rows: nothing is read or written for it
+        m = len(pad)
+        p = _portions(counts + [20], [first[i] if part else 0 for i in range(3)] + [0], slots + [-1])
+        at = lambda t: t[pad].contiguous().to(DEV)                   # noqa: E731,B023
+        o, den = torch.full((m, H, DV), 9.0, device=DEV), torch.full((m, H), 9.0, device=DEV)
+        if mode == ops.SCAN_DELTA:
+            sc = torch.full((m, H, 4), 9.0, device=DEV)
+            sc[..., 3] = at(beta)
+            ops.scan(mode, F32, 4, H, KH, D, DV, at(q), at(k), at(v), None, None, state, p, g=at(decay), scalars=sc, out=o)
+        elif mode == ops.SCAN_MLSTM:
+            ops.scan(mode, F32, 4, H, KH, D, DV, at(q), at(k), at(v), at(li), at(lf), state, p, mstate=mst, out=o, den=den)
+        else:
+            ops.scan(mode, F32, 4, H, KH, D, DV, at(q), at(k), at(v), at(decay[..., 1]), at(beta), state, p, out=o, skip=skip.to(DEV))
+        assert float((o[-20:] - 9).abs().max()) == 0
+        got_o[rows], got_d[rows] = o[:-20].cpu(), den[:-20].cpu()
+    assert pkg._lib.device_status() == 0
+    assert float((state[[1, 4]] - 5).abs().max()) == 0
+    for i in range(3):
+        r = slice(base[i], base[i + 1])
+        qq, kk, vv = (t[r].double().repeat_interleave(rep, 1) if t is not v else t[r].double() for t in (q, k, v))
+        if mode == ops.SCAN_DELTA:
+            ref = orc.delta_scan(qq, kk, vv, decay[r].double(), beta[r].double())
+            assert rel(got_o[r], ref) < 2e-6, i
+        elif mode == ops.SCAN_MLSTM:
+            # numerator and denominator by themselves: their quotient is as ill-conditioned as |n . q| is small
+            num, den = mlstm_parts(qq, kk, vv, li[r].double(), lf[r].double())
+            assert rel(got_o[r], num) < 2e-6 and rel(got_d[r], den) < 2e-6, i
+        else:
+            S, ref = torch.zeros(H, DV, D, dtype=F64), []
+            for t in range(len(qq)):
+                S = decay[r][t, :, 1].double()[:, None, None] * S + beta[r][t].double()[:, None, None] * vv[t][:, :, None] * kk[t][:, None]
+                ref.append(torch.einsum("hvd,hd->hv", S, qq[t]) + skip.double()[:, None] * vv[t])
+            assert rel(got_o[r], torch.stack(ref)) < 2e-6, i
+            assert rel(state[slots[i]], S) < 2e-6, i
+
+
+def test_scan_in_blocks_keeps_the_future_out():
+    """Values behind a token, whatever they are, do not reach its output."""
+    H, D, DV, T = 2, 128, 40, 32
+    q, k, v = (torch.randn(T, H, n, generator=gen(i), device="cpu") for i, n in enumerate((D, D, DV)))
+    v[21] = float("inf")
+    o = torch.zeros(T, H, DV, device=DEV)
+    ops.scan(ops.SCAN_DECAY, F32, 1, H, H, D, DV, q.to(DEV), k.to(DEV), v.to(DEV), torch.full((T, H), 0.9, device=DEV), torch.ones(T, H, device=DEV),
+             torch.zeros(1, H, DV, D, device=DEV), _portions([T], [0], [0]), out=o)
+    assert bool(torch.isfinite(o[:21]).all()) and not bool(torch.isfinite(o[21:]).any())
