@@ -573,6 +573,7 @@ typedef struct {
   void* y;
   int64_t ldy;
   const float* skip; /* DECAY */
+  int64_t rows;      /* m, rows of all portions (0: unknown): picks the form of a prompt's scan */
 } mdb_scan_args;
 int mdb_scan(const mdb_scan_args* args, mdb_stream_t stream);
 

@@ -954,6 +954,8 @@ __global__ void __launch_bounds__(COLS / CPT * 16) gated_scan_kernel(const mdb_s
     for (int b = block0; b < blocks && b * kScanBlockCols < w.col0 + COLS; ++b) mstate[b] = run_max;
 }
 
+#include "scan_blocks.cuh"
+
 // One-token form: every sequence brings one token and a CTA owns all columns of a head.  The delta rule's decay is computed
 // from the raw projection; delta rule and mLSTM normalise and gate the head's output and store it as the next projection's
 // input, the decay scan (whose norms span heads) leaves it in fp32.  The state is
@@ -1159,6 +1161,16 @@ int launch_scan_prompt(const mdb_scan_args& a, cudaStream_t st) {
 template <int MODE, int DP>
 int launch_scan_dim(const mdb_scan_args& a, cudaStream_t st) {
   if (a.fused) return a.dtype == MDB_F32 ? launch_scan_token<float, MODE, DP / 32>(a, st) : launch_scan_token<bf16, MODE, DP / 32>(a, st);
+  if constexpr (DP <= 128) {
+    // In blocks of 16 tokens, from portions of 16 tokens on average up; 64 columns per CTA, or 32 or 16 where their CTAs still
+    // run all at once.
+    if (a.rows >= static_cast<int64_t>(kSbTokens) * a.bs) {
+      const int64_t heads = static_cast<int64_t>(a.heads) * a.bs;
+      if ((a.vdim + 15) / 16 * heads <= 148) return launch_scan_blocks<MODE, DP, 2>(a, st);
+      if ((a.vdim + 31) / 32 * heads <= 148) return launch_scan_blocks<MODE, DP, 4>(a, st);
+      return launch_scan_blocks<MODE, DP, 8>(a, st);
+    }
+  }
   // blocks of 32 columns while they fill the SMs, narrower ones (more re-reads of k, q and g) below that
   const int64_t wide = static_cast<int64_t>((a.vdim + 31) / 32) * a.heads * a.bs;
   return wide >= 148 ? launch_scan_prompt<MODE, DP, 32>(a, st) : launch_scan_prompt<MODE, DP, 16>(a, st);

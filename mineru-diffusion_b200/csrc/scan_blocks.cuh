@@ -1,0 +1,528 @@
+// Scans of prompt portions in blocks of 16 tokens, still in fp32 FMAs (included by recurrent.cu, inside its namespace).
+//
+// With G_t the product of the decays of a block's tokens 1 .. t (per key channel in the delta rule, one number per head in the
+// other recurrences) and S the state in front of the block,
+//   u_t = beta_t (v_t - (G_t k_t) S - sum_{j<t} L_tj u_j),      L_tj = k_t . (k_j prod_{j<s<=t} g_s)
+//   o_t = (G_t q_t) S + sum_{j<=t} M_tj u_j,                    M_tj = q_t . (k_j prod_{j<s<=t} g_s)
+//   S  <- G_16 S + sum_j (k_j prod_{s>j} g_s) u_j^T
+// (other recurrences: u_t = b_t v_t, no L).  Every factor is a product of decays, never a quotient, so nothing can overflow and a
+// decay of zero is a zero.  A token then costs three FMAs per state element (two without L) and no sum over lanes of its
+// own; the token-by-token form spends four (three) and a chain of shuffles for every two tokens.
+//
+// What bounds it: FMA and issue slots of one warp per scheduler.  All the states of four prompts of 16 heads are 55 elements per
+// FMA lane of the chip, so a CTA has four warps that keep the state in registers (CPT columns x 1/16 of the channels a
+// thread: a 16-byte read of shared memory feeds 4 CPT FMAs) and four that prepare the next block meanwhile: its operands with
+// cp.async two blocks ahead, the scaled rows, L and M.  COLS = 8 CPT columns per CTA.
+constexpr int kSbTokens = 16, kSbThreads = 256, kSbRing = 3;
+
+template <int MODE, int DP, int CPT>
+struct SbPlan {
+  static constexpr bool DELTA = MODE == kScanDelta;
+  static constexpr int COLS = 8 * CPT, ROW = kSbTokens * DP;
+  // raw operands, a ring of three blocks: k, q (, g) rows, v, two scalars per token
+  static constexpr int RAW_Q = ROW, RAW_G = 2 * ROW, RAW_V = (DELTA ? 3 : 2) * ROW, RAW_S = RAW_V + kSbTokens * COLS, RAW = RAW_S + 2 * kSbTokens;
+  // prepared block, two of them: (delta) scaled k and q, k as the update takes it, G_16; L transposed, M; per token four floats
+  static constexpr int P_QH = DELTA ? ROW : 0, P_KT = 2 * P_QH, P_G = P_KT + (DELTA ? ROW : 0), P_L = P_G + (DELTA ? DP : 0),
+                       P_M = P_L + (DELTA ? 256 : 0), P_T = P_M + 256, PREP = P_T + 4 * kSbTokens;
+  static constexpr int OFF_PREP = kSbRing * RAW, OFF_R = OFF_PREP + 2 * PREP, OFF_U = OFF_R + (DELTA ? 2 : 1) * kSbTokens * COLS,
+                       OFF_N = OFF_U + 2 * kSbTokens * COLS, FLOATS = OFF_N + kSbTokens;
+  static constexpr int kSmemBytes = FLOATS * 4;
+};
+
+template <int WHICH> __device__ __forceinline__ void sb_bar() { asm volatile("bar.sync %0, 128;" ::"n"(WHICH) : "memory"); }
+
+// Sums 32 values over the 32 lanes: lane l returns the total of value l.
+__device__ __forceinline__ float reduce_scatter32(float (&r)[32], int lane) {
+#pragma unroll
+  for (int o = 16, cur = 16; o > 0; o >>= 1, cur >>= 1) {
+    const bool upper = (lane & o) != 0;
+#pragma unroll
+    for (int j = 0; j < cur; ++j) {
+      const float send = upper ? r[j] : r[j + cur], keep = upper ? r[j + cur] : r[j];
+      r[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  return r[0];
+}
+
+// Sums V values over 16 lanes, the lanes at distance O and less still to come: lane l returns the total of value l * V / (2 O).
+template <int V, int O = 8>
+__device__ __forceinline__ float sb_reduce16(const float (&r)[V], int l16) {
+  if constexpr (O == 0) {
+    return r[0];
+  } else if constexpr (V == 1) {
+    const float h[1] = {r[0] + __shfl_xor_sync(0xffffffffu, r[0], O)};
+    return sb_reduce16<1, O / 2>(h, l16);
+  } else {
+    const bool upper = (l16 & O) != 0;
+    float h[V / 2];
+#pragma unroll
+    for (int j = 0; j < V / 2; ++j) {
+      const float send = upper ? r[j] : r[j + V / 2], keep = upper ? r[j + V / 2] : r[j];
+      h[j] = keep + __shfl_xor_sync(0xffffffffu, send, O);
+    }
+    return sb_reduce16<V / 2, O / 2>(h, l16);
+  }
+}
+
+__device__ __forceinline__ float sum2(f32x2 v) { const float2 x = unpack2(v); return x.x + x.y; }
+
+template <int MODE, int DP, int CPT>
+__global__ void __launch_bounds__(kSbThreads, 1) scan_blocks_kernel(const mdb_scan_args a) {
+  using P = SbPlan<MODE, DP, CPT>;
+  constexpr bool DELTA = P::DELTA, MLSTM = MODE == kScanMlstm;
+  constexpr int COLS = P::COLS, T = kSbTokens, NR = DP / 64, NP = DP / 64;      // float4 per lane and column; channel pairs per lane of a row
+  extern __shared__ __align__(16) float sb_smem[];
+  pdl_launch_dependents();
+  pdl_wait();
+  const ScanJob w = scan_job<MODE, DP, COLS>(a);
+  if (!w.live) return;
+  const int blocks16 = (w.columns + kScanBlockCols - 1) / kScanBlockCols, block0 = w.col0 / kScanBlockCols;
+  float* mstate = MLSTM ? a.mstate + (static_cast<int64_t>(w.slot) * a.heads + w.head) * blocks16 : nullptr;
+  const int nblocks = (w.t_end - w.t_begin + T - 1) / T;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float* const R = sb_smem + P::OFF_R;      // (delta: k-side, then) q-side products with the state, [token][column]
+  float* const U = sb_smem + P::OFF_U;      // u as pairs (u, u), [token][column]
+
+  if (warp >= 4) {
+    // ------------------------------------------------------------------------------------------------ preparing warps
+    const int tid = threadIdx.x - 128, pw = warp - 4;
+    const bool v16 = (a.vdim & 3) == 0 && (reinterpret_cast<uintptr_t>(a.v) & 15) == 0;
+    auto fetch = [&](int b) {
+      if (b < nblocks) {
+        const int t0 = w.t_begin + b * T, n = min(T, w.t_end - t0);
+        float* st = sb_smem + (b % kSbRing) * P::RAW;
+        const uint32_t base = smem_u32(st);
+        for (int i = tid; i < T * (DP / 4); i += 128) {
+          const int t = i / (DP / 4), c = i % (DP / 4) * 4;
+          if (t < n) {
+            const int64_t krow = (static_cast<int64_t>(t0 + t) * a.kv_heads + w.kvh) * DP + c;
+            cp_async16(base + (t * DP + c) * 4, a.k + krow);
+            cp_async16(base + (P::RAW_Q + t * DP + c) * 4, a.q + krow);
+            if (DELTA) cp_async16(base + (P::RAW_G + t * DP + c) * 4, a.g + (static_cast<int64_t>(t0 + t) * a.heads + w.head) * DP + c);
+          } else {      // tokens behind the portion: no key, no query, no decay
+            *reinterpret_cast<float4*>(st + t * DP + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+            *reinterpret_cast<float4*>(st + P::RAW_Q + t * DP + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (DELTA) *reinterpret_cast<float4*>(st + P::RAW_G + t * DP + c) = make_float4(1.f, 1.f, 1.f, 1.f);
+          }
+        }
+        const float* v0 = a.v + (static_cast<int64_t>(t0) * a.heads + w.head) * a.vdim + w.col0;
+        const int64_t vstep = static_cast<int64_t>(a.heads) * a.vdim;
+        for (int i = tid; i < T * (COLS / 4); i += 128) {
+          const int t = i / (COLS / 4), c = i % (COLS / 4) * 4;
+          if (v16 && t < n && w.col0 + c < a.vdim) {
+            cp_async16(base + (P::RAW_V + t * COLS + c) * 4, v0 + t * vstep + c);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              if (t < n && w.col0 + c + e < a.vdim) cp_async4(base + (P::RAW_V + t * COLS + c + e) * 4, v0 + t * vstep + c + e);
+              else st[P::RAW_V + t * COLS + c + e] = 0.f;
+            }
+          }
+        }
+        if (tid < T) {
+          const int64_t th = static_cast<int64_t>(t0 + tid) * a.heads + w.head;
+          if (tid < n) {
+            if (DELTA) {
+              cp_async4(base + (P::RAW_S + 2 * tid) * 4, a.scalars + 4 * th + 3);
+            } else {
+              cp_async4(base + (P::RAW_S + 2 * tid) * 4, a.s0 + th);
+              cp_async4(base + (P::RAW_S + 2 * tid + 1) * 4, a.s1 + th);
+            }
+          } else {
+            // delta: no correction; mLSTM: input gate shut, forget gate open; decay scan: no decay, no step
+            st[P::RAW_S + 2 * tid] = DELTA ? 0.f : (MLSTM ? -INFINITY : 1.f);
+            st[P::RAW_S + 2 * tid + 1] = 0.f;
+          }
+        }
+      }
+      cp_async_commit();
+    };
+
+    float run_max = MLSTM && !w.fresh ? mstate[block0] : 0.f;
+    // the normaliser, one more column of the mLSTM's state: only the CTA of the first columns owns it, warp by warp alike
+    const bool norm = MLSTM && w.col0 == 0;
+    f32x2 nv[NP];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      nv[i] = 0ull;
+      if (norm && !w.fresh) {
+        const float2 x = *reinterpret_cast<const float2*>(w.state + static_cast<int64_t>(a.vdim) * DP + lane * 2 * NP + 2 * i);
+        nv[i] = pack2(x.x, x.y);
+      }
+    }
+    // lane's share of a row: NP channel pairs
+    auto row_pairs = [&](const float* row, f32x2 (&x)[NP]) {
+      if (NP == 2) {
+        lds2(row + lane * 4, x[0], x[NP - 1]);
+      } else {
+        x[0] = *reinterpret_cast<const f32x2*>(row + lane * 2);
+      }
+    };
+
+    auto prepare = [&](int b) {
+      const float* raw = sb_smem + (b % kSbRing) * P::RAW;
+      float* prep = sb_smem + P::OFF_PREP + (b & 1) * P::PREP;
+      float4* per_token = reinterpret_cast<float4*>(prep + P::P_T);
+      if (DELTA) {
+        for (int c = tid; c < DP; c += 128) {
+          float kk[T], gg[T], acc = 1.f;
+#pragma unroll
+          for (int t = 0; t < T; ++t) {
+            kk[t] = raw[t * DP + c];
+            gg[t] = raw[P::RAW_G + t * DP + c];
+            acc *= gg[t];
+            prep[t * DP + c] = acc * kk[t];
+            prep[P::P_QH + t * DP + c] = acc * raw[P::RAW_Q + t * DP + c];
+          }
+          prep[P::P_G + c] = acc;
+          acc = 1.f;
+#pragma unroll
+          for (int t = T - 1; t >= 0; --t) {
+            prep[P::P_KT + t * DP + c] = acc * kk[t];
+            acc *= gg[t];
+          }
+        }
+        if (tid < T) per_token[tid].x = raw[P::RAW_S + 2 * tid];      // beta
+        // L and M: a warp takes two neighbouring keys from either end, so that all warps have 36 pairs of tokens
+#pragma unroll 1
+        for (int pass = 0; pass < 2; ++pass) {
+          const int j0 = pass ? T - 2 - 2 * pw : 2 * pw;
+          f32x2 p[2][NP];
+          float acc[2][32];
+#pragma unroll
+          for (int t = 0; t < T; ++t) {
+#pragma unroll
+            for (int jj = 0; jj < 2; ++jj) acc[jj][2 * t] = acc[jj][2 * t + 1] = 0.f;
+            if (t < j0) continue;
+            f32x2 k[NP], q[NP], g[NP];
+            row_pairs(raw + t * DP, k);
+            row_pairs(raw + P::RAW_Q + t * DP, q);
+            row_pairs(raw + P::RAW_G + t * DP, g);
+#pragma unroll
+            for (int jj = 0; jj < 2; ++jj) {
+              if (t < j0 + jj) continue;
+              if (t == j0 + jj) {
+#pragma unroll
+                for (int i = 0; i < NP; ++i) p[jj][i] = k[i];
+              } else {
+                f32x2 s = 0ull;
+#pragma unroll
+                for (int i = 0; i < NP; ++i) {
+                  p[jj][i] = mul2(p[jj][i], g[i]);
+                  s = fma2(p[jj][i], k[i], s);
+                }
+                acc[jj][2 * t] = sum2(s);
+              }
+              f32x2 s = 0ull;
+#pragma unroll
+              for (int i = 0; i < NP; ++i) s = fma2(p[jj][i], q[i], s);
+              acc[jj][2 * t + 1] = sum2(s);
+            }
+          }
+#pragma unroll
+          for (int jj = 0; jj < 2; ++jj) {
+            const float total = reduce_scatter32(acc[jj], lane);
+            const int t = lane >> 1, j = j0 + jj;
+            if (lane & 1) prep[P::P_M + t * T + j] = total;
+            else prep[P::P_L + j * T + t] = raw[P::RAW_S + 2 * t] * total;      // beta_t L_tj
+          }
+        }
+      } else {
+        // gates of the block: forget and input factor per token, in the mLSTM relative to the running maximum
+        float fa = 1.f, fb = 0.f, em = 0.f;
+        {
+          const int l = lane & 15;
+          const float s0 = raw[P::RAW_S + 2 * l], s1 = raw[P::RAW_S + 2 * l + 1];
+          if (MLSTM) {
+            // m_t = max(f_t + m_(t-1), i_t) as a scan of the maps x -> max(x + F, I); tokens behind the portion keep m
+            float F = s1, I = s0;
+#pragma unroll
+            for (int o = 1; o < T; o <<= 1) {
+              const float Fp = __shfl_up_sync(0xffffffffu, F, o, 16), Ip = __shfl_up_sync(0xffffffffu, I, o, 16);
+              if (l >= o) { I = fmaxf(Ip + F, I); F += Fp; }
+            }
+            const float m = fmaxf(F + run_max, I);
+            float mp = __shfl_up_sync(0xffffffffu, m, 1, 16);
+            if (l == 0) mp = run_max;
+            fa = expf(s1 + mp - m);
+            fb = expf(s0 - m);
+            em = expf(-m);
+            run_max = __shfl_sync(0xffffffffu, m, T - 1);
+          } else {
+            fa = s0;
+            fb = s1;
+          }
+        }
+        // every lane: product of the forget factors of tokens 0 .. t, of those behind t, of those behind j up to t
+        const int t = lane & 15, jl = lane >> 4;
+        float head = 1.f, tail = 1.f;
+        float between[2] = {1.f, 1.f};
+#pragma unroll
+        for (int s = 0; s < T; ++s) {
+          const float f = __shfl_sync(0xffffffffu, fa, s);
+          if (s <= t) head *= f;
+          if (s > t) tail *= f;
+#pragma unroll
+          for (int pass = 0; pass < 2; ++pass) {
+            const int j = (pass ? T - 2 - 2 * pw : 2 * pw) + jl;
+            if (s > j && s <= t) between[pass] *= f;
+          }
+        }
+        if (pw == 0 && lane < T) per_token[lane] = make_float4(head, fb * tail, em, 0.f);
+#pragma unroll 1
+        for (int pass = 0; pass < 2; ++pass) {
+          const int j0 = pass ? T - 2 - 2 * pw : 2 * pw;
+          float acc[32];
+          f32x2 k[2][NP];
+          row_pairs(raw + j0 * DP, k[0]);
+          row_pairs(raw + (j0 + 1) * DP, k[1]);
+#pragma unroll
+          for (int t2 = 0; t2 < T; ++t2) {
+            acc[t2] = acc[T + t2] = 0.f;
+            if (t2 < j0) continue;
+            f32x2 q[NP];
+            row_pairs(raw + P::RAW_Q + t2 * DP, q);
+#pragma unroll
+            for (int jj = 0; jj < 2; ++jj) {
+              f32x2 s = 0ull;
+#pragma unroll
+              for (int i = 0; i < NP; ++i) s = fma2(k[jj][i], q[i], s);
+              acc[jj * T + t2] = sum2(s);
+            }
+          }
+          const float total = reduce_scatter32(acc, lane);      // q_t . k_j, t = lane & 15, j = j0 + lane / 16
+          const int j = j0 + jl;
+          const float bj = __shfl_sync(0xffffffffu, fb, j);
+          prep[P::P_M + t * T + j] = j <= t ? (pass ? between[1] : between[0]) * bj * total : 0.f;
+        }
+        if (norm) {
+          // q_t . n for a warp's four tokens, then n moves past the block (every warp alike)
+          float r4[4];
+#pragma unroll
+          for (int i4 = 0; i4 < 4; ++i4) {
+            f32x2 q[NP], s = 0ull;
+            row_pairs(raw + P::RAW_Q + (4 * pw + i4) * DP, q);
+#pragma unroll
+            for (int i = 0; i < NP; ++i) s = fma2(nv[i], q[i], s);
+            r4[i4] = warp_sum(sum2(s));
+          }
+          const float whole = __shfl_sync(0xffffffffu, head, T - 1);
+          f32x2 moved[NP];
+#pragma unroll
+          for (int i = 0; i < NP; ++i) moved[i] = mul2(nv[i], pack2(whole, whole));
+#pragma unroll
+          for (int s = 0; s < T; ++s) {
+            const float wj = __shfl_sync(0xffffffffu, fb * tail, s);
+            f32x2 k[NP];
+            row_pairs(raw + s * DP, k);
+#pragma unroll
+            for (int i = 0; i < NP; ++i) moved[i] = fma2(k[i], pack2(wj, wj), moved[i]);
+          }
+#pragma unroll
+          for (int i = 0; i < NP; ++i) nv[i] = moved[i];
+          sb_bar<2>();                                        // M is whole
+          if (lane < 4) {
+            const int tt = 4 * pw + lane, tok = w.t_begin + b * T + tt;
+            const float mine = lane == 0 ? r4[0] : lane == 1 ? r4[1] : lane == 2 ? r4[2] : r4[3];
+            const float4 pt = per_token[tt];
+            float s = 0.f;
+#pragma unroll
+            for (int j = 0; j < T; ++j) s += prep[P::P_M + tt * T + j];
+            if (tok < w.t_end) a.den[static_cast<int64_t>(tok) * a.heads + w.head] = fmaxf(fabsf(fmaf(pt.x, mine, s)), pt.z) + 1e-6f;
+          }
+        }
+      }
+    };
+
+    fetch(0);
+    fetch(1);
+    cp_async_wait<1>();
+    sb_bar<2>();
+    prepare(0);
+    __syncthreads();
+    for (int b = 0; b < nblocks; ++b) {
+      fetch(b + 2);                     // its place was read for the last time before the barrier
+      if (b + 1 < nblocks) {
+        cp_async_wait<1>();
+        sb_bar<2>();
+        prepare(b + 1);
+      }
+      __syncthreads();
+    }
+    cp_async_wait<0>();
+    if (norm && pw == 0) {
+#pragma unroll
+      for (int i = 0; i < NP; ++i) {
+        const float2 x = unpack2(nv[i]);
+        *reinterpret_cast<float2*>(w.state + static_cast<int64_t>(a.vdim) * DP + lane * 2 * NP + 2 * i) = x;
+      }
+    }
+    if (MLSTM && tid == 0) {
+      // the copies of the running maximum of this CTA's columns; the normaliser's belongs to the first CTA
+      for (int i = block0; i < blocks16 && i * kScanBlockCols < w.col0 + COLS && i * kScanBlockCols < a.vdim; ++i) mstate[i] = run_max;
+      if (norm && a.vdim % kScanBlockCols == 0) mstate[blocks16 - 1] = run_max;
+    }
+    return;
+  }
+
+  // ---------------------------------------------------------------------------------------------------- state warps
+  const int l16 = threadIdx.x & 15, cg = threadIdx.x >> 4, col = cg * CPT, mycol = w.col0 + col;
+  const float skip = MODE == kScanDecay && a.skip != nullptr ? a.skip[w.head] : 0.f;
+  f32x2 S[CPT][2 * NR];
+#pragma unroll
+  for (int i = 0; i < CPT; ++i)
+#pragma unroll
+    for (int c = 0; c < NR; ++c) {
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (!w.fresh && mycol + i < a.vdim)
+        x = *reinterpret_cast<const float4*>(w.state + static_cast<int64_t>(mycol + i) * DP + c * 64 + l16 * 4);
+      S[i][2 * c] = pack2(x.x, x.y);
+      S[i][2 * c + 1] = pack2(x.z, x.w);
+    }
+  __syncthreads();
+  for (int b = 0; b < nblocks; ++b) {
+    const float* raw = sb_smem + (b % kSbRing) * P::RAW;
+    const float* prep = sb_smem + P::OFF_PREP + (b & 1) * P::PREP;
+    const float4* per_token = reinterpret_cast<const float4*>(prep + P::P_T);
+    // products with the state in front of the block: of a token's k and q (delta), or of two tokens' q, per exchange
+    constexpr int ROWS = DELTA ? 2 * T : T;
+#pragma unroll 2
+    for (int r = 0; r < ROWS; r += 2) {
+      const float* x0 = DELTA ? prep + (r >> 1) * DP + l16 * 4 : raw + P::RAW_Q + r * DP + l16 * 4;
+      const float* x1 = DELTA ? prep + P::P_QH + (r >> 1) * DP + l16 * 4 : x0 + DP;
+      f32x2 acc[2][CPT];
+#pragma unroll
+      for (int i = 0; i < CPT; ++i) acc[0][i] = acc[1][i] = 0ull;
+#pragma unroll
+      for (int c = 0; c < NR; ++c) {
+        f32x2 y0[2], y1[2];
+        lds2(x0 + c * 64, y0[0], y0[1]);
+        lds2(x1 + c * 64, y1[0], y1[1]);
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int i = 0; i < CPT; ++i) {
+            acc[0][i] = fma2(S[i][2 * c + e], y0[e], acc[0][i]);
+            acc[1][i] = fma2(S[i][2 * c + e], y1[e], acc[1][i]);
+          }
+      }
+      float v[2 * CPT];
+#pragma unroll
+      for (int i = 0; i < CPT; ++i) {
+        v[i] = sum2(acc[0][i]);
+        v[CPT + i] = sum2(acc[1][i]);
+      }
+      const float total = sb_reduce16<2 * CPT>(v, l16);
+      constexpr int PER = 16 / (2 * CPT);                // lanes that hold the same sum
+      const int at = l16 / PER, which = at / CPT, i = at % CPT;
+      if (l16 % PER == 0) R[DELTA ? (which * T + (r >> 1)) * COLS + col + i : (r + which) * COLS + col + i] = total;
+    }
+    if (!DELTA) {
+      for (int i = threadIdx.x; i < T * COLS; i += 128) {
+        const float u = raw[P::RAW_V + i] * per_token[i / COLS].y;
+        *reinterpret_cast<float2*>(U + 2 * i) = make_float2(u, u);
+      }
+    }
+    sb_bar<1>();
+    if (DELTA) {
+      if (threadIdx.x < COLS) {
+        float u[T];
+#pragma unroll
+        for (int t = 0; t < T; ++t) u[t] = per_token[t].x * (raw[P::RAW_V + t * COLS + threadIdx.x] - R[t * COLS + threadIdx.x]);
+#pragma unroll
+        for (int j = 0; j < T; ++j) {
+          float l[T];
+#pragma unroll
+          for (int c = j / 4; c < T / 4; ++c) *reinterpret_cast<float4*>(l + 4 * c) = *reinterpret_cast<const float4*>(prep + P::P_L + j * T + 4 * c);
+#pragma unroll
+          for (int t = j + 1; t < T; ++t) u[t] = fmaf(-l[t], u[j], u[t]);
+          *reinterpret_cast<float2*>(U + 2 * (j * COLS + threadIdx.x)) = make_float2(u[j], u[j]);
+        }
+      }
+      sb_bar<1>();
+    }
+    // the state moves past the block
+    const float* kt = (DELTA ? prep + P::P_KT : raw) + l16 * 4;
+    if (DELTA) {
+#pragma unroll
+      for (int c = 0; c < NR; ++c) {
+        f32x2 g[2];
+        lds2(prep + P::P_G + l16 * 4 + c * 64, g[0], g[1]);
+#pragma unroll
+        for (int i = 0; i < CPT; ++i) {
+          S[i][2 * c] = mul2(S[i][2 * c], g[0]);
+          S[i][2 * c + 1] = mul2(S[i][2 * c + 1], g[1]);
+        }
+      }
+    } else {
+      const float whole = per_token[T - 1].x;
+      const f32x2 g = pack2(whole, whole);
+#pragma unroll
+      for (int i = 0; i < CPT; ++i)
+#pragma unroll
+        for (int c = 0; c < 2 * NR; ++c) S[i][c] = mul2(S[i][c], g);
+    }
+#pragma unroll 4
+    for (int t = 0; t < T; ++t) {
+      f32x2 u[CPT];
+#pragma unroll
+      for (int i = 0; i < CPT; i += 2) lds2(U + 2 * (t * COLS + col + i), u[i], u[i + 1]);
+#pragma unroll
+      for (int c = 0; c < NR; ++c) {
+        f32x2 k[2];
+        lds2(kt + t * DP + c * 64, k[0], k[1]);
+#pragma unroll
+        for (int i = 0; i < CPT; ++i) {
+          S[i][2 * c] = fma2(k[0], u[i], S[i][2 * c]);
+          S[i][2 * c + 1] = fma2(k[1], u[i], S[i][2 * c + 1]);
+        }
+      }
+    }
+    // outputs: a thread takes every (128 / COLS)-th token of a column
+    {
+      constexpr int STEP = 128 / COLS;
+      const int c = threadIdx.x % COLS, first = threadIdx.x / COLS;
+      float x[T];
+#pragma unroll
+      for (int j = 0; j < T; ++j) x[j] = DELTA ? U[2 * (j * COLS + c)] : raw[P::RAW_V + j * COLS + c];
+#pragma unroll
+      for (int t = first; t < T; t += STEP) {
+        const int tok = w.t_begin + b * T + t;
+        float m[T], o = DELTA ? R[(T + t) * COLS + c] : R[t * COLS + c] * per_token[t].x;
+#pragma unroll
+        for (int j = 0; j < T; j += 4) *reinterpret_cast<float4*>(m + j) = *reinterpret_cast<const float4*>(prep + P::P_M + t * T + j);
+#pragma unroll
+        for (int j = 0; j < T; ++j)
+          if (j <= t) o = fmaf(m[j], x[j], o);      // not behind t, where a value may be anything
+        if (MODE == kScanDecay) o = fmaf(skip, raw[P::RAW_V + t * COLS + c], o);
+        if (tok < w.t_end && w.col0 + c < a.vdim) a.out[(static_cast<int64_t>(tok) * a.heads + w.head) * a.vdim + w.col0 + c] = o;
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < CPT; ++i)
+    if (mycol + i < a.vdim) {
+#pragma unroll
+      for (int c = 0; c < NR; ++c) {
+        const float2 lo = unpack2(S[i][2 * c]), hi = unpack2(S[i][2 * c + 1]);
+        *reinterpret_cast<float4*>(w.state + static_cast<int64_t>(mycol + i) * DP + c * 64 + l16 * 4) = make_float4(lo.x, lo.y, hi.x, hi.y);
+      }
+    }
+}
+
+template <int MODE, int DP, int CPT>
+int launch_scan_blocks(const mdb_scan_args& a, cudaStream_t st) {
+  using P = SbPlan<MODE, DP, CPT>;
+  static_assert(P::kSmemBytes <= 227 * 1024, "shared memory of the scan in blocks");
+  auto kernel = scan_blocks_kernel<MODE, DP, CPT>;
+  static PerDeviceOnce attr_once;
+  const int dev = attr_once.slot();
+  if (dev < 0) return MDB_ERR_CUDA;
+  if (!attr_once.done[dev]) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P::kSmemBytes) != cudaSuccess) return MDB_ERR_CUDA;
+    attr_once.done[dev] = true;
+  }
+  return mdb_launch(kernel, dim3((a.vdim + P::COLS - 1) / P::COLS, a.heads, a.bs), dim3(kSbThreads), P::kSmemBytes, st, a);
+}
