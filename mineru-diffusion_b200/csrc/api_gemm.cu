@@ -65,14 +65,14 @@ int gemm_group_bf16(const mdb_gemm_args& a, cudaStream_t st) {
     t.heads = a.heads;
     t.a_rows = a.m >= kTcBM ? kTcBM : (a.m + 15) / 16 * 16;
     return launch_tc_group(static_cast<const bf16*>(a.x), static_cast<int64_t>(a.heads) * a.k, a.ldx, static_cast<const bf16*>(a.w),
-                           static_cast<int64_t>(a.heads) * a.n, t, st);
+                           static_cast<int64_t>(a.heads) * a.n, t, 0, st);
   }
   t.tile_expert = a.tile_expert;
   t.num_tiles = a.num_tiles;
   const int most = a.max_rows_per_expert;      // rows a tile can hold at most
   t.a_rows = most <= 0 || most >= kTcBM ? kTcBM : (most + 15) / 16 * 16;
   return launch_tc_group(static_cast<const bf16*>(a.x), a.k, a.ldx, static_cast<const bf16*>(a.w),
-                         static_cast<int64_t>(a.experts) * a.n, t, st);
+                         static_cast<int64_t>(a.experts) * a.n, t, a.experts, st);
 }
 
 }  // namespace

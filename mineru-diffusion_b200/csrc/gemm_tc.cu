@@ -30,7 +30,7 @@
 // tile and the number of tiles read from device memory; a step of few rows
 // loads only the rows a tile can hold).
 //
-// PAIR form (taken from 2048 rows on): a cluster of two CTAs owns a tile of
+// PAIR form (taken from 2048 rows on; per expert, from 160 rows an expert on): a cluster of two CTAs owns a tile of
 // 256 step rows x 256 weight rows (tcgen05.mma.cta_group::2).  Each CTA stages
 // its own 128 step rows (A) and its own 128 of the 256 weight rows (B) per k
 // stage -- 32 KB instead of 48 KB for half the output -- and the MMA, issued by
@@ -54,6 +54,7 @@ constexpr int kTcStages = 4;
 constexpr int kTcABytes = kTcBM * kTcBK * 2;   // 16 KB
 constexpr int kTcBBytes = kTcBN * kTcBK * 2;   // 32 KB
 constexpr int kTcPairStages = 6;               // PAIR: 16 KB of A + 16 KB of B per stage and CTA
+constexpr int kTcPairList = 8192;              // GROUP in pairs: row tiles the lists behind the barriers have room for
 constexpr int kTcLmEpiWarps = 16;
 constexpr int kTcLmRecBytes = 2 * kTcLmEpiWarps * 32 * 5 * 4;    // two buffers of per-warp sampler records
 __host__ __device__ constexpr int tc_epi_warps(int epi) { return epi == 2 ? kTcLmEpiWarps : 8; }
@@ -232,9 +233,43 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = misc[0];
+  // GROUP in pairs: first row tile of every pair, bit 15: alone (an expert's last tile); the staging area behind the barriers
+  // is free in this form
+  uint16_t* const pair_list = reinterpret_cast<uint16_t*>(tc_smem_raw + (base - raw) + bars_off + 256);
   if (EPI == kTcGroup && a.heads == 0) {
     pdl_wait();                            // the tile list comes from a preceding kernel
-    tiles = min(*a.num_tiles, a.tiles_m) * a.tiles_n;
+    const int row_tiles = min(*a.num_tiles, a.tiles_m);
+    tiles = row_tiles * a.tiles_n;
+    if (PAIR) {
+      uint16_t* const experts = pair_list + kTcPairList;
+      for (int t = threadIdx.x; t < row_tiles; t += blockDim.x) experts[t] = static_cast<uint16_t>(a.tile_expert[t]);
+      __syncthreads();
+      if (warp == 0) {
+        // an expert's tiles are neighbours: two and two from its first on
+        int run = 0, count = 0;            // first tile of the expert at hand, pairs so far
+        for (int t0 = 0; t0 < row_tiles; t0 += 32) {
+          const int t = t0 + lane;
+          const bool in = t < row_tiles;
+          int first = in && (t == 0 || experts[t] != experts[t - 1]) ? t : run;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, first, o);
+            if (lane >= o) first = max(first, up);
+          }
+          const bool start = in && ((t - first) & 1) == 0;
+          const uint32_t starts = __ballot_sync(0xffffffffu, start);
+          if (start) {
+            const bool alone = t + 1 >= row_tiles || experts[t + 1] != experts[t];
+            pair_list[count + __popc(starts & ((1u << lane) - 1u))] = static_cast<uint16_t>(t | (alone ? 0x8000 : 0));
+          }
+          count += __popc(starts);
+          run = __shfl_sync(0xffffffffu, first, 31);
+        }
+        if (lane == 0) misc[2] = static_cast<uint32_t>(count);
+      }
+      __syncthreads();
+      tiles = static_cast<int>(misc[2]) * a.tiles_n;
+    }
   }
   // GROUP: row tile, column tile and group (head or expert) of work item t
   auto group_tile = [&](int t, int& tn, int& tm, int& g) {
@@ -246,9 +281,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     } else {
       tm = t / a.tiles_n;
       tn = t % a.tiles_n;
+      if (PAIR) tm = pair_list[tm] & 0x7fff;
       g = a.tile_expert[tm];
     }
   };
+  // rows from one row tile to the next (GROUP counts in tiles of 128 rows whatever the form)
+  constexpr int kRowStep = EPI == kTcGroup ? kTcBM : kRowsPerTile;
   // where an epilogue warp reports that it has drained an accumulator buffer
   const uint32_t acc_empty_target = PAIR ? map_to_cta(bar_acc_empty, 0) : bar_acc_empty;
   auto arrive_acc_empty = [&](int acc_buf) {
@@ -281,7 +319,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         // own 128 weight rows (SiLU form: the leader holds the gate rows, the peer the up rows)
         if (rank == 0) mbar_arrive_expect_tx_w(bar_full + 8 * stage, 2 * (kTcABytes + kBBytes));
         const int brow = EPI == kTcSwiglu ? (rank == 0 ? tn * 128 : a.inter + tn * 128)
-                                          : tn * kTcBN + static_cast<int>(rank) * 128;
+                                          : w_row + tn * kTcBN + static_cast<int>(rank) * 128;
         tma_load_2d_pair_w(bdst, &map_w, c * kTcBK, brow, full);
       } else {
         mbar_arrive_expect_tx_w(full, a_bytes + kTcBBytes);
@@ -296,7 +334,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     auto load_rows = [&](int stage, int c, int tm) {
       const uint32_t full = full_target + 8 * stage;
       const uint32_t adst = a_tiles + stage * kTcABytes;
-      if (PAIR) tma_load_2d_pair_w(adst, &map_x, c * kTcBK, tm * kRowsPerTile + static_cast<int>(rank) * kTcBM, full);
+      if (PAIR) tma_load_2d_pair_w(adst, &map_x, c * kTcBK, tm * kRowStep + static_cast<int>(rank) * kTcBM, full);
       else tma_load_2d_w(adst, &map_x, x_col + c * kTcBK, tm * kTcBM, full);
     };
     // Weights are written by no kernel of a step: the first ring-full of weight tiles is requested before the
@@ -416,7 +454,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       tc_fence_after();
       const int quarter = warp & 3;       // the 32 tensor-memory lanes this warp may read
       const uint32_t taddr = tmem_base + acc * kTcBN + (static_cast<uint32_t>(32 * quarter) << 16);
-      const int row = tm * kRowsPerTile + static_cast<int>(rank) * kTcBM + 32 * quarter + lane;
+      int row = tm * kRowStep + static_cast<int>(rank) * kTcBM + 32 * quarter + lane;
+      if (EPI == kTcGroup && PAIR && rank == 1 && (pair_list[t / a.tiles_n] & 0x8000)) row = a.m;      // nothing of this half leaves
       if (EPI == kTcBf16 && ks > 1) {
         // split-k cluster: every MMA of this CTA has completed, so the operand ring is idle (a cluster owns one
         // tile, nothing more will be loaded): park the fp32 partial tile there, one row per thread
@@ -868,6 +907,37 @@ static bool tc_supported(int epi, int m, int n, int k, int64_t ldx, int64_t ldy)
   return n % 8 == 0;
 }
 
+// Clusters of two CTAs, with programmatic dependent launch like every other kernel of the library.
+template <int EPI>
+static int launch_tc_pairs(int tiles, int smem, int sm_count, const CUtensorMap& map_x, const CUtensorMap& map_w, TcArgs& a, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(sm_count / 2 * 2);
+  cfg.blockDim = dim3(tc_threads(EPI));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  // CTA pairs the device holds at once (an odd SM of a processing cluster cannot host a pair)
+  static int max_pairs = 0;
+  if (max_pairs == 0) {
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_tc_kernel<EPI, true>, &cfg) != cudaSuccess || n <= 0) n = sm_count / 2;
+    max_pairs = n;
+  }
+  const int pairs = tiles < max_pairs ? tiles : max_pairs;
+  cfg.gridDim = dim3(2 * pairs);
+  a.grid = 2 * pairs;
+  cfg.numAttrs = g_opt_pdl ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, gemm_tc_kernel<EPI, true>, map_x, map_w, a) == cudaSuccess ? MDB_OK : MDB_ERR_CUDA;
+}
+
 template <int EPI, bool PAIR>
 static int launch_tc_impl(const bf16* x, int64_t ldx, const bf16* w, int w_rows, TcArgs& a, cudaStream_t st) {
   static int sm_count = 0;
@@ -943,41 +1013,41 @@ static int launch_tc_impl(const bf16* x, int64_t ldx, const bf16* w, int w_rows,
       return cudaLaunchKernelEx(&cfg, gemm_tc_kernel<EPI, PAIR>, map_x, map_w, a) == cudaSuccess ? MDB_OK : MDB_ERR_CUDA;
     }
   }
-  if (!PAIR)
+  if constexpr (!PAIR)
     return mdb_launch(gemm_tc_kernel<EPI, PAIR>, dim3(tiles < sm_count ? tiles : sm_count), dim3(tc_threads(EPI)), kSmem,
                       st, map_x, map_w, a);
-  // clusters of two CTAs, with programmatic dependent launch like every other kernel of the library
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(sm_count / 2 * 2);
-  cfg.blockDim = dim3(tc_threads(EPI));
-  cfg.dynamicSmemBytes = kSmem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  // CTA pairs the device holds at once (an odd SM of a processing cluster cannot host a pair)
-  static int max_pairs = 0;
-  if (max_pairs == 0) {
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm_tc_kernel<EPI, PAIR>, &cfg) != cudaSuccess || n <= 0) n = sm_count / 2;
-    max_pairs = n;
-  }
-  const int pairs = tiles < max_pairs ? tiles : max_pairs;
-  cfg.gridDim = dim3(2 * pairs);
-  a.grid = 2 * pairs;
-  cfg.numAttrs = g_opt_pdl ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, gemm_tc_kernel<EPI, PAIR>, map_x, map_w, a) == cudaSuccess ? MDB_OK : MDB_ERR_CUDA;
+  else
+    return launch_tc_pairs<EPI>(tiles, kSmem, sm_count, map_x, map_w, a, st);
 }
 
 // GROUP form: x [rows, x_cols], w [groups * n, k]; a.m = rows (of the buffer, in the per-expert form), a.heads or
 // the tile list, a.a_rows, a.y / a.y32, a.ldy, a.act set by the caller.
-static int launch_tc_group(const bf16* x, int64_t x_cols, int64_t ldx, const bf16* w, int64_t w_rows, TcArgs& a, cudaStream_t st) {
+template <bool PAIR>
+static int launch_tc_group_as(const bf16* x, int64_t x_cols, int64_t ldx, const bf16* w, int64_t w_rows, TcArgs& a, int sm_count, cudaStream_t st) {
+  constexpr int kSmem = 1024 + (PAIR ? kTcPairStages * (kTcABytes + kTcBBytes / 2) : kTcStages * (kTcABytes + kTcBBytes)) + 256 +
+                        tc_epi_warps(kTcGroup) * 4096;
+  CUtensorMap map_x, map_w;
+  if (!get_tensor_map(x, a.m, x_cols, ldx, a.a_rows, &map_x)) return MDB_ERR_CUDA;
+  if (!get_tensor_map(w, w_rows, a.k, a.k, PAIR ? 128 : kTcBN, &map_w)) return MDB_ERR_CUDA;
+  static PerDeviceOnce attr_once;
+  const int dev = attr_once.slot();
+  if (dev < 0) return MDB_ERR_CUDA;
+  if (!attr_once.done[dev]) {
+    if (cudaFuncSetAttribute(gemm_tc_kernel<kTcGroup, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess)
+      return MDB_ERR_CUDA;
+    attr_once.done[dev] = true;
+  }
+  const int64_t tiles = static_cast<int64_t>(a.tiles_m) * a.tiles_n * (a.heads > 0 ? a.heads : 1);
+  if (tiles > (1 << 30)) return MDB_ERR_UNSUPPORTED;
+  if constexpr (PAIR) return launch_tc_pairs<kTcGroup>(static_cast<int>(tiles), kSmem, sm_count, map_x, map_w, a, st);
+  a.grid = tiles < sm_count ? static_cast<int>(tiles) : sm_count;
+  return mdb_launch(gemm_tc_kernel<kTcGroup, false>, dim3(a.grid), dim3(tc_threads(kTcGroup)), kSmem, st, map_x, map_w, a);
+}
+
+// `experts`: how many share the rows (0: per-head form).  CTA pairs where an expert has 160 rows or more on average, so that
+// most have two row tiles: a pair computes two tiles of one expert from one copy of its weights in shared memory, whose
+// bandwidth bounds the single form; an expert's odd last tile leaves half of its pair idle.
+static int launch_tc_group(const bf16* x, int64_t x_cols, int64_t ldx, const bf16* w, int64_t w_rows, TcArgs& a, int experts, cudaStream_t st) {
   static int sm_count = 0;
   if (sm_count == 0) {
     int dev = 0;
@@ -985,25 +1055,14 @@ static int launch_tc_group(const bf16* x, int64_t x_cols, int64_t ldx, const bf1
     cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
     if (sm_count <= 0) sm_count = 148;
   }
-  constexpr int kSmem = 1024 + kTcStages * (kTcABytes + kTcBBytes) + 256 + tc_epi_warps(kTcGroup) * 4096;
   a.tiles_m = (a.m + kTcBM - 1) / kTcBM;
   a.tiles_n = (a.n + kTcBN - 1) / kTcBN;
   a.ksplit = 1;
-  CUtensorMap map_x, map_w;
-  if (!get_tensor_map(x, a.m, x_cols, ldx, a.a_rows, &map_x)) return MDB_ERR_CUDA;
-  if (!get_tensor_map(w, w_rows, a.k, a.k, kTcBN, &map_w)) return MDB_ERR_CUDA;
-  static PerDeviceOnce attr_once;
-  const int dev = attr_once.slot();
-  if (dev < 0) return MDB_ERR_CUDA;
-  if (!attr_once.done[dev]) {
-    if (cudaFuncSetAttribute(gemm_tc_kernel<kTcGroup, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess)
-      return MDB_ERR_CUDA;
-    attr_once.done[dev] = true;
-  }
-  const int64_t tiles = static_cast<int64_t>(a.tiles_m) * a.tiles_n * (a.heads > 0 ? a.heads : 1);
-  if (tiles > (1 << 30)) return MDB_ERR_UNSUPPORTED;
-  a.grid = tiles < sm_count ? static_cast<int>(tiles) : sm_count;
-  return mdb_launch(gemm_tc_kernel<kTcGroup, false>, dim3(a.grid), dim3(tc_threads(kTcGroup)), kSmem, st, map_x, map_w, a);
+  // the buffer holds the rows and up to one tile of padding per expert
+  if (g_opt_gemm_pair != 0 && experts > 0 && a.a_rows == kTcBM && a.tiles_m < kTcPairList && experts < 65536 &&
+      4 * (a.tiles_m - experts) >= 5 * experts)
+    return launch_tc_group_as<true>(x, x_cols, ldx, w, w_rows, a, sm_count, st);
+  return launch_tc_group_as<false>(x, x_cols, ldx, w, w_rows, a, sm_count, st);
 }
 
 // CTA pairs from 2048 rows on (measured: +12 .. 15 % on the bf16-store projections at 4096 and 16384 rows, even at

@@ -83,7 +83,8 @@ __global__ void __launch_bounds__(kRouteWarps * 32) moe_route_kernel(const mdb_m
 
 // One CTA.  counts -> first row of every expert (multiples of 128) -> tile list -> a row for every (token, k) pair.
 // The order of the rows of one expert is not fixed; every row's result is independent of its place.
-constexpr int kPlanThreads = 1024;
+// Bound by the latency of its two walks over the ids, so a thread has kPlanBatch of them in flight.
+constexpr int kPlanThreads = 1024, kPlanBatch = 8;
 __global__ void __launch_bounds__(kPlanThreads) moe_plan_kernel(const mdb_moe_plan_args a) {
   pdl_launch_dependents();
   pdl_wait();
@@ -94,9 +95,13 @@ __global__ void __launch_bounds__(kPlanThreads) moe_plan_kernel(const mdb_moe_pl
   for (int e = threadIdx.x; e < a.experts; e += kPlanThreads) count[e] = 0;
   __syncthreads();
   const int n = a.m * a.top;
-  for (int i = threadIdx.x; i < n; i += kPlanThreads) {
-    const int e = a.ids[i];
-    if (e >= 0 && e < a.experts) atomicAdd(&count[e], 1);
+  for (int i0 = threadIdx.x; i0 < n; i0 += kPlanThreads * kPlanBatch) {
+    int e[kPlanBatch];
+#pragma unroll
+    for (int b = 0; b < kPlanBatch; ++b) e[b] = i0 + b * kPlanThreads < n ? a.ids[i0 + b * kPlanThreads] : -1;
+#pragma unroll
+    for (int b = 0; b < kPlanBatch; ++b)
+      if (e[b] >= 0 && e[b] < a.experts) atomicAdd(&count[e[b]], 1);
   }
   __syncthreads();
   if (threadIdx.x < 32) {
@@ -129,15 +134,22 @@ __global__ void __launch_bounds__(kPlanThreads) moe_plan_kernel(const mdb_moe_pl
   for (int r = threadIdx.x; r < total_rows && r < cap; r += kPlanThreads) a.row_token[r] = -1;
   for (int e = threadIdx.x; e < a.experts; e += kPlanThreads) count[e] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < n; i += kPlanThreads) {
-    const int e = a.ids[i];
-    int slot = -1;
-    if (e >= 0 && e < a.experts) {
-      slot = first[e] + atomicAdd(&count[e], 1);
-      if (slot < cap) a.row_token[slot] = i / a.top;
-      else slot = -1;
+  for (int i0 = threadIdx.x; i0 < n; i0 += kPlanThreads * kPlanBatch) {
+    int e[kPlanBatch];
+#pragma unroll
+    for (int b = 0; b < kPlanBatch; ++b) e[b] = i0 + b * kPlanThreads < n ? a.ids[i0 + b * kPlanThreads] : -1;
+#pragma unroll
+    for (int b = 0; b < kPlanBatch; ++b) {
+      const int i = i0 + b * kPlanThreads;
+      if (i >= n) break;
+      int slot = -1;
+      if (e[b] >= 0 && e[b] < a.experts) {
+        slot = first[e[b]] + atomicAdd(&count[e[b]], 1);
+        if (slot < cap) a.row_token[slot] = i / a.top;
+        else slot = -1;
+      }
+      a.slot[i] = slot;
     }
-    a.slot[i] = slot;
   }
 }
 

@@ -132,12 +132,24 @@ __global__ void __launch_bounds__(kRes32Threads) residual_norm_kernel(const mdb_
     }
     if (a.moe_rows != nullptr) {
       float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int k = 0; k < a.moe_top; ++k) {
-        const int slot = a.moe_slot[row * a.moe_top + k];
-        if (slot < 0) continue;
-        const float w = a.moe_weight[row * a.moe_top + k];
-        const float4 e = act_load4(static_cast<const T*>(a.moe_rows) + slot * a.moe_ld + c);
-        d.x = fmaf(w, e.x, d.x); d.y = fmaf(w, e.y, d.y); d.z = fmaf(w, e.z, d.z); d.w = fmaf(w, e.w, d.w);
+      // four experts' rows at a time: one by one, the slot and the row behind it are two latencies per expert
+      for (int k0 = 0; k0 < a.moe_top; k0 += 4) {
+        int slot[4];
+        float w[4];
+        float4 e[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          slot[k] = k0 + k < a.moe_top ? a.moe_slot[row * a.moe_top + k0 + k] : -1;
+          w[k] = k0 + k < a.moe_top ? a.moe_weight[row * a.moe_top + k0 + k] : 0.f;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          e[k] = slot[k] >= 0 ? act_load4(static_cast<const T*>(a.moe_rows) + slot[k] * a.moe_ld + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (slot[k] < 0) continue;
+          d.x = fmaf(w[k], e[k].x, d.x); d.y = fmaf(w[k], e[k].y, d.y); d.z = fmaf(w[k], e[k].z, d.z); d.w = fmaf(w[k], e[k].w, d.w);
+        }
       }
       x.x += d.x; x.y += d.y; x.z += d.z; x.w += d.w;
     }

@@ -1,0 +1,111 @@
+"""Kernel forms at the edges of their tiles and dispatch rules: pairs of query tiles, shares of latent tiles, pairs of expert
+tiles."""
+import importlib
+
+import pytest
+import torch
+
+pkg = importlib.import_module("mineru-diffusion_b200")
+ops = pkg.ops
+pytestmark = pytest.mark.gpu
+DEV, BF, F64 = "cuda", torch.bfloat16, torch.float64
+
+
+def gen(seed):
+    return torch.Generator(device=DEV).manual_seed(seed)
+
+
+def rel(got, ref):
+    return float((got.double() - ref).norm() / ref.norm().clamp_min(1e-30))
+
+
+def i32(v):
+    return torch.tensor(v, dtype=torch.int32, device=DEV)
+
+
+# One, two and three query tiles per sequence (tiles of 128 / group tokens), a tile alone in its pair before and after whole
+# pairs, few tiles (one per unit) and more units than SMs.  P and the output are bf16: 2^-9 relative each.
+@pytest.mark.parametrize("hq,hkv", [(16, 8), (6, 2), (16, 2), (4, 4)])
+@pytest.mark.parametrize("lens", [[64], [1, 65, 129, 190], [700, 33, 64, 1000, 5, 321] * 4])
+def test_prompt_attention_pairs(hq, hkv, lens):
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    m, g = cu[-1], gen(hq + len(lens))
+    q, k, v = (torch.randn(m, h, 128, generator=g, device=DEV).to(BF) for h in (hq, hkv, hkv))
+    out = torch.zeros_like(q)
+    ops.sparse_attn_varlen(q, k, v, i32(cu), i32(cu), 32, max_seqlen=max(lens), out=out)
+    assert pkg._lib.device_status() == 0
+    for a, b in zip(cu, cu[1:]):
+        t = b - a
+        i = torch.arange(t, device=DEV)
+        pad = -t % 32
+        seen = i[None] < torch.clamp(((i + pad) // 32 + 1) * 32 - pad, max=t)[:, None]
+        kk, vv = (x[a:b].double().repeat_interleave(hq // hkv, 1) for x in (k, v))
+        s = torch.einsum("ihd,jhd->hij", q[a:b].double(), kk) * 128 ** -0.5
+        ref = torch.einsum("hij,jhd->ihd", torch.softmax(s.masked_fill(~seen, float("-inf")), -1), vv)
+        assert rel(out[a:b], ref) < 8e-3, (a, b)
+
+
+# Rows that end inside, on and behind a tile of 64 keys and a page, a padding row, one and two groups of heads, whole rows and
+# parts; whatever lies in the cache behind a context must not matter.  bf16 output: 2^-9.
+@pytest.mark.parametrize("width,heads", [(128, 3), (256, 16), (384, 20), (512, 16), (512, 33)])
+@pytest.mark.parametrize("nsplit", [1, 2, 5])
+def test_latent_attention_shares(width, heads, nsplit):
+    ctx = [1, 64, 65, 0, 256, 257, 1000, 700, 3, 511]
+    need = [(n + 255) // 256 for n in ctx]
+    perm, g = torch.randperm(sum(need), generator=torch.Generator().manual_seed(1)).tolist(), gen(width + heads)
+    table = torch.full((len(ctx), max(need)), -1, dtype=torch.int32)
+    cache = torch.full((sum(need) * 256, width), float("nan"), dtype=BF, device=DEV)
+    at = 0
+    for i, n in enumerate(ctx):
+        for p in range(need[i]):
+            page = perm[at]
+            at += 1
+            table[i, p] = page
+            rows = min(256, n - 256 * p)
+            cache[page * 256:page * 256 + rows] = torch.randn(rows, width, generator=g, device=DEV).to(BF)
+    m = len(ctx)
+    q = torch.randn(m, heads * width, generator=g, device=DEV).to(BF)
+    out = torch.full((m, heads * width), 7.0, dtype=BF, device=DEV)
+    ws = torch.full((max(16, ops.latent_attn_workspace_bytes(m, heads, width, nsplit)),), 255, dtype=torch.uint8, device=DEV)
+    ops.latent_attn(q, cache, table.to(DEV), i32(list(range(m))), i32([n - 1 for n in ctx]), heads, 0.11, out, nsplit, ws)
+    assert pkg._lib.device_status() == 0
+    for i, n in enumerate(ctx):
+        if n == 0:
+            assert float((out[i].float() - 7).abs().max()) == 0
+            continue
+        c = cache.view(-1, 256, width)[table[i, :need[i]].long().to(DEV)].flatten(0, 1)[:n].double()
+        p = torch.softmax(q[i].view(heads, width).double() @ c.T * 0.11, -1)
+        assert rel(out[i].view(heads, width), p @ c) < 4e-3, i
+
+
+# Around the rule for pairs (160 rows per expert), experts of one, two, three and no tiles, output columns that do not fill
+# the last tile, and more ids than the plan has in flight.
+@pytest.mark.parametrize("E,top,m,kind", [(4, 2, 300, "spread"), (4, 2, 400, "spread"), (8, 3, 900, "skewed"), (5, 1, 900, "one"), (64, 6, 2600, "spread")])
+@pytest.mark.parametrize("n", [264, 512])
+def test_expert_tiles_in_pairs(E, top, m, kind, n):
+    k, g = 128, gen(E + m)
+    ids = torch.stack([torch.randperm(E, generator=torch.Generator().manual_seed(i))[:top] for i in range(m)])
+    if kind == "one":
+        ids[:] = 3
+    elif kind == "skewed":
+        ids[: m - 7] = torch.tensor([1, 5, 6])
+    tiles = ops.moe_max_tiles(m, top, E)
+    slot, row_token = torch.full((m, top), -9, dtype=torch.int32, device=DEV), torch.full((tiles * 128,), -9, dtype=torch.int32, device=DEV)
+    tile_expert, num = torch.full((tiles,), -9, dtype=torch.int32, device=DEV), torch.full((1,), 1, dtype=torch.int32, device=DEV)
+    x, w = torch.randn(m, k, generator=g, device=DEV).to(BF), (torch.randn(E, n, k, generator=g, device=DEV) * k ** -0.5).to(BF)
+    xs, y = torch.zeros(tiles * 128, k, dtype=BF, device=DEV), torch.full((tiles * 128 + 1, n), 9.0, dtype=BF, device=DEV)
+    ops.moe_plan(ids.int().to(DEV), E, tiles, slot, row_token, tile_expert, num)
+    ops.moe_gather(x, xs, row_token, num, tiles)
+    ops.gemm_experts(xs, w, y[:-1], tile_expert, num, m)
+    assert pkg._lib.device_status() == 0
+    s = slot.cpu().long()
+    assert len(set(s.flatten().tolist())) == m * top and (tile_expert.cpu()[s // 128] == ids).all()
+    assert float((y[int(num) * 128:].float() - 9).abs().max()) == 0          # rows of no tile stay as they were
+    got = y[s.to(DEV)]
+    for e in range(E):
+        rows, at = (ids == e).nonzero(as_tuple=True)
+        if len(rows):
+            ref = x[rows.to(DEV)].double() @ w[e].double().T
+            assert rel(got[rows.to(DEV), at.to(DEV)], ref) < 4e-3, e
