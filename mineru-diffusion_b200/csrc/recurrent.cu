@@ -1166,9 +1166,8 @@ int launch_scan_dim(const mdb_scan_args& a, cudaStream_t st) {
     // run all at once.
     if (a.rows >= static_cast<int64_t>(kSbTokens) * a.bs) {
       const int64_t heads = static_cast<int64_t>(a.heads) * a.bs;
-      if ((a.vdim + 15) / 16 * heads <= 148) return launch_scan_blocks<MODE, DP, 2>(a, st);
-      if ((a.vdim + 31) / 32 * heads <= 148) return launch_scan_blocks<MODE, DP, 4>(a, st);
-      return launch_scan_blocks<MODE, DP, 8>(a, st);
+      if ((a.vdim + 15) / 16 * heads <= 148) return launch_scan_blocks<MODE, DP, 16, 2>(a, st);
+      return (a.vdim + 31) / 32 * heads <= 148 ? launch_scan_blocks<MODE, DP, 32, 4>(a, st) : launch_scan_blocks<MODE, DP, 64, 4>(a, st);
     }
   }
   // blocks of 32 columns while they fill the SMs, narrower ones (more re-reads of k, q and g) below that

@@ -9,16 +9,17 @@
 // decay of zero is a zero.  A token then costs three FMAs per state element (two without L) and no sum over lanes of its
 // own; the token-by-token form spends four (three) and a chain of shuffles for every two tokens.
 //
-// What bounds it: FMA and issue slots of one warp per scheduler.  All the states of four prompts of 16 heads are 55 elements per
-// FMA lane of the chip, so a CTA has four warps that keep the state in registers (CPT columns x 1/16 of the channels a
+// What bounds it: latency, with few warps per scheduler.  All the states of four prompts of 16 heads are 55 elements per FMA
+// lane of the chip.  A CTA has warps that keep COLS columns of the state in registers (CPT columns x 1/16 of the channels a
 // thread: a 16-byte read of shared memory feeds 4 CPT FMAs) and four that prepare the next block meanwhile: its operands with
-// cp.async two blocks ahead, the scaled rows, L and M.  COLS = 8 CPT columns per CTA.
-constexpr int kSbTokens = 16, kSbThreads = 256, kSbRing = 3;
+// cp.async two blocks ahead, the scaled rows, L and M.
+constexpr int kSbTokens = 16, kSbPrep = 128, kSbRing = 3;
 
-template <int MODE, int DP, int CPT>
+template <int MODE, int DP, int COLS, int CPT>
 struct SbPlan {
   static constexpr bool DELTA = MODE == kScanDelta;
-  static constexpr int COLS = 8 * CPT, ROW = kSbTokens * DP;
+  static constexpr int ROW = kSbTokens * DP;
+  static constexpr int MAIN = COLS / CPT * 16, THREADS = MAIN + kSbPrep;      // threads that keep the state; all
   // raw operands, a ring of three blocks: k, q (, g) rows, v, two scalars per token
   static constexpr int RAW_Q = ROW, RAW_G = 2 * ROW, RAW_V = (DELTA ? 3 : 2) * ROW, RAW_S = RAW_V + kSbTokens * COLS, RAW = RAW_S + 2 * kSbTokens;
   // prepared block, two of them: (delta) scaled k and q, k as the update takes it, G_16; L transposed, M; per token four floats
@@ -29,7 +30,7 @@ struct SbPlan {
   static constexpr int kSmemBytes = FLOATS * 4;
 };
 
-template <int WHICH> __device__ __forceinline__ void sb_bar() { asm volatile("bar.sync %0, 128;" ::"n"(WHICH) : "memory"); }
+template <int WHICH, int THREADS> __device__ __forceinline__ void sb_bar() { asm volatile("bar.sync %0, %1;" ::"n"(WHICH), "n"(THREADS) : "memory"); }
 
 // Sums 32 values over the 32 lanes: lane l returns the total of value l.
 __device__ __forceinline__ float reduce_scatter32(float (&r)[32], int lane) {
@@ -67,11 +68,11 @@ __device__ __forceinline__ float sb_reduce16(const float (&r)[V], int l16) {
 
 __device__ __forceinline__ float sum2(f32x2 v) { const float2 x = unpack2(v); return x.x + x.y; }
 
-template <int MODE, int DP, int CPT>
-__global__ void __launch_bounds__(kSbThreads, 1) scan_blocks_kernel(const mdb_scan_args a) {
-  using P = SbPlan<MODE, DP, CPT>;
+template <int MODE, int DP, int COLS, int CPT>
+__global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_blocks_kernel(const mdb_scan_args a) {
+  using P = SbPlan<MODE, DP, COLS, CPT>;
   constexpr bool DELTA = P::DELTA, MLSTM = MODE == kScanMlstm;
-  constexpr int COLS = P::COLS, T = kSbTokens, NR = DP / 64, NP = DP / 64;      // float4 per lane and column; channel pairs per lane of a row
+  constexpr int MAIN = P::MAIN, T = kSbTokens, NR = DP / 64, NP = DP / 64;      // float4 per lane and column; channel pairs per lane of a row
   extern __shared__ __align__(16) float sb_smem[];
   pdl_launch_dependents();
   pdl_wait();
@@ -84,9 +85,9 @@ __global__ void __launch_bounds__(kSbThreads, 1) scan_blocks_kernel(const mdb_sc
   float* const R = sb_smem + P::OFF_R;      // (delta: k-side, then) q-side products with the state, [token][column]
   float* const U = sb_smem + P::OFF_U;      // u as pairs (u, u), [token][column]
 
-  if (warp >= 4) {
+  if (threadIdx.x >= MAIN) {
     // ------------------------------------------------------------------------------------------------ preparing warps
-    const int tid = threadIdx.x - 128, pw = warp - 4;
+    const int tid = threadIdx.x - MAIN, pw = warp - MAIN / 32;
     const bool v16 = (a.vdim & 3) == 0 && (reinterpret_cast<uintptr_t>(a.v) & 15) == 0;
     auto fetch = [&](int b) {
       if (b < nblocks) {
@@ -321,7 +322,7 @@ __global__ void __launch_bounds__(kSbThreads, 1) scan_blocks_kernel(const mdb_sc
           }
 #pragma unroll
           for (int i = 0; i < NP; ++i) nv[i] = moved[i];
-          sb_bar<2>();                                        // M is whole
+          sb_bar<2, kSbPrep>();                                        // M is whole
           if (lane < 4) {
             const int tt = 4 * pw + lane, tok = w.t_begin + b * T + tt;
             const float mine = lane == 0 ? r4[0] : lane == 1 ? r4[1] : lane == 2 ? r4[2] : r4[3];
@@ -338,14 +339,14 @@ __global__ void __launch_bounds__(kSbThreads, 1) scan_blocks_kernel(const mdb_sc
     fetch(0);
     fetch(1);
     cp_async_wait<1>();
-    sb_bar<2>();
+    sb_bar<2, kSbPrep>();
     prepare(0);
     __syncthreads();
     for (int b = 0; b < nblocks; ++b) {
       fetch(b + 2);                     // its place was read for the last time before the barrier
       if (b + 1 < nblocks) {
         cp_async_wait<1>();
-        sb_bar<2>();
+        sb_bar<2, kSbPrep>();
         prepare(b + 1);
       }
       __syncthreads();
@@ -419,12 +420,12 @@ __global__ void __launch_bounds__(kSbThreads, 1) scan_blocks_kernel(const mdb_sc
       if (l16 % PER == 0) R[DELTA ? (which * T + (r >> 1)) * COLS + col + i : (r + which) * COLS + col + i] = total;
     }
     if (!DELTA) {
-      for (int i = threadIdx.x; i < T * COLS; i += 128) {
+      for (int i = threadIdx.x; i < T * COLS; i += MAIN) {
         const float u = raw[P::RAW_V + i] * per_token[i / COLS].y;
         *reinterpret_cast<float2*>(U + 2 * i) = make_float2(u, u);
       }
     }
-    sb_bar<1>();
+    sb_bar<1, MAIN>();
     if (DELTA) {
       if (threadIdx.x < COLS) {
         float u[T];
@@ -440,7 +441,7 @@ __global__ void __launch_bounds__(kSbThreads, 1) scan_blocks_kernel(const mdb_sc
           *reinterpret_cast<float2*>(U + 2 * (j * COLS + threadIdx.x)) = make_float2(u[j], u[j]);
         }
       }
-      sb_bar<1>();
+      sb_bar<1, MAIN>();
     }
     // the state moves past the block
     const float* kt = (DELTA ? prep + P::P_KT : raw) + l16 * 4;
@@ -479,9 +480,9 @@ __global__ void __launch_bounds__(kSbThreads, 1) scan_blocks_kernel(const mdb_sc
         }
       }
     }
-    // outputs: a thread takes every (128 / COLS)-th token of a column
+    // outputs: a thread takes every (MAIN / COLS)-th token of a column
     {
-      constexpr int STEP = 128 / COLS;
+      constexpr int STEP = MAIN / COLS;
       const int c = threadIdx.x % COLS, first = threadIdx.x / COLS;
       float x[T];
 #pragma unroll
@@ -512,11 +513,11 @@ __global__ void __launch_bounds__(kSbThreads, 1) scan_blocks_kernel(const mdb_sc
     }
 }
 
-template <int MODE, int DP, int CPT>
+template <int MODE, int DP, int COLS, int CPT>
 int launch_scan_blocks(const mdb_scan_args& a, cudaStream_t st) {
-  using P = SbPlan<MODE, DP, CPT>;
+  using P = SbPlan<MODE, DP, COLS, CPT>;
   static_assert(P::kSmemBytes <= 227 * 1024, "shared memory of the scan in blocks");
-  auto kernel = scan_blocks_kernel<MODE, DP, CPT>;
+  auto kernel = scan_blocks_kernel<MODE, DP, COLS, CPT>;
   static PerDeviceOnce attr_once;
   const int dev = attr_once.slot();
   if (dev < 0) return MDB_ERR_CUDA;
@@ -524,5 +525,5 @@ int launch_scan_blocks(const mdb_scan_args& a, cudaStream_t st) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P::kSmemBytes) != cudaSuccess) return MDB_ERR_CUDA;
     attr_once.done[dev] = true;
   }
-  return mdb_launch(kernel, dim3((a.vdim + P::COLS - 1) / P::COLS, a.heads, a.bs), dim3(kSbThreads), P::kSmemBytes, st, a);
+  return mdb_launch(kernel, dim3((a.vdim + COLS - 1) / COLS, a.heads, a.bs), dim3(P::THREADS), P::kSmemBytes, st, a);
 }
