@@ -1,20 +1,11 @@
-// Attention on the 5th-generation tensor cores, in three forms that share one
-// warp-specialised pipeline:
-//   * block attention over the paged KV cache (decode: the masked block of
-//     every request against its committed prefix, every key visible;
-//     flash_attn_with_kvcache as nanovllm/layers/sdar_attention.py:50-55 calls it);
-//   * staircase attention over packed sequences (prefill: a query row sees the
-//     keys up to the right edge of its right-aligned block;
-//     nanovllm/kernels/triton/attention/block_prefill_attention_v2.py:17-166);
-//   * window attention of prompt portions over the paged KV cache (WIN, a kind of
-//     staircase with stairs of one token: a query row sees the last `window` keys
-//     up to its own), with an optional sink in the softmax's denominator, one output
-//     gate per head, and heads of 64 or 128 stored channels.
+// Block attention over the paged KV cache on the 5th-generation tensor cores (decode: the masked block of every request
+// against its committed prefix, every key visible; flash_attn_with_kvcache as nanovllm/layers/sdar_attention.py:50-55
+// calls it).  Prompts have a kernel of their own (attention_prompt.cu), which shares the helpers and arguments of this file.
 //
-// One work unit = the query rows of `tokens x group` (tokens of one request or
-// sequence times the query heads that share a KV head; row = token * group +
+// One work unit = the query rows of `tokens x group` (tokens of one request
+// times the query heads that share a KV head; row = token * group +
 // head_in_group) against a key range.  ROWS = 64 or 128 rows per unit: the MMA
-// is always M = 128.  With ROWS = 64 (paged form) the Q tile holds the rows
+// is always M = 128.  With ROWS = 64 the Q tile holds the rows
 // twice, so that S carries every row in two tensor-memory lanes and the softmax
 // of a tile is spread over four warps, two per row, 64 keys each; the P tile has
 // the 64 real rows only (the upper operand rows of P V are whatever follows in
@@ -35,7 +26,7 @@
 //            O) partial to the split workspace.
 // Tensor memory: S0 | S1 | O, 128 columns each.
 //
-// HBM traffic of the paged form is K and V once: 512 bytes per key per KV head.
+// HBM traffic is K and V once: 512 bytes per key per KV head.
 #include "mdb_common.cuh"
 
 namespace mdb {
@@ -48,22 +39,19 @@ constexpr int kAtMaxRanked = 512;                     // batches above this are 
 
 // Shared-memory plan for ROWS query rows per unit (224 KB of tiles either way).
 //
-// DUP (64-row units of the paged form): the softmax of a 128-key tile is bound by the exponential unit of the
+// DUP (64-row units): the softmax of a 128-key tile is bound by the exponential unit of the
 // sub-partitions that hold the softmax warps (128 ex2 per row on a quarter-rate pipe), so the 64 rows are spread
 // over all four: the Q tile holds the 64 rows twice (operand rows 64..127 repeat rows 0..63), S = Q K^T therefore
 // carries every row in two tensor-memory lanes, and the thread of lane r takes keys 0..63 of the tile while the
 // thread of lane r + 64 takes keys 64..127 of the same row.  The two exchange their row maximum through shared
 // memory, write their halves of the same P row, and add up their partial sums at the end of the unit.
-template <int ROWS, bool DUP = false, bool STAIR = false>
+template <int ROWS, bool DUP = false>
 struct AtPlan {
   static_assert(!DUP || ROWS == 64, "row duplication exists for the 64-row units");
   static constexpr int kQRows = DUP ? 128 : ROWS;     // rows of the Q operand tile
   static constexpr int kQBufs = (ROWS == 64 && !DUP) ? 2 : 1;
-  // Staircase form: one P buffer is enough (the P V of a tile is long over when the next tile's softmax wants to
-  // write), which buys the K ring a third stage: 4 x 4096 tokens 407 -> 396 us, one sequence of 16384 tokens
-  // 1366 -> 1297 us.  (The paged form with 128-row units loses 3 % with the same trade and keeps two and two.)
-  static constexpr int kPBufs = STAIR ? 1 : 2;
-  static constexpr int kKStages = STAIR ? 3 : 2;
+  static constexpr int kPBufs = 2;
+  static constexpr int kKStages = 2;
   static constexpr int kVStages = ROWS == 64 ? 3 : 2;
   static constexpr int kQBytes = 2 * kQRows * 128;    // two channel halves of [kQRows][128 B]
   static constexpr int kPBytes = 2 * ROWS * 128;      // two key halves of [ROWS][128 B]
@@ -88,7 +76,7 @@ struct AtPlan {
 enum {
   kAtBarQFull = 0, kAtBarQEmpty = 2, kAtBarKFull = 4, kAtBarKEmpty = 7, kAtBarVFull = 10, kAtBarVEmpty = 13,
   kAtBarSFull = 16, kAtBarSEmpty = 18, kAtBarPFull = 20, kAtBarPEmpty = 22, kAtBarOFull = 24, kAtBarOEmpty = 25,
-  kAtBarQReady = 26, kAtBarCount = 28      // up to three K and three V stages
+  kAtBarCount = 28      // up to three K and three V stages
 };
 
 struct AtArgs {
@@ -108,7 +96,7 @@ struct AtArgs {
   const int32_t* cu_seqlens;   // rows of the keys
   const int32_t* cu_seqlens_q; // rows of the queries: the last ones of every sequence (NULL: all of them)
   int64_t out_stride;
-  int nseq, max_qtiles, log2_stairs;
+  int nseq, max_qtiles, tiles_per_unit, log2_stairs;
   float q_scale;            // applied to q and rounded to bf16: log2(e) / sqrt(D) as the reference kernel does, or 1
   // window form (with the page table above and cu_seqlens_q)
   const int32_t* start;     // position of every sequence's first query
@@ -173,62 +161,24 @@ __device__ __forceinline__ uint64_t umma_desc_sw128_mn(uint32_t smem_addr) {
 
 // The unit list every role walks the same way.
 //
-// Paged form: requests are ranked by context length (longest first; the ranks
+// Requests are ranked by context length (longest first; the ranks
 // sit in shared memory) and the ranked units are dealt to the CTAs in
 // alternating direction, wave by wave, so that every CTA gets about the same
 // number of key tiles however ragged the batch is.
-// Staircase form: units are (query tile, sequence, KV head) with the late
-// (long) query tiles first.
 struct AtUnit {
   bool valid;
   int ntiles;       // 128-key tiles
   int kbeg, kend;   // keys [kbeg, kend)
   int kvh;
   int q_tok0;       // row of the unit's first token in the q tensor
-  int req, split, tok0;        // paged: request, key-range part, first token of the block covered
-  bool ctx_clamped;            // paged: the context length exceeded what the page table can address
-  int seq_start, T;            // staircase: first packed key row of the sequence, its length
-  int q_start, q_off, m0, Tq;  // ... first packed query row, tokens in front of it, first query of the unit, number of queries
+  int req, split, tok0;        // request, key-range part, first token of the block covered
+  bool ctx_clamped;            // the context length exceeded what the page table can address
 };
 
-template <bool STAIR, bool WIN = false>
 __device__ __forceinline__ AtUnit at_unit(const AtArgs& a, const uint16_t* order, int units, int wave,
                                           int max_ranked = kAtMaxRanked) {
   AtUnit w = {};
   const int G = static_cast<int>(gridDim.x), c = static_cast<int>(blockIdx.x);
-  if (STAIR) {
-    const int p = wave * G + c;
-    if (p >= units) return w;
-    const int per_tile = a.nseq * a.hkv;
-    const int qt = a.max_qtiles - 1 - p / per_tile;
-    const int rest = p % per_tile;
-    const int seq = rest / a.hkv;
-    w.kvh = rest % a.hkv;
-    w.m0 = qt * a.tokens_per_unit;
-    const int32_t* cu_q = a.cu_seqlens_q != nullptr ? a.cu_seqlens_q : a.cu_seqlens;
-    w.q_start = cu_q[seq];
-    w.Tq = cu_q[seq + 1] - w.q_start;
-    if (WIN) {
-      w.req = seq;
-      w.q_off = a.start[seq];
-      w.T = w.q_off + w.Tq;
-    } else {
-      w.seq_start = a.cu_seqlens[seq];
-      w.T = a.cu_seqlens[seq + 1] - w.seq_start;
-      w.q_off = w.T - w.Tq;
-    }
-    if (w.m0 >= w.Tq) return w;
-    w.valid = true;
-    w.q_tok0 = w.q_start + w.m0;
-    const int S = 1 << a.log2_stairs;
-    const int pad = ((w.T + S - 1) >> a.log2_stairs << a.log2_stairs) - w.T;
-    const int last = w.q_off + min(w.m0 + a.tokens_per_unit, w.Tq) - 1;
-    // window form: from the tile that holds the first query's first key
-    w.kbeg = WIN && a.window > 0 ? max(0, w.q_off + w.m0 - a.window + 1) / kAtKeys * kAtKeys : 0;
-    w.kend = min(w.T, ((((last + pad) >> a.log2_stairs) + 1) << a.log2_stairs) - pad);
-    w.ntiles = (w.kend - w.kbeg + kAtKeys - 1) / kAtKeys;
-    return w;
-  }
   const int p = wave * G + ((wave & 1) ? G - 1 - c : c);
   if (p >= units) return w;
   w.valid = true;
@@ -284,14 +234,11 @@ __device__ __forceinline__ bool at_swap(volatile unsigned long long* xch, int la
   }
 }
 
-template <int ROWS, bool STAIR, bool DUP = false, bool WIN = false>
-__global__ void __launch_bounds__(AtPlan<ROWS, DUP, STAIR>::kThreads, 1)
+template <int ROWS, bool DUP = false>
+__global__ void __launch_bounds__(AtPlan<ROWS, DUP>::kThreads, 1)
 attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                const __grid_constant__ CUtensorMap map_v, const AtArgs a, const int units) {
-  using P = AtPlan<ROWS, DUP, STAIR>;
-  static_assert(!(DUP && STAIR), "row duplication is a paged-form layout");
-  static_assert(!WIN || STAIR, "the window form is a staircase with paged keys");
-  const int halves = WIN ? a.halves : 2;      // 64-channel halves of a stored head
+  using P = AtPlan<ROWS, DUP>;
   extern __shared__ __align__(1024) unsigned char at_smem_raw[];
   const uint32_t raw = smem_u32(at_smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -316,7 +263,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 
   if (threadIdx.x == 0) trace_event(30, 0);
   pdl_launch_dependents();
-  if (!STAIR && a.bs <= P::kMaxRanked) {
+  if (a.bs <= P::kMaxRanked) {
     // context lengths are step inputs, not written by the kernels this one is chained to
     for (int r = threadIdx.x; r < a.bs; r += P::kThreads) {
       const int mine = a.ctx_lens[r];
@@ -335,7 +282,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   if (threadIdx.x == 0) {
     for (int s = 0; s < kAtBarCount; ++s) {
       const bool by_softmax = (s >= kAtBarSEmpty && s < kAtBarSEmpty + 2) || (s >= kAtBarPFull && s < kAtBarPFull + 2) ||
-                              s == kAtBarOEmpty || s >= kAtBarQReady;
+                              s == kAtBarOEmpty;
       mbar_init(bar(s), by_softmax ? P::kSoftmaxWarps : 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -366,25 +313,25 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         if (!mbar_wait(bar(empty0 + r.stage), r.phase ^ 1)) return false;
         const uint32_t full = bar(full0 + r.stage);
         const uint32_t dst = tiles0 + r.stage * kAtTileBytes;
-        mbar_arrive_expect_tx(full, halves * kAtHalfBytes);
-        tma_load_2d(dst, map, kvh * 64 * halves, token_row, full);
-        if (halves > 1) tma_load_2d(dst + kAtHalfBytes, map, kvh * kHeadDim + 64, token_row, full);
+        mbar_arrive_expect_tx(full, 2 * kAtHalfBytes);
+        tma_load_2d(dst, map, kvh * kHeadDim, token_row, full);
+        tma_load_2d(dst + kAtHalfBytes, map, kvh * kHeadDim + 64, token_row, full);
         pend |= 1u << r.stage;
         par = (par & ~(1u << r.stage)) | (r.phase << r.stage);
         r.advance(stages);
         return true;
       };
       for (int wave = 0; wave < waves && ok; ++wave) {
-        const AtUnit w = at_unit<STAIR, WIN>(a, order, units, wave, P::kMaxRanked);
+        const AtUnit w = at_unit(a, order, units, wave, P::kMaxRanked);
         if (w.ctx_clamped) report_status(MDB_STATUS_BAD_PAGE);
         if (w.ntiles == 0) continue;
         if (!mbar_wait(bar(kAtBarQEmpty + qr.stage), qr.phase ^ 1)) { ok = false; break; }
         {
           const uint32_t full = bar(kAtBarQFull + qr.stage);
           const uint32_t dst = base + P::kOffQ + qr.stage * P::kQBytes;
-          mbar_arrive_expect_tx(full, static_cast<uint32_t>(rows_used) * (DUP ? 512u : 128u * halves));
+          mbar_arrive_expect_tx(full, static_cast<uint32_t>(rows_used) * (DUP ? 512u : 256u));
           tma_load_3d(dst, &map_q, 0, w.kvh * group, w.q_tok0, full);
-          if (halves > 1) tma_load_3d(dst + P::kQRows * 128, &map_q, 64, w.kvh * group, w.q_tok0, full);
+          tma_load_3d(dst + P::kQRows * 128, &map_q, 64, w.kvh * group, w.q_tok0, full);
           if (DUP) {      // the same rows once more as operand rows 64..
             tma_load_3d(dst + 64 * 128, &map_q, 0, w.kvh * group, w.q_tok0, full);
             tma_load_3d(dst + P::kQRows * 128 + 64 * 128, &map_q, 64, w.kvh * group, w.q_tok0, full);
@@ -395,8 +342,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         }
         auto token_row = [&](int tile) {
           const int key0 = w.kbeg + tile * kAtKeys;
-          if (STAIR && !WIN) return w.seq_start + key0;
-          int page = !WIN || key0 / kPage < a.table_stride ? a.block_table[static_cast<int64_t>(w.req) * a.table_stride + key0 / kPage] : -1;
+          int page = a.block_table[static_cast<int64_t>(w.req) * a.table_stride + key0 / kPage];
           if (page < 0 || page >= a.num_pages) {
             report_status(MDB_STATUS_BAD_PAGE);
             page = 0;
@@ -431,15 +377,14 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kAtKeys >> 3) << 17) |
                                (static_cast<uint32_t>(128 >> 4) << 24);
       const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) |
-                               (static_cast<uint32_t>(halves * 8) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
+                               (static_cast<uint32_t>(kHeadDim >> 3) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
       AtRing kr, vr, qr, sr, pr;        // sr: S buffer the next S = Q K^T goes to; pr: P buffer of the next P V
       uint32_t o_phase = 0;             // parity of the o_empty phase to wait for
       bool ok = true;
       for (int wave = 0; wave < waves && ok; ++wave) {
-        const AtUnit w = at_unit<STAIR, WIN>(a, order, units, wave, P::kMaxRanked);
+        const AtUnit w = at_unit(a, order, units, wave, P::kMaxRanked);
         if (w.ntiles == 0) continue;
-        // staircase form: the softmax warps scale q in place first
-        if (!mbar_wait_w(bar((STAIR && !WIN ? kAtBarQReady : kAtBarQFull) + qr.stage), qr.phase)) { ok = false; break; }
+        if (!mbar_wait_w(bar(kAtBarQFull + qr.stage), qr.phase)) { ok = false; break; }
         const uint32_t q_tile = base + P::kOffQ + qr.stage * P::kQBytes;
         auto issue_s = [&](int j) {
           if (!mbar_wait_w(bar(kAtBarKFull + kr.stage), kr.phase)) return false;
@@ -449,7 +394,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           const uint32_t d_tmem = tmem_base + sr.stage * kAtKeys;
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {
-            if (WIN && kk >= 4 * halves) break;
             const uint64_t adesc = umma_desc_sw128(q_tile + (kk >> 2) * (P::kQRows * 128)) + 2 * (kk & 3);
             const uint64_t bdesc = umma_desc_sw128(k_tile + (kk >> 2) * kAtHalfBytes) + 2 * (kk & 3);
             umma_bf16_w(d_tmem, adesc, bdesc, idesc_s, kk > 0 ? 1u : 0u);
@@ -502,34 +446,21 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     const uint32_t lane_field = static_cast<uint32_t>(32 * warp) << 16;
     volatile unsigned long long* xch = reinterpret_cast<volatile unsigned long long*>(gen_base + P::kOffXch);
     uint32_t xseq = 0;                                     // DUP: running number of the swaps of this thread
-    AtRing sr, pr, vr, qr;             // positions of the tile being handled in the S, P, V and Q rings
+    AtRing sr, pr, vr;                 // positions of the tile being handled in the S, P and V rings
     uint32_t prev_p_stage = 0, prev_p_phase = 0;   // P ring position of the previous tile (its P V frees O for a rescale)
     uint32_t o_phase = 0;
     bool ok = true;
     for (int wave = 0; wave < waves && ok; ++wave) {
-      const AtUnit w = at_unit<STAIR, WIN>(a, order, units, wave, P::kMaxRanked);
+      const AtUnit w = at_unit(a, order, units, wave, P::kMaxRanked);
       if (!w.valid) continue;
       const int head = w.kvh * group + head_in_group;
       bool row_valid = row < rows_used;
-      int limit = 0, first = 0;      // staircase form: last (window form: and first) key this row sees
-      bf16* out_row;
-      int64_t prow = 0;
-      if (STAIR) {
-        const int qi = w.m0 + tok_local, i = w.q_off + qi;
-        row_valid = row_valid && qi < w.Tq;
-        const int S = 1 << a.log2_stairs;
-        const int pad = ((w.T + S - 1) >> a.log2_stairs << a.log2_stairs) - w.T;
-        limit = row_valid ? min(w.T - 1, ((((i + pad) >> a.log2_stairs) + 1) << a.log2_stairs) - 1 - pad) : -1;
-        if (WIN && a.window > 0) first = i - a.window + 1;
-        out_row = a.out + static_cast<int64_t>(w.q_start + (row_valid ? qi : 0)) * a.out_stride + head * (WIN ? a.dim : kHeadDim);
-      } else {
-        const int tok = w.tok0 + tok_local;
-        row_valid = row_valid && tok < a.block;
-        const int tk = row_valid ? tok : 0;
-        prow = ((static_cast<int64_t>(w.req) * a.nsplit + w.split) * a.hq + head) * a.block + tk;
-        out_row = a.out + ((static_cast<int64_t>(w.req) * a.block + tk) * a.hq + head) * kHeadDim;
-      }
-      if (w.ntiles == 0) {           // paged form only: an empty key range
+      const int tok = w.tok0 + tok_local;
+      row_valid = row_valid && tok < a.block;
+      const int tk = row_valid ? tok : 0;
+      const int64_t prow = ((static_cast<int64_t>(w.req) * a.nsplit + w.split) * a.hq + head) * a.block + tk;
+      bf16* out_row = a.out + ((static_cast<int64_t>(w.req) * a.block + tk) * a.hq + head) * kHeadDim;
+      if (w.ntiles == 0) {           // an empty key range
         if (row_valid && half == 0) {
           if (a.nsplit == 1) {
 #pragma unroll
@@ -543,30 +474,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         }
         continue;
       }
-      if (STAIR && !WIN) {
-        // q * log2(e)/sqrt(D) rounded to bf16, in place (elementwise, so the swizzle does not matter)
-        ok = mbar_wait(bar(kAtBarQFull + qr.stage), qr.phase);
-        if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
-        if (row < rows_used) {
-          const uint32_t q_row = base + P::kOffQ + qr.stage * P::kQBytes + row * 128;
-#pragma unroll
-          for (int c = 0; c < 16; ++c) {
-            const uint32_t addr = q_row + (c >> 3) * (ROWS * 128) + (c & 7) * 16;
-            uint32_t x[4];
-            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]) : "r"(addr));
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float2 f = unpack_bf16x2(x[e]);
-              x[e] = pack_bf16x2(f.x * a.q_scale, f.y * a.q_scale);
-            }
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]) : "memory");
-          }
-        }
-        fence_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(kAtBarQReady + qr.stage));
-        qr.advance(P::kQBufs);
-      }
       float m_ref = -INFINITY, l = 0.f;
       for (int j = 0; j < w.ntiles; ++j) {
         ok = mbar_wait(bar(kAtBarSFull + sr.stage), sr.phase);
@@ -574,8 +481,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         tc_fence_after();
         const uint32_t s_addr = tmem_base + sr.stage * kAtKeys + lane_field;
         const int key0 = w.kbeg + j * kAtKeys;
-        // keys of this tile the row sees: [0, nvalid)
-        const int nvalid = STAIR ? max(0, min(kAtKeys, limit + 1 - key0)) : min(kAtKeys, w.kend - key0);
+        // keys of this tile that belong to the context: [0, nvalid)
+        const int nvalid = min(kAtKeys, w.kend - key0);
         // the thread's share of the score row into registers, then the S buffer goes back to the MMA warp
         float s[NC];
 #pragma unroll
@@ -588,10 +495,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         if (nv < NC) {
 #pragma unroll
           for (int i = 0; i < NC; ++i) if (i >= nv) s[i] = -INFINITY;   // also replaces NaN from stale rows
-        }
-        if (WIN && first > key0) {
-#pragma unroll
-          for (int i = 0; i < NC; ++i) if (i < first - key0) s[i] = -INFINITY;
         }
         // eight independent chains: the warp is alone on its sub-partition, nothing else hides the ALU latency
         float mxv[8];
@@ -612,7 +515,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         }
         if (!row_valid) mx = 0.f;                             // rows past the block hold whatever the tile held
         const float m_tile = mx * a.scale_log2;
-        // a row that sees no key of this tile (staircase form, rows above the tile's diagonal) keeps its state
         const bool grow = m_tile > m_ref + kAtRescaleStep || (m_ref == -INFINITY && m_tile != -INFINITY);
         if (__any_sync(0xffffffffu, grow)) {
           const float m_new = fmaxf(m_ref, m_tile);
@@ -664,13 +566,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                        "r"(pk[4 * q]), "r"(pk[4 * q + 1]), "r"(pk[4 * q + 2]), "r"(pk[4 * q + 3])
                        : "memory");
         }
-        const int held = WIN ? w.kend - key0 : nvalid;      // keys of the tile that belong to the context
-        if ((!STAIR || WIN) && held < kAtKeys) {
+        if (nvalid < kAtKeys) {
           // stale cache rows past the context end must not reach O through 0 * (Inf or NaN): clear them in V
           ok = mbar_wait(bar(kAtBarVFull + vr.stage), vr.phase);
           if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
           const uint32_t v_tile = base + P::kOffV + vr.stage * kAtTileBytes;
-          for (int r = held + lane_row; r < kAtKeys; r += 32 * P::kSoftmaxWarps) {
+          for (int r = nvalid + lane_row; r < kAtKeys; r += 32 * P::kSoftmaxWarps) {
 #pragma unroll
             for (int h = 0; h < 2; ++h)
 #pragma unroll
@@ -703,28 +604,14 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       }
       if (half != 0) {
         // DUP: lanes 64..127 of O belong to operand rows nobody wrote; the rows' outputs leave from lanes 0..63
-      } else if (STAIR || a.nsplit == 1) {
-        float inv;
-        if (WIN) {
-          // the sink's term exp(0) in the units of the running reference
-          const float den = a.sink ? l + ex2_approx(-m_ref) : l;
-          float z = a.out_scale;
-          if (row_valid && rows_present(a.gate)) z *= sigmoid_f(rows_at<bf16>(a.gate, w.q_start + w.m0 + tok_local, head));
-          inv = den > 0.f ? z / den : 0.f;
-        } else {
-          inv = l > 0.f ? 1.0f / l : 0.f;
-        }
-        const bool ragged = WIN && a.dim != 64 * halves;      // fewer channels leave than are stored
+      } else if (a.nsplit == 1) {
+        const float inv = l > 0.f ? 1.0f / l : 0.f;
 #pragma unroll 1
-        for (int c = 0; c < 2 * halves; ++c) {
+        for (int c = 0; c < 4; ++c) {
           float o[32];
           tmem_ld32(tmem_o + lane_field + 32 * c, o);
           tmem_ld_wait();
-          if (row_valid && ragged) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (32 * c + i < a.dim) out_row[32 * c + i] = __float2bfloat16_rn(o[i] * inv);
-          } else if (row_valid) {
+          if (row_valid) {
 #pragma unroll
             for (int q4 = 0; q4 < 4; ++q4)
               reinterpret_cast<uint4*>(out_row + 32 * c)[q4] =
@@ -820,15 +707,15 @@ static int at_sm_count() {
   return sm_count;
 }
 
-template <int ROWS, bool STAIR, bool DUP = false, bool WIN = false>
+template <int ROWS, bool DUP = false>
 static int at_launch(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const AtArgs& a,
                      int64_t units, cudaStream_t st) {
-  using P = AtPlan<ROWS, DUP, STAIR>;
+  using P = AtPlan<ROWS, DUP>;
   static PerDeviceOnce attr_once;
   const int dev = attr_once.slot();
   if (dev < 0) return MDB_ERR_CUDA;
   if (!attr_once.done[dev]) {
-    if (cudaFuncSetAttribute(attn_tc_kernel<ROWS, STAIR, DUP, WIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(attn_tc_kernel<ROWS, DUP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              P::kSmemBytes) != cudaSuccess)
       return MDB_ERR_CUDA;
     attr_once.done[dev] = true;
@@ -836,7 +723,7 @@ static int at_launch(const CUtensorMap& map_q, const CUtensorMap& map_k, const C
   if (units > (1 << 30)) return MDB_ERR_UNSUPPORTED;
   const int sms = at_sm_count();
   const int grid = units < sms ? static_cast<int>(units) : sms;
-  return mdb_launch(attn_tc_kernel<ROWS, STAIR, DUP, WIN>, dim3(grid), dim3(P::kThreads), P::kSmemBytes, st, map_q, map_k,
+  return mdb_launch(attn_tc_kernel<ROWS, DUP>, dim3(grid), dim3(P::kThreads), P::kSmemBytes, st, map_q, map_k,
                     map_v, a, static_cast<int>(units));
 }
 
@@ -873,73 +760,8 @@ static int attn_tc_launch(const AttnPagedArgs& pa, int bs, cudaStream_t st) {
   if (!get_tensor_map(pa.k_cache, cache_rows, pa.hkv * kHeadDim, pa.hkv * kHeadDim, kAtKeys, &map_k)) return MDB_ERR_CUDA;
   if (!get_tensor_map(pa.v_cache, cache_rows, pa.hkv * kHeadDim, pa.hkv * kHeadDim, kAtKeys, &map_v)) return MDB_ERR_CUDA;
   const int64_t units = static_cast<int64_t>(bs) * pa.hkv * a.row_blocks * pa.nsplit;
-  return rows == 64 ? at_launch<64, false, true>(map_q, map_k, map_v, a, units, st)
-                    : at_launch<128, false>(map_q, map_k, map_v, a, units, st);
-}
-
-// ---- staircase form ----
-static bool attn_stair_tc_supported(int hq, int hkv, int64_t q_stride, int64_t k_stride, int64_t v_stride) {
-  if (hkv <= 0 || hq % hkv != 0 || hq / hkv > 128) return false;
-  return q_stride % 8 == 0 && k_stride % 8 == 0 && v_stride % 8 == 0;
-}
-
-static int attn_stair_tc_launch(const AttnStairArgs& sa, int nseq, int max_seqlen, int64_t total_q, int64_t total_tokens,
-                                cudaStream_t st) {
-  AtArgs a = {};
-  a.q = sa.q;
-  a.out = sa.out;
-  a.hq = sa.hq; a.hkv = sa.hkv; a.group = sa.hq / sa.hkv;
-  a.scale_log2 = sa.scale_log2;
-  a.q_scale = sa.q_scale;
-  a.cu_seqlens = sa.cu_seqlens;
-  a.cu_seqlens_q = sa.cu_seqlens_q;
-  a.out_stride = sa.out_stride;
-  a.nseq = nseq;
-  a.log2_stairs = sa.log2_stairs;
-  a.tokens_per_unit = 128 / a.group;
-  a.max_qtiles = (max_seqlen + a.tokens_per_unit - 1) / a.tokens_per_unit;
-  a.nsplit = 1;
-  CUtensorMap map_q, map_k, map_v;
-  if (!get_q_tensor_map(sa.q, total_q, sa.q_stride, sa.hq, a.group, a.tokens_per_unit, &map_q)) return MDB_ERR_CUDA;
-  if (!get_tensor_map(sa.k, total_tokens, sa.hkv * kHeadDim, sa.k_stride, kAtKeys, &map_k)) return MDB_ERR_CUDA;
-  if (!get_tensor_map(sa.v, total_tokens, sa.hkv * kHeadDim, sa.v_stride, kAtKeys, &map_v)) return MDB_ERR_CUDA;
-  const int64_t units = static_cast<int64_t>(a.max_qtiles) * nseq * sa.hkv;
-  return at_launch<128, true>(map_q, map_k, map_v, a, units, st);
-}
-
-// ---- window form ----
-static bool attn_win_tc_supported(const mdb_window_attn_args& w) {
-  return w.dtype == MDB_BF16 && (w.dim_pad == 64 || w.dim_pad == 128) && w.heads / w.kv_heads <= 128 && w.scale > 0.f && w.cu_q && w.start;
-}
-
-static int attn_win_tc_launch(const mdb_window_attn_args& w, cudaStream_t st) {
-  AtArgs a = {};
-  a.q = static_cast<const bf16*>(w.q);
-  a.out = static_cast<bf16*>(w.out);
-  a.hq = w.heads; a.hkv = w.kv_heads; a.group = w.heads / w.kv_heads;
-  a.scale_log2 = w.scale * 1.4426950408889634f;
-  a.q_scale = 1.0f;
-  a.cu_seqlens_q = w.cu_q;
-  a.start = w.start;
-  a.block_table = w.block_table;
-  a.table_stride = w.table_stride;
-  a.num_pages = w.num_pages;
-  a.out_stride = w.ld_out;
-  a.nseq = w.bs;
-  a.tokens_per_unit = 128 / a.group;
-  a.max_qtiles = (w.max_q + a.tokens_per_unit - 1) / a.tokens_per_unit;
-  a.nsplit = 1;
-  a.window = w.window; a.sink = w.sink;
-  a.dim = w.dim; a.halves = w.dim_pad / 64;
-  a.out_scale = w.out_scale;
-  a.gate = w.gate;
-  CUtensorMap map_q, map_k, map_v;
-  const int64_t cache_rows = static_cast<int64_t>(w.num_pages) * kPage;
-  const int cols = w.kv_heads * w.dim_pad;
-  if (!get_q_tensor_map(w.q, w.m, static_cast<int64_t>(w.heads) * w.dim_pad, w.heads, a.group, a.tokens_per_unit, &map_q, w.dim_pad)) return MDB_ERR_CUDA;
-  if (!get_tensor_map(w.k_cache, cache_rows, cols, cols, kAtKeys, &map_k)) return MDB_ERR_CUDA;
-  if (!get_tensor_map(w.v_cache, cache_rows, cols, cols, kAtKeys, &map_v)) return MDB_ERR_CUDA;
-  return at_launch<128, true, false, true>(map_q, map_k, map_v, a, static_cast<int64_t>(a.max_qtiles) * w.bs * w.kv_heads, st);
+  return rows == 64 ? at_launch<64, true>(map_q, map_k, map_v, a, units, st)
+                    : at_launch<128>(map_q, map_k, map_v, a, units, st);
 }
 
 }  // namespace mdb
