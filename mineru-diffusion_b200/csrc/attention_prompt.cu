@@ -7,15 +7,16 @@
 //
 // A tile is 128 query rows, `tokens x group` of one sequence and KV head (row = token * group + head in group); a unit is two
 // neighbouring tiles A and B of one sequence, which walk the same key tiles of 128 keys.  Roles: a TMA warp (both Q tiles, K and
-// V rings), an MMA warp, and four softmax warps per tile, one query row per thread.
+// V rings) and, per tile, an MMA warp and four softmax warps, one query row per thread.
 //
 // What bounds it: the chain of a tile (S ready, scores to registers, maximum, exponentials, P back, P V) took 1.7 us for
 // 128 keys and 0.27 us of products while one tile had the SM to itself.  Here one tile's softmax runs under the other's products,
 // and each tile goes in steps of 64 keys with two score buffers, so that the scores of the next step are there when a softmax
 // ends; P goes back into the tensor memory of the scores it came from (bf16 pairs, the left operand of P V): no shared
 // memory for P and no proxy fence.  The products of one thread run in the order of issue, so new scores may follow P V into the
-// same columns without a wait.  4 x 4096 tokens, 16 query
-// and 8 KV heads: 418 -> 313 us (880 TFLOP/s of visible products); one tile per SM with single score buffers 322 us.
+// same columns without a wait.  One warp issuing for both tiles spent 2000 cycles per step of both on its waits and issues, twice
+// what the exponentials take, hence a warp per tile.  4 x 4096 tokens, 16 query and 8 KV heads: 404 -> 299 us (923 TFLOP/s of
+// visible products; one issuing warp 313, one score buffer of 128 keys per tile 322).
 //
 // Tensor memory: S_A (P_A) two steps | S_B (P_B) two steps, 64 columns each | O_A | O_B, 128 columns each.
 #include "mdb_common.cuh"
@@ -25,7 +26,7 @@ namespace mdb {
 struct ApPlan {
   static constexpr int kKStages = 3, kVStages = 2;
   static constexpr int kQBytes = 2 * 128 * 128;             // a tile: two channel halves of [128 rows][128 B]
-  static constexpr int kProducerWarp = 8, kMmaWarp = 9, kThreads = 320;
+  static constexpr int kProducerWarp = 8, kMmaWarp = 9 /* tile A; B: the next */, kThreads = 352;
   static constexpr int kOffK = 2 * kQBytes;
   static constexpr int kOffV = kOffK + kKStages * kAtTileBytes;
   static constexpr int kOffBars = kOffV + kVStages * kAtTileBytes;
@@ -150,7 +151,8 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   if (threadIdx.x == 0) {
     for (int s = 0; s < kApBarCount; ++s) {
       const bool by_softmax = s == kApBarQReady || s == kApBarQReady + 1 || (s >= kApBarPFull && s < kApBarPFull + 4) || s >= kApBarOEmpty;
-      mbar_init(bar(s), by_softmax ? 4 : 1);
+      const bool by_products = s == kApBarQEmpty || (s >= kApBarKEmpty && s < kApBarVFull) || (s >= kApBarVEmpty && s < kApBarSFull);
+      mbar_init(bar(s), by_softmax ? 4 : by_products ? 2 : 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -228,46 +230,39 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         if (pend_q) mbar_wait(bar(kApBarQFull), par_q);
       }
     }
-  } else if (warp == P::kMmaWarp) {
-    // ----------------------------------------------------------------- MMA issue (all lanes, one elected)
+  } else if (warp >= P::kMmaWarp) {
+    // ----------------------------------------------------------------- MMA issue (all lanes, one elected), a warp per tile
+    const int x = warp - P::kMmaWarp;
     // bf16 x bf16 -> fp32, M = 128, N = 64 keys, or 64 or 128 channels; bit 16 set: B operand MN-major
     const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kApStep >> 3) << 17) |
                              (static_cast<uint32_t>(128 >> 4) << 24);
     const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) |
                              (static_cast<uint32_t>(halves * 8) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
+    const uint32_t s_cols = tmem_base + x * 128, o_cols = tmem_base + 256 + x * 128;
     AtRing kr, vr;
-    uint32_t q_phase[2] = {0, 0}, p_phase = 0 /* bit 2 x + buffer */, o_phase[2] = {0, 0};
-    uint32_t qfull_phase = 0;
+    uint32_t q_phase = 0, p_phase = 0 /* bit per buffer */, o_phase = 0;
     bool ok = true;
     for (int wave = 0; wave < waves && ok; ++wave) {
       const ApUnit w = ap_unit<WIN>(a, units, wave);
       if (w.ntiles == 0) continue;
-      if (WIN) {
-        if (!mbar_wait_w(bar(kApBarQFull), qfull_phase)) { ok = false; break; }
-        qfull_phase ^= 1;
-      } else {
-        // staircase form: the softmax warps scale q in place first
-#pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          if (!w.t[x].valid) continue;
-          if (ok && !mbar_wait_w(bar(kApBarQReady + x), q_phase[x])) ok = false;
-          q_phase[x] ^= 1;
-        }
-        if (!ok) break;
-      }
-      // scores of step h of every tile that takes it, from the K tile at the ring's position
+      const ApTile t = x == 0 ? w.t[0] : w.t[1];
       const int steps = w.t[1].valid ? w.t[1].last : w.t[0].last;
+      // staircase form: the softmax warps scale q in place first.  (Window form: seen by both, whether they have a tile or not,
+      // since the next phase is told from this one by parity.)
+      if (WIN || t.valid) {
+        if (!mbar_wait_w(bar(WIN ? kApBarQFull : kApBarQReady + x), q_phase)) { ok = false; break; }
+        q_phase ^= 1;
+      }
+      // Both warps walk all the key tiles and release them, with products of their own or not.
       auto issue_s = [&](int h) {
         if ((h & 1) == 0 && !mbar_wait_w(bar(kApBarKFull + kr.stage), kr.phase)) return false;
-        tc_fence_after();
-        const uint32_t k_rows = base + P::kOffK + kr.stage * kAtTileBytes + (h & 1) * (kApStep * 128);
-#pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          if (!w.t[x].valid || h < w.t[x].first || h >= w.t[x].last) continue;
+        if (t.valid && h >= t.first && h < t.last) {
+          tc_fence_after();
+          const uint32_t k_rows = base + P::kOffK + kr.stage * kAtTileBytes + (h & 1) * (kApStep * 128);
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             if (WIN && c >= halves) break;
-            umma_bf16_x4_w(tmem_base + x * 128 + (h & 1) * kApStep, umma_desc_sw128(base + x * P::kQBytes + c * (128 * 128)), 2,
+            umma_bf16_x4_w(s_cols + (h & 1) * kApStep, umma_desc_sw128(base + x * P::kQBytes + c * (128 * 128)), 2,
                            umma_desc_sw128(k_rows + c * kAtHalfBytes), 2, idesc_s, c);
           }
           umma_commit_w(bar(kApBarSFull + 2 * x + (h & 1)));
@@ -284,25 +279,21 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         // (the buffer of step h + 1 held step h - 1, whose P V has been issued)
         if (h + 1 < steps && !issue_s(h + 1)) { ok = false; break; }
         if ((h & 1) == 0 && !mbar_wait_w(bar(kApBarVFull + vr.stage), vr.phase)) { ok = false; break; }
-        const uint32_t v_rows = base + P::kOffV + vr.stage * kAtTileBytes + (h & 1) * (kApStep * 128);
-#pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          if (!w.t[x].valid || h < w.t[x].first || h >= w.t[x].last) continue;
-          if (h == w.t[x].first) {
+        if (t.valid && h >= t.first && h < t.last) {
+          if (h == t.first) {
             // the previous unit's accumulator must have been read out
-            if (!mbar_wait_w(bar(kApBarOEmpty + x), o_phase[x] ^ 1)) { ok = false; break; }
-            o_phase[x] ^= 1;
+            if (!mbar_wait_w(bar(kApBarOEmpty + x), o_phase ^ 1)) { ok = false; break; }
+            o_phase ^= 1;
           }
-          const int buf = 2 * x + (h & 1);
-          if (!mbar_wait_w(bar(kApBarPFull + buf), p_phase >> buf & 1)) { ok = false; break; }
-          p_phase ^= 1u << buf;
+          if (!mbar_wait_w(bar(kApBarPFull + 2 * x + (h & 1)), p_phase >> (h & 1) & 1)) { ok = false; break; }
+          p_phase ^= 1u << (h & 1);
           tc_fence_after();
-          umma_bf16_ts_x4_w(tmem_base + 256 + x * 128, tmem_base + x * 128 + (h & 1) * kApStep, umma_desc_sw128_mn(v_rows), 128, idesc_o,
-                            h > w.t[x].first ? 1u : 0u);
+          umma_bf16_ts_x4_w(o_cols, s_cols + (h & 1) * kApStep,
+                            umma_desc_sw128_mn(base + P::kOffV + vr.stage * kAtTileBytes + (h & 1) * (kApStep * 128)), 128, idesc_o,
+                            h > t.first ? 1u : 0u);
           umma_commit_w(bar(kApBarPDone + x));
-          if (h == w.t[x].last - 1) umma_commit_w(bar(kApBarOFull + x));
+          if (h == t.last - 1) umma_commit_w(bar(kApBarOFull + x));
         }
-        if (!ok) break;
         if ((h & 1) || h == steps - 1) {
           umma_commit_w(bar(kApBarVEmpty + vr.stage));
           vr.advance(P::kVStages);
