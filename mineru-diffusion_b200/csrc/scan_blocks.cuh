@@ -11,15 +11,17 @@
 //
 // What bounds it: latency, with few warps per scheduler.  All the states of four prompts of 16 heads are 55 elements per FMA
 // lane of the chip.  A CTA has warps that keep COLS columns of the state in registers (CPT columns x 1/16 of the channels a
-// thread: a 16-byte read of shared memory feeds 4 CPT FMAs) and four that prepare the next block meanwhile: its operands with
+// thread: a 16-byte read of shared memory feeds 4 CPT FMAs) and others that prepare the next block meanwhile: its operands with
 // cp.async two blocks ahead, the scaled rows, L and M.
-constexpr int kSbTokens = 16, kSbPrep = 128, kSbRing = 3;
+constexpr int kSbTokens = 16, kSbRing = 3;
 
 template <int MODE, int DP, int COLS, int CPT>
 struct SbPlan {
   static constexpr bool DELTA = MODE == kScanDelta;
   static constexpr int ROW = kSbTokens * DP;
-  static constexpr int MAIN = COLS / CPT * 16, THREADS = MAIN + kSbPrep;      // threads that keep the state; all
+  // threads that prepare: L and M of the delta rule, or a block next to few columns, keep eight warps busy
+  static constexpr int PREP_THREADS = DELTA || COLS == 16 ? 256 : 128;
+  static constexpr int MAIN = COLS / CPT * 16, THREADS = MAIN + PREP_THREADS;      // threads that keep the state; all
   // raw operands, a ring of three blocks: k, q (, g) rows, v, two scalars per token
   static constexpr int RAW_Q = ROW, RAW_G = 2 * ROW, RAW_V = (DELTA ? 3 : 2) * ROW, RAW_S = RAW_V + kSbTokens * COLS, RAW = RAW_S + 2 * kSbTokens;
   // prepared block, two of them: (delta) scaled k and q, k as the update takes it, G_16; L transposed, M; per token four floats
@@ -72,7 +74,7 @@ template <int MODE, int DP, int COLS, int CPT>
 __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_blocks_kernel(const mdb_scan_args a) {
   using P = SbPlan<MODE, DP, COLS, CPT>;
   constexpr bool DELTA = P::DELTA, MLSTM = MODE == kScanMlstm;
-  constexpr int MAIN = P::MAIN, T = kSbTokens, NR = DP / 64, NP = DP / 64;      // float4 per lane and column; channel pairs per lane of a row
+  constexpr int MAIN = P::MAIN, T = kSbTokens, PW = P::PREP_THREADS / 32, PASSES = T / 2 / PW, TPW = T / PW, NR = DP / 64, NP = DP / 64;      // float4 per lane and column; channel pairs per lane of a row
   extern __shared__ __align__(16) float sb_smem[];
   pdl_launch_dependents();
   pdl_wait();
@@ -94,7 +96,7 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
         const int t0 = w.t_begin + b * T, n = min(T, w.t_end - t0);
         float* st = sb_smem + (b % kSbRing) * P::RAW;
         const uint32_t base = smem_u32(st);
-        for (int i = tid; i < T * (DP / 4); i += 128) {
+        for (int i = tid; i < T * (DP / 4); i += P::PREP_THREADS) {
           const int t = i / (DP / 4), c = i % (DP / 4) * 4;
           if (t < n) {
             const int64_t krow = (static_cast<int64_t>(t0 + t) * a.kv_heads + w.kvh) * DP + c;
@@ -109,7 +111,7 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
         }
         const float* v0 = a.v + (static_cast<int64_t>(t0) * a.heads + w.head) * a.vdim + w.col0;
         const int64_t vstep = static_cast<int64_t>(a.heads) * a.vdim;
-        for (int i = tid; i < T * (COLS / 4); i += 128) {
+        for (int i = tid; i < T * (COLS / 4); i += P::PREP_THREADS) {
           const int t = i / (COLS / 4), c = i % (COLS / 4) * 4;
           if (v16 && t < n && w.col0 + c < a.vdim) {
             cp_async16(base + (P::RAW_V + t * COLS + c) * 4, v0 + t * vstep + c);
@@ -166,7 +168,8 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
       float* prep = sb_smem + P::OFF_PREP + (b & 1) * P::PREP;
       float4* per_token = reinterpret_cast<float4*>(prep + P::P_T);
       if (DELTA) {
-        for (int c = tid; c < DP; c += 128) {
+        if (tid < DP) {
+          const int c = tid;
           float kk[T], gg[T], acc = 1.f;
 #pragma unroll
           for (int t = 0; t < T; ++t) {
@@ -185,10 +188,10 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
           }
         }
         if (tid < T) per_token[tid].x = raw[P::RAW_S + 2 * tid];      // beta
-        // L and M: a warp takes two neighbouring keys from either end, so that all warps have 36 pairs of tokens
-#pragma unroll 1
-        for (int pass = 0; pass < 2; ++pass) {
-          const int j0 = pass ? T - 2 - 2 * pw : 2 * pw;
+        // L and M: a warp takes two neighbouring keys; the first warps, who also scale the rows, those with few tokens behind them
+        static_assert(!DELTA || PASSES == 1, "a pair of keys per warp");
+        const int j0 = pw >= 4 ? 2 * (pw - 4) : T - 2 - 2 * pw;
+        {
           f32x2 p[2][NP];
           float acc[2][32];
 #pragma unroll
@@ -258,22 +261,24 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
         // every lane: product of the forget factors of tokens 0 .. t, of those behind t, of those behind j up to t
         const int t = lane & 15, jl = lane >> 4;
         float head = 1.f, tail = 1.f;
-        float between[2] = {1.f, 1.f};
+        // the two keys a warp takes in a pass: from either end, so that the tokens behind them even out
+        auto first_key = [&](int pass) { return pass ? T - 2 - 2 * pw : 2 * pw; };
+        float between[PASSES];
+#pragma unroll
+        for (int pass = 0; pass < PASSES; ++pass) between[pass] = 1.f;
 #pragma unroll
         for (int s = 0; s < T; ++s) {
           const float f = __shfl_sync(0xffffffffu, fa, s);
           if (s <= t) head *= f;
           if (s > t) tail *= f;
 #pragma unroll
-          for (int pass = 0; pass < 2; ++pass) {
-            const int j = (pass ? T - 2 - 2 * pw : 2 * pw) + jl;
-            if (s > j && s <= t) between[pass] *= f;
-          }
+          for (int pass = 0; pass < PASSES; ++pass)
+            if (s > first_key(pass) + jl && s <= t) between[pass] *= f;
         }
         if (pw == 0 && lane < T) per_token[lane] = make_float4(head, fb * tail, em, 0.f);
-#pragma unroll 1
-        for (int pass = 0; pass < 2; ++pass) {
-          const int j0 = pass ? T - 2 - 2 * pw : 2 * pw;
+#pragma unroll
+        for (int pass = 0; pass < PASSES; ++pass) {
+          const int j0 = first_key(pass), j = j0 + jl;
           float acc[32];
           f32x2 k[2][NP];
           row_pairs(raw + j0 * DP, k[0]);
@@ -293,20 +298,20 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
             }
           }
           const float total = reduce_scatter32(acc, lane);      // q_t . k_j, t = lane & 15, j = j0 + lane / 16
-          const int j = j0 + jl;
           const float bj = __shfl_sync(0xffffffffu, fb, j);
-          prep[P::P_M + t * T + j] = j <= t ? (pass ? between[1] : between[0]) * bj * total : 0.f;
+          prep[P::P_M + t * T + j] = j <= t ? between[pass] * bj * total : 0.f;
         }
         if (norm) {
-          // q_t . n for a warp's four tokens, then n moves past the block (every warp alike)
-          float r4[4];
+          // q_t . n for a warp's tokens, then n moves past the block (every warp alike)
+          float mine = 0.f;
 #pragma unroll
-          for (int i4 = 0; i4 < 4; ++i4) {
+          for (int i2 = 0; i2 < TPW; ++i2) {
             f32x2 q[NP], s = 0ull;
-            row_pairs(raw + P::RAW_Q + (4 * pw + i4) * DP, q);
+            row_pairs(raw + P::RAW_Q + (TPW * pw + i2) * DP, q);
 #pragma unroll
             for (int i = 0; i < NP; ++i) s = fma2(nv[i], q[i], s);
-            r4[i4] = warp_sum(sum2(s));
+            const float qn = warp_sum(sum2(s));
+            if (lane == i2) mine = qn;
           }
           const float whole = __shfl_sync(0xffffffffu, head, T - 1);
           f32x2 moved[NP];
@@ -322,10 +327,9 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
           }
 #pragma unroll
           for (int i = 0; i < NP; ++i) nv[i] = moved[i];
-          sb_bar<2, kSbPrep>();                                        // M is whole
-          if (lane < 4) {
-            const int tt = 4 * pw + lane, tok = w.t_begin + b * T + tt;
-            const float mine = lane == 0 ? r4[0] : lane == 1 ? r4[1] : lane == 2 ? r4[2] : r4[3];
+          sb_bar<2, P::PREP_THREADS>();                                        // M is whole
+          if (lane < TPW) {
+            const int tt = TPW * pw + lane, tok = w.t_begin + b * T + tt;
             const float4 pt = per_token[tt];
             float s = 0.f;
 #pragma unroll
@@ -339,14 +343,14 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
     fetch(0);
     fetch(1);
     cp_async_wait<1>();
-    sb_bar<2, kSbPrep>();
+    sb_bar<2, P::PREP_THREADS>();
     prepare(0);
     __syncthreads();
     for (int b = 0; b < nblocks; ++b) {
       fetch(b + 2);                     // its place was read for the last time before the barrier
       if (b + 1 < nblocks) {
         cp_async_wait<1>();
-        sb_bar<2, kSbPrep>();
+        sb_bar<2, P::PREP_THREADS>();
         prepare(b + 1);
       }
       __syncthreads();
