@@ -52,26 +52,42 @@ __global__ void __launch_bounds__(F32Plan<BM, BN, TM, TN, KS, STAGES>::kThreads,
   const int n0 = blockIdx.x * kCols;
   const uint32_t smem = smem_u32(f32_smem);
 
-  // 16-byte pieces of a stage: [group][x rows, then weight rows][eight of four k]; what lies outside arrives as zeros
-  auto fill = [&](int step) {
-    const uint32_t st = smem + (step % STAGES) * P::kStage * 4;
-    const int k_step = step * KS * kF32K;
-    for (int i = threadIdx.x; i < KS * P::kRows * (kF32K / 4); i += P::kThreads) {
-      const int c = i % (kF32K / 4), r = i / (kF32K / 4) % P::kRows, g = i / (kF32K / 4) / P::kRows;
-      const int k = k_step + g * kF32K + c * 4;
-      const float* src = x;
-      bool in = k < a.k;
-      if (r < BM) {
-        in = in && row0 + r < a.m;
-        src = x + (row0 + r) * a.ldx + k;
-      } else {
-        const int rw = r - BM, up = GLU && rw >= kCols ? 1 : 0, col = n0 + rw - up * kCols;
-        in = in && col < a.n;
-        src = w + (w_row0 + col + (up ? a.n : 0)) * a.k + k;
+  // 16-byte pieces of a stage: [group][x rows, then weight rows][eight of four k].  A thread fetches the same piece of the same NR
+  // rows of every group and stage, so their addresses are worked out once; what lies outside arrives as zeros.
+  constexpr int RS = P::kThreads / 8, NR = P::kRows / RS;
+  static_assert(P::kRows % RS == 0, "whole rounds over the rows of a stage");
+  const int piece = (threadIdx.x & 7) * 4;
+  const float* src[NR];
+  uint32_t live = 0;
+#pragma unroll
+  for (int q = 0; q < NR; ++q) {
+    const int r = static_cast<int>(threadIdx.x >> 3) + RS * q;
+    src[q] = static_cast<const float*>(a.w) + piece;
+    if (r < BM) {
+      if (row0 + r < a.m) {
+        src[q] = x + (row0 + r) * a.ldx + piece;
+        live |= 1u << q;
       }
-      const uint32_t bytes = in ? 16u : 0u;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(st + ((g * P::kRows + r) * kF32Ld + c * 4) * 4),
-                   "l"(in ? src : static_cast<const float*>(a.w)), "r"(bytes) : "memory");
+    } else {
+      const int rw = r - BM, up = GLU && rw >= kCols ? 1 : 0, col = n0 + rw - up * kCols;
+      if (col < a.n) {
+        src[q] = w + (w_row0 + col + (up ? a.n : 0)) * a.k + piece;
+        live |= 1u << q;
+      }
+    }
+  }
+  const uint32_t dst0 = smem + ((threadIdx.x >> 3) * kF32Ld + piece) * 4;
+  auto fill = [&](int step) {
+    const uint32_t dst = dst0 + (step % STAGES) * P::kStage * 4;
+#pragma unroll
+    for (int g = 0; g < KS; ++g) {
+      const int k = (step * KS + g) * kF32K;
+#pragma unroll
+      for (int q = 0; q < NR; ++q) {
+        const bool in = (live >> q & 1u) && k + piece < a.k;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (g * P::kRows + RS * q) * kF32Ld * 4),
+                     "l"(in ? src[q] + k : static_cast<const float*>(a.w)), "r"(in ? 16u : 0u) : "memory");
+      }
     }
   };
 
@@ -95,7 +111,7 @@ __global__ void __launch_bounds__(F32Plan<BM, BN, TM, TN, KS, STAGES>::kThreads,
     const float* st = f32_smem + (s % STAGES) * P::kStage + group * P::kRows * kF32Ld;
     const float* xs = st + ty * kF32Ld;
     const float* ws = st + (BM + tx) * kF32Ld;
-#pragma unroll 2
+#pragma unroll 4
     for (int k = 0; k < kF32K; k += 4) {
       ulonglong2 xr[TM];
 #pragma unroll
