@@ -2,11 +2,13 @@
 // three forms as the grouped tcgen05 kernel: plain, one weight per head (column blocks of x and y), one weight per expert (row
 // tiles of 128).  GLU: half of a tile's weight rows are gate rows, the other half the up rows n further.
 //
-// Bound by the FMA units: 8 x 8 outputs per thread in packed pairs.  A pair holds the sums over even and over odd k, so that both
-// operands are pairs as they lie in memory (k contiguous): no transposing, no duplicating, 16-byte cp.async into a ring and
-// 16-byte reads out of it, 128 packed FMAs for 16 reads.  Rows of a stage are 36 floats long: the eight lanes that read eight
-// neighbouring rows meet eight different groups of banks.  The KS groups of a CTA take 32 k each of a stage and add their sums up
-// in shared memory in a fixed order: a tile of 64 x 64 then has 256 threads, and 500 rows x 1024 columns already give 128 CTAs.
+// Bound by shared memory and the FMA units alike: 8 x 8 outputs per thread, operands as they lie in memory (k contiguous): no
+// transposing, 16-byte cp.async into a ring and 16-byte reads out of it, 256 FMAs for 16 reads.  Scalar FMAs: the packed form is
+// bound by the register file (67 against 114 FMA per cycle and SM in a loop of 8 x 8 outputs).  Rows of a stage are 36 floats
+// long: the eight lanes that read eight neighbouring rows meet eight different groups of banks.  The KS groups of a CTA take 32
+// k each of a stage and add their sums up in shared memory in a fixed order: a tile of 64 x 64 then has 256 threads, and 500
+// rows x 1024 columns already give 128 CTAs.  A prompt of 500 tokens through three layers of width 1024, scans and attention
+// included: 3.19 -> 1.54 ms, of 16 tokens 1.61 -> 0.63 ms.  (8 x 16 outputs per thread, a quarter fewer reads: 1.60 ms.)
 #include "mdb_common.cuh"
 
 namespace mdb {
@@ -21,12 +23,6 @@ struct F32Plan {
   static_assert(TX % 8 == 0 && (KS == 1 || TM % KS == 0), "eight lanes share a row of x; the last sums are dealt out by rows");
   static_assert(KS * BM * BN <= STAGES * kStage, "the groups' sums fit where the operands were");
 };
-
-__device__ __forceinline__ unsigned long long f32_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
 
 template <int BM, int BN, int TM, int TN, int KS, int STAGES, bool GLU>
 __global__ void __launch_bounds__(F32Plan<BM, BN, TM, TN, KS, STAGES>::kThreads, 1) gemm_f32_kernel(const mdb_gemm_args a) {
@@ -92,11 +88,11 @@ __global__ void __launch_bounds__(F32Plan<BM, BN, TM, TN, KS, STAGES>::kThreads,
   };
 
   const int group = threadIdx.x / P::kGroup, lid = threadIdx.x % P::kGroup, tx = lid % P::TX, ty = lid / P::TX;
-  unsigned long long acc[TM][TN];
+  float acc[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
   const int steps = (a.k + KS * kF32K - 1) / (KS * kF32K);
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
@@ -113,16 +109,20 @@ __global__ void __launch_bounds__(F32Plan<BM, BN, TM, TN, KS, STAGES>::kThreads,
     const float* ws = st + (BM + tx) * kF32Ld;
 #pragma unroll 4
     for (int k = 0; k < kF32K; k += 4) {
-      ulonglong2 xr[TM];
+      float4 xr[TM];
 #pragma unroll
-      for (int i = 0; i < TM; ++i) xr[i] = *reinterpret_cast<const ulonglong2*>(xs + i * P::TY * kF32Ld + k);
+      for (int i = 0; i < TM; ++i) xr[i] = *reinterpret_cast<const float4*>(xs + i * P::TY * kF32Ld + k);
 #pragma unroll
       for (int j = 0; j < TN; ++j) {
-        const ulonglong2 wr = *reinterpret_cast<const ulonglong2*>(ws + j * P::TX * kF32Ld + k);
+        const float4 wr = *reinterpret_cast<const float4*>(ws + j * P::TX * kF32Ld + k);
 #pragma unroll
-        for (int i = 0; i < TM; ++i) acc[i][j] = f32_fma2(xr[i].x, wr.x, acc[i][j]);
+        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(xr[i].x, wr.x, acc[i][j]);
 #pragma unroll
-        for (int i = 0; i < TM; ++i) acc[i][j] = f32_fma2(xr[i].y, wr.y, acc[i][j]);
+        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(xr[i].y, wr.y, acc[i][j]);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(xr[i].z, wr.z, acc[i][j]);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(xr[i].w, wr.w, acc[i][j]);
       }
     }
   }
@@ -142,13 +142,12 @@ __global__ void __launch_bounds__(F32Plan<BM, BN, TM, TN, KS, STAGES>::kThreads,
       y[row * a.ldy + y_col + col] = z;
     }
   };
-  auto sum = [](unsigned long long p) { return __uint_as_float(static_cast<uint32_t>(p)) + __uint_as_float(static_cast<uint32_t>(p >> 32)); };
   if (KS == 1) {
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
       float v[TN];
 #pragma unroll
-      for (int j = 0; j < TN; ++j) v[j] = sum(acc[i][j]);
+      for (int j = 0; j < TN; ++j) v[j] = acc[i][j];
       leave(i, v);
     }
     return;
@@ -157,7 +156,7 @@ __global__ void __launch_bounds__(F32Plan<BM, BN, TM, TN, KS, STAGES>::kThreads,
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) f32_smem[((group * TM + i) * TN + j) * P::kGroup + lid] = sum(acc[i][j]);
+    for (int j = 0; j < TN; ++j) f32_smem[((group * TM + i) * TN + j) * P::kGroup + lid] = acc[i][j];
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < (KS == 1 ? 1 : TM / KS); ++r) {
