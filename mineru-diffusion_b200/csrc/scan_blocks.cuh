@@ -392,7 +392,8 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
     const float4* per_token = reinterpret_cast<const float4*>(prep + P::P_T);
     // products with the state in front of the block: of a token's k and q (delta), or of two tokens' q, per exchange
     constexpr int ROWS = DELTA ? 2 * T : T;
-#pragma unroll 2
+    constexpr int AHEAD = CPT <= 2 ? 8 : 2;      // chains of sums over lanes in flight, as registers allow
+#pragma unroll AHEAD
     for (int r = 0; r < ROWS; r += 2) {
       const float* x0 = DELTA ? prep + (r >> 1) * DP + l16 * 4 : raw + P::RAW_Q + r * DP + l16 * 4;
       const float* x1 = DELTA ? prep + P::P_QH + (r >> 1) * DP + l16 * 4 : x0 + DP;
@@ -468,7 +469,7 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
 #pragma unroll
         for (int c = 0; c < 2 * NR; ++c) S[i][c] = mul2(S[i][c], g);
     }
-#pragma unroll 4
+#pragma unroll 8
     for (int t = 0; t < T; ++t) {
       f32x2 u[CPT];
 #pragma unroll
