@@ -12,7 +12,9 @@
 // What bounds it: latency, with few warps per scheduler.  All the states of four prompts of 16 heads are 55 elements per FMA
 // lane of the chip.  A CTA has warps that keep COLS columns of the state in registers (CPT columns x 1/16 of the channels a
 // thread: a 16-byte read of shared memory feeds 4 CPT FMAs) and others that prepare the next block meanwhile: its operands with
-// cp.async two blocks ahead, the scaled rows, L and M.
+// cp.async two blocks ahead, the scaled rows, L and M.  Against the token-by-token form, 2048 tokens: mLSTM, 8 heads of 128 x 256,
+// one, two and four sequences 478 / 635 / 681 -> 315 / 350 / 470 us; delta rule with its decays, 16 heads of 128 x 128, 840 / 857
+// / 1399 -> 485 / 611 / 820 us.
 constexpr int kSbTokens = 16, kSbRing = 3;
 
 template <int MODE, int DP, int COLS, int CPT>
