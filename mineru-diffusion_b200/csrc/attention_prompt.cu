@@ -7,18 +7,17 @@
 //
 // A tile is 128 query rows, `tokens x group` of one sequence and KV head (row = token * group + head in group); a unit is two
 // neighbouring tiles A and B of one sequence, which walk the same key tiles of 128 keys.  Roles: a TMA warp (both Q tiles, K and
-// V rings) and, per tile, an MMA warp and four softmax warps, one query row per thread.
+// V rings), an MMA warp, and four softmax warps per tile, one query row per thread.
 //
 // What bounds it: the chain of a tile (S ready, scores to registers, maximum, exponentials, P back, P V) took 1.7 us for
 // 128 keys and 0.27 us of products while one tile had the SM to itself.  Here one tile's softmax runs under the other's products,
-// and each tile goes in steps of 64 keys with two score buffers, so that the scores of the next step are there when a softmax
-// ends; P goes back into the tensor memory of the scores it came from (bf16 pairs, the left operand of P V): no shared
-// memory for P and no proxy fence.  The products of one thread run in the order of issue, so new scores may follow P V into the
-// same columns without a wait.  One warp issuing for both tiles spent 2000 cycles per step of both on its waits and issues, twice
-// what the exponentials take, hence a warp per tile.  4 x 4096 tokens, 16 query and 8 KV heads: 404 -> 299 us (923 TFLOP/s of
-// visible products; one issuing warp 313, one score buffer of 128 keys per tile 322).
+// and P goes back into the tensor memory of the scores it came from (bf16 pairs, the left operand of P V): no shared memory for P
+// and no proxy fence.  The products of one thread run in the order of issue, so new scores may follow P V into the same columns
+// without a wait.  A unit of one tile (see the launch) takes both score buffers in turn, the next scores ahead of P V.
+// 4 x 4096 tokens, 16 query and 8 KV heads: 418 -> 322 us, the same bits.  (Steps of 64 keys with two score buffers per tile, and an
+// issuing warp per tile: 299 us alone, 329 in a loop at the power limit, and other roundings; an issuing warp per tile here: 351.)
 //
-// Tensor memory: S_A (P_A) two steps | S_B (P_B) two steps, 64 columns each | O_A | O_B, 128 columns each.
+// Tensor memory: S_A (P_A) | S_B (P_B) | O_A | O_B, 128 columns each; with one tile S of even | odd key tiles | O.
 #include "mdb_common.cuh"
 
 namespace mdb {
@@ -26,7 +25,10 @@ namespace mdb {
 struct ApPlan {
   static constexpr int kKStages = 3, kVStages = 2;
   static constexpr int kQBytes = 2 * 128 * 128;             // a tile: two channel halves of [128 rows][128 B]
-  static constexpr int kProducerWarp = 8, kMmaWarp = 9 /* tile A; B: the next */, kThreads = 352;
+  static constexpr int kProducerWarp = 8, kMmaWarp = 9, kThreads = 384;      // three warpgroups; two warps idle
+  // registers: 384 threads x 168 at launch = 256 x 216 (softmax) + 128 x 72
+  static constexpr int kSoftmaxRegs = 216, kOtherRegs = 72;
+  static_assert(256 * kSoftmaxRegs + 128 * kOtherRegs <= kThreads * 168, "registers after the split");
   static constexpr int kOffK = 2 * kQBytes;
   static constexpr int kOffV = kOffK + kKStages * kAtTileBytes;
   static constexpr int kOffBars = kOffV + kVStages * kAtTileBytes;
@@ -34,12 +36,11 @@ struct ApPlan {
 };
 static_assert(ApPlan::kSmemBytes <= 227 * 1024, "shared memory of the prompt attention");
 
-// barrier slots; those of a tile (A, B) come in pairs, scores and P per tile and buffer
+// barrier slots; those of a tile (A, B) or of a score buffer come in pairs
 enum {
   kApBarQFull = 0, kApBarQEmpty = 1, kApBarQReady = 2, kApBarKFull = 4, kApBarKEmpty = 7, kApBarVFull = 10, kApBarVEmpty = 12,
-  kApBarSFull = 14 /* [tile][buffer] */, kApBarPFull = 18, kApBarPDone = 22, kApBarOFull = 24, kApBarOEmpty = 26, kApBarCount = 28
+  kApBarSFull = 14, kApBarPFull = 16, kApBarPDone = 18, kApBarOFull = 20, kApBarOEmpty = 22, kApBarCount = 24
 };
-constexpr int kApStep = 64;      // keys of a step
 
 // Four products in a row with one elected lane: left operand steps of `a_step`, right operand steps of `b_step` (descriptor
 // units of 16 bytes).
@@ -77,7 +78,7 @@ __device__ __forceinline__ void umma_bf16_ts_x4_w(uint32_t d_tmem, uint32_t a_tm
 struct ApTile {
   bool valid;
   int m0;             // first query
-  int first, last;    // steps of 64 keys [first, last) of the unit
+  int first, last;    // key tiles [first, last) of the unit
 };
 struct ApUnit {
   int seq, kvh, q_start, Tq, q_off, T, seq_start;
@@ -122,9 +123,9 @@ __device__ __forceinline__ ApUnit ap_unit(const AtArgs& a, int units, int wave) 
     const int beg = WIN && a.window > 0 ? max(0, w.q_off + t.m0 - a.window + 1) : 0;
     if (x == 0) w.kbeg = beg / kAtKeys * kAtKeys;
     w.kend = end;
-    t.first = (beg - w.kbeg) / kApStep;
-    t.last = (end - w.kbeg + kApStep - 1) / kApStep;
-    w.ntiles = (end - w.kbeg + kAtKeys - 1) / kAtKeys;
+    t.first = (beg - w.kbeg) / kAtKeys;
+    t.last = (end - w.kbeg + kAtKeys - 1) / kAtKeys;
+    w.ntiles = t.last;
   }
   return w;
 }
@@ -150,9 +151,8 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   pdl_launch_dependents();
   if (threadIdx.x == 0) {
     for (int s = 0; s < kApBarCount; ++s) {
-      const bool by_softmax = s == kApBarQReady || s == kApBarQReady + 1 || (s >= kApBarPFull && s < kApBarPFull + 4) || s >= kApBarOEmpty;
-      const bool by_products = s == kApBarQEmpty || (s >= kApBarKEmpty && s < kApBarVFull) || (s >= kApBarVEmpty && s < kApBarSFull);
-      mbar_init(bar(s), by_softmax ? 4 : by_products ? 2 : 1);
+      const bool by_softmax = s == kApBarQReady || s == kApBarQReady + 1 || (s >= kApBarPFull && s < kApBarPFull + 2) || s >= kApBarOEmpty;
+      mbar_init(bar(s), by_softmax ? 4 : 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -167,149 +167,176 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   const uint32_t tmem_base = misc[0];
   pdl_wait();   // q and the K/V rows of this step come from the preceding kernels
 
-  if (warp == P::kProducerWarp) {
-    // ------------------------------------------------------------------ producer
-    if (lane == 0) {
+  if (warp >= P::kProducerWarp) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(P::kOtherRegs));
+    if (warp == P::kProducerWarp) {
+      // ------------------------------------------------------------------ producer
+      if (lane == 0) {
+        AtRing kr, vr;
+        uint32_t q_phase = 0;
+        uint32_t pend_k = 0, pend_v = 0, pend_q = 0;          // stages with a copy in flight, and the parity it completes
+        uint32_t par_k = 0, par_v = 0, par_q = 0;
+        bool ok = true;
+        auto load_tile = [&](const CUtensorMap* map, uint32_t tiles0, int full0, int empty0, int stages, AtRing& r,
+                             uint32_t& pend, uint32_t& par, int kvh, int token_row) {
+          if (!mbar_wait(bar(empty0 + r.stage), r.phase ^ 1)) return false;
+          const uint32_t full = bar(full0 + r.stage);
+          const uint32_t dst = tiles0 + r.stage * kAtTileBytes;
+          mbar_arrive_expect_tx(full, halves * kAtHalfBytes);
+          tma_load_2d(dst, map, kvh * 64 * halves, token_row, full);
+          if (halves > 1) tma_load_2d(dst + kAtHalfBytes, map, kvh * kHeadDim + 64, token_row, full);
+          pend |= 1u << r.stage;
+          par = (par & ~(1u << r.stage)) | (r.phase << r.stage);
+          r.advance(stages);
+          return true;
+        };
+        for (int wave = 0; wave < waves && ok; ++wave) {
+          const ApUnit w = ap_unit<WIN>(a, units, wave);
+          if (w.ntiles == 0) continue;
+          if (!mbar_wait(bar(kApBarQEmpty), q_phase ^ 1)) { ok = false; break; }
+          {
+            const uint32_t full = bar(kApBarQFull);
+            mbar_arrive_expect_tx(full, static_cast<uint32_t>(rows_used) * 128u * halves * (w.t[1].valid ? 2u : 1u));
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+              if (!w.t[x].valid) continue;
+              const uint32_t dst = base + x * P::kQBytes;
+              tma_load_3d(dst, &map_q, 0, w.kvh * group, w.q_start + w.t[x].m0, full);
+              if (halves > 1) tma_load_3d(dst + 128 * 128, &map_q, 64, w.kvh * group, w.q_start + w.t[x].m0, full);
+            }
+            pend_q = 1u;
+            par_q = q_phase;
+            q_phase ^= 1;
+          }
+          auto token_row = [&](int tile) {
+            const int key0 = w.kbeg + tile * kAtKeys;
+            if (!WIN) return w.seq_start + key0;
+            int page = key0 / kPage < a.table_stride ? a.block_table[static_cast<int64_t>(w.seq) * a.table_stride + key0 / kPage] : -1;
+            if (page < 0 || page >= a.num_pages) {
+              report_status(MDB_STATUS_BAD_PAGE);
+              page = 0;
+            }
+            return page * kPage + key0 % kPage;
+          };
+          for (int j = 0; j < w.ntiles && ok; ++j) {
+            ok = load_tile(&map_k, base + P::kOffK, kApBarKFull, kApBarKEmpty, P::kKStages, kr, pend_k, par_k, w.kvh, token_row(j));
+            if (ok)
+              ok = load_tile(&map_v, base + P::kOffV, kApBarVFull, kApBarVEmpty, P::kVStages, vr, pend_v, par_v, w.kvh, token_row(j));
+          }
+        }
+        if (!ok) {
+          report_status(MDB_STATUS_WAIT_TIMEOUT);
+          // let the copies already issued land before the CTA gives its shared memory back
+          for (int s = 0; s < P::kKStages; ++s) if (pend_k >> s & 1) mbar_wait(bar(kApBarKFull + s), par_k >> s & 1);
+          for (int s = 0; s < P::kVStages; ++s) if (pend_v >> s & 1) mbar_wait(bar(kApBarVFull + s), par_v >> s & 1);
+          if (pend_q) mbar_wait(bar(kApBarQFull), par_q);
+        }
+      }
+    } else if (warp == P::kMmaWarp) {
+      // ----------------------------------------------------------------- MMA issue (all lanes, one elected)
+      const bool single = a.tiles_per_unit == 1;
+      // bf16 x bf16 -> fp32, M = 128, N = 128 (or 64 channels); bit 16 set: B operand MN-major
+      const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kAtKeys >> 3) << 17) |
+                               (static_cast<uint32_t>(128 >> 4) << 24);
+      const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) |
+                               (static_cast<uint32_t>(halves * 8) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
       AtRing kr, vr;
-      uint32_t q_phase = 0;
-      uint32_t pend_k = 0, pend_v = 0, pend_q = 0;          // stages with a copy in flight, and the parity it completes
-      uint32_t par_k = 0, par_v = 0, par_q = 0;
+      uint32_t q_phase[2] = {0, 0}, p_phase = 0 /* bit per score buffer */, o_phase[2] = {0, 0};
+      uint32_t qfull_phase = 0;
       bool ok = true;
-      auto load_tile = [&](const CUtensorMap* map, uint32_t tiles0, int full0, int empty0, int stages, AtRing& r,
-                           uint32_t& pend, uint32_t& par, int kvh, int token_row) {
-        if (!mbar_wait(bar(empty0 + r.stage), r.phase ^ 1)) return false;
-        const uint32_t full = bar(full0 + r.stage);
-        const uint32_t dst = tiles0 + r.stage * kAtTileBytes;
-        mbar_arrive_expect_tx(full, halves * kAtHalfBytes);
-        tma_load_2d(dst, map, kvh * 64 * halves, token_row, full);
-        if (halves > 1) tma_load_2d(dst + kAtHalfBytes, map, kvh * kHeadDim + 64, token_row, full);
-        pend |= 1u << r.stage;
-        par = (par & ~(1u << r.stage)) | (r.phase << r.stage);
-        r.advance(stages);
-        return true;
-      };
       for (int wave = 0; wave < waves && ok; ++wave) {
         const ApUnit w = ap_unit<WIN>(a, units, wave);
         if (w.ntiles == 0) continue;
-        if (!mbar_wait(bar(kApBarQEmpty), q_phase ^ 1)) { ok = false; break; }
-        {
-          const uint32_t full = bar(kApBarQFull);
-          mbar_arrive_expect_tx(full, static_cast<uint32_t>(rows_used) * 128u * halves * (w.t[1].valid ? 2u : 1u));
+        if (WIN) {
+          if (!mbar_wait_w(bar(kApBarQFull), qfull_phase)) { ok = false; break; }
+          qfull_phase ^= 1;
+        } else {
+          // staircase form: the softmax warps scale q in place first
 #pragma unroll
           for (int x = 0; x < 2; ++x) {
             if (!w.t[x].valid) continue;
-            const uint32_t dst = base + x * P::kQBytes;
-            tma_load_3d(dst, &map_q, 0, w.kvh * group, w.q_start + w.t[x].m0, full);
-            if (halves > 1) tma_load_3d(dst + 128 * 128, &map_q, 64, w.kvh * group, w.q_start + w.t[x].m0, full);
+            if (ok && !mbar_wait_w(bar(kApBarQReady + x), q_phase[x])) ok = false;
+            q_phase[x] ^= 1;
           }
-          pend_q = 1u;
-          par_q = q_phase;
-          q_phase ^= 1;
+          if (!ok) break;
         }
-        auto token_row = [&](int tile) {
-          const int key0 = w.kbeg + tile * kAtKeys;
-          if (!WIN) return w.seq_start + key0;
-          int page = key0 / kPage < a.table_stride ? a.block_table[static_cast<int64_t>(w.seq) * a.table_stride + key0 / kPage] : -1;
-          if (page < 0 || page >= a.num_pages) {
-            report_status(MDB_STATUS_BAD_PAGE);
-            page = 0;
-          }
-          return page * kPage + key0 % kPage;
-        };
-        for (int j = 0; j < w.ntiles && ok; ++j) {
-          ok = load_tile(&map_k, base + P::kOffK, kApBarKFull, kApBarKEmpty, P::kKStages, kr, pend_k, par_k, w.kvh, token_row(j));
-          if (ok)
-            ok = load_tile(&map_v, base + P::kOffV, kApBarVFull, kApBarVEmpty, P::kVStages, vr, pend_v, par_v, w.kvh, token_row(j));
-        }
-      }
-      if (!ok) {
-        report_status(MDB_STATUS_WAIT_TIMEOUT);
-        // let the copies already issued land before the CTA gives its shared memory back
-        for (int s = 0; s < P::kKStages; ++s) if (pend_k >> s & 1) mbar_wait(bar(kApBarKFull + s), par_k >> s & 1);
-        for (int s = 0; s < P::kVStages; ++s) if (pend_v >> s & 1) mbar_wait(bar(kApBarVFull + s), par_v >> s & 1);
-        if (pend_q) mbar_wait(bar(kApBarQFull), par_q);
-      }
-    }
-  } else if (warp >= P::kMmaWarp) {
-    // ----------------------------------------------------------------- MMA issue (all lanes, one elected), a warp per tile
-    const int x = warp - P::kMmaWarp;
-    // bf16 x bf16 -> fp32, M = 128, N = 64 keys, or 64 or 128 channels; bit 16 set: B operand MN-major
-    const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kApStep >> 3) << 17) |
-                             (static_cast<uint32_t>(128 >> 4) << 24);
-    const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) |
-                             (static_cast<uint32_t>(halves * 8) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
-    const uint32_t s_cols = tmem_base + x * 128, o_cols = tmem_base + 256 + x * 128;
-    AtRing kr, vr;
-    uint32_t q_phase = 0, p_phase = 0 /* bit per buffer */, o_phase = 0;
-    bool ok = true;
-    for (int wave = 0; wave < waves && ok; ++wave) {
-      const ApUnit w = ap_unit<WIN>(a, units, wave);
-      if (w.ntiles == 0) continue;
-      const ApTile t = x == 0 ? w.t[0] : w.t[1];
-      const int steps = w.t[1].valid ? w.t[1].last : w.t[0].last;
-      // staircase form: the softmax warps scale q in place first.  (Window form: seen by both, whether they have a tile or not,
-      // since the next phase is told from this one by parity.)
-      if (WIN || t.valid) {
-        if (!mbar_wait_w(bar(WIN ? kApBarQFull : kApBarQReady + x), q_phase)) { ok = false; break; }
-        q_phase ^= 1;
-      }
-      // Both warps walk all the key tiles and release them, with products of their own or not.
-      auto issue_s = [&](int h) {
-        if ((h & 1) == 0 && !mbar_wait_w(bar(kApBarKFull + kr.stage), kr.phase)) return false;
-        if (t.valid && h >= t.first && h < t.last) {
-          tc_fence_after();
-          const uint32_t k_rows = base + P::kOffK + kr.stage * kAtTileBytes + (h & 1) * (kApStep * 128);
+        auto issue_s = [&](int x, int buf) {           // scores of tile x with the K tile at the ring's position
+          const uint32_t q_tile = base + x * P::kQBytes, k_tile = base + P::kOffK + kr.stage * kAtTileBytes;
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             if (WIN && c >= halves) break;
-            umma_bf16_x4_w(s_cols + (h & 1) * kApStep, umma_desc_sw128(base + x * P::kQBytes + c * (128 * 128)), 2,
-                           umma_desc_sw128(k_rows + c * kAtHalfBytes), 2, idesc_s, c);
+            umma_bf16_x4_w(tmem_base + buf * 128, umma_desc_sw128(q_tile + c * (128 * 128)), 2, umma_desc_sw128(k_tile + c * kAtHalfBytes), 2,
+                           idesc_s, c);
           }
-          umma_commit_w(bar(kApBarSFull + 2 * x + (h & 1)));
-        }
-        if ((h & 1) || h == steps - 1) {
+          umma_commit_w(bar(kApBarSFull + buf));
+        };
+        auto release_k = [&](int j) {
           umma_commit_w(bar(kApBarKEmpty + kr.stage));
           kr.advance(P::kKStages);
-        }
-        if (h == steps - 1) umma_commit_w(bar(kApBarQEmpty));
-        return true;
-      };
-      ok = issue_s(0);
-      for (int h = 0; h < steps && ok; ++h) {
-        // (the buffer of step h + 1 held step h - 1, whose P V has been issued)
-        if (h + 1 < steps && !issue_s(h + 1)) { ok = false; break; }
-        if ((h & 1) == 0 && !mbar_wait_w(bar(kApBarVFull + vr.stage), vr.phase)) { ok = false; break; }
-        if (t.valid && h >= t.first && h < t.last) {
-          if (h == t.first) {
-            // the previous unit's accumulator must have been read out
-            if (!mbar_wait_w(bar(kApBarOEmpty + x), o_phase ^ 1)) { ok = false; break; }
-            o_phase ^= 1;
+          if (j == w.ntiles - 1) umma_commit_w(bar(kApBarQEmpty));
+        };
+        if (!mbar_wait_w(bar(kApBarKFull + kr.stage), kr.phase)) { ok = false; break; }
+        tc_fence_after();
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+          if (w.t[x].valid && w.t[x].first == 0) issue_s(x, x);
+        release_k(0);
+        for (int j = 0; j < w.ntiles && ok; ++j) {
+          const bool more = j + 1 < w.ntiles;
+          bool k_there = false;
+          if (single && more) {
+            // the other buffer held the last key tile, whose P V has been issued
+            if (!mbar_wait_w(bar(kApBarKFull + kr.stage), kr.phase)) { ok = false; break; }
+            tc_fence_after();
+            issue_s(0, (j + 1) & 1);
+            release_k(j + 1);
           }
-          if (!mbar_wait_w(bar(kApBarPFull + 2 * x + (h & 1)), p_phase >> (h & 1) & 1)) { ok = false; break; }
-          p_phase ^= 1u << (h & 1);
-          tc_fence_after();
-          umma_bf16_ts_x4_w(o_cols, s_cols + (h & 1) * kApStep,
-                            umma_desc_sw128_mn(base + P::kOffV + vr.stage * kAtTileBytes + (h & 1) * (kApStep * 128)), 128, idesc_o,
-                            h > t.first ? 1u : 0u);
-          umma_commit_w(bar(kApBarPDone + x));
-          if (h == t.last - 1) umma_commit_w(bar(kApBarOFull + x));
-        }
-        if ((h & 1) || h == steps - 1) {
+          if (!mbar_wait_w(bar(kApBarVFull + vr.stage), vr.phase)) { ok = false; break; }
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            if (!w.t[x].valid) continue;
+            if (j >= w.t[x].first && j < w.t[x].last) {
+              const int buf = single ? j & 1 : x;
+              if (j == w.t[x].first) {
+                // the previous unit's accumulator must have been read out
+                if (!mbar_wait_w(bar(kApBarOEmpty + x), o_phase[x] ^ 1)) { ok = false; break; }
+                o_phase[x] ^= 1;
+              }
+              if (!mbar_wait_w(bar(kApBarPFull + buf), p_phase >> buf & 1)) { ok = false; break; }
+              p_phase ^= 1u << buf;
+              tc_fence_after();
+              const uint32_t v_tile = base + P::kOffV + vr.stage * kAtTileBytes, p = tmem_base + buf * 128, o = tmem_base + 256 + x * 128;
+              umma_bf16_ts_x4_w(o, p, umma_desc_sw128_mn(v_tile), 128, idesc_o, j > w.t[x].first ? 1u : 0u);
+              umma_bf16_ts_x4_w(o, p + 32, umma_desc_sw128_mn(v_tile + 4 * 2048), 128, idesc_o, 1u);
+              umma_commit_w(bar(kApBarPDone + x));
+              if (j == w.t[x].last - 1) umma_commit_w(bar(kApBarOFull + x));
+            }
+            if (!single && more && j + 1 >= w.t[x].first && j + 1 < w.t[x].last) {
+              if (!k_there && !mbar_wait_w(bar(kApBarKFull + kr.stage), kr.phase)) { ok = false; break; }
+              k_there = true;
+              tc_fence_after();
+              issue_s(x, x);
+            }
+          }
+          if (!ok) break;
           umma_commit_w(bar(kApBarVEmpty + vr.stage));
           vr.advance(P::kVStages);
+          if (!single && more) release_k(j + 1);      // (the key tiles of A and B overlap or touch: every one is used by a tile)
         }
       }
+      if (!ok && lane == 0) report_status(MDB_STATUS_WAIT_TIMEOUT);
     }
-    if (!ok && lane == 0) report_status(MDB_STATUS_WAIT_TIMEOUT);
   } else {
     // ------------------------------------------------------------------- softmax
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(P::kSoftmaxRegs));
     const int x = warp >> 2;                               // tile A or B
     const int row = threadIdx.x & 127;                     // query row of the tile, and its tensor-memory lane
     const int tok_local = row / group, head_in_group = row % group;
     const uint32_t lane_field = static_cast<uint32_t>(32 * (warp & 3)) << 16;
-    const uint32_t s_addr = tmem_base + x * 128 + lane_field, o_addr = s_addr + 256;
+    const bool single = a.tiles_per_unit == 1;
+    const uint32_t o_addr = tmem_base + 256 + x * 128 + lane_field;
     AtRing vr;                          // V ring position of the unit's first key tile
-    uint32_t s_phase = 0 /* bit per buffer */, o_phase = 0, q_phase = 0, done_phase = 0;      // done: of the last step's P V
+    uint32_t s_phase = 0 /* bit per buffer */, o_phase = 0, q_phase = 0, done_phase = 0;      // done: of the last P V
     bool ok = true;
     for (int wave = 0; wave < waves && ok; ++wave) {
       const ApUnit w = ap_unit<WIN>(a, units, wave);
@@ -360,44 +387,45 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       q_phase ^= 1;
       float m_ref = -INFINITY, l = 0.f;
       for (int j = t.first; j < t.last; ++j) {
-        const int buf = j & 1;
-        ok = mbar_wait(bar(kApBarSFull + 2 * x + buf), s_phase >> buf & 1);
+        const int buf = single ? j & 1 : x;
+        const uint32_t s_addr = tmem_base + buf * 128 + lane_field;
+        ok = mbar_wait(bar(kApBarSFull + buf), s_phase >> buf & 1);
         if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
         s_phase ^= 1u << buf;
         tc_fence_after();
-        const int key0 = w.kbeg + j * kApStep;
-        float s[kApStep];
+        const int key0 = w.kbeg + j * kAtKeys;
+        float s[kAtKeys];
 #pragma unroll
-        for (int c = 0; c < 2; ++c) tmem_ld32(s_addr + buf * kApStep + 32 * c, s + 32 * c);
+        for (int c = 0; c < 4; ++c) tmem_ld32(s_addr + 32 * c, s + 32 * c);
         tmem_ld_wait();
-        const int nv = limit + 1 - key0;            // keys of this step the row sees: [0, nv)
-        if (nv < kApStep) {
+        const int nv = limit + 1 - key0;            // keys of this tile the row sees: [0, nv)
+        if (nv < kAtKeys) {
 #pragma unroll
-          for (int c = 0; c < kApStep; ++c) if (c >= nv) s[c] = -INFINITY;   // also replaces NaN from stale rows
+          for (int c = 0; c < kAtKeys; ++c) if (c >= nv) s[c] = -INFINITY;   // also replaces NaN from stale rows
         }
         if (WIN && first > key0) {
 #pragma unroll
-          for (int c = 0; c < kApStep; ++c) if (c < first - key0) s[c] = -INFINITY;
+          for (int c = 0; c < kAtKeys; ++c) if (c < first - key0) s[c] = -INFINITY;
         }
         float mxv[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) mxv[k] = s[k];
 #pragma unroll
-        for (int c = 8; c < kApStep; c += 8) {
+        for (int c = 8; c < kAtKeys; c += 8) {
 #pragma unroll
           for (int k = 0; k < 8; ++k) mxv[k] = fmaxf(mxv[k], s[c + k]);
         }
         float mx = fmaxf(fmaxf(fmaxf(mxv[0], mxv[1]), fmaxf(mxv[2], mxv[3])), fmaxf(fmaxf(mxv[4], mxv[5]), fmaxf(mxv[6], mxv[7])));
         if (!row_valid) mx = 0.f;                             // rows past the portion hold whatever the tile held
         const float m_tile = mx * a.scale_log2;
-        // a row that sees no key of this step (above the tile's diagonal) keeps its state
+        // a row that sees no key of this tile (above the diagonal) keeps its state
         const bool grow = m_tile > m_ref + kAtRescaleStep || (m_ref == -INFINITY && m_tile != -INFINITY);
         if (__any_sync(0xffffffffu, grow)) {
           const float m_new = fmaxf(m_ref, m_tile);
           const float f = m_ref == -INFINITY ? 0.f : ex2_approx(m_ref - m_new);
           l *= f;
           if (j > t.first) {
-            // O is quiet once the last step's P V has completed (the one before completed before these scores)
+            // O is quiet once the last key tile's P V has completed (the one before completed before these scores)
             ok = mbar_wait(bar(kApBarPDone + x), done_phase ^ 1);
             if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
             tc_fence_after();
@@ -416,34 +444,37 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         // P = 2^(s * scale - m_ref) rounded to bf16; a masked key gives 2^-inf = 0
         const float m_use = m_ref == -INFINITY ? 0.f : m_ref;   // nothing seen yet: every s is -inf, P = 0
         float lv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        float pk[32];                                           // 64 keys, two per word
 #pragma unroll
-        for (int c = 0; c < kApStep; c += 8) {
-          float pv[8];
+        for (int h = 0; h < 2; ++h) {
+          float pk[32];                                         // 64 keys, two per word
 #pragma unroll
-          for (int k = 0; k < 8; ++k) pv[k] = ex2_approx(fmaf(s[c + k], a.scale_log2, -m_use));
+          for (int c = 0; c < 64; c += 8) {
+            float pv[8];
 #pragma unroll
-          for (int k = 0; k < 8; ++k) lv[k] += pv[k];
+            for (int k = 0; k < 8; ++k) pv[k] = ex2_approx(fmaf(s[64 * h + c + k], a.scale_log2, -m_use));
 #pragma unroll
-          for (int k = 0; k < 8; k += 2) pk[(c + k) >> 1] = __uint_as_float(pack_bf16x2(pv[k], pv[k + 1]));
+            for (int k = 0; k < 8; ++k) lv[k] += pv[k];
+#pragma unroll
+            for (int k = 0; k < 8; k += 2) pk[(c + k) >> 1] = __uint_as_float(pack_bf16x2(pv[k], pv[k + 1]));
+          }
+          tmem_st32(s_addr + 32 * h, pk);
         }
-        tmem_st32(s_addr + buf * kApStep, pk);
         l += ((lv[0] + lv[1]) + (lv[2] + lv[3])) + ((lv[4] + lv[5]) + (lv[6] + lv[7]));
-        if (WIN && w.kend - key0 < kApStep) {
+        if (WIN && w.kend - key0 < kAtKeys) {
           // stale cache rows past the context end must not reach O through 0 * (Inf or NaN): clear them in V.  Both tiles'
-          // warps do (where both take this step), each before its own P V.
+          // warps do (where both take this key tile), each before its own P V.
           AtRing v = vr;
-          for (int n = 0; n < j >> 1; ++n) v.advance(P::kVStages);
+          for (int n = 0; n < j; ++n) v.advance(P::kVStages);
           ok = mbar_wait(bar(kApBarVFull + v.stage), v.phase);
           if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
-          const uint32_t v_rows = base + P::kOffV + v.stage * kAtTileBytes + buf * (kApStep * 128);
+          const uint32_t v_tile = base + P::kOffV + v.stage * kAtTileBytes;
           const int r = w.kend - key0 + row;
-          if (r < kApStep) {
+          if (r < kAtKeys) {
 #pragma unroll
             for (int h = 0; h < 2; ++h)
 #pragma unroll
               for (int c = 0; c < 8; ++c)
-                asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(v_rows + h * kAtHalfBytes + r * 128 + c * 16),
+                asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(v_tile + h * kAtHalfBytes + r * 128 + c * 16),
                              "r"(0u)
                              : "memory");
           }
@@ -452,7 +483,7 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar(kApBarPFull + 2 * x + buf));
+        if (lane == 0) mbar_arrive(bar(kApBarPFull + buf));
         done_phase ^= 1;
       }
       if (!ok) break;
