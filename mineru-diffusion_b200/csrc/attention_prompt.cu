@@ -14,8 +14,9 @@
 // and P goes back into the tensor memory of the scores it came from (bf16 pairs, the left operand of P V): no shared memory for P
 // and no proxy fence.  The products of one thread run in the order of issue, so new scores may follow P V into the same columns
 // without a wait.  A unit of one tile (see the launch) takes both score buffers in turn, the next scores ahead of P V.
-// 4 x 4096 tokens, 16 query and 8 KV heads: 418 -> 322 us, the same bits.  (Steps of 64 keys with two score buffers per tile, and an
-// issuing warp per tile: 299 us alone, 329 in a loop at the power limit, and other roundings; an issuing warp per tile here: 351.)
+// 4 x 4096 tokens, 16 query and 8 KV heads: 400 -> 301 us alone, 417 -> 335 in a loop at the power limit, the same bits.  (Steps of
+// 64 keys with two score buffers per tile and an issuing warp per tile: 299 us alone, 329 in a loop, other roundings; an issuing
+// warp per tile with these steps: 351.)
 //
 // Tensor memory: S_A (P_A) | S_B (P_B) | O_A | O_B, 128 columns each; with one tile S of even | odd key tiles | O.
 #include "mdb_common.cuh"
@@ -547,7 +548,7 @@ static int ap_launch(const CUtensorMap& map_q, const CUtensorMap& map_k, const C
     attr_once.done[dev] = true;
   }
   // Tiles that can all have an SM of their own take one: two on one SM wait for one another (one prompt of 1056
-  // tokens, 136 tiles: 24.8 us in pairs, 21.1 us alone).
+  // tokens, 136 tiles: 24.8 us in pairs, 20.4 us alone).
   const int sms = at_sm_count();
   a.tiles_per_unit = static_cast<int64_t>(a.max_qtiles) * a.nseq * a.hkv <= sms ? 1 : 2;
   const int64_t units = static_cast<int64_t>((a.max_qtiles + a.tiles_per_unit - 1) / a.tiles_per_unit) * a.nseq * a.hkv;
