@@ -242,7 +242,7 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) |
                                (static_cast<uint32_t>(halves * 8) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
       AtRing kr, vr;
-      uint32_t q_phase[2] = {0, 0}, p_phase = 0 /* bit per score buffer */, o_phase[2] = {0, 0};
+      uint32_t p_phase = 0 /* bit per score buffer */, o_phase[2] = {0, 0};
       uint32_t qfull_phase = 0;
       bool ok = true;
       for (int wave = 0; wave < waves && ok; ++wave) {
@@ -252,14 +252,10 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           if (!mbar_wait_w(bar(kApBarQFull), qfull_phase)) { ok = false; break; }
           qfull_phase ^= 1;
         } else {
-          // staircase form: the softmax warps scale q in place first
-#pragma unroll
-          for (int x = 0; x < 2; ++x) {
-            if (!w.t[x].valid) continue;
-            if (ok && !mbar_wait_w(bar(kApBarQReady + x), q_phase[x])) ok = false;
-            q_phase[x] ^= 1;
-          }
-          if (!ok) break;
+          // staircase form: the softmax warps scale q in place first.  Those of a tile that is not there have only seen it: the
+          // next unit's q may not arrive before all have, or they would miss a phase and wait for a later one.
+          if (!mbar_wait_w(bar(kApBarQReady), qfull_phase) || !mbar_wait_w(bar(kApBarQReady + 1), qfull_phase)) { ok = false; break; }
+          qfull_phase ^= 1;
         }
         auto issue_s = [&](int x, int buf) {           // scores of tile x with the K tile at the ring's position
           const uint32_t q_tile = base + x * P::kQBytes, k_tile = base + P::kOffK + kr.stage * kAtTileBytes;
@@ -344,10 +340,11 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       if (w.ntiles == 0) continue;
       const ApTile t = x == 0 ? w.t[0] : w.t[1];
       if (!t.valid) {
-        // (a phase must have been seen complete before the next one can be waited for by parity)
         if (!WIN) {
+          // a phase must have been seen complete before the next one can be waited for by parity
           ok = mbar_wait(bar(kApBarQFull), q_phase);
           if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+          if (lane == 0) mbar_arrive(bar(kApBarQReady + x));
         }
         q_phase ^= 1;
         if (WIN) for (int j = 0; j < w.ntiles; ++j) vr.advance(P::kVStages);

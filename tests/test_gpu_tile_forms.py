@@ -28,6 +28,16 @@ def i32(v):
 @pytest.mark.parametrize("hq,hkv", [(16, 8), (6, 2), (16, 2), (4, 4)])
 @pytest.mark.parametrize("lens", [[64], [1, 65, 129, 190], [700, 33, 64, 1000, 5, 321] * 4])
 def test_prompt_attention_pairs(hq, hkv, lens):
+    _prompts(hq, hkv, lens)
+
+
+# Several waves of CTAs in which a unit of one tile and one tile of keys comes behind a whole pair, behind its like, and in front of
+# a pair: the warps of the tile that is not there have to see every unit's queries arrive.
+def test_prompt_attention_tiles_alone_behind_pairs():
+    _prompts(2, 1, [128] * 150 + [40] * 460 + [100] * 150 + [7] * 150)
+
+
+def _prompts(hq, hkv, lens):
     cu = [0]
     for n in lens:
         cu.append(cu[-1] + n)
