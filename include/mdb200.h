@@ -573,9 +573,12 @@ typedef struct {
   void* y;
   int64_t ldy;
   const float* skip; /* DECAY */
-  int64_t rows;      /* m, rows of all portions (0: unknown): picks the form of a prompt's scan */
 } mdb_scan_args;
 int mdb_scan(const mdb_scan_args* args, mdb_stream_t stream);
+/* The same, told how many rows the portions have together (since version 102; 0: unknown, as in mdb_scan): from 16 tokens a
+ * portion on average up, heads of up to 128 channels are scanned in blocks of 16 tokens.  The sums of a row are rounded in the
+ * order of the form that is taken. */
+int mdb_scan_rows(const mdb_scan_args* args, int64_t rows, mdb_stream_t stream);
 
 /* The decay scan over prompt portions in chunks of 64 tokens on the tensor cores: bf16 rows of ldq / ldk elements with head
  * g of q and k at column g * dim (dim a multiple of 8, missing channels up to dim_pad count as zeros) and rows of ldv elements

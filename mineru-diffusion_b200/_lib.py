@@ -73,7 +73,7 @@ ScanArgs = _struct("ScanArgs", [(n, _i) for n in (
     ("state_slot_stride", _i64), ("num_slots", _i64), ("mstate", _p), ("scalars", _p),
     ("den", _p), ("cu_q", _p), ("start", _p),
     ("state_slot", _p), ("out", _p), ("raw_decay", Rows), ("a_log", _p), ("dt_bias", _p), ("gate", Rows), ("norm", _p),
-    ("norm_head_stride", _i64), ("y", _p), ("ldy", _i64), ("skip", _p), ("rows", _i64)])
+    ("norm_head_stride", _i64), ("y", _p), ("ldy", _i64), ("skip", _p)])
 ChunkScanArgs = _struct("ChunkScanArgs", [(n, _i) for n in ("m", "bs", "heads", "kv_heads", "dim", "dim_pad", "vdim", "max_q")] + [
     ("q", _p), ("k", _p), ("v", _p), ("ldq", _i64), ("ldk", _i64), ("ldv", _i64), ("ld_scalars", _i64), ("log_decay", _p), ("step", _p), ("skip", _p), ("state", _p), ("state_slot_stride", _i64),
     ("num_slots", _i64), ("cu_q", _p), ("start", _p), ("state_slot", _p), ("out", _p)])
@@ -143,6 +143,7 @@ SIGNATURES = {
     "mdb_channel_decay": (_i, [C.POINTER(DecayArgs), _p]),
     "mdb_mlstm_prep": (_i, [C.POINTER(MlstmPrepArgs), _p]),
     "mdb_scan": (_i, [C.POINTER(ScanArgs), _p]),
+    "mdb_scan_rows": (_i, [C.POINTER(ScanArgs), _i64, _p]),
     "mdb_chunk_scan_supported": (_i, [_i, _i]),
     "mdb_chunk_scan": (_i, [C.POINTER(ChunkScanArgs), _p]),
     "mdb_moe_route": (_i, [C.POINTER(MoeRouteArgs), _p]),

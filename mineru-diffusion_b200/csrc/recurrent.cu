@@ -1161,14 +1161,14 @@ int launch_scan_prompt(const mdb_scan_args& a, cudaStream_t st) {
 }
 
 template <int MODE, int DP>
-int launch_scan_dim(const mdb_scan_args& a, cudaStream_t st) {
+int launch_scan_dim(const mdb_scan_args& a, int64_t rows, cudaStream_t st) {
   if (a.fused) return a.dtype == MDB_F32 ? launch_scan_token<float, MODE, DP / 32>(a, st) : launch_scan_token<bf16, MODE, DP / 32>(a, st);
   if constexpr (DP <= 128) {
     // In blocks of 16 tokens, from portions of 16 tokens on average up (65 tokens of 4 heads: delta rule with its decays 29.0 us
     // against 29.7 token by token, mLSTM of 2 heads 16.8 against 17.7; 100 tokens of 4 x 16 heads 52.9 against 77.4); shorter
     // ones would leave most of a block empty.  64 columns per CTA, or 32 or 16 where their CTAs still run all at once: a block
     // of the delta rule takes 3.6 us with 16 columns, 4.5 with 32, 5.9 with 64.
-    if (a.rows >= static_cast<int64_t>(kSbTokens) * a.bs) {
+    if (rows >= static_cast<int64_t>(kSbTokens) * a.bs) {
       const int64_t heads = static_cast<int64_t>(a.heads) * a.bs;
       if ((a.vdim + 15) / 16 * heads <= 148) return launch_scan_blocks<MODE, DP, 16, 2>(a, st);
       return (a.vdim + 31) / 32 * heads <= 148 ? launch_scan_blocks<MODE, DP, 32, 4>(a, st) : launch_scan_blocks<MODE, DP, 64, 4>(a, st);
@@ -1180,13 +1180,13 @@ int launch_scan_dim(const mdb_scan_args& a, cudaStream_t st) {
 }
 
 template <int MODE>
-int launch_scan(const mdb_scan_args& a, cudaStream_t st) {
+int launch_scan(const mdb_scan_args& a, int64_t rows, cudaStream_t st) {
   switch (a.dim_pad) {
-    case 64: return launch_scan_dim<MODE, 64>(a, st);
-    case 128: return launch_scan_dim<MODE, 128>(a, st);
-    case 192: return launch_scan_dim<MODE, 192>(a, st);
-    case 256: return launch_scan_dim<MODE, 256>(a, st);
-    case 512: return launch_scan_dim<MODE, 512>(a, st);
+    case 64: return launch_scan_dim<MODE, 64>(a, rows, st);
+    case 128: return launch_scan_dim<MODE, 128>(a, rows, st);
+    case 192: return launch_scan_dim<MODE, 192>(a, rows, st);
+    case 256: return launch_scan_dim<MODE, 256>(a, rows, st);
+    case 512: return launch_scan_dim<MODE, 512>(a, rows, st);
     default: return MDB_ERR_UNSUPPORTED;
   }
 }
@@ -1330,8 +1330,10 @@ int mdb_mlstm_prep(const mdb_mlstm_prep_args* args, mdb_stream_t stream) {
                : mdb_launch(mlstm_prep_kernel<bf16, true, false>, grid, dim3(256), 0, st, a);
 }
 
-int mdb_scan(const mdb_scan_args* args, mdb_stream_t stream) {
-  MDB_REQUIRE(args != nullptr, MDB_ERR_ARG);
+int mdb_scan(const mdb_scan_args* args, mdb_stream_t stream) { return mdb_scan_rows(args, 0, stream); }
+
+int mdb_scan_rows(const mdb_scan_args* args, int64_t rows, mdb_stream_t stream) {
+  MDB_REQUIRE(args != nullptr && rows >= 0, MDB_ERR_ARG);
   const mdb_scan_args a = *args;
   MDB_REQUIRE(a.mode >= MDB_SCAN_DELTA && a.mode <= MDB_SCAN_DECAY, MDB_ERR_ARG);
   MDB_REQUIRE(a.bs >= 0 && a.heads > 0 && a.kv_heads > 0 && a.heads % a.kv_heads == 0 && a.dim > 0 && a.vdim > 0, MDB_ERR_ARG);
@@ -1351,8 +1353,8 @@ int mdb_scan(const mdb_scan_args* args, mdb_stream_t stream) {
               MDB_ERR_ALIGN);
   MDB_REQUIRE(a.heads <= 65535 && a.bs <= 65535, MDB_ERR_UNSUPPORTED);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (a.mode == MDB_SCAN_DECAY) return launch_scan<kScanDecay>(a, st);
-  return a.mode == MDB_SCAN_DELTA ? launch_scan<kScanDelta>(a, st) : launch_scan<kScanMlstm>(a, st);
+  if (a.mode == MDB_SCAN_DECAY) return launch_scan<kScanDecay>(a, rows, st);
+  return a.mode == MDB_SCAN_DELTA ? launch_scan<kScanDelta>(a, rows, st) : launch_scan<kScanMlstm>(a, rows, st);
 }
 
 }  // extern "C"

@@ -762,8 +762,8 @@ def scan(mode: int, dtype: torch.dtype, bs: int, heads: int, kv_heads: int, dim:
         mstate=_ptr(mstate), scalars=_ptr(scalars), den=_ptr(den), cu_q=cu_q.data_ptr(), start=start.data_ptr(), state_slot=slot.data_ptr(),
         out=_ptr(out), raw_decay=_rows_c(raw_decay), a_log=_ptr(a_log), dt_bias=_ptr(dt_bias), gate=_rows_c(gate),
         norm=_ptr(norm), norm_head_stride=vdim if per_head_norm else 0, y=_ptr(y), ldy=0 if y is None else _rows(y, "y"),
-        skip=_ptr(skip), rows=q.shape[0])
-    _lib.check(_lib.lib().mdb_scan(a, _stream()), "mdb_scan")
+        skip=_ptr(skip))
+    _lib.check(_lib.lib().mdb_scan_rows(a, q.shape[0], _stream()), "mdb_scan_rows")
 
 
 def chunk_scan_supported(dim_pad: int, vdim: int) -> bool:

@@ -94,3 +94,52 @@ def test_argument_blocks_match_the_header(tmp_path):
         assert int(out[n]) == ctypes.sizeof(t), n
         for f, _ in t._fields_:
             assert int(out[f"{n}.{f}"]) == getattr(t, f).offset, f"{n}.{f}"
+
+
+# Callers built against an earlier header pass blocks of these sizes; a call reads no further.
+BLOCK_BYTES = {"mdb_rows": 40, "mdb_gemm_args": 104, "mdb_residual_norm_args": 216, "mdb_rms_segment": 96, "mdb_gated_norm_args": 104,
+               "mdb_part_norm_args": 104, "mdb_delta_prep_args": 376, "mdb_decay_args": 112, "mdb_mlstm_prep_args": 288, "mdb_decay_prep_args": 344,
+               "mdb_scan_args": 304, "mdb_chunk_scan_args": 168, "mdb_moe_route_args": 88, "mdb_moe_plan_args": 56, "mdb_rotary_commit_args": 224,
+               "mdb_window_attn_args": 200}
+
+
+def test_argument_blocks_keep_their_size():
+    import importlib
+    lib = importlib.import_module("mineru-diffusion_b200._lib")
+    for n, size in BLOCK_BYTES.items():
+        assert ctypes.sizeof(getattr(lib, "".join(p.capitalize() for p in n[len("mdb_"):].split("_")))) == size, n
+
+
+# A scan's block at the very end of a readable page.  The head count is past what a launch takes, so the call reads the whole block
+# and is refused on the host.
+SCAN_AT_PAGE_END = """
+import ctypes as C, importlib, mmap, sys
+sys.path.insert(0, {root!r})
+lib = importlib.import_module("mineru-diffusion_b200._lib")
+page = mmap.PAGESIZE
+mem = mmap.mmap(-1, 2 * page)
+base = C.addressof(C.c_char.from_buffer(mem))
+libc = C.CDLL(None, use_errno=True)
+assert libc.mprotect(C.c_void_p(base + page), C.c_size_t(page), 0) == 0
+block = lib.ScanArgs()
+block.mode, block.bs, block.heads, block.kv_heads, block.dim, block.dim_pad, block.vdim = 2, 1, 65536, 65536, 128, 128, 64
+for name in ("q", "k", "v", "s0", "s1", "state", "cu_q", "start", "state_slot", "out"):
+    setattr(block, name, 64)
+at = base + page - {size}
+C.memmove(at, C.addressof(block), {size})
+handle = C.CDLL(lib.LIB_PATH)
+handle.mdb_scan.argtypes = [C.c_void_p, C.c_void_p]
+print(handle.mdb_scan(at, None), flush=True)
+import os
+os._exit(0)
+"""
+
+
+def test_a_scan_reads_no_further_than_its_block(built):
+    import subprocess
+    import sys
+    code = SCAN_AT_PAGE_END.format(root=ROOT, size=BLOCK_BYTES["mdb_scan_args"])
+    run = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, (run.returncode, run.stderr[-400:])
+    unsupported = int(re.search(r"MDB_ERR_UNSUPPORTED\s*=?\s*\(?(-?\d+)", open(HEADER).read()).group(1))
+    assert int(run.stdout) == unsupported
