@@ -79,11 +79,13 @@ __device__ __forceinline__ void umma_bf16_ts_x4_w(uint32_t d_tmem, uint32_t a_tm
 struct ApTile {
   bool valid;
   int m0;             // first query
+  int end;            // keys in front of it are seen by a row of the tile
   int first, last;    // key tiles [first, last) of the unit
 };
 struct ApUnit {
   int seq, kvh, q_start, Tq, q_off, T, seq_start;
-  int kbeg, kend, ntiles;      // ntiles 0: nothing to do
+  int kbeg, ntiles;      // ntiles 0: nothing to do
+  int cut;               // window form: key tile inside which tile A's keys end and B's go on (-1: none)
   ApTile t[2];
 };
 
@@ -92,6 +94,7 @@ struct ApUnit {
 template <bool WIN>
 __device__ __forceinline__ ApUnit ap_unit(const AtArgs& a, int units, int wave) {
   ApUnit w = {};
+  w.cut = -1;
   const int G = static_cast<int>(gridDim.x), c = static_cast<int>(blockIdx.x);
   const int p = wave * G + ((wave & 1) ? G - 1 - c : c);
   if (p >= units) return w;
@@ -123,11 +126,12 @@ __device__ __forceinline__ ApUnit ap_unit(const AtArgs& a, int units, int wave) 
     // window form: from the tile of keys that holds the first query's first key
     const int beg = WIN && a.window > 0 ? max(0, w.q_off + t.m0 - a.window + 1) : 0;
     if (x == 0) w.kbeg = beg / kAtKeys * kAtKeys;
-    w.kend = end;
+    t.end = end;
     t.first = (beg - w.kbeg) / kAtKeys;
     t.last = (end - w.kbeg + kAtKeys - 1) / kAtKeys;
     w.ntiles = t.last;
   }
+  if (WIN && w.t[1].valid && w.t[0].end < w.kbeg + w.t[0].last * kAtKeys) w.cut = w.t[0].last - 1;
   return w;
 }
 
@@ -221,7 +225,7 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           };
           for (int j = 0; j < w.ntiles && ok; ++j) {
             ok = load_tile(&map_k, base + P::kOffK, kApBarKFull, kApBarKEmpty, P::kKStages, kr, pend_k, par_k, w.kvh, token_row(j));
-            if (ok)
+            for (int copy = 0; copy < (WIN && j == w.cut ? 2 : 1) && ok; ++copy)
               ok = load_tile(&map_v, base + P::kOffV, kApBarVFull, kApBarVEmpty, P::kVStages, vr, pend_v, par_v, w.kvh, token_row(j));
           }
         }
@@ -292,6 +296,11 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 #pragma unroll
           for (int x = 0; x < 2; ++x) {
             if (!w.t[x].valid) continue;
+            if (WIN && x == 1 && j == w.cut) {      // B's copy of the values
+              umma_commit_w(bar(kApBarVEmpty + vr.stage));
+              vr.advance(P::kVStages);
+              if (!mbar_wait_w(bar(kApBarVFull + vr.stage), vr.phase)) { ok = false; break; }
+            }
             if (j >= w.t[x].first && j < w.t[x].last) {
               const int buf = single ? j & 1 : x;
               if (j == w.t[x].first) {
@@ -333,6 +342,7 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     const bool single = a.tiles_per_unit == 1;
     const uint32_t o_addr = tmem_base + 256 + x * 128 + lane_field;
     AtRing vr;                          // V ring position of the unit's first key tile
+    auto skip_v = [&](const ApUnit& w) { if (WIN) for (int j = 0; j < w.ntiles + (w.cut >= 0 ? 1 : 0); ++j) vr.advance(P::kVStages); };
     uint32_t s_phase = 0 /* bit per buffer */, o_phase = 0, q_phase = 0, done_phase = 0;      // done: of the last P V
     bool ok = true;
     for (int wave = 0; wave < waves && ok; ++wave) {
@@ -347,7 +357,7 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           if (lane == 0) mbar_arrive(bar(kApBarQReady + x));
         }
         q_phase ^= 1;
-        if (WIN) for (int j = 0; j < w.ntiles; ++j) vr.advance(P::kVStages);
+        skip_v(w);
         continue;
       }
       const int head = w.kvh * group + head_in_group;
@@ -458,15 +468,15 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           tmem_st32(s_addr + 32 * h, pk);
         }
         l += ((lv[0] + lv[1]) + (lv[2] + lv[3])) + ((lv[4] + lv[5]) + (lv[6] + lv[7]));
-        if (WIN && w.kend - key0 < kAtKeys) {
-          // stale cache rows past the context end must not reach O through 0 * (Inf or NaN): clear them in V.  Both tiles'
-          // warps do (where both take this key tile), each before its own P V.
+        if (WIN && t.end - key0 < kAtKeys) {
+          // values behind the tile's last key (stale cache rows, or tokens that only tile B sees) must not reach O through
+          // 0 * (Inf or NaN): clear them.  Where A's keys end and B's go on, each has a copy of its own.
           AtRing v = vr;
-          for (int n = 0; n < j; ++n) v.advance(P::kVStages);
+          for (int n = 0; n < j + (x == 1 && w.cut >= 0 ? 1 : 0); ++n) v.advance(P::kVStages);
           ok = mbar_wait(bar(kApBarVFull + v.stage), v.phase);
           if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
           const uint32_t v_tile = base + P::kOffV + v.stage * kAtTileBytes;
-          const int r = w.kend - key0 + row;
+          const int r = t.end - key0 + row;
           if (r < kAtKeys) {
 #pragma unroll
             for (int h = 0; h < 2; ++h)
@@ -485,7 +495,7 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         done_phase ^= 1;
       }
       if (!ok) break;
-      if (WIN) for (int j = 0; j < w.ntiles; ++j) vr.advance(P::kVStages);
+      skip_v(w);
       // ------------------------------------------------------------- outputs of the tile
       ok = mbar_wait(bar(kApBarOFull + x), o_phase);
       if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }

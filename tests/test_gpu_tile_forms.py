@@ -119,3 +119,63 @@ def test_expert_tiles_in_pairs(E, top, m, kind, n):
         if len(rows):
             ref = x[rows.to(DEV)].double() @ w[e].double().T
             assert rel(got[rows.to(DEV), at.to(DEV)], ref) < 4e-3, e
+
+
+def _window_case(H, KH, D, portions, starts, window, sink, edit=None):
+    """Outputs of ops.window_attn for portions behind cached tokens, pages in any order and rubbish behind every context, and of
+    the same attention in 64 bits; ``edit(values, start)`` may change a sequence's values [tokens, KH, D]."""
+    bs, g, dp = len(portions), gen(H + D + window), (D + 63) // 64 * 64
+    ctx = [a + b for a, b in zip(portions, starts)]
+    need = [(n + 255) // 256 for n in ctx]
+    perm, at = torch.randperm(sum(need), generator=torch.Generator().manual_seed(3)).tolist(), 0
+    table = torch.full((bs, max(need)), -1, dtype=torch.int32)
+    kc, vc = (torch.full((sum(need) * 256, KH, dp), float("nan"), dtype=BF, device=DEV) for _ in range(2))
+    scale, qs, refs = 1.5 * D ** -0.5, [], []
+    for i, n in enumerate(ctx):
+        table[i, :need[i]] = torch.tensor(perm[at:at + need[i]])
+        at += need[i]
+        q, k, v = (torch.randn(t, h, D, generator=g, device=DEV).to(BF) for t, h in ((portions[i], H), (n, KH), (n, KH)))
+        if edit is not None:
+            edit(v, starts[i])
+        slots = (table[i, :need[i]].long()[:, None] * 256 + torch.arange(256)).flatten()[:n].to(DEV)
+        for c, x in ((kc, k), (vc, v)):
+            c[slots] = 0
+            c[slots, :, :D] = x
+        qs.append(torch.zeros(portions[i], H, dp, dtype=BF, device=DEV))
+        qs[-1][..., :D] = q
+        p, j = torch.arange(starts[i], n, device=DEV)[:, None], torch.arange(n, device=DEV)[None]
+        seen = (j <= p) & (j > p - window) if window else j <= p
+        kk, vv = (x.double().repeat_interleave(H // KH, 1) for x in (k, v))
+        s = (torch.einsum("ihd,jhd->hij", q.double(), kk) * scale).masked_fill(~seen, float("-inf"))
+        if sink:
+            s = torch.cat([s, torch.zeros_like(s[..., :1])], -1)
+        w = torch.softmax(s, -1)[..., :n]
+        # a value that is not seen does not count, whatever it is
+        ref = torch.einsum("hij,jhd->ihd", w, torch.nan_to_num(vv, posinf=0, neginf=0))
+        for t in (~torch.isfinite(v)).any(-1).any(-1).nonzero().flatten().tolist():
+            ref[seen[:, t]] = float("nan")
+        refs.append(ref)
+    cu = [0]
+    for n in portions:
+        cu.append(cu[-1] + n)
+    rows = (i32([i for i, n in enumerate(portions) for _ in range(n)]), i32(cu), i32(starts), i32(list(range(bs))))
+    out = torch.full((cu[-1], (H * D + 7) // 8 * 8), 7.0, dtype=BF, device=DEV)
+    ops.window_attn(torch.cat(qs), kc, vc, table.to(DEV), rows, i32([p for s, n in zip(starts, portions) for p in range(s, s + n)]), max(portions), D,
+                    window, sink, scale, out)
+    assert pkg._lib.device_status() == 0
+    return [out[a:b, :H * D].view(b - a, H, D) for a, b in zip(cu, cu[1:])], refs
+
+
+# A value of a token behind a query tile reaches no row of that tile, whatever it is: not through a key tile that the two query tiles of
+# a pair share either (weights of zero times infinity).  160 tiles of 64 rows: pairs; the tiles meet inside a key tile.
+@pytest.mark.parametrize("window", [0, 50])
+@pytest.mark.parametrize("start", [0, 37])
+def test_window_pairs_keep_the_future_out(window, start):
+    def poison(v, first):
+        v[first + 64 + 5] = float("inf")
+
+    got, ref = _window_case(8, 4, 128, [256] * 10, [start] * 10, window, True, poison)
+    for o, r in zip(got, ref):
+        assert rel(o[:64], r[:64]) < 8e-3
+        hit = torch.isnan(r).flatten(1).any(1)
+        assert not bool(torch.isfinite(o[hit]).all(-1).any())
