@@ -575,9 +575,9 @@ typedef struct {
   const float* skip; /* DECAY */
 } mdb_scan_args;
 int mdb_scan(const mdb_scan_args* args, mdb_stream_t stream);
-/* The same, told how many rows the portions have together (since version 102; 0: unknown, as in mdb_scan): from 16 tokens a
- * portion on average up, heads of up to 128 channels are scanned in blocks of 16 tokens.  The sums of a row are rounded in the
- * order of the form that is taken. */
+/* The same, told how many rows the portions have together (since version 102; 0: unknown, as in mdb_scan): long portions of few
+ * sequences, with heads of up to 128 channels, are scanned in blocks of 16 tokens.  The sums of a row are rounded in the order of
+ * the form that is taken. */
 int mdb_scan_rows(const mdb_scan_args* args, int64_t rows, mdb_stream_t stream);
 
 /* The decay scan over prompt portions in chunks of 64 tokens on the tensor cores: bf16 rows of ldq / ldk elements with head

@@ -15,7 +15,7 @@
 // the same number of FMAs per token with half the dependent shuffle reductions; these products of keys and queries are
 // computed beforehand, with the decays.
 //
-// Portions of 16 tokens and more with heads of up to 128 key channels go in blocks of 16 tokens instead (scan_blocks.cuh).
+// Long portions of few sequences with heads of up to 128 key channels go in blocks of 16 tokens instead (scan_blocks.cuh).
 //
 // The linear recurrence S <- a S + b k v^T, o = S^T q + skip v is the mLSTM's scan with its gates given and no normaliser.
 //
@@ -1160,18 +1160,44 @@ int launch_scan_prompt(const mdb_scan_args& a, cudaStream_t st) {
   return mdb_launch(kernel, dim3((columns + COLS - 1) / COLS, a.heads, a.bs), dim3(threads), smem, st, a);
 }
 
+// Columns per CTA of the scan in blocks of 16 tokens, 0: token by token.
+//
+// The blocks shorten the chain of a sequence but leave an SM to one CTA, so they lose (by 5 to 55 %) once their CTAs no longer run all
+// at once; within that, 64 columns per CTA, or 32 or 16 where those still fit (a block of the delta rule takes 3.6 us with 16
+// columns, 4.5 with 32, 5.9 with 64).  What is left is how many tokens make up for the start and for a last block that is partly
+// empty.  Time of the blocks over the time token by token, with heads of 128 channels, at 96 / 512 tokens (and one token into a new
+// block at the thresholds below: at most 1.0):
+//   delta rule, columns 128: 4 to 16 sequence heads (16) 1.02 / 0.96; 32 (32) 0.99 / 0.90; 48 (64) 0.98 / 0.95; 64 (64) 0.79 / 0.75
+//   mLSTM, columns 256:      4 to 32 sequence heads (16, 32, 64) 0.80 - 0.83 / 0.72 - 0.77
+//   decay scan, columns 64:  up to 32 sequence heads (16) 0.81 / 0.76; 48 (32) 0.96 / 0.91; 80 (64) 0.96 / 0.90; 128 (64) 0.82 / 0.78
+// and of 64 channels: delta rule 1.01 - 1.2 whatever the form; mLSTM, columns 128: 0.75 / 0.67 (16), 0.99 / 0.94 (32), 0.78 / 0.72
+// (64, SMs full); decay scan 0.83 / 0.78 (16), 1.0 - 1.15 (32, 64).
+template <int MODE, int DP>
+int scan_block_columns(const mdb_scan_args& a, int64_t rows) {
+  if (DP > 128 || (DP == 64 && MODE == kScanDelta)) return 0;
+  const int64_t heads = static_cast<int64_t>(a.heads) * a.bs, sms = at_sm_count();
+  auto ctas = [&](int cols) { return (a.vdim + cols - 1) / cols * heads; };
+  if (ctas(64) > sms) return 0;
+  const int cols = ctas(16) <= sms ? 16 : ctas(32) <= sms ? 32 : 64;
+  if (MODE == kScanDecay && DP == 64 && cols != 16) return 0;
+  int least;                                       // tokens of a sequence on average
+  if (cols == 16) least = MODE == kScanDelta ? 448 : 80;
+  else if (MODE == kScanMlstm && DP == 128) least = 80;
+  else if (cols == 64 && 4 * ctas(64) >= 3 * sms) least = 96;
+  else if (cols == 64) least = MODE == kScanDelta ? 448 : 256;
+  else least = MODE == kScanMlstm ? 448 : 256;
+  return rows >= static_cast<int64_t>(least) * a.bs ? cols : 0;
+}
+
 template <int MODE, int DP>
 int launch_scan_dim(const mdb_scan_args& a, int64_t rows, cudaStream_t st) {
   if (a.fused) return a.dtype == MDB_F32 ? launch_scan_token<float, MODE, DP / 32>(a, st) : launch_scan_token<bf16, MODE, DP / 32>(a, st);
-  if constexpr (DP <= 128) {
-    // In blocks of 16 tokens, from portions of 16 tokens on average up (65 tokens of 4 heads: delta rule with its decays 29.0 us
-    // against 29.7 token by token, mLSTM of 2 heads 16.8 against 17.7; 100 tokens of 4 x 16 heads 52.9 against 77.4); shorter
-    // ones would leave most of a block empty.  64 columns per CTA, or 32 or 16 where their CTAs still run all at once: a block
-    // of the delta rule takes 3.6 us with 16 columns, 4.5 with 32, 5.9 with 64.
-    if (rows >= static_cast<int64_t>(kSbTokens) * a.bs) {
-      const int64_t heads = static_cast<int64_t>(a.heads) * a.bs;
-      if ((a.vdim + 15) / 16 * heads <= 148) return launch_scan_blocks<MODE, DP, 16, 2>(a, st);
-      return (a.vdim + 31) / 32 * heads <= 148 ? launch_scan_blocks<MODE, DP, 32, 4>(a, st) : launch_scan_blocks<MODE, DP, 64, 4>(a, st);
+  const int cols = scan_block_columns<MODE, DP>(a, rows);
+  if constexpr (DP == 128 || (DP == 64 && MODE != kScanDelta)) {
+    if (cols == 16) return launch_scan_blocks<MODE, DP, 16, 2>(a, st);
+    if constexpr (DP == 128 || MODE == kScanMlstm) {
+      if (cols == 32) return launch_scan_blocks<MODE, DP, 32, 4>(a, st);
+      if (cols == 64) return launch_scan_blocks<MODE, DP, 64, 4>(a, st);
     }
   }
   // blocks of 32 columns while they fill the SMs, narrower ones (more re-reads of k, q and g) below that

@@ -63,9 +63,13 @@ def mlstm_parts(q, k, v, li, lf):
 
 # token counts around a block, two portions one behind the other, a padding entry; columns that fill 16, 32 and 64 wide CTAs or
 # do not; one and several heads per key head; enough heads for the wide CTAs.  2e-6: thrice what the token by token form shows.
+# Portions this short go token by token; a padding entry of 2000 rows lifts the average to where blocks are taken (not with the 80 and
+# 160 sequence heads of two cases, whose CTAs would not run all at once; the last cases are as wide as fits).
+@pytest.mark.parametrize("padding", [20, 2000])
 @pytest.mark.parametrize("mode", [ops.SCAN_DELTA, ops.SCAN_MLSTM, ops.SCAN_DECAY])
-@pytest.mark.parametrize("H,KH,D,DV,bs", [(2, 1, 64, 24, 3), (3, 3, 128, 33, 3), (8, 4, 128, 80, 3), (20, 20, 128, 128, 3), (40, 40, 64, 70, 3)])
-def test_scan_in_blocks(mode, H, KH, D, DV, bs):
+@pytest.mark.parametrize("H,KH,D,DV,bs", [(2, 1, 64, 24, 3), (3, 3, 128, 33, 3), (8, 4, 128, 80, 3), (20, 20, 128, 128, 3), (40, 40, 64, 70, 3),
+                                          (8, 8, 64, 80, 3), (16, 16, 128, 128, 3), (18, 18, 64, 100, 3)])
+def test_scan_in_blocks(mode, H, KH, D, DV, bs, padding):
     if mode == ops.SCAN_MLSTM:
         KH = H
     first, second, slots = [47, 16, 1], [17, 33, 31], [2, 0, 3]
@@ -86,21 +90,22 @@ def test_scan_in_blocks(mode, H, KH, D, DV, bs):
     got_o, got_d = torch.zeros(sum(total), H, DV), torch.ones(sum(total), H)
     for part, counts in enumerate((first, second)):
         rows = torch.cat([torch.arange(base[i] + (first[i] if part else 0), base[i] + (first[i] if part else 0) + n) for i, n in enumerate(counts)])
-        pad = torch.cat([rows, rows[:20]])                           # a padding entry of 20 rows: nothing is read or written for it
+        pad = torch.cat([rows, rows[torch.arange(padding) % len(rows)]])      # the padding entry: nothing is read or written for it
         m = len(pad)
-        p = _portions(counts + [20], [first[i] if part else 0 for i in range(3)] + [0], slots + [-1])
+        p = _portions(counts + [padding], [first[i] if part else 0 for i in range(3)] + [0], slots + [-1])
         at = lambda t: t[pad].contiguous().to(DEV)                   # noqa: E731,B023
         o, den = torch.full((m, H, DV), 9.0, device=DEV), torch.full((m, H), 9.0, device=DEV)
         if mode == ops.SCAN_DELTA:
-            sc = torch.full((m, H, 4), 9.0, device=DEV)
-            sc[..., 3] = at(beta)
+            kk, qq = (t[pad].double().repeat_interleave(rep, 1) for t in (k, q))
+            before = decay[pad].double() * kk.roll(1, 0)             # (read for the second token of a pair only)
+            sc = torch.stack([(kk * qq).sum(-1), (before * kk).sum(-1), (before * qq).sum(-1), beta[pad].double()], -1).float().to(DEV)
             ops.scan(mode, F32, 4, H, KH, D, DV, at(q), at(k), at(v), None, None, state, p, g=at(decay), scalars=sc, out=o)
         elif mode == ops.SCAN_MLSTM:
             ops.scan(mode, F32, 4, H, KH, D, DV, at(q), at(k), at(v), at(li), at(lf), state, p, mstate=mst, out=o, den=den)
         else:
             ops.scan(mode, F32, 4, H, KH, D, DV, at(q), at(k), at(v), at(decay[..., 1]), at(beta), state, p, out=o, skip=skip.to(DEV))
-        assert float((o[-20:] - 9).abs().max()) == 0
-        got_o[rows], got_d[rows] = o[:-20].cpu(), den[:-20].cpu()
+        assert float((o[-padding:] - 9).abs().max()) == 0
+        got_o[rows], got_d[rows] = o[:-padding].cpu(), den[:-padding].cpu()
     assert pkg._lib.device_status() == 0
     assert float((state[[1, 4]] - 5).abs().max()) == 0
     for i in range(3):
@@ -124,10 +129,10 @@ def test_scan_in_blocks(mode, H, KH, D, DV, bs):
 
 def test_scan_in_blocks_keeps_the_future_out():
     """Values behind a token, whatever they are, do not reach its output."""
-    H, D, DV, T = 2, 128, 40, 32
-    q, k, v = (torch.randn(T, H, n, generator=gen(i), device="cpu") for i, n in enumerate((D, D, DV)))
+    H, D, DV, T, rows = 2, 128, 40, 32, 600      # rows behind the portion: as many as make blocks worth while
+    q, k, v = (torch.randn(rows, H, n, generator=gen(i), device="cpu") for i, n in enumerate((D, D, DV)))
     v[21] = float("inf")
-    o = torch.zeros(T, H, DV, device=DEV)
-    ops.scan(ops.SCAN_DECAY, F32, 1, H, H, D, DV, q.to(DEV), k.to(DEV), v.to(DEV), torch.full((T, H), 0.9, device=DEV), torch.ones(T, H, device=DEV),
+    o = torch.zeros(rows, H, DV, device=DEV)
+    ops.scan(ops.SCAN_DECAY, F32, 1, H, H, D, DV, q.to(DEV), k.to(DEV), v.to(DEV), torch.full((rows, H), 0.9, device=DEV), torch.ones(rows, H, device=DEV),
              torch.zeros(1, H, DV, D, device=DEV), _portions([T], [0], [0]), out=o)
-    assert bool(torch.isfinite(o[:21]).all()) and not bool(torch.isfinite(o[21:]).any())
+    assert bool(torch.isfinite(o[:21]).all()) and not bool(torch.isfinite(o[21:T]).any()) and float(o[T:].abs().max()) == 0
