@@ -14,12 +14,14 @@
 namespace mdb {
 
 constexpr int kF32K = 32, kF32Ld = kF32K + 4;      // k of a group's stage; floats between rows
+constexpr int kF32Chains = 4;                      // an output is the sum of four chains, whatever the tile
 
 template <int BM, int BN, int TM, int TN, int KS, int STAGES>
 struct F32Plan {
   static constexpr int TX = BN / TN, TY = BM / TM, kGroup = TX * TY, kThreads = kGroup * KS;
   static constexpr int kRows = BM + BN, kStage = KS * kRows * kF32Ld;                       // floats
   static constexpr int kSmemBytes = STAGES * kStage * 4;
+  static_assert(KS == 1 || KS == kF32Chains, "a chain per group, or one behind another");
   static_assert(TX % 8 == 0 && (KS == 1 || TM % KS == 0), "eight lanes share a row of x; the last sums are dealt out by rows");
   static_assert(KS * BM * BN <= STAGES * kStage, "the groups' sums fit where the operands were");
 };
@@ -73,11 +75,20 @@ __global__ void __launch_bounds__(F32Plan<BM, BN, TM, TN, KS, STAGES>::kThreads,
     }
   }
   const uint32_t dst0 = smem + ((threadIdx.x >> 3) * kF32Ld + piece) * 4;
+  // KS 1: the blocks of 32 k in the order of the chains, chain c from step first_of(c) on
+  const int blocks = (a.k + kF32K - 1) / kF32K;
+  auto first_of = [&](int c) { return c * (blocks / kF32Chains) + min(c, blocks % kF32Chains); };
+  auto block_of = [&](int step) {
+    int c = 0;
+#pragma unroll
+    for (int i = 1; i < kF32Chains; ++i) c += step >= first_of(i) ? 1 : 0;
+    return (step - first_of(c)) * kF32Chains + c;
+  };
   auto fill = [&](int step) {
     const uint32_t dst = dst0 + (step % STAGES) * P::kStage * 4;
 #pragma unroll
     for (int g = 0; g < KS; ++g) {
-      const int k = (step * KS + g) * kF32K;
+      const int k = (KS == 1 ? block_of(step) : step * KS + g) * kF32K;
 #pragma unroll
       for (int q = 0; q < NR; ++q) {
         const bool in = (live >> q & 1u) && k + piece < a.k;
@@ -93,7 +104,24 @@ __global__ void __launch_bounds__(F32Plan<BM, BN, TM, TN, KS, STAGES>::kThreads,
   for (int i = 0; i < TM; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-  const int steps = (a.k + KS * kF32K - 1) / (KS * kF32K);
+  float sum[KS == 1 ? TM : 1][KS == 1 ? TN : 1];           // of the chains that have ended
+  if (KS == 1) {
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) sum[KS == 1 ? i : 0][KS == 1 ? j : 0] = 0.f;
+  }
+  auto end_chain = [&]() {
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) {
+        sum[KS == 1 ? i : 0][KS == 1 ? j : 0] += acc[i][j];
+        acc[i][j] = 0.f;
+      }
+  };
+  const int steps = KS == 1 ? blocks : (a.k + KS * kF32K - 1) / (KS * kF32K);
+  int chain = 1, chain_end = first_of(1);
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
     if (s < steps) fill(s);
@@ -104,6 +132,10 @@ __global__ void __launch_bounds__(F32Plan<BM, BN, TM, TN, KS, STAGES>::kThreads,
     __syncthreads();                                       // stage s is there for everyone, and stage s - 1 has been read
     if (s + STAGES - 1 < steps) fill(s + STAGES - 1);
     asm volatile("cp.async.commit_group;" ::: "memory");
+    if (KS == 1 && s == chain_end) {
+      end_chain();
+      chain_end = first_of(++chain);
+    }
     const float* st = f32_smem + (s % STAGES) * P::kStage + group * P::kRows * kF32Ld;
     const float* xs = st + ty * kF32Ld;
     const float* ws = st + (BM + tx) * kF32Ld;
@@ -143,11 +175,12 @@ __global__ void __launch_bounds__(F32Plan<BM, BN, TM, TN, KS, STAGES>::kThreads,
     }
   };
   if (KS == 1) {
+    end_chain();
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
       float v[TN];
 #pragma unroll
-      for (int j = 0; j < TN; ++j) v[j] = acc[i][j];
+      for (int j = 0; j < TN; ++j) v[j] = sum[KS == 1 ? i : 0][KS == 1 ? j : 0];
       leave(i, v);
     }
     return;
@@ -189,13 +222,14 @@ static int gemm_f32_run(const mdb_gemm_args& a, cudaStream_t st) {
   return mdb_launch(kernel, grid, dim3(P::kThreads), P::kSmemBytes, st, a);
 }
 
-// Rounds of 148 tiles times the FMA time of a tile per k: 128 cycles for 128 x 128 (a tenth less, it reads half as much through
+// Rounds of a tile per SM times the FMA time of a tile per k: 128 cycles for 128 x 128 (a tenth less, it reads half as much through
 // L2), 32 for 64 x 64, and 8 for 16 x 32, whose 4 x 4 outputs per thread are bound by shared memory at half the FMA rate.
 template <bool GLU>
 static int gemm_f32_dispatch(const mdb_gemm_args& a, cudaStream_t st) {
   const int64_t z = a.form == MDB_GEMM_HEADS ? a.heads : 1, n = GLU ? 2LL * a.n : a.n;
+  const int64_t sms = at_sm_count();
   auto rounds = [&](int bm, int bn) {
-    return (((static_cast<int64_t>(a.m) + bm - 1) / bm) * ((n + bn - 1) / bn) * z + 147) / 148;
+    return (((static_cast<int64_t>(a.m) + bm - 1) / bm) * ((n + bn - 1) / bn) * z + sms - 1) / sms;
   };
   const int64_t wide = rounds(128, 128) * 115, mid = rounds(64, 64) * 32, narrow = rounds(16, 32) * 8;
   // grids reach 65535 row tiles: as many rows as tiles of 64 allowed

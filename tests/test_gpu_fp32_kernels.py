@@ -42,6 +42,16 @@ def test_fp32_product_tiles(m, n, k, act):
     assert pkg._lib.device_status() == 0
 
 
+# The tile goes by the number of rows, the order of a row's sums does not: the same bits alone and beside any other rows.
+@pytest.mark.parametrize("n,k", [(36, 16), (3072, 112), (1024, 176), (1024, 1024), (260, 2000)])
+@pytest.mark.parametrize("act", [ops.ACT_NONE, ops.ACT_RELU_GLU])
+def test_fp32_product_of_a_row_does_not_depend_on_the_others(n, k, act):
+    x, w = torch.randn(4100, k, generator=gen(3)).to(DEV), torch.randn(2 * n if act == ops.ACT_RELU_GLU else n, k, generator=gen(4)).to(DEV)
+    whole = ops.gemm(x, w, torch.zeros(4100, n, device=DEV), act=act)
+    for m in (1, 16, 33, 64, 100, 500, 1000, 2050):
+        assert torch.equal(ops.gemm(x[:m], w, torch.zeros(m, n, device=DEV), act=act), whole[:m]), m
+
+
 def _portions(counts, starts, slots):
     cu = torch.tensor([0] + list(counts)).cumsum(0)
     row_seq = torch.cat([torch.full((n,), i) for i, n in enumerate(counts)])
