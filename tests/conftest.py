@@ -31,8 +31,8 @@ def mdb():
     return importlib.import_module("mineru-diffusion_b200")
 
 
-# Where the GPU tests leave their parity figures (one JSON object per line), if that folder exists.
-RECORD_DIR = os.environ.get("MDB200_RECORD_DIR", os.path.join(ROOT, "gpurun_out"))
+# Where the GPU tests leave their parity figures (one JSON object per line), if it is set and that folder exists.
+RECORD_DIR = os.environ.get("MDB200_RECORD_DIR", "")
 
 
 def record_parity(name: str, **figures) -> None:
