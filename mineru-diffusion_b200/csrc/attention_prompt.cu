@@ -18,30 +18,45 @@
 // 64 keys with two score buffers per tile and an issuing warp per tile: 299 us alone, 329 in a loop, other roundings; an issuing
 // warp per tile with these steps: 351.)
 //
-// Tensor memory: S_A (P_A) | S_B (P_B) | O_A | O_B, 128 columns each; with one tile S of even | odd key tiles | O.
+// Tensor memory: S_A (P_A) | S_B (P_B) | O_A | O_B, 128 columns each; with one tile S of even key tiles | - | O | S of odd ones.
 #include "mdb_common.cuh"
 
 namespace mdb {
 
+// Times of a unit, in sixteenths of a key tile of one query tile: a key tile, and the start and end of a unit.  Fitted to both forms'
+// times of 100 calls (one to 64 prompts of 64 to 4096 tokens, alike and not); the worst choice left is 11 % off the better.
+constexpr int kApTileStep = 16, kApTileUnit = 32, kApPairStep = 23, kApPairUnit = 32;
+
 struct ApPlan {
   static constexpr int kKStages = 3, kVStages = 2;
   static constexpr int kQBytes = 2 * 128 * 128;             // a tile: two channel halves of [128 rows][128 B]
-  static constexpr int kProducerWarp = 8, kMmaWarp = 9, kThreads = 384;      // three warpgroups; two warps idle
-  // registers: 384 threads x 168 at launch = 256 x 216 (softmax) + 128 x 72
-  static constexpr int kSoftmaxRegs = 216, kOtherRegs = 72;
+  static constexpr int kThreads = 384;                      // three warpgroups; two warps idle
+  // registers: 384 threads x 168 at launch = 256 x 208 (softmax) + 128 x 88
+  static constexpr int kSoftmaxRegs = 208, kOtherRegs = 88;
   static_assert(256 * kSoftmaxRegs + 128 * kOtherRegs <= kThreads * 168, "registers after the split");
   static constexpr int kOffK = 2 * kQBytes;
   static constexpr int kOffV = kOffK + kKStages * kAtTileBytes;
   static constexpr int kOffBars = kOffV + kVStages * kAtTileBytes;
-  static constexpr int kSmemBytes = 1024 + kOffBars + 256;
+  static constexpr int kOffList = kOffBars + 256;            // the sorted list of items
+  static constexpr int kMaxItems = 256, kMaxSeqs = 1024;
+  static constexpr int kSmemBytes = 1024 + kOffList + kMaxItems * 4;
 };
 static_assert(ApPlan::kSmemBytes <= 227 * 1024, "shared memory of the prompt attention");
 
-// barrier slots; those of a tile (A, B) or of a score buffer come in pairs
+// The softmax warps, four for every tile there may be, then the other roles.
+template <bool DEAL>
+struct ApRoles {
+  static constexpr int kProducer = DEAL ? 8 : 4, kMma = DEAL ? 9 : 5, kThreads = DEAL ? ApPlan::kThreads : 192;
+};
+
+// barrier slots; those of a tile (A, B) come in pairs, those of a score buffer in threes
 enum {
   kApBarQFull = 0, kApBarQEmpty = 1, kApBarQReady = 2, kApBarKFull = 4, kApBarKEmpty = 7, kApBarVFull = 10, kApBarVEmpty = 12,
-  kApBarSFull = 14, kApBarPFull = 16, kApBarPDone = 18, kApBarOFull = 20, kApBarOEmpty = 22, kApBarCount = 24
+  kApBarSFull = 14, kApBarPFull = 17, kApBarPDone = 20, kApBarOFull = 22, kApBarOEmpty = 24, kApBarCount = 26
 };
+// Score buffers: of tile A, of tile B, and the second one of a unit without tile B, in B's output columns
+constexpr int kApAlone = 2;
+__device__ __forceinline__ uint32_t ap_score_col(int buf) { return buf == kApAlone ? 384u : 128u * buf; }
 
 // Four products in a row with one elected lane: left operand steps of `a_step`, right operand steps of `b_step` (descriptor
 // units of 16 bytes).
@@ -89,57 +104,181 @@ struct ApUnit {
   ApTile t[2];
 };
 
-// Units are (pair of query tiles, sequence, KV head), the late (long) pairs first, dealt to the CTAs in alternating direction;
-// with tiles_per_unit 1 there is no tile B.
+// Where a sequence's queries and keys lie.
+struct ApSeq {
+  int q_start, Tq, q_off, T, seq_start;
+};
 template <bool WIN>
-__device__ __forceinline__ ApUnit ap_unit(const AtArgs& a, int units, int wave) {
+__device__ __forceinline__ ApSeq ap_seq(const AtArgs& a, int seq) {
+  ApSeq w = {};
+  const int32_t* cu_q = a.cu_seqlens_q != nullptr ? a.cu_seqlens_q : a.cu_seqlens;
+  w.q_start = cu_q[seq];
+  w.Tq = cu_q[seq + 1] - w.q_start;
+  if (WIN) {
+    w.q_off = a.start[seq];
+    w.T = w.q_off + w.Tq;
+  } else {
+    w.seq_start = a.cu_seqlens[seq];
+    w.T = a.cu_seqlens[seq + 1] - w.seq_start;
+    w.q_off = w.T - w.Tq;
+  }
+  return w;
+}
+// Keys [x, y) that the rows of the query tile from query m0 on see.
+template <bool WIN>
+__host__ __device__ __forceinline__ int2 ap_keys(const AtArgs& a, const ApSeq& w, int m0) {
+  const int S = 1 << a.log2_stairs;
+  const int pad = ((w.T + S - 1) >> a.log2_stairs << a.log2_stairs) - w.T;
+  const int last = w.q_off + min(m0 + a.tokens_per_unit, w.Tq) - 1;
+  return make_int2(WIN && a.window > 0 ? max(0, w.q_off + m0 - a.window + 1) : 0,
+                   min(w.T, ((((last + pad) >> a.log2_stairs) + 1) << a.log2_stairs) - pad));
+}
+
+// How the units of a launch are dealt out: `tiles` query tiles each; either the sorted list of `items` (sequence, tile or pair) for
+// every KV head, or (items 0) all that the longest sequence allows for, the late ones first.
+struct ApDeal {
+  int tiles, items, units;
+};
+// Time of a unit of the query tiles from tile `first` on.
+template <bool WIN>
+__host__ __device__ __forceinline__ int ap_cost(const AtArgs& a, const ApSeq& w, int first, bool pair) {
+  const int m0 = first * a.tokens_per_unit, m1 = m0 + a.tokens_per_unit;
+  pair = pair && m1 < w.Tq;
+  const int2 k0 = ap_keys<WIN>(a, w, m0);
+  const int end = pair ? ap_keys<WIN>(a, w, m1).y : k0.y, steps = (end + kAtKeys - 1) / kAtKeys - k0.x / kAtKeys;
+  return pair ? kApPairStep * steps + kApPairUnit : kApTileStep * steps + kApTileUnit;
+}
+
+// Where the sequences differ, by all threads: picks tiles alone or pairs and sorts the units by their time, so that dealing them in
+// alternating direction gives every CTA about the same.  Sequences of few queries and many keys beside prompts, and batches
+// in which one sequence is the longest by far, would leave the list of all that is possible nearly empty and its order the wrong
+// one (8 sequences, a prompt of 512 tokens and 7 rows behind 4000 keys: 103 us unsorted in pairs, 59 us; [1000] and 40 times 60
+// tokens 57 -> 43 us).  It takes 1.2 us.  `answer`: two words of shared memory; `scratch`: memory of the operand tiles, not in use yet.
+template <bool WIN>
+__device__ __forceinline__ ApDeal ap_deal(const AtArgs& a, int* answer, uint32_t* scratch, uint32_t* list) {
+  const int tid = threadIdx.x, lane = tid & 31, G = static_cast<int>(gridDim.x);
+  int* const first_item = reinterpret_cast<int*>(scratch); // [nseq]
+  uint32_t* const keys = scratch + ApPlan::kMaxSeqs;
+  auto tiles_of = [&](const ApSeq& w) { return min(a.max_qtiles, (max(w.Tq, 0) + a.tokens_per_unit - 1) / a.tokens_per_unit); };
+  const int per_rank = a.nseq * a.hkv;
+  if (a.tiles_per_unit > 0) return {a.tiles_per_unit, 0, (a.max_qtiles + a.tiles_per_unit - 1) / a.tiles_per_unit * per_rank};
+  if (tid < 32) {
+    // tiles of the sequences, their time in all, its extremes; the same in pairs
+    int v[8] = {0, 0, 0, 0x7fffffff, 0, 0, 0, 0x7fffffff};
+    for (int s = lane; s < a.nseq; s += 32) {
+      const ApSeq w = ap_seq<WIN>(a, s);
+      const int nt = tiles_of(w), np = (nt + 1) / 2;
+      if (s < ApPlan::kMaxSeqs) first_item[s] = nt;
+      if (nt > 0) {
+        const int t0 = ap_cost<WIN>(a, w, 0, false), t1 = ap_cost<WIN>(a, w, nt - 1, false);
+        const int p0 = ap_cost<WIN>(a, w, 0, true), p1 = ap_cost<WIN>(a, w, 2 * np - 2, true);
+        v[0] += nt; v[1] += nt * ((t0 + t1) / 2); v[2] = max(v[2], max(t0, t1)); v[3] = min(v[3], min(t0, t1));
+        v[4] += np; v[5] += np * ((p0 + p1) / 2); v[6] = max(v[6], max(p0, p1)); v[7] = min(v[7], min(p0, p1));
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      v[i] = (i & 3) < 2 ? __reduce_add_sync(0xffffffffu, v[i]) : (i & 3) == 2 ? __reduce_max_sync(0xffffffffu, v[i]) : __reduce_min_sync(0xffffffffu, v[i]);
+    // units of equal times take whole rounds; the more they differ, the better the rounds even out
+    auto time = [&](int n, int all, int most, int least) {
+      const float rounds = fmaxf(n, 1) * a.hkv / G, alike = most > 0 ? static_cast<float>(least) / most : 1.f;
+      return fmaxf(most, all / fmaxf(n, 1) * (rounds + alike * (ceilf(rounds) - rounds)));
+    };
+    const int per = time(v[0], v[1], v[2], v[3]) <= time(v[4], v[5], v[6], v[7]) ? 1 : 2;
+    const int items = per == 1 ? v[0] : v[4];
+    const bool sorted = a.nseq <= ApPlan::kMaxSeqs && items <= ApPlan::kMaxItems;
+    if (lane == 0) { answer[0] = per; answer[1] = sorted ? items : 0; }
+    int before = 0;
+    for (int s0 = 0; sorted && s0 < a.nseq; s0 += 32) {
+      const int s = s0 + lane, mine = s < a.nseq ? (first_item[s] + per - 1) / per : 0;
+      int upto = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += up;
+      }
+      if (s < a.nseq) first_item[s] = before + upto - mine;
+      before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+  }
+  __syncthreads();
+  const int per = answer[0], items = answer[1];
+  uint32_t item = 0, key = 0;
+  if (tid < items) {
+    int lo = 0, hi = a.nseq;                               // the last sequence whose first item is not behind this one
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) / 2;
+      if (first_item[mid] <= tid) lo = mid;
+      else hi = mid;
+    }
+    // (of sequences without items the one behind them has the same first item, and is the later one)
+    const int at = tid - first_item[lo];
+    item = static_cast<uint32_t>(lo) << 16 | static_cast<uint32_t>(at);
+    key = static_cast<uint32_t>(min(ap_cost<WIN>(a, ap_seq<WIN>(a, lo), at * per, per == 2), 0xffffff)) << 8 | static_cast<uint32_t>(255 - tid);
+  }
+  if (tid < ApPlan::kMaxItems) keys[tid] = key;            // (0: behind all items)
+  __syncthreads();
+  if (tid < items) {
+    int rank = 0;
+#pragma unroll 4
+    for (int i = 0; i < items; i += 4) {
+      const uint4 k = *reinterpret_cast<const uint4*>(keys + i);
+      rank += (k.x > key) + (k.y > key) + (k.z > key) + (k.w > key);
+    }
+    list[rank] = item;
+  }
+  fence_async_smem();
+  __syncthreads();
+  return {per, items, items > 0 ? items * a.hkv : (a.max_qtiles + per - 1) / per * per_rank};
+}
+
+// Unit of this CTA in a wave.
+template <bool WIN, bool DEAL>
+__device__ __forceinline__ ApUnit ap_unit(const AtArgs& a, const ApDeal& deal, const uint32_t* list, int wave) {
   ApUnit w = {};
   w.cut = -1;
   const int G = static_cast<int>(gridDim.x), c = static_cast<int>(blockIdx.x);
   const int p = wave * G + ((wave & 1) ? G - 1 - c : c);
-  if (p >= units) return w;
-  const int per_pair = a.nseq * a.hkv, pairs = (a.max_qtiles + a.tiles_per_unit - 1) / a.tiles_per_unit;
-  const int pair = pairs - 1 - p / per_pair, rest = p % per_pair;
-  w.seq = rest / a.hkv;
-  w.kvh = rest % a.hkv;
-  const int32_t* cu_q = a.cu_seqlens_q != nullptr ? a.cu_seqlens_q : a.cu_seqlens;
-  w.q_start = cu_q[w.seq];
-  w.Tq = cu_q[w.seq + 1] - w.q_start;
-  if (WIN) {
-    w.q_off = a.start[w.seq];
-    w.T = w.q_off + w.Tq;
+  if (p >= deal.units) return w;
+  int at;                                                  // first tile / tiles of a unit
+  if (DEAL && deal.items > 0) {
+    const uint32_t item = list[p / a.hkv];
+    w.seq = static_cast<int>(item >> 16);
+    at = static_cast<int>(item & 0xffffu);
+    w.kvh = p % a.hkv;
   } else {
-    w.seq_start = a.cu_seqlens[w.seq];
-    w.T = a.cu_seqlens[w.seq + 1] - w.seq_start;
-    w.q_off = w.T - w.Tq;
+    const int per_rank = a.nseq * a.hkv, rest = p % per_rank;
+    at = (a.max_qtiles + deal.tiles - 1) / deal.tiles - 1 - p / per_rank;
+    w.seq = rest / a.hkv;
+    w.kvh = rest % a.hkv;
   }
-  const int S = 1 << a.log2_stairs;
-  const int pad = ((w.T + S - 1) >> a.log2_stairs << a.log2_stairs) - w.T;
+  const ApSeq q = ap_seq<WIN>(a, w.seq);
+  w.q_start = q.q_start; w.Tq = q.Tq; w.q_off = q.q_off; w.T = q.T; w.seq_start = q.seq_start;
 #pragma unroll
   for (int x = 0; x < 2; ++x) {
     ApTile& t = w.t[x];
-    t.m0 = (a.tiles_per_unit * pair + x) * a.tokens_per_unit;
-    t.valid = x < a.tiles_per_unit && t.m0 < w.Tq;
+    t.m0 = (deal.tiles * at + x) * a.tokens_per_unit;
+    t.valid = x < (DEAL ? deal.tiles : 1) && t.m0 < w.Tq;
     if (!t.valid) continue;
-    const int last = w.q_off + min(t.m0 + a.tokens_per_unit, w.Tq) - 1;
-    const int end = min(w.T, ((((last + pad) >> a.log2_stairs) + 1) << a.log2_stairs) - pad);
+    const int2 keys = ap_keys<WIN>(a, q, t.m0);
     // window form: from the tile of keys that holds the first query's first key
-    const int beg = WIN && a.window > 0 ? max(0, w.q_off + t.m0 - a.window + 1) : 0;
-    if (x == 0) w.kbeg = beg / kAtKeys * kAtKeys;
-    t.end = end;
-    t.first = (beg - w.kbeg) / kAtKeys;
-    t.last = (end - w.kbeg + kAtKeys - 1) / kAtKeys;
+    if (x == 0) w.kbeg = keys.x / kAtKeys * kAtKeys;
+    t.end = keys.y;
+    t.first = (keys.x - w.kbeg) / kAtKeys;
+    t.last = (keys.y - w.kbeg + kAtKeys - 1) / kAtKeys;
     w.ntiles = t.last;
   }
   if (WIN && w.t[1].valid && w.t[0].end < w.kbeg + w.t[0].last * kAtKeys) w.cut = w.t[0].last - 1;
   return w;
 }
 
-template <bool WIN>
-__global__ void __launch_bounds__(ApPlan::kThreads, 1)
+// DEAL: more tiles than SMs, in sequences of more than one
+template <bool WIN, bool DEAL>
+__global__ void __launch_bounds__(ApRoles<DEAL>::kThreads, 1)
 attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                    const __grid_constant__ CUtensorMap map_v, const AtArgs a, const int units) {
   using P = ApPlan;
+  constexpr int kProducerWarp = ApRoles<DEAL>::kProducer, kMmaWarp = ApRoles<DEAL>::kMma;
   const int halves = WIN ? a.halves : 2;      // 64-channel halves of a stored head
   extern __shared__ __align__(1024) unsigned char ap_smem_raw[];
   const uint32_t raw = smem_u32(ap_smem_raw);
@@ -148,7 +287,6 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   const uint32_t bars = base + P::kOffBars;
   auto bar = [&](int slot) { return bars + 8u * static_cast<uint32_t>(slot); };
   volatile uint32_t* misc = reinterpret_cast<volatile uint32_t*>(gen_base + P::kOffBars + 8 * kApBarCount);
-  const int waves = (units + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = a.group;
   const int rows_used = group * a.tokens_per_unit;      // <= 128
@@ -156,12 +294,12 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   pdl_launch_dependents();
   if (threadIdx.x == 0) {
     for (int s = 0; s < kApBarCount; ++s) {
-      const bool by_softmax = s == kApBarQReady || s == kApBarQReady + 1 || (s >= kApBarPFull && s < kApBarPFull + 2) || s >= kApBarOEmpty;
+      const bool by_softmax = s == kApBarQReady || s == kApBarQReady + 1 || (s >= kApBarPFull && s < kApBarPFull + 3) || s >= kApBarOEmpty;
       mbar_init(bar(s), by_softmax ? 4 : 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == P::kMmaWarp) {
+  if (warp == kMmaWarp) {
     const uint32_t slot = smem_u32(const_cast<uint32_t*>(&misc[0]));
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -171,10 +309,16 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   tc_fence_after();
   const uint32_t tmem_base = misc[0];
   pdl_wait();   // q and the K/V rows of this step come from the preceding kernels
+  const uint32_t* const list = reinterpret_cast<const uint32_t*>(gen_base + P::kOffList);
+  ApDeal deal = {1, 0, units};
+  if (DEAL)
+    deal = ap_deal<WIN>(a, reinterpret_cast<int*>(gen_base + P::kOffBars + 8 * kApBarCount + 8), reinterpret_cast<uint32_t*>(gen_base + P::kOffK),
+                        reinterpret_cast<uint32_t*>(gen_base + P::kOffList));
+  const int waves = (deal.units + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
 
-  if (warp >= P::kProducerWarp) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(P::kOtherRegs));
-    if (warp == P::kProducerWarp) {
+  if (warp >= kProducerWarp) {
+    if (DEAL) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(P::kOtherRegs));
+    if (warp == kProducerWarp) {
       // ------------------------------------------------------------------ producer
       if (lane == 0) {
         AtRing kr, vr;
@@ -196,7 +340,7 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           return true;
         };
         for (int wave = 0; wave < waves && ok; ++wave) {
-          const ApUnit w = ap_unit<WIN>(a, units, wave);
+          const ApUnit w = ap_unit<WIN, DEAL>(a, deal, list, wave);
           if (w.ntiles == 0) continue;
           if (!mbar_wait(bar(kApBarQEmpty), q_phase ^ 1)) { ok = false; break; }
           {
@@ -237,9 +381,8 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           if (pend_q) mbar_wait(bar(kApBarQFull), par_q);
         }
       }
-    } else if (warp == P::kMmaWarp) {
+    } else if (warp == kMmaWarp) {
       // ----------------------------------------------------------------- MMA issue (all lanes, one elected)
-      const bool single = a.tiles_per_unit == 1;
       // bf16 x bf16 -> fp32, M = 128, N = 128 (or 64 channels); bit 16 set: B operand MN-major
       const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kAtKeys >> 3) << 17) |
                                (static_cast<uint32_t>(128 >> 4) << 24);
@@ -250,15 +393,16 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       uint32_t qfull_phase = 0;
       bool ok = true;
       for (int wave = 0; wave < waves && ok; ++wave) {
-        const ApUnit w = ap_unit<WIN>(a, units, wave);
+        const ApUnit w = ap_unit<WIN, DEAL>(a, deal, list, wave);
         if (w.ntiles == 0) continue;
+        const bool alone = !w.t[1].valid;
         if (WIN) {
           if (!mbar_wait_w(bar(kApBarQFull), qfull_phase)) { ok = false; break; }
           qfull_phase ^= 1;
         } else {
           // staircase form: the softmax warps scale q in place first.  Those of a tile that is not there have only seen it: the
           // next unit's q may not arrive before all have, or they would miss a phase and wait for a later one.
-          if (!mbar_wait_w(bar(kApBarQReady), qfull_phase) || !mbar_wait_w(bar(kApBarQReady + 1), qfull_phase)) { ok = false; break; }
+          if (!mbar_wait_w(bar(kApBarQReady), qfull_phase) || (DEAL && !mbar_wait_w(bar(kApBarQReady + 1), qfull_phase))) { ok = false; break; }
           qfull_phase ^= 1;
         }
         auto issue_s = [&](int x, int buf) {           // scores of tile x with the K tile at the ring's position
@@ -266,7 +410,7 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             if (WIN && c >= halves) break;
-            umma_bf16_x4_w(tmem_base + buf * 128, umma_desc_sw128(q_tile + c * (128 * 128)), 2, umma_desc_sw128(k_tile + c * kAtHalfBytes), 2,
+            umma_bf16_x4_w(tmem_base + ap_score_col(buf), umma_desc_sw128(q_tile + c * (128 * 128)), 2, umma_desc_sw128(k_tile + c * kAtHalfBytes), 2,
                            idesc_s, c);
           }
           umma_commit_w(bar(kApBarSFull + buf));
@@ -285,11 +429,12 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         for (int j = 0; j < w.ntiles && ok; ++j) {
           const bool more = j + 1 < w.ntiles;
           bool k_there = false;
-          if (single && more) {
-            // the other buffer held the last key tile, whose P V has been issued
+          if (alone && more) {
+            // the other buffer held the last key tile, whose P V has been issued; or an output of tile B that must have been read out
+            if (j == 0 && !mbar_wait_w(bar(kApBarOEmpty + 1), o_phase[1] ^ 1)) { ok = false; break; }
             if (!mbar_wait_w(bar(kApBarKFull + kr.stage), kr.phase)) { ok = false; break; }
             tc_fence_after();
-            issue_s(0, (j + 1) & 1);
+            issue_s(0, j & 1 ? 0 : kApAlone);
             release_k(j + 1);
           }
           if (!mbar_wait_w(bar(kApBarVFull + vr.stage), vr.phase)) { ok = false; break; }
@@ -302,7 +447,7 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
               if (!mbar_wait_w(bar(kApBarVFull + vr.stage), vr.phase)) { ok = false; break; }
             }
             if (j >= w.t[x].first && j < w.t[x].last) {
-              const int buf = single ? j & 1 : x;
+              const int buf = alone && (j & 1) ? kApAlone : x;
               if (j == w.t[x].first) {
                 // the previous unit's accumulator must have been read out
                 if (!mbar_wait_w(bar(kApBarOEmpty + x), o_phase[x] ^ 1)) { ok = false; break; }
@@ -311,13 +456,13 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
               if (!mbar_wait_w(bar(kApBarPFull + buf), p_phase >> buf & 1)) { ok = false; break; }
               p_phase ^= 1u << buf;
               tc_fence_after();
-              const uint32_t v_tile = base + P::kOffV + vr.stage * kAtTileBytes, p = tmem_base + buf * 128, o = tmem_base + 256 + x * 128;
+              const uint32_t v_tile = base + P::kOffV + vr.stage * kAtTileBytes, p = tmem_base + ap_score_col(buf), o = tmem_base + 256 + x * 128;
               umma_bf16_ts_x4_w(o, p, umma_desc_sw128_mn(v_tile), 128, idesc_o, j > w.t[x].first ? 1u : 0u);
               umma_bf16_ts_x4_w(o, p + 32, umma_desc_sw128_mn(v_tile + 4 * 2048), 128, idesc_o, 1u);
               umma_commit_w(bar(kApBarPDone + x));
               if (j == w.t[x].last - 1) umma_commit_w(bar(kApBarOFull + x));
             }
-            if (!single && more && j + 1 >= w.t[x].first && j + 1 < w.t[x].last) {
+            if (!alone && more && j + 1 >= w.t[x].first && j + 1 < w.t[x].last) {
               if (!k_there && !mbar_wait_w(bar(kApBarKFull + kr.stage), kr.phase)) { ok = false; break; }
               k_there = true;
               tc_fence_after();
@@ -327,37 +472,39 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           if (!ok) break;
           umma_commit_w(bar(kApBarVEmpty + vr.stage));
           vr.advance(P::kVStages);
-          if (!single && more) release_k(j + 1);      // (the key tiles of A and B overlap or touch: every one is used by a tile)
+          if (!alone && more) release_k(j + 1);      // (the key tiles of A and B overlap or touch: every one is used by a tile)
         }
       }
       if (!ok && lane == 0) report_status(MDB_STATUS_WAIT_TIMEOUT);
     }
   } else {
     // ------------------------------------------------------------------- softmax
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(P::kSoftmaxRegs));
+    if (DEAL) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(P::kSoftmaxRegs));
     const int x = warp >> 2;                               // tile A or B
     const int row = threadIdx.x & 127;                     // query row of the tile, and its tensor-memory lane
     const int tok_local = row / group, head_in_group = row % group;
     const uint32_t lane_field = static_cast<uint32_t>(32 * (warp & 3)) << 16;
-    const bool single = a.tiles_per_unit == 1;
     const uint32_t o_addr = tmem_base + 256 + x * 128 + lane_field;
     AtRing vr;                          // V ring position of the unit's first key tile
     auto skip_v = [&](const ApUnit& w) { if (WIN) for (int j = 0; j < w.ntiles + (w.cut >= 0 ? 1 : 0); ++j) vr.advance(P::kVStages); };
     uint32_t s_phase = 0 /* bit per buffer */, o_phase = 0, q_phase = 0, done_phase = 0;      // done: of the last P V
     bool ok = true;
+    ApUnit next = ap_unit<WIN, DEAL>(a, deal, list, 0);
     for (int wave = 0; wave < waves && ok; ++wave) {
-      const ApUnit w = ap_unit<WIN>(a, units, wave);
-      if (w.ntiles == 0) continue;
+      const ApUnit w = next;
       const ApTile t = x == 0 ? w.t[0] : w.t[1];
-      if (!t.valid) {
-        if (!WIN) {
-          // a phase must have been seen complete before the next one can be waited for by parity
-          ok = mbar_wait(bar(kApBarQFull), q_phase);
-          if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
-          if (lane == 0) mbar_arrive(bar(kApBarQReady + x));
+      if (w.ntiles == 0 || !t.valid) {
+        if (w.ntiles > 0) {
+          if (!WIN && DEAL) {
+            // a phase must have been seen complete before the next one can be waited for by parity
+            ok = mbar_wait(bar(kApBarQFull), q_phase);
+            if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+            if (lane == 0) mbar_arrive(bar(kApBarQReady + x));
+          }
+          q_phase ^= 1;
+          skip_v(w);
         }
-        q_phase ^= 1;
-        skip_v(w);
+        next = ap_unit<WIN, DEAL>(a, deal, list, wave + 1);
         continue;
       }
       const int head = w.kvh * group + head_in_group;
@@ -395,8 +542,8 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       q_phase ^= 1;
       float m_ref = -INFINITY, l = 0.f;
       for (int j = t.first; j < t.last; ++j) {
-        const int buf = single ? j & 1 : x;
-        const uint32_t s_addr = tmem_base + buf * 128 + lane_field;
+        const int buf = !w.t[1].valid && (j & 1) ? kApAlone : x;
+        const uint32_t s_addr = tmem_base + ap_score_col(buf) + lane_field;
         ok = mbar_wait(bar(kApBarSFull + buf), s_phase >> buf & 1);
         if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
         s_phase ^= 1u << buf;
@@ -496,6 +643,7 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       }
       if (!ok) break;
       skip_v(w);
+      next = ap_unit<WIN, DEAL>(a, deal, list, wave + 1);      // under the last products
       // ------------------------------------------------------------- outputs of the tile
       ok = mbar_wait(bar(kApBarOFull + x), o_phase);
       if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
@@ -538,31 +686,59 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 
   tc_fence_before();
   __syncthreads();
-  if (warp == P::kMmaWarp) {
+  if (warp == kMmaWarp) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
   }
 }
 
-template <bool WIN>
-static int ap_launch(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, AtArgs& a, cudaStream_t st) {
+template <bool WIN, bool DEAL>
+static int ap_run(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const AtArgs& a, int units, int grid, cudaStream_t st) {
   static PerDeviceOnce attr_once;
   const int dev = attr_once.slot();
   if (dev < 0) return MDB_ERR_CUDA;
   if (!attr_once.done[dev]) {
-    if (cudaFuncSetAttribute(attn_prompt_kernel<WIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, ApPlan::kSmemBytes) != cudaSuccess)
+    if (cudaFuncSetAttribute(attn_prompt_kernel<WIN, DEAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, ApPlan::kSmemBytes) != cudaSuccess)
       return MDB_ERR_CUDA;
     attr_once.done[dev] = true;
   }
-  // Tiles that can all have an SM of their own take one: two on one SM wait for one another (one prompt of 1056
-  // tokens, 136 tiles: 24.8 us in pairs, 20.4 us alone).
+  return mdb_launch(attn_prompt_kernel<WIN, DEAL>, dim3(grid), dim3(ApRoles<DEAL>::kThreads), ApPlan::kSmemBytes, st, map_q, map_k, map_v, a, units);
+}
+
+// Tiles per unit for sequences of the same `queries` and `keys` (each of the first behind keys - queries tokens): the shorter time of
+// the longest of every fourth CTA.  One prompt of 1280 to 2304 tokens (160 to 288 tiles): 28 - 49 us in pairs, 21 - 39 us alone; of 3072
+// tokens, or 8 of 256, the other way round (61 against 64, 17 against 19 us).
+template <bool WIN>
+static int ap_tiles_alike(const AtArgs& a, int queries, int keys, int sms) {
+  const int per_rank = a.nseq * a.hkv;
+  if (a.max_qtiles == 1) return 1;
+  if (static_cast<int64_t>(a.max_qtiles) * per_rank > 4 * sms) return 2;
+  const ApSeq w = {0, queries, keys - queries, keys, 0};
+  int most[2] = {0, 0};
+  for (int per = 1; per <= 2; ++per) {
+    const int n = (a.max_qtiles + per - 1) / per;
+    for (int c = 0; c < sms; c += 4) {
+      int t = 0;
+      for (int p0 = 0, odd = 0; p0 < n * per_rank; p0 += sms, odd ^= 1) {
+        const int p = p0 + (odd ? sms - 1 - c : c);
+        if (p < n * per_rank) t += ap_cost<WIN>(a, w, (n - 1 - p / per_rank) * per, per == 2);
+      }
+      if (t > most[per - 1]) most[per - 1] = t;
+    }
+  }
+  return most[0] <= most[1] ? 1 : 2;
+}
+
+// Tiles that can all have an SM of their own take one: two on one SM wait for one another (one prompt of 1056 tokens, 136 tiles:
+// 24.8 us in pairs, 19.0 us alone).  With more, a.tiles_per_unit is the answer for sequences that are alike, or 0: the kernel decides.
+template <bool WIN>
+static int ap_launch(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const AtArgs& a, cudaStream_t st) {
   const int sms = at_sm_count();
-  a.tiles_per_unit = static_cast<int64_t>(a.max_qtiles) * a.nseq * a.hkv <= sms ? 1 : 2;
-  const int64_t units = static_cast<int64_t>((a.max_qtiles + a.tiles_per_unit - 1) / a.tiles_per_unit) * a.nseq * a.hkv;
-  if (units > (1 << 30)) return MDB_ERR_UNSUPPORTED;
-  const int grid = units < sms ? static_cast<int>(units) : sms;
-  return mdb_launch(attn_prompt_kernel<WIN>, dim3(grid), dim3(ApPlan::kThreads), ApPlan::kSmemBytes, st, map_q, map_k, map_v, a,
-                    static_cast<int>(units));
+  const int64_t tiles = static_cast<int64_t>(a.max_qtiles) * a.nseq * a.hkv;
+  if (tiles > (1 << 30)) return MDB_ERR_UNSUPPORTED;
+  const int units = static_cast<int>(tiles), grid = units < sms ? units : sms;
+  return units <= sms || a.tiles_per_unit == 1 ? ap_run<WIN, false>(map_q, map_k, map_v, a, units, grid, st)
+                                               : ap_run<WIN, true>(map_q, map_k, map_v, a, units, grid, st);
 }
 
 // ---- staircase form ----
@@ -586,6 +762,10 @@ static int attn_stair_tc_launch(const AttnStairArgs& sa, int nseq, int max_seqle
   a.log2_stairs = sa.log2_stairs;
   a.tokens_per_unit = 128 / a.group;
   a.max_qtiles = (max_seqlen + a.tokens_per_unit - 1) / a.tokens_per_unit;
+  // one sequence, or prompts of one length (an odd last tile would be first in the order, and not the longest unit); one tile each
+  if (a.max_qtiles == 1 || (nseq == 1 && total_q == max_seqlen && total_tokens >= total_q) ||
+      (a.max_qtiles % 2 == 0 && total_q == static_cast<int64_t>(nseq) * max_seqlen && total_q == total_tokens))
+    a.tiles_per_unit = ap_tiles_alike<false>(a, max_seqlen, nseq == 1 ? static_cast<int>(total_tokens) : max_seqlen, at_sm_count());
   a.nsplit = 1;
   CUtensorMap map_q, map_k, map_v;
   if (!get_q_tensor_map(sa.q, total_q, sa.q_stride, sa.hq, a.group, a.tokens_per_unit, &map_q)) return MDB_ERR_CUDA;
@@ -615,6 +795,9 @@ static int attn_win_tc_launch(const mdb_window_attn_args& w, cudaStream_t st) {
   a.nseq = w.bs;
   a.tokens_per_unit = 128 / a.group;
   a.max_qtiles = (w.max_q + a.tokens_per_unit - 1) / a.tokens_per_unit;
+  // one tile each; portions of one length under a narrow window, which makes their tiles alike, wherever they start
+  if (a.max_qtiles == 1 || (a.max_qtiles % 2 == 0 && w.m == static_cast<int64_t>(w.bs) * w.max_q && w.window > 0 && w.window <= 2 * kAtKeys))
+    a.tiles_per_unit = ap_tiles_alike<true>(a, w.max_q, w.max_q + w.window, at_sm_count());
   a.nsplit = 1;
   a.window = w.window; a.sink = w.sink;
   a.dim = w.dim; a.halves = w.dim_pad / 64;

@@ -74,9 +74,9 @@ struct AtPlan {
 
 // barrier slots (8 bytes each) after the tiles
 enum {
-  kAtBarQFull = 0, kAtBarQEmpty = 2, kAtBarKFull = 4, kAtBarKEmpty = 7, kAtBarVFull = 10, kAtBarVEmpty = 13,
-  kAtBarSFull = 16, kAtBarSEmpty = 18, kAtBarPFull = 20, kAtBarPEmpty = 22, kAtBarOFull = 24, kAtBarOEmpty = 25,
-  kAtBarCount = 28      // up to three K and three V stages
+  kAtBarQFull = 0, kAtBarQEmpty = 2, kAtBarKFull = 4, kAtBarKEmpty = 6, kAtBarVFull = 8, kAtBarVEmpty = 11,
+  kAtBarSFull = 14, kAtBarSEmpty = 16, kAtBarPFull = 18, kAtBarPEmpty = 20, kAtBarOFull = 22, kAtBarOEmpty = 23,
+  kAtBarCount = 24      // two K and up to three V stages
 };
 
 struct AtArgs {

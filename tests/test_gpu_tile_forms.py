@@ -37,6 +37,36 @@ def test_prompt_attention_tiles_alone_behind_pairs():
     _prompts(2, 1, [128] * 150 + [40] * 460 + [100] * 150 + [7] * 150)
 
 
+# More tiles than SMs: prompts of one length, in pairs and alone in several rounds; an odd last tile; sequences that differ, sorted by
+# their time; more items than are sorted, and more sequences, which go as they come.
+@pytest.mark.parametrize("hq,hkv,lens", [(16, 8, [256] * 8), (16, 8, [1500]), (16, 8, [1500, 1500]), (8, 8, [600] * 7), (8, 8, [129, 700, 3, 250] * 5),
+                                         (2, 2, list(range(130, 430))), (1, 1, [5, 300] + [1, 17] * 520)])
+def test_prompt_attention_dealt_out(hq, hkv, lens):
+    _prompts(hq, hkv, lens)
+
+
+# Portions behind cached tokens, the queries being the last rows of each sequence: pairs, tiles alone beside them, rows of one token
+# with many keys beside a prompt, in one round and in several.  P and the output are bf16: 2^-9 relative each.
+@pytest.mark.parametrize("hq,hkv", [(16, 8), (8, 8)])
+@pytest.mark.parametrize("portions,cached", [([512] * 3, [700, 0, 1500]), ([300, 1, 65, 700, 130, 1] * 3, [0, 2000, 511, 100, 900, 3] * 3), ([600], [1333]),
+                                             ([256] + [1] * 40, [0] + [1000] * 40)])
+def test_causal_attention_behind_cached_tokens(hq, hkv, portions, cached):
+    ends, cu_q, cu_k, g = [a + b for a, b in zip(portions, cached)], [0], [0], gen(len(portions))
+    for n, t in zip(portions, ends):
+        cu_q.append(cu_q[-1] + n)
+        cu_k.append(cu_k[-1] + t)
+    q, k, v = (torch.randn(m, h, 128, generator=g, device=DEV).to(BF) for m, h in ((cu_q[-1], hq), (cu_k[-1], hkv), (cu_k[-1], hkv)))
+    out = torch.zeros_like(q)
+    ops.causal_attn_varlen(q, k, v, i32(cu_q), i32(cu_k), len(portions), max(portions), 0.1, out)
+    assert pkg._lib.device_status() == 0
+    for i, (n, t) in enumerate(zip(portions, ends)):
+        kk, vv = (x[cu_k[i]:cu_k[i + 1]].double().repeat_interleave(hq // hkv, 1) for x in (k, v))
+        s = torch.einsum("ihd,jhd->hij", q[cu_q[i]:cu_q[i + 1]].double(), kk) * 0.1
+        seen = torch.arange(t, device=DEV)[None] <= torch.arange(t - n, t, device=DEV)[:, None]
+        ref = torch.einsum("hij,jhd->ihd", torch.softmax(s.masked_fill(~seen, float("-inf")), -1), vv)
+        assert rel(out[cu_q[i]:cu_q[i + 1]], ref) < 8e-3, i
+
+
 def _prompts(hq, hkv, lens):
     cu = [0]
     for n in lens:
@@ -179,3 +209,14 @@ def test_window_pairs_keep_the_future_out(window, start):
         assert rel(o[:64], r[:64]) < 8e-3
         hit = torch.isnan(r).flatten(1).any(1)
         assert not bool(torch.isfinite(o[hit]).all(-1).any())
+
+
+# Pairs of window attention in several rounds: one and two channel halves, channels that do not fill them, ragged portions behind cached
+# tokens, windows narrower than a tile, of a tile and one, and none; rubbish behind every context.
+@pytest.mark.parametrize("H,KH,D", [(8, 4, 128), (8, 4, 64), (6, 6, 96), (12, 4, 40)])
+@pytest.mark.parametrize("window", [0, 50, 129])
+@pytest.mark.parametrize("portions,starts", [([300, 20, 700, 65, 128] * 4, [0, 1000, 37, 255, 600] * 4), ([256] * 12, [100] * 12)])
+def test_window_pairs(H, KH, D, window, portions, starts):
+    got, ref = _window_case(H, KH, D, portions, starts, window, True)
+    for i, (o, r) in enumerate(zip(got, ref)):
+        assert rel(o, r) < 8e-3, i
