@@ -52,7 +52,8 @@ int mdb_version(void);
  * fault isolation).  MDB_OPT_PDL: 1 = kernels are chained with programmatic
  * dependent launch (default), 0 = plain stream order.  MDB_OPT_GEMM_PAIR: GEMMs
  * of many rows on pairs of CTAs (tcgen05.mma.cta_group::2, tiles of 256 x 256):
- * 1 = from 2048 rows (default), 2 = from 256 rows, 0 = never.
+ * 1 = from 2048 rows (default), 2 = from 256 rows, 0 = never; products per
+ * expert: 1 = from 160 rows an expert where it gains, 2 = from there on always.
  * MDB_OPT_WAIT_LIMIT_US: how long a wait inside a kernel (mbarrier, peer flag)
  * may last before it gives up and raises MDB_STATUS_WAIT_TIMEOUT, in
  * microseconds (default 2 000 000); written to the current device, blocking. */

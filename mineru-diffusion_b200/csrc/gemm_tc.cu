@@ -30,7 +30,7 @@
 // tile and the number of tiles read from device memory; a step of few rows
 // loads only the rows a tile can hold).
 //
-// PAIR form (taken from 2048 rows on; per expert, from 160 rows an expert on): a cluster of two CTAs owns a tile of
+// PAIR form (taken from 2048 rows on; per expert, from 160 rows an expert on where it gains): a cluster of two CTAs owns a tile of
 // 256 step rows x 256 weight rows (tcgen05.mma.cta_group::2).  Each CTA stages
 // its own 128 step rows (A) and its own 128 of the 256 weight rows (B) per k
 // stage -- 32 KB instead of 48 KB for half the output -- and the MMA, issued by
@@ -43,6 +43,7 @@
 // peer's epilogue warps arrive on the leader's "accumulator empty" barrier
 // through its cluster address, and a cluster barrier before the tensor memory
 // is freed keeps either CTA's shared memory alive while the other may read it.
+#include <cmath>
 #include "mdb_common.cuh"
 
 namespace mdb {
@@ -1044,9 +1045,29 @@ static int launch_tc_group_as(const bf16* x, int64_t x_cols, int64_t ldx, const 
   return mdb_launch(gemm_tc_kernel<kTcGroup, false>, dim3(a.grid), dim3(tc_threads(kTcGroup)), kSmem, st, map_x, map_w, a);
 }
 
-// `experts`: how many share the rows (0: per-head form).  CTA pairs where an expert has 160 rows or more on average, so that
-// most have two row tiles: a pair computes two tiles of one expert from one copy of its weights in shared memory, whose
-// bandwidth bounds the single form; an expert's odd last tile leaves half of its pair idle.
+// Whether CTA pairs are the faster form of expert products with `rows` rows an expert on average: a pair computes two row tiles of one
+// expert from one copy of its weights in shared memory, whose bandwidth bounds the single form, but an expert's odd last tile leaves
+// half of its pair idle.  A round of pairs takes 0.8 (k 2048) to 0.9 (k 1024) of a round of as many single tiles; with shorter k the
+// epilogue decides and pairs always lost (by a fifth on average over 8 to 128 experts of 165 to 1500 rows).  16 experts of 256 rows, 1024 x 2048: 36.0 -> 31.6 us; 64 of
+// 192: 76 -> 70 us; 32 of 300, 4096 x 2048: 198 -> 208, 8 of 175, 512 x 2048: 16.6 -> 18.2, which stay single.  The rows of
+// an expert are spread like the sum of independent choices: five points of that spread.
+static bool group_pairs_gain(double rows, int experts, int tiles_n, int k, int sm_count) {
+  if (k < 1024) return false;
+  double single = 0, pair = 0;
+  for (const double z : {-1.28, -0.52, 0.0, 0.52, 1.28}) {
+    const int t = static_cast<int>(std::ceil((rows + z * std::sqrt(rows)) / kTcBM));
+    single += 0.2 * t;
+    pair += 0.2 * ((t + 1) / 2);
+  }
+  single *= static_cast<double>(experts) * tiles_n / sm_count;
+  pair *= static_cast<double>(experts) * tiles_n / (sm_count / 2);
+  if (single <= 1.0) return false;
+  auto rounds = [](double x) { return x < 8 ? std::ceil(x - 0.05) : x + 0.3; };      // many rounds even out
+  return rounds(pair) * (k < 2048 ? 0.9 : 0.8) <= rounds(single);
+}
+
+// `experts`: how many share the rows (0: per-head form).  CTA pairs from 160 rows an expert on average, so that most have two row
+// tiles, where they gain.
 static int launch_tc_group(const bf16* x, int64_t x_cols, int64_t ldx, const bf16* w, int64_t w_rows, TcArgs& a, int experts, cudaStream_t st) {
   static int sm_count = 0;
   if (sm_count == 0) {
@@ -1059,8 +1080,10 @@ static int launch_tc_group(const bf16* x, int64_t x_cols, int64_t ldx, const bf1
   a.tiles_n = (a.n + kTcBN - 1) / kTcBN;
   a.ksplit = 1;
   // the buffer holds the rows and up to one tile of padding per expert
-  if (g_opt_gemm_pair != 0 && experts > 0 && a.a_rows == kTcBM && a.tiles_m < kTcPairList && experts < 65536 &&
-      4 * (a.tiles_m - experts) >= 5 * experts)
+  const int row_tiles = a.tiles_m - experts;
+  const bool can = experts > 0 && a.a_rows == kTcBM && a.tiles_m < kTcPairList && experts < 65536 && 4 * row_tiles >= 5 * experts;
+  if (can && (g_opt_gemm_pair == 2 ||
+              (g_opt_gemm_pair == 1 && group_pairs_gain(static_cast<double>(row_tiles) * kTcBM / experts, experts, a.tiles_n, a.k, sm_count))))
     return launch_tc_group_as<true>(x, x_cols, ldx, w, w_rows, a, sm_count, st);
   return launch_tc_group_as<false>(x, x_cols, ldx, w, w_rows, a, sm_count, st);
 }

@@ -120,11 +120,12 @@ def test_latent_attention_shares(width, heads, nsplit):
         assert rel(out[i].view(heads, width), p @ c) < 4e-3, i
 
 
-# Around the rule for pairs (160 rows per expert), experts of one, two, three and no tiles, output columns that do not fill
-# the last tile, and more ids than the plan has in flight.
+# Around the rule for pairs (160 rows per expert; option 2 takes them from there on, whatever they gain), experts of one, two, three and
+# no tiles, output columns that do not fill the last tile, and more ids than the plan has in flight.
+@pytest.mark.parametrize("pairs", [1, 2])
 @pytest.mark.parametrize("E,top,m,kind", [(4, 2, 300, "spread"), (4, 2, 400, "spread"), (8, 3, 900, "skewed"), (5, 1, 900, "one"), (64, 6, 2600, "spread")])
 @pytest.mark.parametrize("n", [264, 512])
-def test_expert_tiles_in_pairs(E, top, m, kind, n):
+def test_expert_tiles_in_pairs(E, top, m, kind, n, pairs):
     k, g = 128, gen(E + m)
     ids = torch.stack([torch.randperm(E, generator=torch.Generator().manual_seed(i))[:top] for i in range(m)])
     if kind == "one":
@@ -138,7 +139,11 @@ def test_expert_tiles_in_pairs(E, top, m, kind, n):
     xs, y = torch.zeros(tiles * 128, k, dtype=BF, device=DEV), torch.full((tiles * 128 + 1, n), 9.0, dtype=BF, device=DEV)
     ops.moe_plan(ids.int().to(DEV), E, tiles, slot, row_token, tile_expert, num)
     ops.moe_gather(x, xs, row_token, num, tiles)
-    ops.gemm_experts(xs, w, y[:-1], tile_expert, num, m)
+    ops.set_option(ops.OPT_GEMM_PAIR, pairs)
+    try:
+        ops.gemm_experts(xs, w, y[:-1], tile_expert, num, m)
+    finally:
+        ops.set_option(ops.OPT_GEMM_PAIR, 1)
     assert pkg._lib.device_status() == 0
     s = slot.cpu().long()
     assert len(set(s.flatten().tolist())) == m * top and (tile_expert.cpu()[s // 128] == ids).all()
