@@ -92,7 +92,8 @@ constexpr int kRes32Threads = 256;
 // One CTA per row.  residual (scaled or, with ids, = embed[id] * scale) + up to two projections + the weighted sum of
 // the chosen experts' rows; y = residual / rms * weight.  POST: the norm replaces the residual, and y is the new residual or
 // its norm with a second weight.  NV float4 chunks of the row per thread; PARTS: a projection may come as split-k slices.
-template <typename T, int NV, bool POST, bool PARTS>
+// AHEAD: four of the chosen experts' rows requested together
+template <typename T, int NV, bool POST, bool PARTS, bool AHEAD>
 __global__ void __launch_bounds__(kRes32Threads) residual_norm_kernel(const mdb_residual_norm_args a) {
   pdl_launch_dependents();
   pdl_wait();
@@ -132,23 +133,33 @@ __global__ void __launch_bounds__(kRes32Threads) residual_norm_kernel(const mdb_
     }
     if (a.moe_rows != nullptr) {
       float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
-      // four experts' rows at a time: one by one, the slot and the row behind it are two latencies per expert
-      for (int k0 = 0; k0 < a.moe_top; k0 += 4) {
-        int slot[4];
-        float w[4];
-        float4 e[4];
+      if (AHEAD) {
+        // one by one, the slot and the row behind it are two latencies per expert
+        for (int k0 = 0; k0 < a.moe_top; k0 += 4) {
+          int slot[4];
+          float w[4];
+          float4 e[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          slot[k] = k0 + k < a.moe_top ? a.moe_slot[row * a.moe_top + k0 + k] : -1;
-          w[k] = k0 + k < a.moe_top ? a.moe_weight[row * a.moe_top + k0 + k] : 0.f;
+          for (int k = 0; k < 4; ++k) {
+            slot[k] = k0 + k < a.moe_top ? a.moe_slot[row * a.moe_top + k0 + k] : -1;
+            w[k] = k0 + k < a.moe_top ? a.moe_weight[row * a.moe_top + k0 + k] : 0.f;
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            e[k] = slot[k] >= 0 ? act_load4(static_cast<const T*>(a.moe_rows) + slot[k] * a.moe_ld + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            if (slot[k] < 0) continue;
+            d.x = fmaf(w[k], e[k].x, d.x); d.y = fmaf(w[k], e[k].y, d.y); d.z = fmaf(w[k], e[k].z, d.z); d.w = fmaf(w[k], e[k].w, d.w);
+          }
         }
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          e[k] = slot[k] >= 0 ? act_load4(static_cast<const T*>(a.moe_rows) + slot[k] * a.moe_ld + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          if (slot[k] < 0) continue;
-          d.x = fmaf(w[k], e[k].x, d.x); d.y = fmaf(w[k], e[k].y, d.y); d.z = fmaf(w[k], e[k].z, d.z); d.w = fmaf(w[k], e[k].w, d.w);
+      } else {
+        for (int k = 0; k < a.moe_top; ++k) {
+          const int slot = a.moe_slot[row * a.moe_top + k];
+          if (slot < 0) continue;
+          const float w = a.moe_weight[row * a.moe_top + k];
+          const float4 e = act_load4(static_cast<const T*>(a.moe_rows) + slot * a.moe_ld + c);
+          d.x = fmaf(w, e.x, d.x); d.y = fmaf(w, e.y, d.y); d.z = fmaf(w, e.z, d.z); d.w = fmaf(w, e.w, d.w);
         }
       }
       x.x += d.x; x.y += d.y; x.z += d.z; x.w += d.w;
@@ -493,19 +504,22 @@ bool rows_ok(const mdb_rows& s) {
                               (s.parts == nullptr || (s.nparts >= 1 && s.part_stride % 4 == 0)));
 }
 
-template <typename T, bool POST, bool PARTS>
+template <typename T, bool POST, bool PARTS, bool AHEAD>
 int launch_residual_norm_of(const mdb_residual_norm_args& a, cudaStream_t st) {
   const int chunks = (a.width_pad / 4 + kRes32Threads - 1) / kRes32Threads;
-  if (chunks <= 1) return mdb_launch(residual_norm_kernel<T, 1, POST, PARTS>, dim3(a.m), dim3(kRes32Threads), 0, st, a);
-  if (chunks <= 2) return mdb_launch(residual_norm_kernel<T, 2, POST, PARTS>, dim3(a.m), dim3(kRes32Threads), 0, st, a);
-  if (chunks <= 4) return mdb_launch(residual_norm_kernel<T, 4, POST, PARTS>, dim3(a.m), dim3(kRes32Threads), 0, st, a);
-  if (chunks <= 8) return mdb_launch(residual_norm_kernel<T, 8, POST, PARTS>, dim3(a.m), dim3(kRes32Threads), 0, st, a);
+  if (chunks <= 1) return mdb_launch(residual_norm_kernel<T, 1, POST, PARTS, AHEAD>, dim3(a.m), dim3(kRes32Threads), 0, st, a);
+  if (chunks <= 2) return mdb_launch(residual_norm_kernel<T, 2, POST, PARTS, AHEAD>, dim3(a.m), dim3(kRes32Threads), 0, st, a);
+  if (chunks <= 4) return mdb_launch(residual_norm_kernel<T, 4, POST, PARTS, AHEAD>, dim3(a.m), dim3(kRes32Threads), 0, st, a);
+  if (chunks <= 8) return mdb_launch(residual_norm_kernel<T, 8, POST, PARTS, AHEAD>, dim3(a.m), dim3(kRes32Threads), 0, st, a);
   return MDB_ERR_UNSUPPORTED;
 }
 template <typename T, bool POST>
 int launch_residual_norm(const mdb_residual_norm_args& a, cudaStream_t st) {
-  return a.add[0].parts != nullptr || a.add[1].parts != nullptr ? launch_residual_norm_of<T, POST, true>(a, st)
-                                                                : launch_residual_norm_of<T, POST, false>(a, st);
+  if (a.add[0].parts != nullptr || a.add[1].parts != nullptr) return launch_residual_norm_of<T, POST, true, false>(a, st);
+  // Chosen rows that L2 does not hold whole: behind their product, 2048 tokens of six rows of 2048 (50 MB) 26 us one by one, 23 four at a
+  // time.  Out of L2 the longer form is the slower one: 700 tokens of two rows 5.6 against 7.7 us, 64 of six 5.1 against 5.9.
+  const int64_t chosen = a.moe_rows == nullptr ? 0 : static_cast<int64_t>(a.m) * a.moe_top * a.moe_ld * static_cast<int64_t>(sizeof(T));
+  return chosen >= (48 << 20) ? launch_residual_norm_of<T, POST, false, true>(a, st) : launch_residual_norm_of<T, POST, false, false>(a, st);
 }
 }  // namespace
 
