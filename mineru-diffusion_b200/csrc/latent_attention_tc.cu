@@ -11,7 +11,8 @@
 //
 // What bounds it: memory; a tile is read from shared memory twice (1024 cycles at 64 KB) and written once.  A CTA per SM takes
 // an equal share of all the step's key tiles, cut where they fall (a row of a step has at most nsplit parts; with one part
-// rows stay whole), so a ragged batch leaves no SM behind; the next row's tiles arrive while this one's output leaves.
+// rows stay whole), so with three parts a row and more a ragged batch leaves no SM behind; with two a share is at least the longest
+// row, and 99 to 148 rows keep as many SMs busy.  The next row's tiles arrive while this one's output leaves.
 // With the merge of the parts, 16 heads, width 512: 32 requests of 2048 to 4096 keys 47.3 -> 31.7 us, 60 requests 79.9 -> 46.1,
 // one request of 8000 keys 32.2 -> 28.4, of 300 keys 17.9 -> 18.1; 64 requests of 4000 to 8000 keys, 32 heads, 263 -> 169 us.
 #include "mdb_common.cuh"

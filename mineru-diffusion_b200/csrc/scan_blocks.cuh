@@ -1,4 +1,5 @@
-// Scans of prompt portions in blocks of 16 tokens, still in fp32 FMAs (included by recurrent.cu, inside its namespace).
+// Scans of long prompt portions of few sequences in blocks of 16 tokens, still in fp32 FMAs (included by recurrent.cu, inside its
+// namespace, which has the rule for when).
 //
 // With G_t the product of the decays of a block's tokens 1 .. t (per key channel in the delta rule, one number per head in the
 // other recurrences) and S the state in front of the block,
@@ -12,9 +13,9 @@
 // What bounds it: latency, with few warps per scheduler.  All the states of four prompts of 16 heads are 55 elements per FMA
 // lane of the chip.  A CTA has warps that keep COLS columns of the state in registers (CPT columns x 1/16 of the channels a
 // thread: a 16-byte read of shared memory feeds 4 CPT FMAs) and others that prepare the next block meanwhile: its operands with
-// cp.async two blocks ahead, the scaled rows, L and M.  Against the token-by-token form, 2048 tokens: mLSTM, 8 heads of 128 x 256,
-// one, two and four sequences 478 / 635 / 681 -> 315 / 350 / 470 us; delta rule with its decays, 16 heads of 128 x 128, 840 / 857
-// / 1399 -> 485 / 611 / 820 us.
+// cp.async two blocks ahead, the scaled rows, L and M.  Against the token-by-token form, the scan alone, 2048 tokens: mLSTM, 8 heads
+// of 128 x 256, one, two and four sequences 438 / 474 / 624 -> 315 / 350 / 471 us (3.7 us a block of 64 columns, three warps per
+// scheduler); delta rule, 16 heads of 128 x 128, 490 / 647 / 1024 -> 465 / 576 / 756 us (5.9 us a block, four warps per scheduler).
 constexpr int kSbTokens = 16, kSbRing = 3;
 
 template <int MODE, int DP, int COLS, int CPT>

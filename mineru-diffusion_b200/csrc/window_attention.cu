@@ -1,6 +1,6 @@
 // Rotary grouped-query attention over paged K and V caches, with a window and a sink: the kernel in front of it (per-head
 // norms, rotation, cache rows) and the forms that take a few tokens of a sequence, decoding above all.  Prompt portions
-// go to the window form of the tensor-memory kernel (attention_tc.cu).
+// go to the window form of the tensor-memory kernel (attention_prompt.cu).
 //
 //   rotary_commit_kernel     a CTA per token: sines and cosines once, then a warp per head.
 //   window_attn_mma_kernel   bf16: a CTA takes up to 16 query heads of one KV head of one token and a range of its keys (split

@@ -47,7 +47,8 @@ def pad_head(dim: int) -> int:
 
 def key_parts(ctas: int, keys: int) -> int:
     """Key-range parts of an attention of ``ctas`` CTAs over up to ``keys`` keys each: about two CTAs per SM, parts of at least
-    128 keys."""
+    128 keys.  The window attention's decoding kernel cuts every row into so many; the latent attention, whose CTAs take shares of all
+    rows, at most so many, which leaves SMs idle where it is 1 or 2 (from 99 rows of 16 heads on)."""
     return max(1, min(296 // max(1, ctas), keys // 128, 64))
 
 
