@@ -14,7 +14,7 @@
 // and P goes back into the tensor memory of the scores it came from (bf16 pairs, the left operand of P V): no shared memory for P
 // and no proxy fence.  The products of one thread run in the order of issue, so new scores may follow P V into the same columns
 // without a wait.  A unit of one tile (see the launch) takes both score buffers in turn, the next scores ahead of P V.
-// 4 x 4096 tokens, 16 query and 8 KV heads: 400 -> 301 us alone, 417 -> 335 in a loop at the power limit, the same bits.  (Steps of
+// 4 x 4096 tokens, 16 query and 8 KV heads: 400 -> 289 us alone, 417 -> 333 - 337 in a loop at the power limit, the same bits.  (Steps of
 // 64 keys with two score buffers per tile and an issuing warp per tile: 299 us alone, 329 in a loop, other roundings; an issuing
 // warp per tile with these steps: 351.)
 //
@@ -31,8 +31,8 @@ struct ApPlan {
   static constexpr int kKStages = 3, kVStages = 2;
   static constexpr int kQBytes = 2 * 128 * 128;             // a tile: two channel halves of [128 rows][128 B]
   static constexpr int kThreads = 384;                      // three warpgroups; two warps idle
-  // registers: 384 threads x 168 at launch = 256 x 208 (softmax) + 128 x 88
-  static constexpr int kSoftmaxRegs = 208, kOtherRegs = 88;
+  // registers: 384 threads x 168 at launch = 256 x 216 (softmax) + 128 x 72, no spills (208 / 88: 291 against 289 us)
+  static constexpr int kSoftmaxRegs = 216, kOtherRegs = 72;
   static_assert(256 * kSoftmaxRegs + 128 * kOtherRegs <= kThreads * 168, "registers after the split");
   static constexpr int kOffK = 2 * kQBytes;
   static constexpr int kOffV = kOffK + kKStages * kAtTileBytes;
@@ -153,7 +153,7 @@ __host__ __device__ __forceinline__ int ap_cost(const AtArgs& a, const ApSeq& w,
 // alternating direction gives every CTA about the same.  Sequences of few queries and many keys beside prompts, and batches
 // in which one sequence is the longest by far, would leave the list of all that is possible nearly empty and its order the wrong
 // one (8 sequences, a prompt of 512 tokens and 7 rows behind 4000 keys: 103 us unsorted in pairs, 59 us; [1000] and 40 times 60
-// tokens 57 -> 43 us).  It takes 1.2 us.  `answer`: two words of shared memory; `scratch`: memory of the operand tiles, not in use yet.
+// tokens 57 -> 36 us).  It takes 1.2 us.  `answer`: two words of shared memory; `scratch`: memory of the operand tiles, not in use yet.
 template <bool WIN>
 __device__ __forceinline__ ApDeal ap_deal(const AtArgs& a, int* answer, uint32_t* scratch, uint32_t* list) {
   const int tid = threadIdx.x, lane = tid & 31, G = static_cast<int>(gridDim.x);
@@ -489,9 +489,10 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     auto skip_v = [&](const ApUnit& w) { if (WIN) for (int j = 0; j < w.ntiles + (w.cut >= 0 ? 1 : 0); ++j) vr.advance(P::kVStages); };
     uint32_t s_phase = 0 /* bit per buffer */, o_phase = 0, q_phase = 0, done_phase = 0;      // done: of the last P V
     bool ok = true;
+    // where there is one tile per unit, the next unit is looked up under the last products; with two it would cost registers
     ApUnit next = ap_unit<WIN, DEAL>(a, deal, list, 0);
     for (int wave = 0; wave < waves && ok; ++wave) {
-      const ApUnit w = next;
+      const ApUnit w = DEAL ? ap_unit<WIN, DEAL>(a, deal, list, wave) : next;
       const ApTile t = x == 0 ? w.t[0] : w.t[1];
       if (w.ntiles == 0 || !t.valid) {
         if (w.ntiles > 0) {
@@ -504,7 +505,7 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           q_phase ^= 1;
           skip_v(w);
         }
-        next = ap_unit<WIN, DEAL>(a, deal, list, wave + 1);
+        if (!DEAL) next = ap_unit<WIN, DEAL>(a, deal, list, wave + 1);
         continue;
       }
       const int head = w.kvh * group + head_in_group;
@@ -643,7 +644,7 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       }
       if (!ok) break;
       skip_v(w);
-      next = ap_unit<WIN, DEAL>(a, deal, list, wave + 1);      // under the last products
+      if (!DEAL) next = ap_unit<WIN, DEAL>(a, deal, list, wave + 1);
       // ------------------------------------------------------------- outputs of the tile
       ok = mbar_wait(bar(kApBarOFull + x), o_phase);
       if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
@@ -706,8 +707,8 @@ static int ap_run(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUte
 }
 
 // Tiles per unit for sequences of the same `queries` and `keys` (each of the first behind keys - queries tokens): the shorter time of
-// the longest of every fourth CTA.  One prompt of 1280 to 2304 tokens (160 to 288 tiles): 28 - 49 us in pairs, 21 - 39 us alone; of 3072
-// tokens, or 8 of 256, the other way round (61 against 64, 17 against 19 us).
+// the longest of every fourth CTA.  One prompt of 1280 to 2304 tokens (160 to 288 tiles): 31 - 49 us in pairs, 19 - 35 us alone; of 4096
+// tokens, or 8 of 256, the other way round (79 against 84, 17 against 19 us).
 template <bool WIN>
 static int ap_tiles_alike(const AtArgs& a, int queries, int keys, int sms) {
   const int per_rank = a.nseq * a.hkv;
@@ -726,7 +727,8 @@ static int ap_tiles_alike(const AtArgs& a, int queries, int keys, int sms) {
       if (t > most[per - 1]) most[per - 1] = t;
     }
   }
-  return most[0] <= most[1] ? 1 : 2;
+  // (a launch of tiles alone, with 192 threads, takes 0.87 of the time of one that could have had pairs: 30.5 against 35.1 us for 2048)
+  return 7 * most[0] <= 8 * most[1] ? 1 : 2;
 }
 
 // Tiles that can all have an SM of their own take one: two on one SM wait for one another (one prompt of 1056 tokens, 136 tiles:
