@@ -1,4 +1,4 @@
-// y = x W^T in true fp32 (no tensor-core mode has a 24-bit significand), for the fp32 mode of the models that have one.  Same
+// y = x W^T in true fp32, for the fp32 mode of the models that have one, on FMAs (a long k: gemm_f32_tc.cu).  Same
 // three forms as the grouped tcgen05 kernel: plain, one weight per head (column blocks of x and y), one weight per expert (row
 // tiles of 128).  GLU: half of a tile's weight rows are gate rows, the other half the up rows n further.
 //
@@ -245,6 +245,10 @@ static int gemm_f32_dispatch(const mdb_gemm_args& a, cudaStream_t st) {
 static int gemm_f32_launch(const mdb_gemm_args& a, cudaStream_t st) {
   if (a.k % 16 != 0) return MDB_ERR_UNSUPPORTED;
   if ((static_cast<int64_t>(a.m) + 63) / 64 > 65535 || a.heads > 65535) return MDB_ERR_UNSUPPORTED;
+  // Above this k on the tensor cores, by k alone, so that a row's bits do not depend on how many rows there are.  Their form takes 6 to 9
+  // us for the smallest product: at k 512, 16 rows x 2048 columns lose by it (5.2 -> 7.0 us) and 500 rows gain; at k 1024 all but
+  // the narrowest gain, and its error, not k's root but level, is the smaller one.
+  if (a.k >= 768) return gemm_f32_tc_launch(a, st);
   return a.act == MDB_ACT_RELU_GLU ? gemm_f32_dispatch<true>(a, st) : gemm_f32_dispatch<false>(a, st);
 }
 

@@ -43,13 +43,6 @@ __device__ __forceinline__ uint64_t lt_desc_mn(uint32_t smem_addr) {
   return static_cast<uint64_t>((smem_addr >> 4) & 0x3FFF) | (static_cast<uint64_t>(kLtBox >> 4) << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) |
          (static_cast<uint64_t>(1) << 46) | (static_cast<uint64_t>(2) << 61);
 }
-__device__ __forceinline__ void tmem_stf16(uint32_t taddr, const float (&v)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "f"(v[0]), "f"(v[1]),
-      "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]), "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]),
-      "f"(v[14]), "f"(v[15])
-      : "memory");
-}
 
 // The share of a CTA: `count` key tiles of the rows laid end to end, from tile `off` of row `row`, which begins at `base`.
 struct LtShare {

@@ -151,6 +151,41 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
+// ---- pairs of fp32 numbers ---------------------------------------------------
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// The three bf16 parts of a pair of numbers: 24 significant bits are the exact sum of three times eight, cut and not rounded (the
+// upper half of x, that of what is left, the rest).  Numbers below 2^-110 lose their last bits: no bf16 number is below 2^-133.
+__device__ __forceinline__ void split3(f32x2 xy, uint32_t (&part)[3]) {
+  const f32x2 minus = pack2(-1.0f, -1.0f);
+#pragma unroll
+  for (int p = 0; p < 3; ++p) {
+    const float2 v = unpack2(xy);
+    const uint32_t a = __float_as_uint(v.x), b = __float_as_uint(v.y);
+    part[p] = __byte_perm(a, b, 0x7632);
+    if (p < 2) xy = fma2(pack2(__uint_as_float(a & 0xffff0000u), __uint_as_float(b & 0xffff0000u)), minus, xy);
+  }
+}
+
 // Named barrier over `threads` threads that also ANDs a predicate across them.
 __device__ __forceinline__ bool named_bar_and(int id, int threads, bool pred) {
   uint32_t r;

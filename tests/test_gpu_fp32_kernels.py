@@ -146,3 +146,59 @@ def test_scan_in_blocks_keeps_the_future_out():
     ops.scan(ops.SCAN_DECAY, F32, 1, H, H, D, DV, q.to(DEV), k.to(DEV), v.to(DEV), torch.full((rows, H), 0.9, device=DEV), torch.ones(rows, H, device=DEV),
              torch.zeros(1, H, DV, D, device=DEV), _portions([T], [0], [0]), out=o)
     assert bool(torch.isfinite(o[:21]).all()) and not bool(torch.isfinite(o[21:T]).any()) and float(o[T:].abs().max()) == 0
+
+
+# From k = 768 on the products run on the tensor cores: tiles of 128 weight rows (64 with GLU) x 32 or 64 rows, chunks of 64 k, one to four
+# CTAs for a tile's k.  Sums of 64 products are cut off four times (2^-23 of a sum that is 1/16 of the whole in its square and
+# less) and added up in fp32: 2e-7 by measurement; 4e-7 leaves room for the activation, which doubles it.
+@pytest.mark.parametrize("m,n,k", [(1, 4, 768), (31, 132, 784), (33, 1000, 1040), (64, 260, 1552), (65, 4100, 768), (500, 1028, 3072), (1030, 2300, 816)])
+@pytest.mark.parametrize("act", [ops.ACT_NONE, ops.ACT_RELU2, ops.ACT_RELU_GLU, ops.ACT_SILU])
+def test_fp32_product_on_tensor_cores(m, n, k, act):
+    x, w = torch.randn(m, k + 4 if m % 2 else k, generator=gen(1)), torch.randn(2 * n if act == ops.ACT_RELU_GLU else n, k, generator=gen(2)) * k ** -0.5
+    y = torch.full((m + 1, n + 4), 7.0, device=DEV)
+    wide = torch.zeros(m, k + 8, device=DEV)
+    wide[:, 4 * (m % 2):4 * (m % 2) + k] = x[:, :k].to(DEV)                  # odd m: rows on a boundary of 16 bytes only
+    rows = wide[:, 4 * (m % 2):4 * (m % 2) + k]
+    ops.gemm(rows, w.to(DEV), y[:m, :n], act=act, act_from=4 if act == ops.ACT_SILU else 0)
+    z = x[:, :k].to(DEV, F64) @ w.to(DEV, F64).T
+    if act == ops.ACT_RELU2:
+        z = torch.relu(z) ** 2
+    elif act == ops.ACT_RELU_GLU:
+        z = torch.relu(z[:, :n]) * z[:, n:]
+    elif act == ops.ACT_SILU:
+        z[:, 4:] = torch.nn.functional.silu(z[:, 4:])
+    assert rel(y[:m, :n], z) < 4e-7
+    assert float((y[:m, n:] - 7).abs().max()) == 0 and float((y[m] - 7).abs().max()) == 0
+    assert pkg._lib.device_status() == 0
+
+
+def test_fp32_product_per_head_and_per_expert_on_tensor_cores():
+    heads, n, k, m = 3, 200, 1024, 70
+    x, w = torch.randn(m, heads * k, generator=gen(5)).to(DEV), torch.randn(heads, n, k, generator=gen(6)).to(DEV)
+    y = ops.gemm_heads(x, w, torch.zeros(m, heads * n, device=DEV))
+    ref = torch.einsum("mhk,hnk->mhn", x.double().view(m, heads, k), w.double()).reshape(m, -1)
+    assert rel(y, ref) < 4e-7
+    tiles = torch.tensor([2, 0, 2], dtype=torch.int32, device=DEV)
+    x = torch.randn(4 * 128, k, generator=gen(7)).to(DEV)
+    y = torch.full((4 * 128, n), 7.0, device=DEV)
+    ops.gemm_experts(x, w, y, tiles, torch.tensor([3, 0, 0, 0], dtype=torch.int32, device=DEV), 128)
+    for i, e in enumerate(tiles.tolist()):
+        assert rel(y[128 * i:128 * i + 128], x[128 * i:128 * i + 128].double() @ w[e].double().T) < 4e-7
+    assert float((y[384:] - 7).abs().max()) == 0 and pkg._lib.device_status() == 0
+
+
+@pytest.mark.parametrize("m", [5, 400])
+def test_fp32_product_of_numbers_that_are_not_finite(m):
+    """Infinities and NaN reach the outputs that an fp32 sum gives them, and no others; numbers near the largest stay finite."""
+    n, k = 300, 1024
+    x, w = torch.randn(m, k, generator=gen(8)), torch.randn(n, k, generator=gen(9))
+    x[1, 5], x[2, 7], x[3, 8] = float("inf"), float("nan"), 3e38
+    w[4, 5], w[11, 0], w[12, 8], w[13] = 0.0, -float("inf"), 0.5, 0.0
+    y = ops.gemm(x.to(DEV), w.to(DEV), torch.zeros(m, n, device=DEV)).cpu()
+    ref = x.double() @ w.double().T                                     # inf * 0 is NaN there too
+    kind = lambda t: torch.where(t.isnan(), 3.0, torch.where(t.isinf(), t.sign(), 2.0 * torch.ones_like(t)))      # noqa: E731
+    big = ref.abs() > 3.4e38
+    ref[big & ref.isfinite()] = ref[big & ref.isfinite()].sign() * float("inf")
+    assert torch.equal(kind(y.double()), kind(ref))
+    assert rel(y[4][ref[4].isfinite()], ref[4][ref[4].isfinite()]) < 4e-7
+    assert pkg._lib.device_status() == 0
