@@ -1142,15 +1142,13 @@ int launch_scan_prompt(const mdb_scan_args& a, cudaStream_t st) {
 // Columns per CTA of the scan in blocks of 16 tokens, 0: token by token.
 //
 // The blocks shorten the chain of a sequence but leave an SM to one CTA, so they lose (by 5 to 55 %) once their CTAs no longer run all
-// at once; within that, 64 columns per CTA, or 32 or 16 where those still fit (a block of the delta rule takes 3.6 us with 16
-// columns, 4.5 with 32, 5.9 with 64).  What is left is how many tokens make up for the start and for a last block that is partly
-// empty.  Time of the blocks over the time token by token, with heads of 128 channels, at 96 / 512 tokens (and one token into a new
-// block at the thresholds below: at most 1.0):
-//   delta rule, columns 128: 4 to 16 sequence heads (16) 1.02 / 0.96; 32 (32) 0.99 / 0.90; 48 (64) 0.98 / 0.95; 64 (64) 0.79 / 0.75
-//   mLSTM, columns 256:      4 to 32 sequence heads (16, 32, 64) 0.80 - 0.83 / 0.72 - 0.77
-//   decay scan, columns 64:  up to 32 sequence heads (16) 0.81 / 0.76; 48 (32) 0.96 / 0.91; 80 (64) 0.96 / 0.90; 128 (64) 0.82 / 0.78
-// and of 64 channels: delta rule 1.01 - 1.2 whatever the form; mLSTM, columns 128: 0.75 / 0.67 (16), 0.99 / 0.94 (32), 0.78 / 0.72
-// (64, SMs full); decay scan 0.83 / 0.78 (16), 1.0 - 1.15 (32, 64).
+// at once; within that, 64 columns per CTA, or 32 or 16 where those still fit.  What is left is how many tokens make up for the
+// start and for a last block that is partly empty.  us token by token and in blocks, one token into a new block, 33 / 49 / 65 tokens:
+//   delta rule, columns 128: 16 heads (16 columns a CTA) 11.2 12.1 / 15.3 15.2 / 19.4 18.0; 32 (32) 14.9 15.5 / 20.7 19.9 / 26.2 24.1;
+//                            48 (64) 17.5 19.2 / 26.1 24.4 / 34.4 29.7; 64 (64) 23.0 19.2 / 33.0 24.5 / 42 30
+//   mLSTM, columns 256:      8 heads (16) 10.0 9.0 / 13.4 10.9; 16 (32) 11.8 10.4 / 16 12.7; 32 (64) 14.5 14.1 / 19.6 17.3
+//   decay scan, columns 64:  16 heads (16) 8.8 7.6 / 11.6 9.4; 48 (32) 10.4 9.7 / 13.6 11.9; 80 (64) 13.8 12.9; 128 (64) 13.8 13.3
+// and of 64 channels: delta rule 1.0 - 1.2 of the time whatever the form; decay scan 7.1 6.1 (16), no better with 32 and 64.
 template <int MODE, int DP>
 int scan_block_columns(const mdb_scan_args& a, int64_t rows) {
   if (DP > 128 || (DP == 64 && MODE == kScanDelta)) return 0;
@@ -1159,12 +1157,10 @@ int scan_block_columns(const mdb_scan_args& a, int64_t rows) {
   if (ctas(64) > sms) return 0;
   const int cols = ctas(16) <= sms ? 16 : ctas(32) <= sms ? 32 : 64;
   if (MODE == kScanDecay && DP == 64 && cols != 16) return 0;
-  int least;                                       // tokens of a sequence on average
-  if (cols == 16) least = MODE == kScanDelta ? 448 : 80;
-  else if (MODE == kScanMlstm && DP == 128) least = 80;
-  else if (cols == 64 && 4 * ctas(64) >= 3 * sms) least = 96;
-  else if (cols == 64) least = MODE == kScanDelta ? 448 : 256;
-  else least = MODE == kScanMlstm ? 448 : 256;
+  // tokens of a sequence on average
+  int least = 32;
+  if (MODE == kScanDelta && 4 * ctas(64) < 3 * sms) least = 64;
+  if (MODE == kScanMlstm && DP == 64 && cols != 16) least = 80;
   return rows >= static_cast<int64_t>(least) * a.bs ? cols : 0;
 }
 

@@ -10,12 +10,16 @@
 // decay of zero is a zero.  A token then costs three FMAs per state element (two without L) and no sum over lanes of its
 // own; the token-by-token form spends four (three) and a chain of shuffles for every two tokens.
 //
-// What bounds it: latency, with few warps per scheduler.  All the states of four prompts of 16 heads are 55 elements per FMA
-// lane of the chip.  A CTA has warps that keep COLS columns of the state in registers (CPT columns x 1/16 of the channels a
-// thread: a 16-byte read of shared memory feeds 4 CPT FMAs) and others that prepare the next block meanwhile: its operands with
-// cp.async two blocks ahead, the scaled rows, L and M.  Against the token-by-token form, the scan alone, 2048 tokens: mLSTM, 8 heads
-// of 128 x 256, one, two and four sequences 438 / 474 / 624 -> 315 / 350 / 471 us (3.7 us a block of 64 columns, three warps per
-// scheduler); delta rule, 16 heads of 128 x 128, 490 / 647 / 1024 -> 465 / 576 / 756 us (5.9 us a block, four warps per scheduler).
+// What bounds it: latency, with few warps per scheduler; a delta rule with 64 columns a CTA by the rate of packed FMAs and shared memory.
+// All the states of four prompts of 16 heads are 55 elements per FMA lane of the chip.  A CTA has warps that keep COLS columns of
+// the state in registers (CPT columns x 1/16 of the channels a thread: a 16-byte read of shared memory feeds 4 CPT FMAs) and others
+// that prepare the next block meanwhile: its operands with cp.async two blocks ahead, the scaled rows, L and M.  Loads stand in
+// front of stores: every store might be to what the next load reads, for all the compiler knows, and with a store in each turn of a loop
+// the turns come one behind the other (sums of products with the state, u, outputs, scaled rows: 755 -> 665 us for the delta
+// rule below); places in memory are worked out once; the mLSTM's normaliser lies in shared memory, a channel per thread.
+// The scan alone, 2048 tokens, with those changes: mLSTM, 8 heads of 128 x 256, one, two and four sequences 315 / 350 / 469 -> 250 / 280 /
+// 412 us; delta rule, 16 heads of 128 x 128, 463 / 576 / 755 -> 370 / 530 / 644 us.  (Scalar FMAs for the products with the state: 682,
+// 444.  The same blocks on tcgen05, operands in three bf16 parts, 128 columns a CTA: 560 and 403, no better for up to 32 sequence heads.)
 constexpr int kSbTokens = 16, kSbRing = 3;
 
 template <int MODE, int DP, int COLS, int CPT>
@@ -31,7 +35,7 @@ struct SbPlan {
   static constexpr int P_QH = DELTA ? ROW : 0, P_KT = 2 * P_QH, P_G = P_KT + (DELTA ? ROW : 0), P_L = P_G + (DELTA ? DP : 0),
                        P_M = P_L + (DELTA ? 256 : 0), P_T = P_M + 256, PREP = P_T + 4 * kSbTokens;
   static constexpr int OFF_PREP = kSbRing * RAW, OFF_R = OFF_PREP + 2 * PREP, OFF_U = OFF_R + (DELTA ? 2 : 1) * kSbTokens * COLS,
-                       OFF_N = OFF_U + 2 * kSbTokens * COLS, FLOATS = OFF_N + kSbTokens;
+                       OFF_N = OFF_U + 2 * kSbTokens * COLS, FLOATS = OFF_N + DP;
   static constexpr int kSmemBytes = FLOATS * 4;
 };
 
@@ -94,38 +98,55 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
     // ------------------------------------------------------------------------------------------------ preparing warps
     const int tid = threadIdx.x - MAIN, pw = warp - MAIN / 32;
     const bool v16 = (a.vdim & 3) == 0 && (reinterpret_cast<uintptr_t>(a.v) & 15) == 0;
-    auto fetch = [&](int b) {
+    // places of a thread's 16-byte pieces, worked out once: KP rows of k, q and g, VP of v
+    constexpr int KT = P::PREP_THREADS / (DP / 4), KP = T / KT, VT = P::PREP_THREADS / (COLS / 4), VP = T > VT ? T / VT : 1;
+    static_assert(KT <= T && T % KT == 0 && (VT >= T || T % VT == 0), "whole rounds over a block's rows");
+    const int ft = tid / (DP / 4), fc = tid % (DP / 4) * 4, vt = tid / (COLS / 4), vc = tid % (COLS / 4) * 4;
+    const int64_t kstep = static_cast<int64_t>(a.kv_heads) * DP, gstep = static_cast<int64_t>(a.heads) * DP, vstep = static_cast<int64_t>(a.heads) * a.vdim;
+    const int64_t k_at = static_cast<int64_t>(w.kvh) * DP + (w.t_begin + ft) * kstep + fc;
+    const float* kp = a.k + k_at;
+    const float* qp = a.q + k_at;
+    const float* gp = DELTA ? a.g + static_cast<int64_t>(w.head) * DP + (w.t_begin + ft) * gstep + fc : nullptr;
+    const float* vp = a.v + static_cast<int64_t>(w.head) * a.vdim + w.col0 + (w.t_begin + vt) * vstep + vc;
+    const bool v_whole = v16 && w.col0 + vc < a.vdim;
+    auto fetch = [&](int b) {                                   // blocks one after the other
       if (b < nblocks) {
         const int t0 = w.t_begin + b * T, n = min(T, w.t_end - t0);
         float* st = sb_smem + (b % kSbRing) * P::RAW;
         const uint32_t base = smem_u32(st);
-        for (int i = tid; i < T * (DP / 4); i += P::PREP_THREADS) {
-          const int t = i / (DP / 4), c = i % (DP / 4) * 4;
+#pragma unroll
+        for (int i = 0; i < KP; ++i) {
+          const int t = ft + i * KT;
           if (t < n) {
-            const int64_t krow = (static_cast<int64_t>(t0 + t) * a.kv_heads + w.kvh) * DP + c;
-            cp_async16(base + (t * DP + c) * 4, a.k + krow);
-            cp_async16(base + (P::RAW_Q + t * DP + c) * 4, a.q + krow);
-            if (DELTA) cp_async16(base + (P::RAW_G + t * DP + c) * 4, a.g + (static_cast<int64_t>(t0 + t) * a.heads + w.head) * DP + c);
+            cp_async16(base + (t * DP + fc) * 4, kp + i * KT * kstep);
+            cp_async16(base + (P::RAW_Q + t * DP + fc) * 4, qp + i * KT * kstep);
+            if (DELTA) cp_async16(base + (P::RAW_G + t * DP + fc) * 4, gp + i * KT * gstep);
           } else {      // tokens behind the portion: no key, no query, no decay
-            *reinterpret_cast<float4*>(st + t * DP + c) = make_float4(0.f, 0.f, 0.f, 0.f);
-            *reinterpret_cast<float4*>(st + P::RAW_Q + t * DP + c) = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (DELTA) *reinterpret_cast<float4*>(st + P::RAW_G + t * DP + c) = make_float4(1.f, 1.f, 1.f, 1.f);
+            *reinterpret_cast<float4*>(st + t * DP + fc) = make_float4(0.f, 0.f, 0.f, 0.f);
+            *reinterpret_cast<float4*>(st + P::RAW_Q + t * DP + fc) = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (DELTA) *reinterpret_cast<float4*>(st + P::RAW_G + t * DP + fc) = make_float4(1.f, 1.f, 1.f, 1.f);
           }
         }
-        const float* v0 = a.v + (static_cast<int64_t>(t0) * a.heads + w.head) * a.vdim + w.col0;
-        const int64_t vstep = static_cast<int64_t>(a.heads) * a.vdim;
-        for (int i = tid; i < T * (COLS / 4); i += P::PREP_THREADS) {
-          const int t = i / (COLS / 4), c = i % (COLS / 4) * 4;
-          if (v16 && t < n && w.col0 + c < a.vdim) {
-            cp_async16(base + (P::RAW_V + t * COLS + c) * 4, v0 + t * vstep + c);
+#pragma unroll
+        for (int i = 0; i < VP; ++i) {
+          const int t = vt + i * VT;
+          if (t >= T) break;
+          float* vs = st + P::RAW_V + t * COLS + vc;
+          const float* from = vp + i * VT * vstep;
+          if (v_whole && t < n) {
+            cp_async16(smem_u32(vs), from);
           } else {
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              if (t < n && w.col0 + c + e < a.vdim) cp_async4(base + (P::RAW_V + t * COLS + c + e) * 4, v0 + t * vstep + c + e);
-              else st[P::RAW_V + t * COLS + c + e] = 0.f;
+              if (t < n && w.col0 + vc + e < a.vdim) cp_async4(smem_u32(vs + e), from + e);
+              else vs[e] = 0.f;
             }
           }
         }
+        kp += T * kstep;
+        qp += T * kstep;
+        gp += T * gstep;
+        vp += T * vstep;
         if (tid < T) {
           const int64_t th = static_cast<int64_t>(t0 + tid) * a.heads + w.head;
           if (tid < n) {
@@ -146,17 +167,11 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
     };
 
     float run_max = MLSTM && !w.fresh ? mstate[block0] : 0.f;
-    // the normaliser, one more column of the mLSTM's state: only the CTA of the first columns owns it, warp by warp alike
+    // the normaliser, one more column of the mLSTM's state: only the CTA of the first columns has it, a channel per thread
     const bool norm = MLSTM && w.col0 == 0;
-    f32x2 nv[NP];
-#pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      nv[i] = 0ull;
-      if (norm && !w.fresh) {
-        const float2 x = *reinterpret_cast<const float2*>(w.state + static_cast<int64_t>(a.vdim) * DP + lane * 2 * NP + 2 * i);
-        nv[i] = pack2(x.x, x.y);
-      }
-    }
+    float* const nrm = sb_smem + P::OFF_N;
+    static_assert(!MLSTM || P::PREP_THREADS >= DP, "a thread per channel of the normaliser");
+    if (norm && tid < DP) nrm[tid] = w.fresh ? 0.f : w.state[static_cast<int64_t>(a.vdim) * DP + tid];
     // lane's share of a row: NP channel pairs
     auto row_pairs = [&](const float* row, f32x2 (&x)[NP]) {
       if (NP == 2) {
@@ -173,14 +188,18 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
       if (DELTA) {
         if (tid < DP) {
           const int c = tid;
-          float kk[T], gg[T], acc = 1.f;
+          float kk[T], gg[T], qq[T], acc = 1.f;
 #pragma unroll
           for (int t = 0; t < T; ++t) {
             kk[t] = raw[t * DP + c];
             gg[t] = raw[P::RAW_G + t * DP + c];
+            qq[t] = raw[P::RAW_Q + t * DP + c];
+          }
+#pragma unroll
+          for (int t = 0; t < T; ++t) {
             acc *= gg[t];
             prep[t * DP + c] = acc * kk[t];
-            prep[P::P_QH + t * DP + c] = acc * raw[P::RAW_Q + t * DP + c];
+            prep[P::P_QH + t * DP + c] = acc * qq[t];
           }
           prep[P::P_G + c] = acc;
           acc = 1.f;
@@ -198,33 +217,37 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
           f32x2 p[2][NP];
           float acc[2][32];
 #pragma unroll
-          for (int t = 0; t < T; ++t) {
+          for (int i = 0; i < NP; ++i) p[0][i] = p[1][i] = 0ull;
+          // (a branch for four tokens at a time: what lies in front of it is not fetched ahead)
 #pragma unroll
-            for (int jj = 0; jj < 2; ++jj) acc[jj][2 * t] = acc[jj][2 * t + 1] = 0.f;
-            if (t < j0) continue;
-            f32x2 k[NP], q[NP], g[NP];
-            row_pairs(raw + t * DP, k);
-            row_pairs(raw + P::RAW_Q + t * DP, q);
-            row_pairs(raw + P::RAW_G + t * DP, g);
+          for (int t4 = 0; t4 < T; t4 += 4) {
+            if (t4 + 3 < j0) {
 #pragma unroll
-            for (int jj = 0; jj < 2; ++jj) {
-              if (t < j0 + jj) continue;
-              if (t == j0 + jj) {
+              for (int i = 0; i < 8; ++i) acc[0][2 * t4 + i] = acc[1][2 * t4 + i] = 0.f;
+              continue;
+            }
+            f32x2 k[4][NP], q[4][NP], g[4][NP];
 #pragma unroll
-                for (int i = 0; i < NP; ++i) p[jj][i] = k[i];
-              } else {
-                f32x2 s = 0ull;
+            for (int e = 0; e < 4; ++e) {
+              row_pairs(raw + (t4 + e) * DP, k[e]);
+              row_pairs(raw + P::RAW_Q + (t4 + e) * DP, q[e]);
+              row_pairs(raw + P::RAW_G + (t4 + e) * DP, g[e]);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int t = t4 + e;
+#pragma unroll
+              for (int jj = 0; jj < 2; ++jj) {
+                f32x2 l = 0ull, m = 0ull;
 #pragma unroll
                 for (int i = 0; i < NP; ++i) {
-                  p[jj][i] = mul2(p[jj][i], g[i]);
-                  s = fma2(p[jj][i], k[i], s);
+                  p[jj][i] = t == j0 + jj ? k[e][i] : mul2(p[jj][i], g[e][i]);      // nothing in front of the key itself
+                  l = fma2(p[jj][i], k[e][i], l);
+                  m = fma2(p[jj][i], q[e][i], m);
                 }
-                acc[jj][2 * t] = sum2(s);
+                acc[jj][2 * t] = sum2(l);
+                acc[jj][2 * t + 1] = sum2(m);
               }
-              f32x2 s = 0ull;
-#pragma unroll
-              for (int i = 0; i < NP; ++i) s = fma2(p[jj][i], q[i], s);
-              acc[jj][2 * t + 1] = sum2(s);
             }
           }
 #pragma unroll
@@ -305,8 +328,10 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
           prep[P::P_M + t * T + j] = j <= t ? between[pass] * bj * total : 0.f;
         }
         if (norm) {
-          // q_t . n for a warp's tokens, then n moves past the block (every warp alike)
+          // q_t . n for a warp's tokens; when all have read it n moves past the block
           float mine = 0.f;
+          f32x2 nv[NP];
+          row_pairs(nrm, nv);
 #pragma unroll
           for (int i2 = 0; i2 < TPW; ++i2) {
             f32x2 q[NP], s = 0ull;
@@ -316,21 +341,13 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
             const float qn = warp_sum(sum2(s));
             if (lane == i2) mine = qn;
           }
-          const float whole = __shfl_sync(0xffffffffu, head, T - 1);
-          f32x2 moved[NP];
+          sb_bar<2, P::PREP_THREADS>();                                        // and M is whole
+          if (tid < DP) {
+            float n = nrm[tid] * per_token[T - 1].x;
 #pragma unroll
-          for (int i = 0; i < NP; ++i) moved[i] = mul2(nv[i], pack2(whole, whole));
-#pragma unroll
-          for (int s = 0; s < T; ++s) {
-            const float wj = __shfl_sync(0xffffffffu, fb * tail, s);
-            f32x2 k[NP];
-            row_pairs(raw + s * DP, k);
-#pragma unroll
-            for (int i = 0; i < NP; ++i) moved[i] = fma2(k[i], pack2(wj, wj), moved[i]);
+            for (int s = 0; s < T; ++s) n = fmaf(raw[s * DP + tid], per_token[s].y, n);
+            nrm[tid] = n;
           }
-#pragma unroll
-          for (int i = 0; i < NP; ++i) nv[i] = moved[i];
-          sb_bar<2, P::PREP_THREADS>();                                        // M is whole
           if (lane < TPW) {
             const int tt = TPW * pw + lane, tok = w.t_begin + b * T + tt;
             const float4 pt = per_token[tt];
@@ -359,13 +376,7 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
       __syncthreads();
     }
     cp_async_wait<0>();
-    if (norm && pw == 0) {
-#pragma unroll
-      for (int i = 0; i < NP; ++i) {
-        const float2 x = unpack2(nv[i]);
-        *reinterpret_cast<float2*>(w.state + static_cast<int64_t>(a.vdim) * DP + lane * 2 * NP + 2 * i) = x;
-      }
-    }
+    if (norm && tid < DP) w.state[static_cast<int64_t>(a.vdim) * DP + tid] = nrm[tid];
     if (MLSTM && tid == 0) {
       // the copies of the running maximum of this CTA's columns; the normaliser's belongs to the first CTA
       for (int i = block0; i < blocks16 && i * kScanBlockCols < w.col0 + COLS && i * kScanBlockCols < a.vdim; ++i) mstate[i] = run_max;
@@ -395,8 +406,8 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
     const float4* per_token = reinterpret_cast<const float4*>(prep + P::P_T);
     // products with the state in front of the block: of a token's k and q (delta), or of two tokens' q, per exchange
     constexpr int ROWS = DELTA ? 2 * T : T;
-    constexpr int AHEAD = CPT <= 2 ? 8 : 2;      // chains of sums over lanes in flight, as registers allow
-#pragma unroll AHEAD
+    float totals[ROWS / 2];
+#pragma unroll
     for (int r = 0; r < ROWS; r += 2) {
       const float* x0 = DELTA ? prep + (r >> 1) * DP + l16 * 4 : raw + P::RAW_Q + r * DP + l16 * 4;
       const float* x1 = DELTA ? prep + P::P_QH + (r >> 1) * DP + l16 * 4 : x0 + DP;
@@ -422,16 +433,27 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
         v[i] = sum2(acc[0][i]);
         v[CPT + i] = sum2(acc[1][i]);
       }
-      const float total = sb_reduce16<2 * CPT>(v, l16);
+      totals[r / 2] = sb_reduce16<2 * CPT>(v, l16);
+    }
+    {
       constexpr int PER = 16 / (2 * CPT);                // lanes that hold the same sum
       const int at = l16 / PER, which = at / CPT, i = at % CPT;
-      if (l16 % PER == 0) R[DELTA ? (which * T + (r >> 1)) * COLS + col + i : (r + which) * COLS + col + i] = total;
+      if (l16 % PER == 0) {
+#pragma unroll
+        for (int r = 0; r < ROWS; r += 2) R[DELTA ? (which * T + (r >> 1)) * COLS + col + i : (r + which) * COLS + col + i] = totals[r / 2];
+      }
     }
     if (!DELTA) {
-      for (int i = threadIdx.x; i < T * COLS; i += MAIN) {
-        const float u = raw[P::RAW_V + i] * per_token[i / COLS].y;
-        *reinterpret_cast<float2*>(U + 2 * i) = make_float2(u, u);
+      constexpr int N = (T * COLS + MAIN - 1) / MAIN;
+      float u[N];
+#pragma unroll
+      for (int n = 0; n < N; ++n) {
+        const int i = min(static_cast<int>(threadIdx.x) + n * MAIN, T * COLS - 1);
+        u[n] = raw[P::RAW_V + i] * per_token[i / COLS].y;
       }
+#pragma unroll
+      for (int n = 0; n < N; ++n)
+        if (threadIdx.x + n * MAIN < T * COLS) *reinterpret_cast<float2*>(U + 2 * (threadIdx.x + n * MAIN)) = make_float2(u[n], u[n]);
     }
     sb_bar<1, MAIN>();
     if (DELTA) {
@@ -446,8 +468,9 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
           for (int c = j / 4; c < T / 4; ++c) *reinterpret_cast<float4*>(l + 4 * c) = *reinterpret_cast<const float4*>(prep + P::P_L + j * T + 4 * c);
 #pragma unroll
           for (int t = j + 1; t < T; ++t) u[t] = fmaf(-l[t], u[j], u[t]);
-          *reinterpret_cast<float2*>(U + 2 * (j * COLS + threadIdx.x)) = make_float2(u[j], u[j]);
         }
+#pragma unroll
+        for (int j = 0; j < T; ++j) *reinterpret_cast<float2*>(U + 2 * (j * COLS + threadIdx.x)) = make_float2(u[j], u[j]);
       }
       sb_bar<1, MAIN>();
     }
@@ -495,9 +518,11 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
       float x[T];
 #pragma unroll
       for (int j = 0; j < T; ++j) x[j] = DELTA ? U[2 * (j * COLS + c)] : raw[P::RAW_V + j * COLS + c];
+      constexpr int N = T / STEP;
+      float out[N];
 #pragma unroll
-      for (int t = first; t < T; t += STEP) {
-        const int tok = w.t_begin + b * T + t;
+      for (int n = 0; n < N; ++n) {
+        const int t = first + n * STEP;
         float m[T], o = DELTA ? R[(T + t) * COLS + c] : R[t * COLS + c] * per_token[t].x;
 #pragma unroll
         for (int j = 0; j < T; j += 4) *reinterpret_cast<float4*>(m + j) = *reinterpret_cast<const float4*>(prep + P::P_M + t * T + j);
@@ -505,7 +530,12 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
         for (int j = 0; j < T; ++j)
           if (j <= t) o = fmaf(m[j], x[j], o);      // not behind t, where a value may be anything
         if (MODE == kScanDecay) o = fmaf(skip, raw[P::RAW_V + t * COLS + c], o);
-        if (tok < w.t_end && w.col0 + c < a.vdim) a.out[(static_cast<int64_t>(tok) * a.heads + w.head) * a.vdim + w.col0 + c] = o;
+        out[n] = o;
+      }
+#pragma unroll
+      for (int n = 0; n < N; ++n) {
+        const int tok = w.t_begin + b * T + first + n * STEP;
+        if (tok < w.t_end && w.col0 + c < a.vdim) a.out[(static_cast<int64_t>(tok) * a.heads + w.head) * a.vdim + w.col0 + c] = out[n];
       }
     }
     __syncthreads();
