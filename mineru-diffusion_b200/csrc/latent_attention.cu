@@ -105,25 +105,46 @@ __global__ void __launch_bounds__(128) latent_attn_rows_kernel(const LatentArgs 
     if (c < a.width) qv[i] = act_load4(q + c);
   }
   float m = -INFINITY, l = 0.f;
-  for (int key = warp; key <= pos; key += 4) {
-    const T* kr = static_cast<const T*>(a.cache) + latent_slot(a, table, key) * a.width;
-    float4 kv[NV];
-    float s = 0.f;
+  // several keys at a time, as registers allow: their rows are in flight together and share a new maximum
+  constexpr int KEYS = NV <= 2 ? 4 : NV <= 4 ? 2 : 1;
+  for (int key = warp; key <= pos; key += 4 * KEYS) {
+    float4 kv[KEYS][NV];
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      kv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      const int c = (lane + 32 * i) * 4;
-      if (c < a.width) kv[i] = act_load4(kr + c);
-      s += qv[i].x * kv[i].x + qv[i].y * kv[i].y + qv[i].z * kv[i].z + qv[i].w * kv[i].w;
+    for (int j = 0; j < KEYS; ++j) {
+      const T* kr = static_cast<const T*>(a.cache) + latent_slot(a, table, min(key + 4 * j, pos)) * a.width;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        kv[j][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        const int c = (lane + 32 * i) * 4;
+        if (c < a.width) kv[j][i] = act_load4(kr + c);
+      }
     }
-    s = warp_sum(s) * a.scale_log2;
-    const float m_new = fmaxf(m, s), f = exp2f(m - m_new), p = exp2f(s - m_new);
-    m = m_new;
-    l = l * f + p;
+    float s[KEYS], m_new = m;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      o[i].x = fmaf(p, kv[i].x, o[i].x * f); o[i].y = fmaf(p, kv[i].y, o[i].y * f);
-      o[i].z = fmaf(p, kv[i].z, o[i].z * f); o[i].w = fmaf(p, kv[i].w, o[i].w * f);
+    for (int j = 0; j < KEYS; ++j) {
+      s[j] = 0.f;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) s[j] += qv[i].x * kv[j][i].x + qv[i].y * kv[j][i].y + qv[i].z * kv[j][i].z + qv[i].w * kv[j][i].w;
+    }
+#pragma unroll
+    for (int j = 0; j < KEYS; ++j) {
+      s[j] = key + 4 * j <= pos ? warp_sum(s[j]) * a.scale_log2 : -INFINITY;
+      m_new = fmaxf(m_new, s[j]);
+    }
+    const float f = exp2f(m - m_new);
+    m = m_new;
+    l *= f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) { o[i].x *= f; o[i].y *= f; o[i].z *= f; o[i].w *= f; }
+#pragma unroll
+    for (int j = 0; j < KEYS; ++j) {
+      const float p = exp2f(s[j] - m);
+      l += p;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        o[i].x = fmaf(p, kv[j][i].x, o[i].x); o[i].y = fmaf(p, kv[j][i].y, o[i].y);
+        o[i].z = fmaf(p, kv[j][i].z, o[i].z); o[i].w = fmaf(p, kv[j][i].w, o[i].w);
+      }
     }
   }
   if (lane == 0) { sm[warp] = m; sl[warp] = l; }

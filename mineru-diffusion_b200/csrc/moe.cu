@@ -83,10 +83,11 @@ __global__ void __launch_bounds__(kRouteWarps * 32) moe_route_kernel(const mdb_m
 
 // One CTA.  counts -> first row of every expert (multiples of 128) -> tile list -> a row for every (token, k) pair.
 // The order of the rows of one expert is not fixed; every row's result is independent of its place.
-// Bound by the latency of its two walks over the ids, so a thread has kPlanBatch of them in flight (1 where there is no more than an
-// id per thread: 256 pairs 3.0 against 3.2 us).
-constexpr int kPlanThreads = 1024;
-template <int kPlanBatch>
+// Bound by latencies one behind the other: the ids, the counts, the rows.  With up to KEEP ids per thread the count that a pair
+// finds is its place among its expert's rows, and stays in a register with its expert: one walk over the ids and one over the rows'
+// list; beyond that (KEEP 0) the ids are read twice.  Rows that stay empty are marked by a warp per expert.
+constexpr int kPlanThreads = 1024, kPlanBatch = 8;
+template <int KEEP>
 __global__ void __launch_bounds__(kPlanThreads) moe_plan_kernel(const mdb_moe_plan_args a) {
   pdl_launch_dependents();
   pdl_wait();
@@ -94,16 +95,30 @@ __global__ void __launch_bounds__(kPlanThreads) moe_plan_kernel(const mdb_moe_pl
   int* count = plan_smem;              // [experts]
   int* first = plan_smem + a.experts;  // [experts]
   __shared__ int total_rows;
+  const int n = a.m * a.top;
+  int id[KEEP > 0 ? KEEP : 1], place[KEEP > 0 ? KEEP : 1];
+  if (KEEP > 0) {
+#pragma unroll
+    for (int b = 0; b < KEEP; ++b) {
+      const int i = static_cast<int>(threadIdx.x) + b * kPlanThreads;
+      id[b] = a.ids[min(i, n - 1)];
+      if (i >= n || id[b] < 0 || id[b] >= a.experts) id[b] = -1;
+    }
+  }
   for (int e = threadIdx.x; e < a.experts; e += kPlanThreads) count[e] = 0;
   __syncthreads();
-  const int n = a.m * a.top;
-  for (int i0 = threadIdx.x; i0 < n; i0 += kPlanThreads * kPlanBatch) {
-    int e[kPlanBatch];
+  if (KEEP > 0) {
 #pragma unroll
-    for (int b = 0; b < kPlanBatch; ++b) e[b] = i0 + b * kPlanThreads < n ? a.ids[i0 + b * kPlanThreads] : -1;
+    for (int b = 0; b < KEEP; ++b) place[b] = id[b] >= 0 ? atomicAdd(&count[id[b]], 1) : 0;
+  } else {
+    for (int i0 = threadIdx.x; i0 < n; i0 += kPlanThreads * kPlanBatch) {
+      int e[kPlanBatch];
 #pragma unroll
-    for (int b = 0; b < kPlanBatch; ++b)
-      if (e[b] >= 0 && e[b] < a.experts) atomicAdd(&count[e[b]], 1);
+      for (int b = 0; b < kPlanBatch; ++b) e[b] = i0 + b * kPlanThreads < n ? a.ids[i0 + b * kPlanThreads] : -1;
+#pragma unroll
+      for (int b = 0; b < kPlanBatch; ++b)
+        if (e[b] >= 0 && e[b] < a.experts) atomicAdd(&count[e[b]], 1);
+    }
   }
   __syncthreads();
   if (threadIdx.x < 32) {
@@ -118,12 +133,7 @@ __global__ void __launch_bounds__(kPlanThreads) moe_plan_kernel(const mdb_moe_pl
         const int v = __shfl_up_sync(0xffffffffu, incl, o);
         if (static_cast<int>(threadIdx.x) >= o) incl += v;
       }
-      if (e < a.experts) {
-        const int t0 = base + incl - tiles;
-        first[e] = t0 * kMoeTileRows;
-        for (int t = 0; t < tiles; ++t)
-          if (t0 + t < a.max_tiles) a.tile_expert[t0 + t] = e;
-      }
+      if (e < a.experts) first[e] = (base + incl - tiles) * kMoeTileRows;
       base += __shfl_sync(0xffffffffu, incl, 31);
     }
     if (threadIdx.x == 0) {
@@ -133,7 +143,24 @@ __global__ void __launch_bounds__(kPlanThreads) moe_plan_kernel(const mdb_moe_pl
   }
   __syncthreads();
   const int cap = a.max_tiles * kMoeTileRows;
-  for (int r = threadIdx.x; r < total_rows && r < cap; r += kPlanThreads) a.row_token[r] = -1;
+  // every expert's tiles, and the rows of its last one that stay empty
+  for (int e = threadIdx.x >> 5; e < a.experts; e += kPlanThreads / 32) {
+    const int r0 = first[e], r1 = r0 + count[e], r2 = r0 + (count[e] + kMoeTileRows - 1) / kMoeTileRows * kMoeTileRows;
+    for (int t = r0 / kMoeTileRows + (threadIdx.x & 31); t < r2 / kMoeTileRows && t < a.max_tiles; t += 32) a.tile_expert[t] = e;
+    for (int r = r1 + (threadIdx.x & 31); r < r2 && r < cap; r += 32) a.row_token[r] = -1;
+  }
+  if (KEEP > 0) {
+#pragma unroll
+    for (int b = 0; b < KEEP; ++b) {
+      const int i = static_cast<int>(threadIdx.x) + b * kPlanThreads;
+      int slot = id[b] >= 0 ? first[id[b]] + place[b] : -1;
+      if (slot >= cap) slot = -1;
+      if (slot >= 0) a.row_token[slot] = i / a.top;
+      if (i < n) a.slot[i] = slot;
+    }
+    return;
+  }
+  __syncthreads();
   for (int e = threadIdx.x; e < a.experts; e += kPlanThreads) count[e] = 0;
   __syncthreads();
   for (int i0 = threadIdx.x; i0 < n; i0 += kPlanThreads * kPlanBatch) {
@@ -163,14 +190,26 @@ __global__ void __launch_bounds__(128) moe_gather_kernel(const T* x, int64_t ldx
                                                          const int32_t* num_tiles) {
   pdl_launch_dependents();
   pdl_wait();
-  const int rows = *num_tiles * kMoeTileRows;
+  // a warp per row, eight pieces of 16 bytes in flight per lane, the next row's place read meanwhile
+  const int rows = *num_tiles * kMoeTileRows, lane = threadIdx.x & 31, step = gridDim.x * 4;
   const int chunks = width * static_cast<int>(sizeof(T)) / 16;
-  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
-    const int t = row_token[r];
-    if (t < 0) continue;                 // padding rows keep whatever they hold; nobody reads their results
-    const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<int64_t>(t) * ldx);
-    uint4* dst = reinterpret_cast<uint4*>(out + static_cast<int64_t>(r) * width);
-    for (int c = threadIdx.x; c < chunks; c += 128) dst[c] = src[c];
+  int r = blockIdx.x * 4 + (threadIdx.x >> 5);
+  int t = r < rows ? row_token[r] : -1;
+  for (; r < rows; r += step) {
+    const int next = r + step < rows ? row_token[r + step] : -1;
+    if (t >= 0) {                        // padding rows keep whatever they hold; nobody reads their results
+      const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<int64_t>(t) * ldx);
+      uint4* dst = reinterpret_cast<uint4*>(out + static_cast<int64_t>(r) * width);
+      for (int c0 = 0; c0 < chunks; c0 += 256) {
+        uint4 v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = src[min(c0 + 32 * i + lane, chunks - 1)];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (c0 + 32 * i + lane < chunks) dst[c0 + 32 * i + lane] = v[i];
+      }
+    }
+    t = next;
   }
 }
 
@@ -207,8 +246,10 @@ int mdb_moe_plan(const mdb_moe_plan_args* args, mdb_stream_t stream) {
   MDB_REQUIRE(a.m >= 0 && a.experts > 0 && a.top > 0 && a.max_tiles > 0, MDB_ERR_ARG);
   MDB_REQUIRE(a.ids && a.slot && a.row_token && a.tile_expert && a.num_tiles, MDB_ERR_ARG);
   MDB_REQUIRE(a.experts <= 4096 && static_cast<int64_t>(a.m) * a.top < (1 << 30), MDB_ERR_UNSUPPORTED);
-  return mdb_launch(a.m * a.top > kPlanThreads ? moe_plan_kernel<8> : moe_plan_kernel<1>, dim3(1), dim3(kPlanThreads), sizeof(int) * 2 * a.experts,
-                    static_cast<cudaStream_t>(stream), a);
+  const int each = (a.m * a.top + kPlanThreads - 1) / kPlanThreads;
+  void (*const kernel)(mdb_moe_plan_args) = each < 1 ? moe_plan_kernel<0> : each <= 1 ? moe_plan_kernel<1> : each <= 4 ? moe_plan_kernel<4> : each <= 12 ? moe_plan_kernel<12>
+                                            : each <= 24 ? moe_plan_kernel<24> : moe_plan_kernel<0>;
+  return mdb_launch(kernel, dim3(1), dim3(kPlanThreads), sizeof(int) * 2 * a.experts, static_cast<cudaStream_t>(stream), a);
 }
 
 int mdb_moe_gather(int dtype, const void* x, int64_t ldx, void* out, int width, const int32_t* row_token,

@@ -164,9 +164,15 @@ __global__ void __launch_bounds__(kRes32Threads) residual_norm_kernel(const mdb_
       }
       x.x += d.x; x.y += d.y; x.z += d.z; x.w += d.w;
     }
-    if (!POST) *reinterpret_cast<float4*>(res + c) = x;
     v[i] = x;
     ss += x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;      // columns past width hold zeros
+  }
+  if (!POST) {      // (behind all loads: each store would hold back the loads that follow it)
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = (threadIdx.x + i * kRes32Threads) * 4;
+      if (c < a.width_pad) *reinterpret_cast<float4*>(res + c) = v[i];
+    }
   }
   if (!POST && a.y == nullptr) return;
   T* y = static_cast<T*>(a.y) + row * a.ldy;
