@@ -18,7 +18,7 @@
 // the turns come one behind the other (sums of products with the state, u, outputs, scaled rows: 755 -> 665 us for the delta
 // rule below); places in memory are worked out once; the mLSTM's normaliser lies in shared memory, a channel per thread.
 // The scan alone, 2048 tokens, with those changes: mLSTM, 8 heads of 128 x 256, one, two and four sequences 315 / 350 / 469 -> 250 / 280 /
-// 412 us; delta rule, 16 heads of 128 x 128, 463 / 576 / 755 -> 370 / 530 / 644 us.  (Scalar FMAs for the products with the state: 682,
+// 412 us; delta rule, 16 heads of 128 x 128, 463 / 576 / 755 -> 370 / 500 / 639 us.  (Scalar FMAs for the products with the state: 682,
 // 444.  The same blocks on tcgen05, operands in three bf16 parts, 128 columns a CTA: 560 and 403, no better for up to 32 sequence heads.)
 constexpr int kSbTokens = 16, kSbRing = 3;
 
@@ -218,24 +218,26 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
           float acc[2][32];
 #pragma unroll
           for (int i = 0; i < NP; ++i) p[0][i] = p[1][i] = 0ull;
-          // (a branch for four tokens at a time: what lies in front of it is not fetched ahead)
+          // A branch for AT tokens at a time, whose loads go out together: four next to 16 columns, one next to more, where the
+          // other warps want the issue slots (64 columns 639 against 664 us for 4 x 2048 tokens, 16 columns 383 against 371 for 1 x 2048).
+          constexpr int AT = COLS == 16 ? 4 : 1;
 #pragma unroll
-          for (int t4 = 0; t4 < T; t4 += 4) {
-            if (t4 + 3 < j0) {
+          for (int t0 = 0; t0 < T; t0 += AT) {
+            if (t0 + AT - 1 < j0) {
 #pragma unroll
-              for (int i = 0; i < 8; ++i) acc[0][2 * t4 + i] = acc[1][2 * t4 + i] = 0.f;
+              for (int i = 0; i < 2 * AT; ++i) acc[0][2 * t0 + i] = acc[1][2 * t0 + i] = 0.f;
               continue;
             }
-            f32x2 k[4][NP], q[4][NP], g[4][NP];
+            f32x2 k[AT][NP], q[AT][NP], g[AT][NP];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              row_pairs(raw + (t4 + e) * DP, k[e]);
-              row_pairs(raw + P::RAW_Q + (t4 + e) * DP, q[e]);
-              row_pairs(raw + P::RAW_G + (t4 + e) * DP, g[e]);
+            for (int e = 0; e < AT; ++e) {
+              row_pairs(raw + (t0 + e) * DP, k[e]);
+              row_pairs(raw + P::RAW_Q + (t0 + e) * DP, q[e]);
+              row_pairs(raw + P::RAW_G + (t0 + e) * DP, g[e]);
             }
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const int t = t4 + e;
+            for (int e = 0; e < AT; ++e) {
+              const int t = t0 + e;
 #pragma unroll
               for (int jj = 0; jj < 2; ++jj) {
                 f32x2 l = 0ull, m = 0ull;
