@@ -14,8 +14,13 @@ from . import _lib
 _BF16 = torch.bfloat16
 
 
+# The handle of the calling thread's current stream.  torch.cuda.current_stream() builds a Stream object for it, a third of the host time
+# of a prompt step of 37 launches; this is where it gets the handle from.
+_device, _raw_stream = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
+
+
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_device())
 
 
 def _ptr(t: torch.Tensor | None) -> int | None:
