@@ -3,16 +3,14 @@
 // tiles of 128).  GLU: half of a tile's weight rows are gate rows, the other half the up rows n further.
 //
 // 8 x 8 outputs per thread, operands as they lie in memory (k contiguous): no transposing, 16-byte cp.async into a ring and
-// 16-byte reads out of it, 256 FMAs for 16 reads.  What bounds it: latency with two warps per scheduler (500 x 3072 x 1024: 95 us, 33
-// TFLOP/s, 0.45 of the FMA rate; a loop of 8 x 8 independent outputs reaches 114 FMA per cycle and SM scalar, 67 packed, which the
-// register file bounds).  Rows of a stage are 36 floats long: the eight lanes that read eight neighbouring rows meet eight
-// different groups of banks.
+// 16-byte reads out of it, 256 FMAs for 16 reads.  What bounds it: latency with two warps per scheduler, and the start and the end of
+// a k this short (500 x 1536 x 384: 27 us, 22 TFLOP/s; at k 1024 33; a loop of 8 x 8 independent outputs reaches 114 FMA per cycle and
+// SM scalar, 67 packed, which the register file bounds).  Rows of a stage are 36 floats long: the eight lanes that read eight
+// neighbouring rows meet eight different groups of banks.
 //
 // An output is the sum of four chains over the blocks of 32 k, block by block in turn, whatever the tile: a row's bits do not depend on
 // the other rows.  Where a CTA has four groups they take a chain each and add up in shared memory; one group runs the chains one
 // behind the other.  So a tile of 64 x 64 has 256 threads, and 500 rows x 1024 columns already give 128 CTAs.
-// A prompt of 500 tokens through three layers of width 1024, scans and attention included: 3.17 -> 1.51 ms, of 16 tokens 1.61 -> 0.63
-// ms.  (8 x 16 outputs per thread, a quarter fewer reads: 1.60 ms.)
 #include "mdb_common.cuh"
 
 namespace mdb {

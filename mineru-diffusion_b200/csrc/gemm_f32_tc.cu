@@ -14,10 +14,11 @@
 // warps add up.  Four chains over k, each a quarter of the chunks: a cluster of one, two or four CTAs shares them out, and they are
 // added in the same order whoever ran them, so that the bits of a row do not depend on the other rows.
 //
-// What bounds it: shared memory and L1, which share their 128 bytes a cycle: per chunk of 128 x 64 outputs the parts are written (72
-// KB) and read by the products (100 KB), and the operands come through L1 (48 KB, in and out): 2100 cycles, of which the products
-// themselves take 770.  500 rows, n x k 4352 x 1024: 117 us on FMAs -> 45; 1024 x 3072: 92 -> 35; 1024 x 1024: 33 -> 18; 16 rows
-// of the same: 13.0 -> 12.7, 20.7 -> 15.5, 7.9 -> 8.9.
+// What bounds it: bringing the operands in and turning them round.  A chunk of 128 x 64 outputs takes 2100 cycles, of which the
+// products need 770: its 48 KB come out of L2 (6 TB/s with all SMs), the parts are written to shared memory (72 KB) and read by the
+// products (100 KB).  500 rows, n x k 4352 x 1024, 45 us: without the loads 32, with a third of the parts' stores 35, without
+// splitting 41, without the products of a2 and a3 42.  On FMAs it took 117; 1024 x 3072: 92 -> 35; 1024 x 1024: 33 -> 18; 16
+// rows of the same: 13.0 -> 12.7, 20.7 -> 15.5, 7.9 -> 8.9.
 #include "mdb_common.cuh"
 
 namespace mdb {

@@ -85,7 +85,8 @@ __global__ void __launch_bounds__(kRouteWarps * 32) moe_route_kernel(const mdb_m
 // The order of the rows of one expert is not fixed; every row's result is independent of its place.
 // Bound by latencies one behind the other: the ids, the counts, the rows.  With up to KEEP ids per thread the count that a pair
 // finds is its place among its expert's rows, and stays in a register with its expert: one walk over the ids and one over the rows'
-// list; beyond that (KEEP 0) the ids are read twice.  Rows that stay empty are marked by a warp per expert.
+// list; beyond that (KEEP 0) the ids are read twice.  Rows that stay empty are marked by a warp per expert.  2048 tokens of six
+// of 64 experts: 12.2 us with two walks, 11.1.
 constexpr int kPlanThreads = 1024, kPlanBatch = 8;
 template <int KEEP>
 __global__ void __launch_bounds__(kPlanThreads) moe_plan_kernel(const mdb_moe_plan_args a) {
@@ -182,6 +183,8 @@ __global__ void __launch_bounds__(kPlanThreads) moe_plan_kernel(const mdb_moe_pl
   }
 }
 
+// Bound by memory and by a row's latencies, its place and its pieces.  2048 tokens of 4 KB to 12288 rows: 13.5 us with a CTA per row
+// and a piece in flight per thread, 10.8 now.
 // (No __restrict__ on these pointers: a load the compiler may treat as invariant, like *num_tiles, moves above
 // griddepcontrol.wait and then reads what the previous plan left.)
 template <typename T>

@@ -15,7 +15,7 @@
 // the same number of FMAs per token with half the dependent shuffle reductions; these products of keys and queries are
 // computed beforehand, with the decays.
 //
-// Long portions of few sequences with heads of up to 128 key channels go in blocks of 16 tokens instead (scan_blocks.cuh).
+// Portions of 32 tokens and more of few sequences with heads of up to 128 key channels go in blocks of 16 tokens instead (scan_blocks.cuh).
 //
 // The linear recurrence S <- a S + b k v^T, o = S^T q + skip v is the mLSTM's scan with its gates given and no normaliser.
 //

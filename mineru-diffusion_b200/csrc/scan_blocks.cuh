@@ -18,7 +18,7 @@
 // the turns come one behind the other (sums of products with the state, u, outputs, scaled rows: 755 -> 665 us for the delta
 // rule below); places in memory are worked out once; the mLSTM's normaliser lies in shared memory, a channel per thread.
 // The scan alone, 2048 tokens, with those changes: mLSTM, 8 heads of 128 x 256, one, two and four sequences 315 / 350 / 469 -> 250 / 280 /
-// 412 us; delta rule, 16 heads of 128 x 128, 463 / 576 / 755 -> 370 / 500 / 639 us.  (Scalar FMAs for the products with the state: 682,
+// 412 us; delta rule, 16 heads of 128 x 128, 463 / 576 / 755 -> 371 / 521 / 640 us.  (Scalar FMAs for the products with the state: 682,
 // 444.  The same blocks on tcgen05, operands in three bf16 parts, 128 columns a CTA: 560 and 403, no better for up to 32 sequence heads.)
 constexpr int kSbTokens = 16, kSbRing = 3;
 
@@ -218,9 +218,10 @@ __global__ void __launch_bounds__(SbPlan<MODE, DP, COLS, CPT>::THREADS, 1) scan_
           float acc[2][32];
 #pragma unroll
           for (int i = 0; i < NP; ++i) p[0][i] = p[1][i] = 0ull;
-          // A branch for AT tokens at a time, whose loads go out together: four next to 16 columns, one next to more, where the
-          // other warps want the issue slots (64 columns 639 against 664 us for 4 x 2048 tokens, 16 columns 383 against 371 for 1 x 2048).
-          constexpr int AT = COLS == 16 ? 4 : 1;
+          // A branch for AT tokens at a time, whose loads go out together: four next to 16 or 32 columns, one next to 64, where the
+          // other warps want the issue slots (4 x 2048 tokens 640 against 664 us; 2 x 2048, 32 columns, 539 against 521; 1 x 2048, 16
+          // columns, 383 against 371).
+          constexpr int AT = COLS == 64 ? 1 : 4;
 #pragma unroll
           for (int t0 = 0; t0 < T; t0 += AT) {
             if (t0 + AT - 1 < j0) {

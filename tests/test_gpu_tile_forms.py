@@ -225,3 +225,44 @@ def test_window_pairs(H, KH, D, window, portions, starts):
     got, ref = _window_case(H, KH, D, portions, starts, window, True)
     for i, (o, r) in enumerate(zip(got, ref)):
         assert rel(o, r) < 8e-3, i
+
+
+# Ids per thread of the plan: one, up to 4, 12 and 24 in registers, more in two walks; some pairs go nowhere.  Gathered rows of one piece, of
+# a warp's eight rounds of pieces, and of one more.  Whole numbers and copies: exact.
+@pytest.mark.parametrize("m,top,experts", [(1, 1, 3), (512, 2, 64), (513, 2, 40), (1024, 4, 64), (1366, 3, 7), (2048, 6, 64), (2049, 6, 64), (4096, 6, 160),
+                                           (4097, 6, 64)])
+def test_expert_plan_and_gather(m, top, experts):
+    ids = torch.rand(m, experts, generator=gen(m), device=DEV).topk(top, dim=1).indices.int()
+    ids[::97] = -1
+    tiles = ops.moe_max_tiles(m, top, experts)
+    slot, row_token = torch.full((m, top), -9, dtype=torch.int32, device=DEV), torch.full((tiles * 128,), -9, dtype=torch.int32, device=DEV)
+    tile_expert, num = torch.full((tiles,), -9, dtype=torch.int32, device=DEV), i32([0] * 4)
+    ops.moe_plan(ids, experts, tiles, slot, row_token, tile_expert, num)
+    counts = torch.bincount(ids[ids >= 0].long(), minlength=experts)
+    per = ((counts + 127) // 128).tolist()
+    used = sum(per)
+    assert int(num[0]) == used <= tiles and tile_expert[:used].tolist() == [e for e, n in enumerate(per) for _ in range(n)]
+    assert bool((slot[ids < 0] == -1).all()) and bool((slot[ids >= 0] >= 0).all())
+    flat, pairs = slot[ids >= 0].long(), (ids >= 0).nonzero()
+    assert len(flat.unique()) == len(flat)                                           # a row of its own for every pair
+    assert torch.equal(tile_expert[flat // 128], ids[ids >= 0]) and torch.equal(row_token[flat].long(), pairs[:, 0])
+    empty = torch.ones(used * 128, dtype=torch.bool, device=DEV)
+    empty[flat] = False
+    assert bool((row_token[:used * 128][empty] == -1).all())
+    for width in (8, 2048, 2056):
+        x = torch.randn(m, width + 8, generator=gen(1), device=DEV).to(BF)[:, :width]
+        xs = torch.full((tiles * 128, width), 3.0, dtype=BF, device=DEV)
+        ops.moe_gather(x, xs, row_token, num, tiles)
+        assert torch.equal(xs[flat], x[pairs[:, 0]]) and bool((xs[:used * 128][empty] == 3).all())
+
+
+# Several keys at a time (four, two, one by width): contexts that end inside a round of the four warps.  fp32 sums of up to 70 weights.
+@pytest.mark.parametrize("width", [256, 384, 1024])
+def test_fp32_latent_rows(width):
+    pos = [0, 1, 3, 4, 5, 11, 15, 16, 17, 31, 32, 63, 69]
+    q, cache = torch.randn(len(pos), 2, width, generator=gen(1), device=DEV) * 3, torch.randn(256, width, generator=gen(2), device=DEV)
+    out, ws = torch.zeros(len(pos), 2 * width, device=DEV), torch.empty(16, dtype=torch.uint8, device=DEV)
+    ops.latent_attn(q.view(len(pos), -1), cache, i32([[0]]), i32([0] * len(pos)), i32(pos), 2, width ** -0.5, out, 1, ws)
+    for i, p in enumerate(pos):
+        a = torch.softmax(q[i].double() @ cache[:p + 1].double().T * width ** -0.5, -1)
+        assert rel(out[i].view(2, width), a @ cache[:p + 1].double()) < 2e-6, p
