@@ -343,6 +343,9 @@ __global__ void __launch_bounds__(128) channel_decay_kernel(const mdb_decay_args
     const float rate = -expf(a.a_log[head]);
     float kq = 0.f, ck = 0.f, cq = 0.f;
     for (int c = lane * 4; c < a.dim_pad; c += 128) {
+      // everything asked for in front of the store, which might be to what the next load reads
+      const float4 k1 = *reinterpret_cast<const float4*>(k + c), q1 = *reinterpret_cast<const float4*>(q + c);
+      const float4 k0 = *reinterpret_cast<const float4*>((odd ? kp : k) + c);
       float xv[4], bv[4], r[4];
       if (VEC && c + 4 <= a.dim) {
         const float4 x4 = *reinterpret_cast<const float4*>(x + c), b4 = *reinterpret_cast<const float4*>(bias + c);
@@ -358,10 +361,8 @@ __global__ void __launch_bounds__(128) channel_decay_kernel(const mdb_decay_args
 #pragma unroll
       for (int i = 0; i < 4; ++i) r[i] = c + i < a.dim ? expf(rate * softplus_f(xv[i] + bv[i])) : 1.f;
       *reinterpret_cast<float4*>(g + c) = make_float4(r[0], r[1], r[2], r[3]);
-      const float4 k1 = *reinterpret_cast<const float4*>(k + c), q1 = *reinterpret_cast<const float4*>(q + c);
       kq += dot4(k1, q1);
       if (odd) {
-        const float4 k0 = *reinterpret_cast<const float4*>(kp + c);
         const float4 e = make_float4(r[0] * k0.x, r[1] * k0.y, r[2] * k0.z, r[3] * k0.w);
         ck += dot4(e, k1);
         cq += dot4(e, q1);
