@@ -4,7 +4,8 @@
 //
 //   latent_attn_tc_kernel    bf16, widths of 128 to 512 (latent_attention_tc.cu); parts of a context are merged by
 //                            latent_combine_kernel.
-//   latent_attn_rows_kernel  fp32, and widths the first kernel does not take: one CTA per (token, head), a warp per key.
+//   latent_attn_rows_kernel  fp32, and widths the first kernel does not take: one CTA per token and one to four heads, a
+//                            warp per key.
 #include "mdb_common.cuh"
 
 namespace mdb {
@@ -84,100 +85,178 @@ __global__ void __launch_bounds__(128) latent_combine_kernel(const LatentArgs a)
   }
 }
 
-// One CTA of four warps per (head, row); warp w takes keys w, w + 4, ...; a lane owns every 32nd float4 group of four
-// channels.  NV = channels per lane / 4.  What bounds it: every head reads the latents for itself, out of L2 (500 rows of 8 heads, width
-// 256: 1 GB, 116 us; 132 with one key at a time, whose row, sum over lanes and weight follow one another).
-template <typename T, int NV>
+// The sums over a warp's lanes of N values at once: lane v * 32 / N (and those up to the next) has value v.  The lanes' tree is the
+// same for every N.
+template <int N>
+__device__ __forceinline__ float lanes_sum(float (&v)[N], int lane) {
+  int bit = 16;
+#pragma unroll
+  for (int n = N / 2; n >= 1; n /= 2, bit /= 2) {
+    const bool up = lane & bit;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const float send = up ? v[i] : v[i + n];
+      v[i] = (up ? v[i + n] : v[i]) + __shfl_xor_sync(~0u, send, bit);
+    }
+  }
+  for (; bit >= 1; bit /= 2) v[0] += __shfl_xor_sync(~0u, v[0], bit);
+  return v[0];
+}
+
+// One CTA of four warps per (row, HEADS heads); warp w takes keys w, w + 4, ...; a lane owns every 32nd float4 group of four
+// channels.  NV = channels per lane / 4.  Several keys at a time, as registers allow: their rows are in flight together and share a
+// new maximum, and a lane works out the weight of one (head, key).  A head's bits do not depend on HEADS.
+// The longest contexts of a prompt, its last rows, go first.
+// What bounds it: few rows, the latency of a step (a row's place, its loads, the sums, the weights); many, issue slots (16 packed FMAs
+// and about 6 other instructions for a head's key of 256 channels).  500 rows of 8 heads, width 256, a prompt: one head at a time with a
+// sum and a weight per lane and key 112 us, out of L2; HEADS 1, 2, 4: 76, 57, 50.
+template <typename T, int NV, int HEADS>
 __global__ void __launch_bounds__(128) latent_attn_rows_kernel(const LatentArgs a) {
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ float sm[4], sl[4];
-  extern __shared__ float rows_o[];        // [4][width]
-  const int row = blockIdx.y, head = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int KEYS = NV <= 2 ? 4 : NV <= 4 ? 2 : 1, N = HEADS * KEYS, STEP = 32 / N;
+  __shared__ float sm[4][HEADS], sl[4][HEADS];
+  extern __shared__ float rows_o[];        // [4][HEADS][width]
+  const int row = a.m - 1 - blockIdx.y, head0 = blockIdx.x * HEADS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int pos = a.row_pos[row];
   if (pos < 0) return;
   const int32_t* table = a.table + static_cast<int64_t>(a.row_seq[row]) * a.table_stride;
-  const T* q = static_cast<const T*>(a.q) + (static_cast<int64_t>(row) * a.heads + head) * a.width;
-  float4 qv[NV], o[NV];
+  f32x2 qv[HEADS][NV][2], o[HEADS][NV][2];
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    qv[i] = o[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     const int c = (lane + 32 * i) * 4;
-    if (c < a.width) qv[i] = act_load4(q + c);
+#pragma unroll
+    for (int h = 0; h < HEADS; ++h) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c < a.width) v = act_load4(static_cast<const T*>(a.q) + (static_cast<int64_t>(row) * a.heads + min(head0 + h, a.heads - 1)) * a.width + c);
+      qv[h][i][0] = pack2(v.x, v.y);
+      qv[h][i][1] = pack2(v.z, v.w);
+      o[h][i][0] = o[h][i][1] = pack2(0.f, 0.f);
+    }
   }
+  const int mine = lane / STEP % KEYS;      // the key, of the KEYS of a step, whose weight this lane works out
   float m = -INFINITY, l = 0.f;
-  // several keys at a time, as registers allow: their rows are in flight together and share a new maximum
-  constexpr int KEYS = NV <= 2 ? 4 : NV <= 4 ? 2 : 1;
   for (int key = warp; key <= pos; key += 4 * KEYS) {
-    float4 kv[KEYS][NV];
+    f32x2 kv[KEYS][NV][2];
 #pragma unroll
     for (int j = 0; j < KEYS; ++j) {
       const T* kr = static_cast<const T*>(a.cache) + latent_slot(a, table, min(key + 4 * j, pos)) * a.width;
 #pragma unroll
       for (int i = 0; i < NV; ++i) {
-        kv[j][i] = make_float4(0.f, 0.f, 0.f, 0.f);
         const int c = (lane + 32 * i) * 4;
-        if (c < a.width) kv[j][i] = act_load4(kr + c);
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (c < a.width) v = act_load4(kr + c);
+        kv[j][i][0] = pack2(v.x, v.y);
+        kv[j][i][1] = pack2(v.z, v.w);
       }
     }
-    float s[KEYS], m_new = m;
+    float s[N];
 #pragma unroll
-    for (int j = 0; j < KEYS; ++j) {
-      s[j] = 0.f;
+    for (int h = 0; h < HEADS; ++h)
 #pragma unroll
-      for (int i = 0; i < NV; ++i) s[j] += qv[i].x * kv[j][i].x + qv[i].y * kv[j][i].y + qv[i].z * kv[j][i].z + qv[i].w * kv[j][i].w;
-    }
+      for (int j = 0; j < KEYS; ++j) {
+        f32x2 t = pack2(0.f, 0.f);
 #pragma unroll
-    for (int j = 0; j < KEYS; ++j) {
-      s[j] = key + 4 * j <= pos ? warp_sum(s[j]) * a.scale_log2 : -INFINITY;
-      m_new = fmaxf(m_new, s[j]);
-    }
+        for (int i = 0; i < NV; ++i) {
+          t = fma2(qv[h][i][0], kv[j][i][0], t);
+          t = fma2(qv[h][i][1], kv[j][i][1], t);
+        }
+        const float2 u = unpack2(t);
+        s[h * KEYS + j] = u.x + u.y;
+      }
+    float w = lanes_sum<N>(s, lane) * a.scale_log2;
+    w = key + 4 * mine <= pos ? w : -INFINITY;
+    float m_new = w;
+#pragma unroll
+    for (int b = STEP; b < STEP * KEYS; b *= 2) m_new = fmaxf(m_new, __shfl_xor_sync(~0u, m_new, b));
+    m_new = fmaxf(m_new, m);
     const float f = exp2f(m - m_new);
     m = m_new;
-    l *= f;
+    w = exp2f(w - m);
+    l = l * f + w;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) { o[i].x *= f; o[i].y *= f; o[i].z *= f; o[i].w *= f; }
-#pragma unroll
-    for (int j = 0; j < KEYS; ++j) {
-      const float p = exp2f(s[j] - m);
-      l += p;
+    for (int h = 0; h < HEADS; ++h) {
+      const float fs = N == 1 ? f : __shfl_sync(~0u, f, h * KEYS * STEP);
+      const f32x2 fh = pack2(fs, fs);
 #pragma unroll
       for (int i = 0; i < NV; ++i) {
-        o[i].x = fmaf(p, kv[j][i].x, o[i].x); o[i].y = fmaf(p, kv[j][i].y, o[i].y);
-        o[i].z = fmaf(p, kv[j][i].z, o[i].z); o[i].w = fmaf(p, kv[j][i].w, o[i].w);
+        o[h][i][0] = mul2(o[h][i][0], fh);
+        o[h][i][1] = mul2(o[h][i][1], fh);
+      }
+#pragma unroll
+      for (int j = 0; j < KEYS; ++j) {
+        const float ps = N == 1 ? w : __shfl_sync(~0u, w, (h * KEYS + j) * STEP);
+        const f32x2 p = pack2(ps, ps);
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+          o[h][i][0] = fma2(p, kv[j][i][0], o[h][i][0]);
+          o[h][i][1] = fma2(p, kv[j][i][1], o[h][i][1]);
+        }
       }
     }
   }
-  if (lane == 0) { sm[warp] = m; sl[warp] = l; }
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int c = (lane + 32 * i) * 4;
-    if (c < a.width) *reinterpret_cast<float4*>(rows_o + warp * a.width + c) = o[i];
-  }
+  for (int b = STEP; b < STEP * KEYS; b *= 2) l += __shfl_xor_sync(~0u, l, b);
+  if (lane % (STEP * KEYS) == 0) { sm[warp][lane / (STEP * KEYS)] = m; sl[warp][lane / (STEP * KEYS)] = l; }
+#pragma unroll
+  for (int h = 0; h < HEADS; ++h)
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = (lane + 32 * i) * 4;
+      const float2 lo = unpack2(o[h][i][0]), hi = unpack2(o[h][i][1]);
+      if (c < a.width) *reinterpret_cast<float4*>(rows_o + (warp * HEADS + h) * a.width + c) = make_float4(lo.x, lo.y, hi.x, hi.y);
+    }
   __syncthreads();
-  const float mx = fmaxf(fmaxf(sm[0], sm[1]), fmaxf(sm[2], sm[3]));
-  float w[4], total = 0.f;
+  T* out = static_cast<T*>(a.out) + (static_cast<int64_t>(row) * a.heads + head0) * a.width;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    w[i] = sm[i] == -INFINITY ? 0.f : exp2f(sm[i] - mx);
-    total += w[i] * sl[i];
+  for (int h = 0; h < HEADS; ++h) {
+    if (head0 + h >= a.heads) break;
+    const float mx = fmaxf(fmaxf(sm[0][h], sm[1][h]), fmaxf(sm[2][h], sm[3][h]));
+    float w[4], total = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      w[i] = sm[i][h] == -INFINITY ? 0.f : exp2f(sm[i][h] - mx);
+      total += w[i] * sl[i][h];
+    }
+    const float* ro = rows_o + h * a.width;
+    const int part = HEADS * a.width;
+    for (int c = threadIdx.x; c < a.width; c += 128)
+      out[h * a.width + c] = act_from_f<T>((w[0] * ro[c] + w[1] * ro[part + c] + w[2] * ro[2 * part + c] + w[3] * ro[3 * part + c]) / total);
   }
-  T* out = static_cast<T*>(a.out) + (static_cast<int64_t>(row) * a.heads + head) * a.width;
-  for (int c = threadIdx.x; c < a.width; c += 128)
-    out[c] = act_from_f<T>((w[0] * rows_o[c] + w[1] * rows_o[a.width + c] + w[2] * rows_o[2 * a.width + c] + w[3] * rows_o[3 * a.width + c]) / total);
 }
 
 template <int WIDTH> static int latent_tc_launch(const LatentArgs& a, cudaStream_t st);      // latent_attention_tc.cu
 
+template <typename T, int NV, int HEADS>
+static int latent_rows_form(const LatentArgs& a, cudaStream_t st) {
+  return mdb_launch(latent_attn_rows_kernel<T, NV, HEADS>, dim3((a.heads + HEADS - 1) / HEADS, a.m), dim3(128),
+                    4 * sizeof(float) * HEADS * a.width, st, a);
+}
+
+// How many heads share the reading of a key: as many as leave the chip full (heads of 256 channels, us with 1, 2, 4 of them; two where
+// that leaves an SM a CTA, four where it leaves three).
+//   prompt of 500 rows, 8 heads   76   57   50        64 rows behind 3000 keys, 16 heads   233  228  250
+//   prompt of 250, 16 heads       42   32   30        128 behind 2000, 16 heads            296  266  272
+//   prompt of 137, 8 heads        12   12   12        8 behind 2000, 8 heads                83   87  103
+// Heads of 512 channels: 300 rows of 16 heads, a prompt, 100, 86, 77; 40 rows behind 2000 keys 232, 241, 282: two are never the best by
+// much.  Behind 512 channels registers leave no room for a second head (200 rows of 16 heads of 640 channels 90, 101).
+template <typename T, int NV>
+static int latent_rows_few(const LatentArgs& a, cudaStream_t st) {
+  const int64_t sms = at_sm_count(), m = a.m;
+  if (m * (a.heads / 4) >= 3 * sms) return latent_rows_form<T, NV, 4>(a, st);
+  if constexpr (NV < 4) {
+    if (m * (a.heads / 2) >= sms) return latent_rows_form<T, NV, 2>(a, st);
+  }
+  return latent_rows_form<T, NV, 1>(a, st);
+}
+
 template <typename T>
 static int launch_latent_rows(const LatentArgs& a, cudaStream_t st) {
-  const dim3 grid(a.heads, a.m);
-  const size_t smem = 4 * sizeof(float) * a.width;
-  if (a.width <= 128) return mdb_launch(latent_attn_rows_kernel<T, 1>, grid, dim3(128), smem, st, a);
-  if (a.width <= 256) return mdb_launch(latent_attn_rows_kernel<T, 2>, grid, dim3(128), smem, st, a);
-  if (a.width <= 512) return mdb_launch(latent_attn_rows_kernel<T, 4>, grid, dim3(128), smem, st, a);
-  if (a.width <= 1024) return mdb_launch(latent_attn_rows_kernel<T, 8>, grid, dim3(128), smem, st, a);
-  if (a.width <= 2048) return mdb_launch(latent_attn_rows_kernel<T, 16>, grid, dim3(128), smem, st, a);
+  if (a.width <= 128) return latent_rows_few<T, 1>(a, st);
+  if (a.width <= 256) return latent_rows_few<T, 2>(a, st);
+  if (a.width <= 512) return latent_rows_few<T, 4>(a, st);
+  if (a.width <= 1024) return latent_rows_form<T, 8, 1>(a, st);
+  if (a.width <= 2048) return latent_rows_form<T, 16, 1>(a, st);
   return MDB_ERR_UNSUPPORTED;
 }
 

@@ -266,3 +266,25 @@ def test_fp32_latent_rows(width):
     for i, p in enumerate(pos):
         a = torch.softmax(q[i].double() @ cache[:p + 1].double().T * width ** -0.5, -1)
         assert rel(out[i].view(2, width), a @ cache[:p + 1].double()) < 2e-6, p
+
+
+# One, two and four heads per reading of a key (by the number of rows and heads; three leave a group short): a row's bits are the same in
+# each, its error that of fp32 sums.  The row alone takes one head at a time.
+@pytest.mark.parametrize("m,heads,width", [(460, 4, 256), (460, 5, 96), (460, 6, 512), (160, 3, 256), (150, 3, 200)])
+@pytest.mark.parametrize("dtype", [torch.float32, BF])
+def test_latent_rows_of_several_heads(m, heads, width, dtype):
+    if dtype == BF and width in (256, 512):
+        pytest.skip("a width of the tensor-core form")
+    q = (torch.randn(m, heads * width, generator=gen(1), device=DEV) * 3).to(dtype)
+    cache = torch.randn(512, width, generator=gen(2), device=DEV).to(dtype)
+    pos, table = i32([-1 if r == 7 else r for r in range(m)]), i32([[1, 0]])
+    out, ws = torch.full((m, heads * width), 5.0, dtype=dtype, device=DEV), torch.empty(16, dtype=torch.uint8, device=DEV)
+    ops.latent_attn(q, cache, table, i32([0] * m), pos, heads, width ** -0.5, out, 1, ws)
+    rows = torch.cat([cache[256:], cache[:256]]).double()
+    for r in (0, 1, 17, 255, m - 1):
+        r, one = min(r, m - 1), torch.zeros(1, heads * width, dtype=dtype, device=DEV)
+        ops.latent_attn(q[r:r + 1], cache, table, i32([0]), pos[r:r + 1].contiguous(), heads, width ** -0.5, one, 1, ws)
+        assert torch.equal(one[0], out[r]), r
+        a = torch.softmax(q[r].view(heads, width).double() @ rows[:r + 1].T * width ** -0.5, -1)
+        assert rel(out[r].view(heads, width), a @ rows[:r + 1]) < (2e-6 if dtype == torch.float32 else 4e-3), r
+    assert bool((out[7] == 5).all())
