@@ -2,22 +2,28 @@
 // expert, and GLU (half of a tile's weight rows are gate rows, the other half the up rows n further).
 //
 // A number of 24 significant bits is the exact sum of three bf16 numbers (split3), so with a_i b_j exact in fp32
-//   a b = a1 b1 + (a1 b2 + a2 b1) + (a1 b3 + a2 b2 + a3 b1) + terms below 2^-24 of a b,
-// six products on the tensor cores.  The sums by size go to accumulators of their own, and those of a1 b1, where the tensor cores'
-// cutting off would show, end every 64 k and are added up in fp32 by threads.  Against 64 bits, normal numbers, k 1024 / 3072 / 6144:
-// 1.3e-7 / 1.5e-7 / 1.6e-7 of the result, where chains of FMAs have 2.9e-7 / 5.0e-7 / 7.0e-7 (k 128: 1.2e-7 and 1.1e-7).  A result
-// that is not finite is computed again by FMAs: its parts may be of either sign, or infinity times zero.
+//   a b = a1 b1 + (a1 b2 + a2 b1) + (a1 b3 + a2 b2 + a3 b1) + (a2 b3 + a3 b2) + a3 b3,
+// of which the last, below 2^-30 of a b, is left out: eight products on the tensor cores.  (The parts are cut off, not rounded, so
+// those of size 2^-24 reach 2^-21 of a b, all of its sign.)  The sums by size go to accumulators of their own, and those of a1 b1,
+// where the tensor cores' cutting off would show, end every 64 k and are added up in fp32 by threads.  The small ones are added to
+// one another before they meet a large one: a row with a single number that is not zero has the error of one rounding.
+// Error of an output in 2^-24 of the sum of |a b|, largest and root mean square, beside chains of FMAs, k 768 / 1024 / 3072:
+//   normal numbers   0.52, 0.085 (1.6, 0.24) / 0.48, 0.076 (1.8, 0.24) / 0.31, 0.052 (1.5, 0.24)
+//   their sizes      4.0, 1.5 (7.7, 1.7) / 4.1, 1.6 (8.8, 2.1) / 4.4, 1.8 (13, 3.2): sums of one sign, cut off at every step
+//   16 not zero      1.9, 0.30 (2.9, 0.37) / 1.9, 0.30 (2.4, 0.37) / 2.1, 0.31 (2.2, 0.38)
+//   one not zero     0.99, 0.42 and the same for FMAs
+// A result that is not finite is computed again by FMAs: its parts may be of either sign, or infinity times zero.
 //
 // Tile: 128 weight rows (the left operand) x 32 or 64 rows of x, k in chunks of 64.  Eight warps fetch rows of fp32 into registers a
 // chunk ahead and leave their three parts in shared memory (K-major, 128-byte swizzle; the three parts of x one behind the
-// other, so that one product takes a1 with b1 | b2 | b3, one a2 with b1 | b2, one a3 with b1), a warp issues the products, four
-// warps add up.  Four chains over k, each a quarter of the chunks: a cluster of one, two or four CTAs shares them out, and they are
+// other, so that one product takes a1 or a2 with b1 | b2 | b3, one a3 with b1 | b2), a warp issues the products, four warps add up.
+// A chunk's small products go first: they wait for nothing, and meanwhile the chunk before's sums of a1 b1 are read.  Four chains over k, each a quarter of the chunks: a cluster of one, two or four CTAs shares them out, and they are
 // added in the same order whoever ran them, so that the bits of a row do not depend on the other rows.
 //
 // What bounds it: bringing the operands in and turning them round.  A chunk of 128 x 64 outputs takes 2100 cycles, of which the
-// products need 770: its 48 KB come out of L2 (6 TB/s with all SMs), the parts are written to shared memory (72 KB) and read by the
-// products (100 KB).  500 rows, n x k 4352 x 1024, 45 us: without the loads 32, with a third of the parts' stores 35, without
-// splitting 41, without the products of a2 and a3 42.  On FMAs it took 117; 1024 x 3072: 92 -> 35; 1024 x 1024: 33 -> 18; 16
+// products need 1030: its 48 KB come out of L2 (6 TB/s with all SMs), the parts are written to shared memory (72 KB) and read by the
+// products (116 KB).  500 rows, n x k 4352 x 1024, 45 us with eight products and with six; with six 32 without the loads, 35 with a
+// third of the parts' stores, 41 without splitting.  On FMAs it took 117; 1024 x 3072: 92 -> 35; 1024 x 1024: 33 -> 18; 16
 // rows of the same: 13.0 -> 12.7, 20.7 -> 15.5, 7.9 -> 8.9.
 #include "mdb_common.cuh"
 
@@ -31,11 +37,11 @@ struct FtPlan {
   static constexpr int kPartA = kFtRows * 128, kPartB = BN * 128, kStage = 3 * (kPartA + kPartB), kStages = 3;
   static constexpr int kSlot = kFtRows * BN * 4;                     // a chain's sums on their way to the other CTAs of the cluster
   static constexpr int kOffBars = kStages * kStage, kBytes = 1024 + kOffBars + 128;
-  // tensor memory: a1 b1 | of size 2^-8 | of size 2^-16, for even and for odd chunks of a chain; sums of the chain before
-  static constexpr uint32_t kSet = 3 * BN, kSum = 6 * BN;
-  static_assert(2 * kSlot <= kStages * kStage && kBytes <= 227 * 1024 && 7 * BN <= 512, "memory of the fp32 product");
+  // tensor memory: a1 b1 of a chunk | of size 2^-8 | of size 2^-16 | of size 2^-24 of a chain | sums of the chains before
+  static constexpr uint32_t kSum = 4 * BN;
+  static_assert(2 * kSlot <= kStages * kStage && kBytes <= 227 * 1024 && 5 * BN <= 512, "memory of the fp32 product");
 };
-enum { kFtFull = 0, kFtEmpty = 3, kFtDFull = 6, kFtDEmpty = 8, kFtBars = 10 };
+enum { kFtFull = 0, kFtEmpty = 3, kFtDFull = 6, kFtDEmpty = 7, kFtBars = 8 };
 
 __device__ __align__(32) const float kFtZeros[8] = {};
 // Eight floats, in one load where they lie on a boundary of 32 bytes (two of 16 bytes read every 32-byte sector twice)
@@ -137,37 +143,37 @@ __global__ void __launch_bounds__(kFtThreads, 1) gemm_f32_tc_kernel(const mdb_ge
     // ---------------------------------------------------------------- products
     const uint32_t tmem = ready();
     const uint32_t id1 = umma_idesc_bf16(BN), id2 = umma_idesc_bf16(2 * BN), id3 = umma_idesc_bf16(3 * BN);
-    uint32_t phase = 0, d_phase = 0;      // a bit per stage, per set
+    uint32_t phase = 0, used = 0;      // a bit per stage; chunks so far
     int stage = 0;
     for (int c = chain0; c < chain1; ++c) {
       const int c0 = first_of(c), c1 = live ? first_of(c + 1) : c0;
       for (int i = c0; i < c1; ++i) {
-        const int set = (i - c0) & 1;
-        const uint32_t d = tmem + set * P::kSet;
-        wait(kFtDEmpty + set, (d_phase >> set & 1u) ^ 1u);
+        if (i == c0) wait(kFtDEmpty, (used & 1u) ^ 1u);      // the small sums of the chain before have been read
         wait(kFtFull + stage, phase >> stage & 1u);
         __syncwarp();
         tc_fence_after();
         if (misc[1] != 0) break;
-        const uint32_t at = base + stage * P::kStage, bt = at + 3 * P::kPartA;
-        const bool fresh = i - c0 < 2;
+        const uint32_t at = base + stage * P::kStage;
+        const uint64_t b1 = umma_desc_sw128(at + 3 * P::kPartA);
+        const uint64_t a1 = umma_desc_sw128(at), a2 = umma_desc_sw128(at + P::kPartA), a3 = umma_desc_sw128(at + 2 * P::kPartA);
 #pragma unroll
         for (int s = 0; s < kFtK / 16; ++s) {
-          const uint64_t b = umma_desc_sw128(bt) + 2 * s;
-          const uint64_t a1 = umma_desc_sw128(at) + 2 * s, a2 = umma_desc_sw128(at + P::kPartA) + 2 * s, a3 = umma_desc_sw128(at + 2 * P::kPartA) + 2 * s;
-          if (s == 0) {
-            umma_bf16_w(d, a1, b, id1, 0u);
-            umma_bf16_w(d + BN, a1, b + (P::kPartB >> 4), id2, fresh ? 0u : 1u);
-          } else {
-            umma_bf16_w(d, a1, b, id3, 1u);
-          }
-          umma_bf16_w(d + BN, a2, b, id2, 1u);
-          umma_bf16_w(d + 2 * BN, a3, b, id1, 1u);
+          umma_bf16_w(tmem + BN, a2 + 2 * s, b1 + 2 * s, id3, i == c0 && s == 0 ? 0u : 1u);
+          umma_bf16_w(tmem + 2 * BN, a3 + 2 * s, b1 + 2 * s, id2, 1u);
         }
+        if (i > c0) {      // the chunk before's sums of a1 b1 have been read
+          wait(kFtDEmpty, (used & 1u) ^ 1u);
+          __syncwarp();
+          tc_fence_after();
+        }
+        umma_bf16_w(tmem, a1, b1, id1, 0u);
+        umma_bf16_w(tmem + BN, a1, b1 + (P::kPartB >> 4), id2, 1u);
+#pragma unroll
+        for (int s = 1; s < kFtK / 16; ++s) umma_bf16_w(tmem, a1 + 2 * s, b1 + 2 * s, id3, 1u);
         umma_commit_w(bars + 8 * (kFtEmpty + stage));
-        umma_commit_w(bars + 8 * (kFtDFull + set));
+        umma_commit_w(bars + 8 * kFtDFull);
         phase ^= 1u << stage;
-        d_phase ^= 1u << set;
+        ++used;
         stage = stage + 1 == P::kStages ? 0 : stage + 1;
       }
     }
@@ -225,7 +231,7 @@ __global__ void __launch_bounds__(kFtThreads, 1) gemm_f32_tc_kernel(const mdb_ge
     // ---------------------------------------------------------------------- sums
     const uint32_t lanes = ready() + (static_cast<uint32_t>(32 * warp) << 16);
     float acc[BN];
-    uint32_t d_phase = 0;
+    uint32_t used = 0;
     bool parked = false;
     auto add = [&](uint32_t col) {
 #pragma unroll
@@ -238,24 +244,39 @@ __global__ void __launch_bounds__(kFtThreads, 1) gemm_f32_tc_kernel(const mdb_ge
         for (int e = 0; e < 32; ++e) acc[j + e] += d[e / 16][e % 16];
       }
     };
+    auto add_small = [&]() {      // a chain's small sums, smallest first
+#pragma unroll
+      for (int j = 0; j < BN; j += 16) {
+        float t[16], u[16];
+        tmem_ld16(lanes + 3 * BN + j, t);
+        tmem_ld16(lanes + 2 * BN + j, u);
+        tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 16; ++e) t[e] += u[e];
+        tmem_ld16(lanes + BN + j, u);
+        tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 16; ++e) acc[j + e] += t[e] + u[e];
+      }
+    };
     for (int c = chain0; c < chain1; ++c) {
       const int c0 = first_of(c), c1 = live ? first_of(c + 1) : c0;
       if (c1 <= c0) continue;
 #pragma unroll
       for (int j = 0; j < BN; ++j) acc[j] = 0.f;
       for (int i = c0; i < c1; ++i) {
-        const int set = (i - c0) & 1;
-        wait(kFtDFull + set, d_phase >> set & 1u);
+        wait(kFtDFull, used & 1u);
         __syncwarp();
         tc_fence_after();
-        // with its last products in a chain a set's small terms, smallest first; at the end the chains before
-        const int adds = i < c1 - 2 ? 1 : 3 + (i == c1 - 1 && rank == 0 && parked ? 1 : 0);
-#pragma unroll 1
-        for (int n = 0; n < adds; ++n) add(n == 3 ? P::kSum : set * P::kSet + (3 - n) % 3 * BN);
+        add(0);
+        if (i == c1 - 1) {
+          add_small();
+          if (rank == 0 && parked) add(P::kSum);
+        }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bars + 8 * (kFtDEmpty + set));
-        d_phase ^= 1u << set;
+        if (lane == 0) mbar_arrive(bars + 8 * kFtDEmpty);
+        ++used;
       }
       const bool last = c == chain1 - 1 || first_of(chain1) == c1;
       if (!last) {      // the operands' memory is still in use: these sums wait in tensor memory

@@ -202,3 +202,38 @@ def test_fp32_product_of_numbers_that_are_not_finite(m):
     assert torch.equal(kind(y.double()), kind(ref))
     assert rel(y[4][ref[4].isfinite()], ref[4][ref[4].isfinite()]) < 4e-7
     assert pkg._lib.device_status() == 0
+
+
+# Outputs one by one, in 2^-24 of the sum of the sizes of their products (against fp64).  Up to 16 products that are not zero: their roundings
+# to 24 bits, half a unit's root mean square and less, however the operands are taken apart; a single one: one rounding, and 2^-6 for
+# the sums of small parts.  Sums of one sign, where a sum cut off (at 2 units of itself, after each 16 of 64 products) falls short by up to
+# (1 + 2 + 3 + 4) / 4 units of itself on average.
+@pytest.mark.parametrize("k", [1024, 3072])
+@pytest.mark.parametrize("kind,rms,largest", [("1", 0.5, 1.1), ("4", 0.5, 4.0), ("16", 0.5, 4.0), ("sizes", 2.5, 16.0), ("full", 2.5, 16.0), ("same", 2.5, 16.0)])
+@pytest.mark.parametrize("form", ["plain", "glu", "experts"])
+def test_fp32_product_output_by_output(k, kind, rms, largest, form):
+    m, n = (128, 200) if form == "experts" else (65, 512)
+    x, w = torch.randn(m, k, generator=gen(10)), torch.randn(n, k, generator=gen(11))
+    if kind.isdigit():      # rows of few numbers that are not zero
+        x *= torch.zeros(m, k).scatter_(1, torch.rand(m, k, generator=gen(12)).topk(int(kind), 1).indices, 1.0)
+    elif kind == "sizes":
+        x, w = x.abs(), w.abs()
+    elif kind == "full":    # of one sign, the last 16 bits of the significand set
+        x, w = (((t.abs() + 1).view(torch.int32) | 0xffff).view(torch.float32) for t in (x, w))
+    else:
+        x, w = (torch.full_like(t, 1 + 65535 / 2 ** 23) for t in (x, w))
+    x, w = x.to(DEV), w.to(DEV)
+    if form == "experts":
+        y = ops.gemm_experts(x, torch.stack([w * 0, w]), torch.zeros(m, n, device=DEV), torch.ones(1, dtype=torch.int32, device=DEV),
+                             torch.ones(4, dtype=torch.int32, device=DEV), 128)
+    else:
+        y = ops.gemm(x, w, torch.zeros(m, n // 2 if form == "glu" else n, device=DEV), act=ops.ACT_RELU_GLU if form == "glu" else ops.ACT_NONE)
+    z, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    if form == "glu":       # an error of each factor reaches the result times the other
+        g, up = torch.relu(z[:, :n // 2]), z[:, n // 2:]
+        z, size = g * up, size[:, :n // 2] * up.abs() * (g > 0) + size[:, n // 2:] * g
+        rms, largest = rms + 0.5, largest + 1      # and their product is rounded
+    some = size > 0
+    e = (y.double() - z)[some] / size[some] * 2 ** 24
+    assert float(e.square().mean().sqrt()) < rms and float(e.abs().max()) < largest
+    assert float(y[~some].abs().max() if bool((~some).any()) else 0) == 0 and pkg._lib.device_status() == 0
