@@ -12,7 +12,9 @@
 //   their sizes      4.0, 1.5 (7.7, 1.7) / 4.1, 1.6 (8.8, 2.1) / 4.4, 1.8 (13, 3.2): sums of one sign, cut off at every step
 //   16 not zero      1.9, 0.30 (2.9, 0.37) / 1.9, 0.30 (2.4, 0.37) / 2.1, 0.31 (2.2, 0.38)
 //   one not zero     0.99, 0.42 and the same for FMAs
-// A result that is not finite is computed again by FMAs: its parts may be of either sign, or infinity times zero.
+// The first part of a number has its sign and is zero only where the number is (or below 2^-133); that of an infinity or NaN is the same, and
+// its other parts are NaN.  So the sum of the a1 b1 is infinite or NaN where that of the a b is, and then the small sums are left
+// out: such a result takes no longer than another.
 //
 // Tile: 128 weight rows (the left operand) x 32 or 64 rows of x, k in chunks of 64.  Eight warps fetch rows of fp32 into registers a
 // chunk ahead and leave their three parts in shared memory (K-major, 128-byte swizzle; the three parts of x one behind the
@@ -58,18 +60,6 @@ __device__ __forceinline__ float f32_activated(const mdb_gemm_args& a, float z, 
   if (a.act == MDB_ACT_SILU && col >= a.act_from) z /= 1.0f + expf(-z);
   return GLU ? fmaxf(z, 0.f) * up : z;
 }
-// An output that is not finite, by FMAs
-template <bool GLU>
-__device__ __noinline__ float f32_by_fma(const mdb_gemm_args& a, const float* x, const float* w, int col) {
-  float z[2] = {0.f, 0.f};
-  for (int h = 0; h < (GLU ? 2 : 1); ++h) {
-    const float* row = w + static_cast<int64_t>(col + h * a.n) * a.k;
-#pragma unroll 1
-    for (int i = 0; i < a.k; ++i) z[h] = fmaf(x[i], row[i], z[h]);
-  }
-  return f32_activated<GLU>(a, z[0], z[1], col);
-}
-
 template <int BN, bool GLU>
 __global__ void __launch_bounds__(kFtThreads, 1) gemm_f32_tc_kernel(const mdb_gemm_args a, const int ctas /* of a cluster */) {
   using P = FtPlan<BN>;
@@ -244,7 +234,7 @@ __global__ void __launch_bounds__(kFtThreads, 1) gemm_f32_tc_kernel(const mdb_ge
         for (int e = 0; e < 32; ++e) acc[j + e] += d[e / 16][e % 16];
       }
     };
-    auto add_small = [&]() {      // a chain's small sums, smallest first
+    auto add_small = [&]() {      // a chain's small sums, smallest first; beside a sum that is not finite they say nothing
 #pragma unroll
       for (int j = 0; j < BN; j += 16) {
         float t[16], u[16];
@@ -256,7 +246,8 @@ __global__ void __launch_bounds__(kFtThreads, 1) gemm_f32_tc_kernel(const mdb_ge
         tmem_ld16(lanes + BN + j, u);
         tmem_ld_wait();
 #pragma unroll
-        for (int e = 0; e < 16; ++e) acc[j + e] += t[e] + u[e];
+        for (int e = 0; e < 16; ++e)
+          if (isfinite(acc[j + e])) acc[j + e] += t[e] + u[e];
       }
     };
     for (int c = chain0; c < chain1; ++c) {
@@ -313,13 +304,9 @@ __global__ void __launch_bounds__(kFtThreads, 1) gemm_f32_tc_kernel(const mdb_ge
       if (out < a.n && (!GLU || warp < kFtSumWarps / 2) && misc[1] == 0) {
         float* const y = static_cast<float*>(a.y) + row0 * a.ldy + y_col + out;
         const int rows = static_cast<int>(min(static_cast<int64_t>(BN), a.m - row0));
-        unsigned long long odd = 0;
 #pragma unroll
-        for (int j = 0; j < BN; ++j) {
-          const float u = GLU ? up[j * kCols] : 0.f;
-          if (!isfinite(acc[j]) || !isfinite(u)) odd |= 1ull << j;
-          if (GLU) acc[j] = fmaxf(acc[j], 0.f) * u;
-        }
+        for (int j = 0; j < BN; ++j)
+          if (GLU) acc[j] = fmaxf(acc[j], 0.f) * up[j * kCols];
         if (a.act == MDB_ACT_RELU2) {
 #pragma unroll
           for (int j = 0; j < BN; ++j) {
@@ -339,9 +326,6 @@ __global__ void __launch_bounds__(kFtThreads, 1) gemm_f32_tc_kernel(const mdb_ge
           for (int j = 0; j < BN; ++j, at += a.ldy)
             if (j < rows) *at = acc[j];
         }
-#pragma unroll 1
-        for (int j = 0; odd != 0 && j < rows; ++j, odd >>= 1)
-          if (odd & 1) y[j * a.ldy] = f32_by_fma<GLU>(a, x + (row0 + j) * a.ldx, w, out);
       }
     }
   }
@@ -386,8 +370,7 @@ __global__ void __launch_bounds__(kFtThreads, 1) gemm_f32_tc_kernel(const mdb_ge
             t[0] += z[i][0];
             t[1] += z[i][GLU ? 1 : 0];
           }
-        const bool odd = !isfinite(t[0]) || !isfinite(t[1]);
-        y[j * a.ldy] = odd ? f32_by_fma<GLU>(a, x + (row0 + j) * a.ldx, w, out) : f32_activated<GLU>(a, t[0], t[1], out);
+        y[j * a.ldy] = f32_activated<GLU>(a, t[0], t[1], out);
       }
     }
   }

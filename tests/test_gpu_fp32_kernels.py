@@ -237,3 +237,31 @@ def test_fp32_product_output_by_output(k, kind, rms, largest, form):
     e = (y.double() - z)[some] / size[some] * 2 ** 24
     assert float(e.square().mean().sqrt()) < rms and float(e.abs().max()) < largest
     assert float(y[~some].abs().max() if bool((~some).any()) else 0) == 0 and pkg._lib.device_status() == 0
+
+
+def test_fp32_product_beside_rows_that_are_not_finite():
+    """Rows nobody reads (the empty rows of an expert's tile hold whatever they held) change neither the other rows nor the time; a NaN
+    is one whatever its bits are."""
+    n, k, tiles = 1024, 1024, 24
+    x, w = torch.randn(tiles * 128, k, generator=gen(13)).to(DEV), torch.randn(1, n, k, generator=gen(14)).to(DEV)
+    plan = torch.zeros(tiles, dtype=torch.int32, device=DEV), torch.full((4,), tiles, dtype=torch.int32, device=DEV)
+    rows = torch.arange(tiles * 128, device=DEV) % 128 < 5
+    odd = x.clone()
+    odd.view(torch.int32)[~rows] = -1                # NaN
+    odd.view(torch.int32)[5::128] = 0x7f800001       # NaN whose upper half is that of an infinity
+    odd[6::128] = float("inf")
+    y = [torch.zeros(tiles * 128, n, device=DEV) for _ in range(2)]
+    took = []
+    for a, b in ((x, y[0]), (odd, y[1])):
+        ops.gemm_experts(a, w, b, *plan, 128)
+        start, end = torch.cuda.Event(True), torch.cuda.Event(True)
+        start.record()
+        for _ in range(5):
+            ops.gemm_experts(a, w, b, *plan, 128)
+        end.record()
+        torch.cuda.synchronize()
+        took.append(start.elapsed_time(end))
+    assert torch.equal(y[0][rows], y[1][rows]) and not bool(torch.isfinite(y[1][~rows]).any())
+    assert bool(y[1][5::128].isnan().all())
+    assert took[1] < 2 * took[0], took               # (hundreds of times as long where a thread forms such a sum again)
+    assert pkg._lib.device_status() == 0
