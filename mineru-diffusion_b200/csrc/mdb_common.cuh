@@ -174,10 +174,13 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
   return r;
 }
 // The three bf16 parts of a pair of numbers: 24 significant bits are the exact sum of three times eight, cut and not rounded (the
-// upper half of x, that of what is left, the rest).  Numbers below 2^-110 lose their last bits: no bf16 number is below 2^-133.  Of an
-// infinity or NaN the first part is the same (by a conversion: the upper half of a NaN may be that of an infinity), the others are NaN.
+// upper half of x, that of what is left, the rest).  The second comes times 2^6, the third times 2^12, as no bf16 number is below 2^-133:
+// numbers from 2^-122 on are taken apart exactly, smaller ones to 2^-145.  (No larger factor: sums of products of first and
+// second parts stay below those of the sizes of the numbers' own products.)  Of an infinity or NaN the first part is the same (by a
+// conversion: the upper half of a NaN may be that of an infinity), the others are NaN.
+constexpr float kSplitUp = 64.0f;
 __device__ __forceinline__ void split3(f32x2 xy, uint32_t (&part)[3]) {
-  const f32x2 minus = pack2(-1.0f, -1.0f);
+  const f32x2 minus = pack2(-1.0f, -1.0f), up = pack2(kSplitUp, kSplitUp);
   const float2 whole = unpack2(xy);
   asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(part[0]) : "f"(whole.y), "f"(whole.x));
 #pragma unroll
@@ -185,7 +188,7 @@ __device__ __forceinline__ void split3(f32x2 xy, uint32_t (&part)[3]) {
     const float2 v = unpack2(xy);
     const uint32_t a = __float_as_uint(v.x), b = __float_as_uint(v.y);
     if (p > 0) part[p] = __byte_perm(a, b, 0x7632);
-    if (p < 2) xy = fma2(pack2(__uint_as_float(a & 0xffff0000u), __uint_as_float(b & 0xffff0000u)), minus, xy);
+    if (p < 2) xy = mul2(fma2(pack2(__uint_as_float(a & 0xffff0000u), __uint_as_float(b & 0xffff0000u)), minus, xy), up);
   }
 }
 

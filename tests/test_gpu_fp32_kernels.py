@@ -265,3 +265,15 @@ def test_fp32_product_beside_rows_that_are_not_finite():
     assert bool(y[1][5::128].isnan().all())
     assert took[1] < 2 * took[0], took               # (hundreds of times as long where a thread forms such a sum again)
     assert pkg._lib.device_status() == 0
+
+
+# Every number down to 2^-122 is taken apart exactly: scaled by a power of two the result has the same error.  Down to the smallest normal number
+# up to four of 24 bits may go, 2^-19 of a number and, with errors of either sign, far less of a sum.  Products far below 1 end at 2^-149.
+@pytest.mark.parametrize("x_exp,w_exp,limit", [(-108, 0, 2e-7), (-114, 0, 2e-7), (-120, 20, 2e-7), (0, -118, 2e-7), (-124, 60, 1e-6), (-60, -60, 2e-7), (90, 20, 2e-7)])
+def test_fp32_product_of_small_and_large_numbers(x_exp, w_exp, limit):
+    m, n, k = 40, 300, 1024
+    x, w = torch.rand(m, k, generator=gen(15)) + 1, torch.rand(n, k, generator=gen(16)) + 1       # sizes in [1, 2), of either sign
+    x, w = x * torch.randn(m, k, generator=gen(17)).sign() * 2.0 ** x_exp, w * torch.randn(n, k, generator=gen(18)).sign() * 2.0 ** w_exp
+    y = ops.gemm(x.to(DEV), w.to(DEV), torch.zeros(m, n, device=DEV))
+    assert rel(y.double() * 2.0 ** -(x_exp + w_exp), x.double() @ w.double().T * 2.0 ** -(x_exp + w_exp)) < limit
+    assert pkg._lib.device_status() == 0
