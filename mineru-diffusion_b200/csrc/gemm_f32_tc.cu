@@ -17,17 +17,20 @@
 // its other parts are NaN.  So the sum of the a1 b1 is infinite or NaN where that of the a b is, and then the small sums are left
 // out: such a result takes no longer than another.
 //
-// Tile: 128 weight rows (the left operand) x 32 or 64 rows of x, k in chunks of 64.  Eight warps fetch rows of fp32 into registers a
-// chunk ahead and leave their three parts in shared memory (K-major, 128-byte swizzle; the three parts of x one behind the
-// other, so that one product takes a1 or a2 with b1 | b2 | b3, one a3 with b1 | b2), a warp issues the products, four warps add up.
-// A chunk's small products go first: they wait for nothing, and meanwhile the chunk before's sums of a1 b1 are read.  Four chains over k, each a quarter of the chunks: a cluster of one, two or four CTAs shares them out, and they are
-// added in the same order whoever ran them, so that the bits of a row do not depend on the other rows.
+// Tile: 128, 64 or 32 weight rows (the left operand) x 64 or 32 rows of x, k in chunks of 64.  Eight warps fetch rows of fp32 into
+// registers a chunk ahead and leave their three parts in shared memory (K-major, 128-byte swizzle; the three parts of x one behind the
+// other, so that one product takes a1 or a2 with b1 | b2 | b3, one a3 with b1 | b2), a warp issues the products, up to four warps add up.
+// A chunk's small products go first: they wait for nothing, and meanwhile the chunk before's sums of a1 b1 are read.  Four chains
+// over k, each a quarter of the chunks: a cluster of one, two or four CTAs shares them out, and they are added in the same order
+// whoever ran them, so that the bits of a row do not depend on the other rows.
 //
 // What bounds it: bringing the operands in and turning them round.  A chunk of 128 x 64 outputs takes 2100 cycles, of which the
 // products need 1030: its 48 KB come out of L2 (6 TB/s with all SMs), the parts are written to shared memory (72 KB) and read by the
 // products (116 KB).  500 rows, n x k 4352 x 1024, 45 us with eight products and with six; with six 32 without the loads, 35 with a
-// third of the parts' stores, 41 without splitting.  On FMAs it took 117; 1024 x 3072: 92 -> 35; 1024 x 1024: 33 -> 18; 16
-// rows of the same: 13.0 -> 12.7, 20.7 -> 15.5, 7.9 -> 8.9.
+// third of the parts' stores, 41 without splitting.  On FMAs it took 117; 1024 x 3072: 92 -> 35; 1024 x 1024: 33 -> 18.
+// Few rows: a chunk's latency, so the weight rows of a tile are as few as still run all at once, and rows of x that are not there are
+// not turned round (8 rows, 1024 x 1024, weights out of HBM: 9.4 us with 128 weight rows, 7.2 with 32; FMAs 7.9).  Not faster: two chunks
+// ahead in registers (9.4 against 8.6 out of L2), weights asked into L2 in front of the dependency wait (8.7 against 7.5).
 #include "mdb_common.cuh"
 
 namespace mdb {
@@ -35,14 +38,16 @@ namespace mdb {
 constexpr int kFtK = 64, kFtRows = 128, kFtChains = 4;
 constexpr int kFtSumWarps = 4, kFtLoadWarps = 8, kFtMma = kFtSumWarps + kFtLoadWarps, kFtThreads = (kFtMma + 1) * 32;
 
-template <int BN>
+template <int BN, int W>
 struct FtPlan {
-  static constexpr int kPartA = kFtRows * 128, kPartB = BN * 128, kStage = 3 * (kPartA + kPartB), kStages = 3;
-  static constexpr int kSlot = kFtRows * BN * 4;                     // a chain's sums on their way to the other CTAs of the cluster
+  static constexpr int kPartA = W * 128, kPartB = BN * 128, kStage = 3 * (kPartA + kPartB), kStages = 3;
+  static constexpr int kSlot = W * BN * 4;                     // a chain's sums on their way to the other CTAs of the cluster
   static constexpr int kOffBars = kStages * kStage, kBytes = 1024 + kOffBars + 128;
   // tensor memory: a1 b1 of a chunk | of size 2^-8 | of size 2^-16 | of size 2^-24 of a chain | sums of the chains before
-  static constexpr uint32_t kSum = 4 * BN;
-  static_assert(2 * kSlot <= kStages * kStage && kBytes <= 227 * 1024 && 5 * BN <= 512, "memory of the fp32 product");
+  static constexpr uint32_t kSum = 4 * BN, kTmemCols = BN == 32 ? 256 : 512;
+  static_assert(2 * kSlot <= kStages * kStage && kBytes <= 227 * 1024 && 5 * BN <= kTmemCols, "memory of the fp32 product");
+  // a product always takes 128 weight rows: behind the W of a part it finds others, whose sums nobody reads
+  static_assert(2 * kPartA + kFtRows * 128 <= kStage, "a product's reads end in its stage");
 };
 enum { kFtFull = 0, kFtEmpty = 3, kFtDFull = 6, kFtDEmpty = 7, kFtBars = 8 };
 
@@ -61,9 +66,9 @@ __device__ __forceinline__ float f32_activated(const mdb_gemm_args& a, float z, 
   if (a.act == MDB_ACT_SILU && col >= a.act_from) z /= 1.0f + expf(-z);
   return GLU ? fmaxf(z, 0.f) * up : z;
 }
-template <int BN, bool GLU>
-__global__ void __launch_bounds__(kFtThreads, 1) gemm_f32_tc_kernel(const mdb_gemm_args a, const int ctas /* of a cluster */) {
-  using P = FtPlan<BN>;
+template <int BN, int W, bool GLU>
+__global__ void __launch_bounds__(kFtThreads, W == 32 ? 2 : 1) gemm_f32_tc_kernel(const mdb_gemm_args a, const int ctas /* of a cluster */) {
+  using P = FtPlan<BN, W>;
   extern __shared__ __align__(1024) unsigned char ft_smem_raw[];
   const uint32_t raw = smem_u32(ft_smem_raw), base = (raw + 1023u) & ~1023u;
   unsigned char* mem = ft_smem_raw + (base - raw);
@@ -71,16 +76,16 @@ __global__ void __launch_bounds__(kFtThreads, 1) gemm_f32_tc_kernel(const mdb_ge
   volatile uint32_t* misc = reinterpret_cast<volatile uint32_t*>(mem + P::kOffBars + 8 * kFtBars);      // tensor memory base, abort flag
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = ctas > 1 ? static_cast<int>(cluster_ctarank()) : 0;
-  constexpr int kCols = GLU ? kFtRows / 2 : kFtRows;                // output columns of a tile
+  constexpr int kCols = GLU ? W / 2 : W, kSumWarps = W / 32;       // output columns of a tile; warps that add up
   const int n0 = static_cast<int>(blockIdx.x) / ctas * kCols;
   const int64_t row0 = static_cast<int64_t>(blockIdx.y) * BN;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kFtBars; ++s) mbar_init(bars + 8 * s, s < kFtEmpty ? kFtLoadWarps : (s < kFtDEmpty ? 1 : kFtSumWarps));
+    for (int s = 0; s < kFtBars; ++s) mbar_init(bars + 8 * s, s < kFtEmpty ? kFtLoadWarps : (s < kFtDEmpty ? 1 : kSumWarps));
     misc[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kFtMma) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(const_cast<uint32_t*>(&misc[0]))), "r"(512u)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(const_cast<uint32_t*>(&misc[0]))), "r"(P::kTmemCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -171,23 +176,23 @@ __global__ void __launch_bounds__(kFtThreads, 1) gemm_f32_tc_kernel(const mdb_ge
   } else if (warp >= kFtSumWarps) {
     // ------------------------------------------------------------------ operands
     // 32 bytes of k of a row per lane, eight lanes a row; a thread has the same piece of NR rows of every chunk
-    constexpr int NR = (kFtRows + BN) / 32;
+    constexpr int NR = (W + BN) / 32;
     const int tid = threadIdx.x - kFtSumWarps * 32, piece = tid & 7, r0 = tid >> 3;
     const float* const x0 = x + (row0 + r0) * a.ldx + 8 * piece;
-    const float* const w0 = w + static_cast<int64_t>(n0 + r0) * a.k + 8 * piece;
+    const float* const w0 = w + static_cast<int64_t>(n0 + r0 + (GLU && kCols < 32 && r0 >= kCols ? a.n - kCols : 0)) * a.k + 8 * piece;
     uint32_t there = 0;
 #pragma unroll
     for (int q = 0; q < NR; ++q) {
       const int r = r0 + 32 * q;
-      if (r < kFtRows ? n0 + r % kCols < a.n : row0 + r - kFtRows < a.m) there |= 1u << q;
+      if (r < W ? n0 + r % kCols < a.n : row0 + r - W < a.m) there |= 1u << q;
     }
     const float* const zeros = kFtZeros;      // what lies outside
     const bool wide = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 31) == 0;      // rows of 16 k, or 8 of x
     f32x2 v[NR][4];
     auto fetch = [&](int q, int chunk) {
       const int k = chunk * kFtK;
-      const float* from = 32 * q >= kFtRows ? x0 + (32 * q - kFtRows) * a.ldx
-                                             : w0 + (static_cast<int64_t>(GLU && 32 * q >= kCols ? a.n - kCols : 0) + 32 * q) * a.k;
+      const float* from = 32 * q >= W ? x0 + (32 * q - W) * a.ldx
+                                             : w0 + (static_cast<int64_t>(GLU && kCols >= 32 && 32 * q >= kCols ? a.n - kCols : 0) + 32 * q) * a.k;
       ldg_f8((there >> q & 1u) && chunk < end && k + 8 * piece < a.k ? from + k : zeros, wide, v[q]);
     };
 #pragma unroll
@@ -201,12 +206,13 @@ __global__ void __launch_bounds__(kFtThreads, 1) gemm_f32_tc_kernel(const mdb_ge
       const uint32_t dst = dst0 + stage * P::kStage;
 #pragma unroll
       for (int q = 0; q < NR; ++q) {
+        if (32 * q >= W && !(there >> q & 1u)) continue;      // a row of x that is not there: its sums go nowhere
         uint32_t p[4][3];
 #pragma unroll
         for (int e = 0; e < 4; ++e) split3(v[q][e], p[e]);
         fetch(q, i + 1);
-        const bool is_w = 32 * q < kFtRows;
-        const uint32_t to = dst + (is_w ? 32 * q * 128 : 3 * P::kPartA + (32 * q - kFtRows) * 128);
+        const bool is_w = 32 * q < W;
+        const uint32_t to = dst + (is_w ? 32 * q * 128 : 3 * P::kPartA + (32 * q - W) * 128);
 #pragma unroll
         for (int e = 0; e < 3; ++e)
           asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(to + e * (is_w ? P::kPartA : P::kPartB)), "r"(p[0][e]), "r"(p[1][e]),
@@ -218,6 +224,8 @@ __global__ void __launch_bounds__(kFtThreads, 1) gemm_f32_tc_kernel(const mdb_ge
       phase ^= 1u << stage;
       stage = stage + 1 == P::kStages ? 0 : stage + 1;
     }
+  } else if (warp >= kSumWarps) {
+    ready();
   } else {
     // ---------------------------------------------------------------------- sums
     const uint32_t lanes = ready() + (static_cast<uint32_t>(32 * warp) << 16);
@@ -288,7 +296,7 @@ __global__ void __launch_bounds__(kFtThreads, 1) gemm_f32_tc_kernel(const mdb_ge
         float* to = reinterpret_cast<float*>(mem + slot * P::kSlot) + 32 * warp + lane;
 #pragma unroll
         for (int j = 0; j < BN; ++j) {
-          to[j * kFtRows] = acc[j];
+          to[j * W] = acc[j];
           acc[j] = 0.f;
         }
         if (slot > 0) add(P::kSum);
@@ -299,13 +307,13 @@ __global__ void __launch_bounds__(kFtThreads, 1) gemm_f32_tc_kernel(const mdb_ge
       const int col = (32 * warp + lane) % kCols, out = n0 + col;
       float* up = reinterpret_cast<float*>(mem) + col;
       if (GLU) {
-        if (warp >= kFtSumWarps / 2) {
+        if (32 * warp + lane >= kCols) {
 #pragma unroll
           for (int j = 0; j < BN; ++j) up[j * kCols] = acc[j];
         }
-        asm volatile("bar.sync 1, %0;" ::"n"(kFtSumWarps * 32) : "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(kSumWarps * 32) : "memory");
       }
-      if (out < a.n && (!GLU || warp < kFtSumWarps / 2) && misc[1] == 0) {
+      if (out < a.n && (!GLU || 32 * warp + lane < kCols) && misc[1] == 0) {
         float* const y = static_cast<float*>(a.y) + row0 * a.ldy + y_col + out;
         const int rows = static_cast<int>(min(static_cast<int64_t>(BN), a.m - row0));
 #pragma unroll
@@ -337,7 +345,7 @@ __global__ void __launch_bounds__(kFtThreads, 1) gemm_f32_tc_kernel(const mdb_ge
   if (ctas > 1) cluster_sync_all();
   else __syncthreads();
   tc_fence_after();
-  if (warp == kFtMma) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(misc[0]), "r"(512u));
+  if (warp == kFtMma) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(misc[0]), "r"(P::kTmemCols));
   if (ctas > 1 && live && misc[1] == 0) {
     // this CTA's rows of the tile: the sums that every CTA has left, in their order
     uint32_t from[kFtChains];
@@ -365,7 +373,7 @@ __global__ void __launch_bounds__(kFtThreads, 1) gemm_f32_tc_kernel(const mdb_ge
           for (int h = 0; h < (GLU ? 2 : 1); ++h) {
             z[i][h] = 0.f;
             if (i < slots)
-              asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(z[i][h]) : "r"(from[i] + (j * kFtRows + h * kCols + col) * 4) : "memory");
+              asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(z[i][h]) : "r"(from[i] + (j * W + h * kCols + col) * 4) : "memory");
           }
         float t[2] = {z[0][0], z[0][GLU ? 1 : 0]};
 #pragma unroll
@@ -378,13 +386,14 @@ __global__ void __launch_bounds__(kFtThreads, 1) gemm_f32_tc_kernel(const mdb_ge
       }
     }
   }
-  if (ctas > 1) cluster_sync_all();      // no CTA leaves while another may still read its shared memory
+  // no CTA leaves while another may still read its shared memory; nothing is handed over here, and what a thread has read it has used
+  if (ctas > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
 
-template <int BN, bool GLU>
+template <int BN, int W, bool GLU>
 static int gemm_f32_tc_run(const mdb_gemm_args& a, int ctas, cudaStream_t st) {
-  using P = FtPlan<BN>;
-  auto kernel = gemm_f32_tc_kernel<BN, GLU>;
+  using P = FtPlan<BN, W>;
+  auto kernel = gemm_f32_tc_kernel<BN, W, GLU>;
   static PerDeviceOnce attr_once;
   const int dev = attr_once.slot();
   if (dev < 0) return MDB_ERR_CUDA;
@@ -392,7 +401,7 @@ static int gemm_f32_tc_run(const mdb_gemm_args& a, int ctas, cudaStream_t st) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P::kBytes) != cudaSuccess) return MDB_ERR_CUDA;
     attr_once.done[dev] = true;
   }
-  const int cols = GLU ? kFtRows / 2 : kFtRows;
+  const int cols = GLU ? W / 2 : W;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((a.n + cols - 1) / cols * ctas, static_cast<unsigned>((static_cast<int64_t>(a.m) + BN - 1) / BN), a.form == MDB_GEMM_HEADS ? a.heads : 1);
   cfg.blockDim = dim3(kFtThreads);
@@ -409,31 +418,37 @@ static int gemm_f32_tc_run(const mdb_gemm_args& a, int ctas, cudaStream_t st) {
   return cudaLaunchKernelEx(&cfg, kernel, a, ctas) == cudaSuccess ? MDB_OK : MDB_ERR_CUDA;
 }
 
-// Rounds of the CTAs times the time of one, in us as measured (32 and 64 rows a tile, clusters of one, two and four): a
-// chunk 0.87 and 1.08, beside it 3.9, 6.1, 5.3 and 5.3, 9.0, 7.9 (of a cluster of two the second CTA leaves two chains).
-// Clusters of four do not fill every SM: 33 run at once on 148.
+// Rounds of the CTAs times the time of one, in hundredths of a us as measured: a chunk, and what is beside it in clusters of one,
+// two and four (of a cluster of two the second CTA leaves two chains).  Clusters of four do not fill every SM: 33 run at once on 148.
+// Of 540 sizes (1 to 1000 rows, 64 to 8192 columns, k 768 to 3072) the form taken was within 8 % of the best of the twelve.
+struct FtForm { int rows, weights, chunk, rest[3]; };
+constexpr FtForm kFtForms[4] = {{64, 128, 108, {530, 900, 790}}, {32, 128, 87, {330, 560, 530}}, {32, 64, 70, {340, 460, 510}}, {32, 32, 58, {440, 540, 520}}};
 template <bool GLU>
 static int gemm_f32_tc_dispatch(const mdb_gemm_args& a, cudaStream_t st) {
-  constexpr int kChunk[2] = {87, 108}, kRest[2][3] = {{390, 610, 530}, {530, 900, 790}};      // hundredths of a us
-  const int cols = GLU ? kFtRows / 2 : kFtRows, chunks = (a.k + kFtK - 1) / kFtK;
-  const int64_t tiles_n = static_cast<int64_t>((a.n + cols - 1) / cols) * (a.form == MDB_GEMM_HEADS ? a.heads : 1), sms = at_sm_count();
+  const int chunks = (a.k + kFtK - 1) / kFtK;
+  const int64_t n = GLU ? 2LL * a.n : a.n, sms = at_sm_count();
   int64_t best = INT64_MAX;
-  int rows = 64, ctas = 1;
-  for (int h = 0; h < 2; ++h) {
-    const int bn = 32 << h;
-    if (a.m > bn * 65535LL) continue;
-    const int64_t tiles = tiles_n * ((static_cast<int64_t>(a.m) + bn - 1) / bn);
+  int form = 0, ctas = 1;
+  for (int f = 0; f < 4; ++f) {
+    const FtForm& p = kFtForms[f];
+    if (a.m > p.rows * 65535LL) continue;
+    const int64_t tiles = (n + p.weights - 1) / p.weights * (a.form == MDB_GEMM_HEADS ? a.heads : 1) * ((static_cast<int64_t>(a.m) + p.rows - 1) / p.rows);
     for (int lg = 0; lg < 3; ++lg) {
       const int c = 1 << lg;
       const int64_t at_once = max(lg == 2 ? sms / 4 - 4 : sms / c, static_cast<int64_t>(1));
-      const int64_t time = (tiles + at_once - 1) / at_once * ((chunks + c - 1) / c * kChunk[h] + kRest[h][lg]);
-      if (time < best) { best = time; rows = bn; ctas = c; }
+      const int64_t time = (tiles + at_once - 1) / at_once * ((chunks + c - 1) / c * p.chunk + p.rest[lg]);
+      if (time < best) { best = time; form = f; ctas = c; }
     }
   }
 #ifdef F32_FORCE
   F32_FORCE
 #endif
-  return rows == 64 ? gemm_f32_tc_run<64, GLU>(a, ctas, st) : gemm_f32_tc_run<32, GLU>(a, ctas, st);
+  switch (form) {
+    case 0: return gemm_f32_tc_run<64, 128, GLU>(a, ctas, st);
+    case 1: return gemm_f32_tc_run<32, 128, GLU>(a, ctas, st);
+    case 2: return gemm_f32_tc_run<32, 64, GLU>(a, ctas, st);
+    default: return gemm_f32_tc_run<32, 32, GLU>(a, ctas, st);
+  }
 }
 
 static int gemm_f32_tc_launch(const mdb_gemm_args& a, cudaStream_t st) {

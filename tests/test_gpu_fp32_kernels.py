@@ -277,3 +277,30 @@ def test_fp32_product_of_small_and_large_numbers(x_exp, w_exp, limit):
     y = ops.gemm(x.to(DEV), w.to(DEV), torch.zeros(m, n, device=DEV))
     assert rel(y.double() * 2.0 ** -(x_exp + w_exp), x.double() @ w.double().T * 2.0 ** -(x_exp + w_exp)) < limit
     assert pkg._lib.device_status() == 0
+
+
+# Few rows take tiles of 128, 64 or 32 weight rows (half of them up rows with GLU) in clusters of one, two or four, by the number of columns: the same
+# bits as beside 600 rows, and the last tile and the last chunk of k may be partly empty.
+@pytest.mark.parametrize("form,n,k", [("plain", 20, 768), ("glu", 20, 768), ("plain", 1028, 1024), ("plain", 2052, 1024), ("glu", 1028, 1040), ("plain", 4352, 1024),
+                                      ("heads", 72, 1040), ("plain", 8200, 832), ("glu", 8, 3088)])
+def test_fp32_product_of_few_rows(form, n, k):
+    heads = 3 if form == "heads" else 1
+    x, w = torch.randn(600, heads * k, generator=gen(19)).to(DEV), torch.randn(heads, 2 * n if form == "glu" else n, k, generator=gen(20)).to(DEV)
+
+    def product(rows):
+        y = torch.full((len(rows) + 1, heads * n), 7.0, device=DEV)
+        if form == "heads":
+            ops.gemm_heads(rows, w, y[:-1])
+        else:
+            ops.gemm(rows, w[0], y[:-1], act=ops.ACT_RELU_GLU if form == "glu" else ops.ACT_NONE)
+        assert float((y[-1] - 7).abs().max()) == 0
+        return y[:-1]
+
+    whole = product(x)
+    z = torch.einsum("mhk,hnk->mhn", x.double().view(600, heads, k), w.double()).reshape(600, -1)
+    if form == "glu":
+        z = torch.relu(z[:, :n]) * z[:, n:]
+    assert rel(whole, z) < 4e-7
+    for m in (1, 9, 33, 64, 100):
+        assert torch.equal(product(x[:m]), whole[:m]), m
+    assert pkg._lib.device_status() == 0
