@@ -440,9 +440,6 @@ static int gemm_f32_tc_dispatch(const mdb_gemm_args& a, cudaStream_t st) {
       if (time < best) { best = time; form = f; ctas = c; }
     }
   }
-#ifdef F32_FORCE
-  F32_FORCE
-#endif
   switch (form) {
     case 0: return gemm_f32_tc_run<64, 128, GLU>(a, ctas, st);
     case 1: return gemm_f32_tc_run<32, 128, GLU>(a, ctas, st);
