@@ -16,10 +16,12 @@ _BF16 = torch.bfloat16
 
 # The handle of the calling thread's current stream.  torch.cuda.current_stream() builds a Stream object for it, a third of the host time
 # of a prompt step of 37 launches; this is where it gets the handle from.
-_device, _raw_stream = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
+_device, _raw_stream = (getattr(torch._C, name, None) for name in ("_cuda_getDevice", "_cuda_getCurrentRawStream"))
 
 
 def _stream() -> int:
+    if _device is None or _raw_stream is None:      # a torch without CUDA, or without these two
+        return torch.cuda.current_stream().cuda_stream
     return _raw_stream(_device())
 
 

@@ -143,3 +143,16 @@ def test_a_scan_reads_no_further_than_its_block(built):
     assert run.returncode == 0, (run.returncode, run.stderr[-400:])
     unsupported = int(re.search(r"MDB_ERR_UNSUPPORTED\s*=?\s*\(?(-?\d+)", open(HEADER).read()).group(1))
     assert int(run.stdout) == unsupported
+
+
+def test_package_imports_without_the_private_stream_calls():
+    """A torch built without CUDA has neither; the stream then comes from where it always may."""
+    import subprocess
+    import sys
+    code = ("import importlib, torch\n"
+            "for n in ('_cuda_getDevice', '_cuda_getCurrentRawStream'):\n"
+            "    if hasattr(torch._C, n): delattr(torch._C, n)\n"
+            "ops = importlib.import_module('mineru-diffusion_b200').ops\n"
+            "torch.cuda.current_stream = lambda: type('S', (), {'cuda_stream': 17})()\n"
+            "assert ops._stream() == 17\n")
+    subprocess.run([sys.executable, "-c", code], cwd=ROOT, check=True, timeout=300)
