@@ -85,10 +85,15 @@ __global__ void __launch_bounds__(kRouteWarps * 32) moe_route_kernel(const mdb_m
 // The order of the rows of one expert is not fixed; every row's result is independent of its place.
 // Bound by latencies one behind the other: the ids, the counts, the rows.  With up to KEEP ids per thread the count that a pair
 // finds is its place among its expert's rows, and stays in a register with its expert: one walk over the ids and one over the rows'
-// list; beyond that (KEEP 0) the ids are read twice.  Rows that stay empty are marked by a warp per expert.  2048 tokens of six
-// of 64 experts: 12.2 us with two walks, 11.1.
+// list; beyond that (KEEP 0) the ids are read twice.  With up to 64 experts (FEW) half a warp has one, lists its tiles and marks the rows
+// that stay empty; with more of them a thread has one, and all rows are marked before they are given out.
+// us, two walks and all rows marked, tiles listed by the scan / now:
+//   8 experts, two a token:    1 token 2.2 / 1.8, 512 2.9 / 2.2, 1365 3.7 / 3.1, 4096 5.6 / 5.3
+//   64 experts, six a token:   1 token 2.8 / 2.3, 128 3.5 / 3.4, 512 5.1 / 4.7, 2048 11.2 / 11.0, 4096 19.8 / 18.7
+//   256 experts, eight a token: 1 token 4.4 / 3.0, 128 7.4 / 5.4, 512 9.5 / 8.3, 2048 17.9 / 16.7
+// (More ids in registers: 2048 tokens of six of 64 experts 10.2 with 12, but with 24 for every number of ids 4.4 for one token.)
 constexpr int kPlanThreads = 1024, kPlanBatch = 8;
-template <int KEEP>
+template <int KEEP, bool FEW>
 __global__ void __launch_bounds__(kPlanThreads) moe_plan_kernel(const mdb_moe_plan_args a) {
   pdl_launch_dependents();
   pdl_wait();
@@ -145,10 +150,16 @@ __global__ void __launch_bounds__(kPlanThreads) moe_plan_kernel(const mdb_moe_pl
   __syncthreads();
   const int cap = a.max_tiles * kMoeTileRows;
   // every expert's tiles, and the rows of its last one that stay empty
-  for (int e = threadIdx.x >> 5; e < a.experts; e += kPlanThreads / 32) {
-    const int r0 = first[e], r1 = r0 + count[e], r2 = r0 + (count[e] + kMoeTileRows - 1) / kMoeTileRows * kMoeTileRows;
-    for (int t = r0 / kMoeTileRows + (threadIdx.x & 31); t < r2 / kMoeTileRows && t < a.max_tiles; t += 32) a.tile_expert[t] = e;
-    for (int r = r1 + (threadIdx.x & 31); r < r2 && r < cap; r += 32) a.row_token[r] = -1;
+  constexpr int kLanes = FEW ? 16 : 1;
+  for (int e = threadIdx.x / kLanes; e < a.experts; e += kPlanThreads / kLanes) {
+    const int l = threadIdx.x % kLanes, r0 = first[e], r1 = r0 + count[e], r2 = r0 + (count[e] + kMoeTileRows - 1) / kMoeTileRows * kMoeTileRows;
+    for (int t = r0 / kMoeTileRows + l; t < r2 / kMoeTileRows && t < a.max_tiles; t += kLanes) a.tile_expert[t] = e;
+    if (FEW)
+      for (int r = r1 + l; r < r2 && r < cap; r += kLanes) a.row_token[r] = -1;
+  }
+  if (!FEW) {
+    for (int r = threadIdx.x; r < total_rows && r < cap; r += kPlanThreads) a.row_token[r] = -1;
+    __syncthreads();
   }
   if (KEEP > 0) {
 #pragma unroll
@@ -250,8 +261,10 @@ int mdb_moe_plan(const mdb_moe_plan_args* args, mdb_stream_t stream) {
   MDB_REQUIRE(a.ids && a.slot && a.row_token && a.tile_expert && a.num_tiles, MDB_ERR_ARG);
   MDB_REQUIRE(a.experts <= 4096 && static_cast<int64_t>(a.m) * a.top < (1 << 30), MDB_ERR_UNSUPPORTED);
   const int each = (a.m * a.top + kPlanThreads - 1) / kPlanThreads;
-  void (*const kernel)(mdb_moe_plan_args) = each < 1 ? moe_plan_kernel<0> : each <= 1 ? moe_plan_kernel<1> : each <= 4 ? moe_plan_kernel<4> : each <= 12 ? moe_plan_kernel<12>
-                                            : each <= 24 ? moe_plan_kernel<24> : moe_plan_kernel<0>;
+  const int keep = each < 1 || each > 4 ? 0 : each > 1 ? 4 : 1;
+  void (*const few)(mdb_moe_plan_args) = keep == 0 ? moe_plan_kernel<0, true> : keep == 1 ? moe_plan_kernel<1, true> : moe_plan_kernel<4, true>;
+  void (*const many)(mdb_moe_plan_args) = keep == 0 ? moe_plan_kernel<0, false> : keep == 1 ? moe_plan_kernel<1, false> : moe_plan_kernel<4, false>;
+  void (*const kernel)(mdb_moe_plan_args) = a.experts <= 64 ? few : many;
   return mdb_launch(kernel, dim3(1), dim3(kPlanThreads), sizeof(int) * 2 * a.experts, static_cast<cudaStream_t>(stream), a);
 }
 

@@ -288,3 +288,9 @@ def test_latent_rows_of_several_heads(m, heads, width, dtype):
         a = torch.softmax(q[r].view(heads, width).double() @ rows[:r + 1].T * width ** -0.5, -1)
         assert rel(out[r].view(heads, width), a @ rows[:r + 1]) < (2e-6 if dtype == torch.float32 else 4e-3), r
     assert bool((out[7] == 5).all())
+
+
+# More experts than there are half warps, with one id per thread, up to four, and more: the same plan and gather.
+@pytest.mark.parametrize("m,top,experts", [(1, 8, 65), (100, 8, 160), (300, 8, 256), (700, 8, 256), (520, 4, 1030), (683, 6, 64), (684, 6, 64)])
+def test_expert_plan_of_many_experts(m, top, experts):
+    test_expert_plan_and_gather(m, top, experts)
