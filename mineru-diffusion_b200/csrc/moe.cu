@@ -194,34 +194,61 @@ __global__ void __launch_bounds__(kPlanThreads) moe_plan_kernel(const mdb_moe_pl
   }
 }
 
-// Bound by memory and by a row's latencies, its place and its pieces.  2048 tokens of 4 KB to 12288 rows: 13.5 us with a CTA per row
-// and a piece in flight per thread, 10.8 now.
+// Bound by memory and by a row's latencies, its place and its pieces; the next place is read meanwhile.  Few rows of up to 8 KB: a CTA per row, two
+// pieces of 16 bytes in flight per thread.  Many: a warp per row, or per eighth round of 512 bytes of it, all eight in flight, in steps that
+// shift a warp by 5/8 of a tile, as a tile's rows lie together and the rest of it is empty.
+// us, a CTA per row and a piece in flight per thread / now (a warp per row in steps of whole tiles beside them):
+//   rows of 4 KB:   2048 tokens of six of 64 experts 11.8 / 9.7 (9.7), 1000 6.2 / 5.8 (5.7), 300 of two of 8 2.0 / 2.1 (2.5)
+//   rows of 8 KB:   700 of eight of 160 11.2 / 10.5 (13.4), 700 of two of 8 3.8 / 3.6 (5.1)
+//   rows of 14 KB:  2048 of six of 64 48.5 / 38 (38), 300 of eight of 160 12.3 / 10.6 (14.7), 128 of two of 8 3.2 / 3.1 (4.9)
 // (No __restrict__ on these pointers: a load the compiler may treat as invariant, like *num_tiles, moves above
-// griddepcontrol.wait and then reads what the previous plan left.)
-template <typename T>
-__global__ void __launch_bounds__(128) moe_gather_kernel(const T* x, int64_t ldx, T* out, int width,
-                                                         const int32_t* row_token,
-                                                         const int32_t* num_tiles) {
+// griddepcontrol.wait and then reads what the previous plan left.  Padding rows keep whatever they hold; nobody reads their results.)
+__global__ void __launch_bounds__(128) moe_gather_few_kernel(const uint4* x, int64_t ldx, uint4* out, int chunks, const int32_t* row_token,
+                                                             const int32_t* num_tiles) {
   pdl_launch_dependents();
   pdl_wait();
-  // a warp per row, eight pieces of 16 bytes in flight per lane, the next row's place read meanwhile
-  const int rows = *num_tiles * kMoeTileRows, lane = threadIdx.x & 31, step = gridDim.x * 4;
-  const int chunks = width * static_cast<int>(sizeof(T)) / 16;
-  int r = blockIdx.x * 4 + (threadIdx.x >> 5);
-  int t = r < rows ? row_token[r] : -1;
-  for (; r < rows; r += step) {
-    const int next = r + step < rows ? row_token[r + step] : -1;
-    if (t >= 0) {                        // padding rows keep whatever they hold; nobody reads their results
-      const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<int64_t>(t) * ldx);
-      uint4* dst = reinterpret_cast<uint4*>(out + static_cast<int64_t>(r) * width);
-      for (int c0 = 0; c0 < chunks; c0 += 256) {
-        uint4 v[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = src[min(c0 + 32 * i + lane, chunks - 1)];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          if (c0 + 32 * i + lane < chunks) dst[c0 + 32 * i + lane] = v[i];
+  const int rows = *num_tiles * kMoeTileRows;
+  int r = blockIdx.x, t = r < rows ? row_token[r] : -1;
+  while (r < rows) {
+    uint4* dst = out + static_cast<int64_t>(r) * chunks;
+    r += gridDim.x;
+    const int next = r < rows ? row_token[r] : -1;
+    if (t >= 0) {
+      const uint4* src = x + static_cast<int64_t>(t) * ldx;
+      for (int c = threadIdx.x; c < chunks; c += 256) {
+        const uint4 v0 = src[c], v1 = src[min(c + 128, chunks - 1)];
+        dst[c] = v0;
+        if (c + 128 < chunks) dst[c + 128] = v1;
       }
+    }
+    t = next;
+  }
+}
+__global__ void __launch_bounds__(128) moe_gather_kernel(const uint4* x, int64_t ldx, uint4* out, int chunks, int parts /* of a row */,
+                                                         const int32_t* row_token, const int32_t* num_tiles) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int rows = *num_tiles * kMoeTileRows, lane = threadIdx.x & 31, step = gridDim.x * 4, first = blockIdx.x * 4 + (threadIdx.x >> 5);
+  int r = first / parts, part = first % parts;
+  int t = r < rows ? row_token[r] : -1;
+  while (r < rows) {
+    const int c0 = part * 256 + lane;
+    uint4* dst = out + static_cast<int64_t>(r) * chunks;
+    r += step / parts;
+    part += step % parts;
+    if (part >= parts) {
+      part -= parts;
+      ++r;
+    }
+    const int next = r < rows ? row_token[r] : -1;
+    if (t >= 0) {
+      const uint4* src = x + static_cast<int64_t>(t) * ldx;
+      uint4 v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = src[min(c0 + 32 * k, chunks - 1)];
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (c0 + 32 * k < chunks) dst[c0 + 32 * k] = v[k];
     }
     t = next;
   }
@@ -274,14 +301,18 @@ int mdb_moe_gather(int dtype, const void* x, int64_t ldx, void* out, int width, 
   if (max_tiles == 0) return MDB_OK;
   MDB_REQUIRE(x && out && row_token && num_tiles, MDB_ERR_ARG);
   MDB_REQUIRE(width % 8 == 0 && ldx % 8 == 0 && mdb_aligned16(x) && mdb_aligned16(out), MDB_ERR_ALIGN);
+  const int per = 16 / (dtype == MDB_F32 ? 4 : 2), chunks = width / per, parts = (chunks + 255) / 256;      // elements of a piece, pieces
   const int64_t rows = static_cast<int64_t>(max_tiles) * kMoeTileRows;
-  const int grid = static_cast<int>(rows < 148 * 16 ? rows : 148 * 16);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (dtype == MDB_F32)
-    return mdb_launch(moe_gather_kernel<float>, dim3(grid), dim3(128), 0, st, static_cast<const float*>(x), ldx,
-                      static_cast<float*>(out), width, row_token, num_tiles);
-  return mdb_launch(moe_gather_kernel<bf16>, dim3(grid), dim3(128), 0, st, static_cast<const bf16*>(x), ldx,
-                    static_cast<bf16*>(out), width, row_token, num_tiles);
+  const uint4* from = static_cast<const uint4*>(x);
+  uint4* to = static_cast<uint4*>(out);
+  int grid = 148 * 16;
+  if (rows <= grid && chunks <= 512)      // (300 of two of 8, 14 KB: 4.7 us so, 4.0 by the other form)
+    return mdb_launch(moe_gather_few_kernel, dim3(static_cast<unsigned>(rows)), dim3(128), 0, st, from, ldx / per, to, chunks, row_token, num_tiles);
+  const int tile = kMoeTileRows / 4 * parts;      // CTAs that a tile's rows keep busy at once
+  if (grid > tile) grid -= (grid - tile * 5 / 8) % tile;
+  if ((rows * parts + 3) / 4 < grid) grid = static_cast<int>((rows * parts + 3) / 4);
+  return mdb_launch(moe_gather_kernel, dim3(grid), dim3(128), 0, st, from, ldx / per, to, chunks, parts, row_token, num_tiles);
 }
 
 }  // extern "C"
