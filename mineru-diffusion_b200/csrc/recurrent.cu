@@ -1140,16 +1140,21 @@ int launch_scan_prompt(const mdb_scan_args& a, cudaStream_t st) {
   return mdb_launch(kernel, dim3((columns + COLS - 1) / COLS, a.heads, a.bs), dim3(threads), smem, st, a);
 }
 
+// Columns per CTA of a prompt's scan token by token: 32 while they fill the SMs, fewer (more re-reads of k, q and g) below that
+bool scan_wide(const mdb_scan_args& a) { return static_cast<int64_t>((a.vdim + 31) / 32) * a.heads * a.bs >= 148; }
+
 // Columns per CTA of the scan in blocks of 16 tokens, 0: token by token.
 //
 // The blocks shorten the chain of a sequence but leave an SM to one CTA, so they lose (by 5 to 55 %) once their CTAs no longer run all
-// at once; within that, 64 columns per CTA, or 32 or 16 where those still fit.  What is left is how many tokens make up for the
-// start and for a last block that is partly empty.  us token by token and in blocks, one token into a new block, 33 / 49 / 65 tokens:
-//   delta rule, columns 128: 16 heads (16 columns a CTA) 11.2 12.1 / 15.3 15.2 / 19.4 18.0; 32 (32) 14.9 15.5 / 20.7 19.9 / 26.2 24.1;
-//                            48 (64) 17.5 19.2 / 26.1 24.4 / 34.4 29.7; 64 (64) 23.0 19.2 / 33.0 24.5 / 42 30
-//   mLSTM, columns 256:      8 heads (16) 10.0 9.0 / 13.4 10.9; 16 (32) 11.8 10.4 / 16 12.7; 32 (64) 14.5 14.1 / 19.6 17.3
-//   decay scan, columns 64:  16 heads (16) 8.8 7.6 / 11.6 9.4; 48 (32) 10.4 9.7 / 13.6 11.9; 80 (64) 13.8 12.9; 128 (64) 13.8 13.3
-// and of 64 channels: delta rule 1.0 - 1.2 of the time whatever the form; decay scan 7.1 6.1 (16), no better with 32 and 64.
+// at once; within that, 64 columns per CTA, or 32 or 16 where those still fit.  What is left is how many tokens make up for the start
+// and for a last block that is partly empty.  Time in blocks over the time token by token, heads of 128 channels, one token into a new block,
+// 33 / 49 / 65 / 97 / 129 tokens, with the number of CTAs that the form token by token has (it is slow where some SMs have one more):
+//   delta rule  16 columns a CTA 1.15 1.05 1.00 0.93 0.89;  32: 160 CTAs 1.26 1.18 1.13 1.08 1.04, 240 - 288 1.18 1.11 1.07 1.00 0.96;
+//               64: 160 - 192 1.13 1.02 0.97 0.91 0.88, 240 - 288 0.99 0.91 0.86 0.81 0.77, two on every SM 1.19 1.08 1.03 0.98 0.95
+//   decay scan  16: 0.90 0.82 0.78 0.72 0.70;  32: 160 - 216 1.11 1.00 0.95 0.88 0.85, 224 - 288 1.00 0.93 0.86 0.78 0.75;
+//               64: 160 - 224 1.12 1.05 0.99 0.93 0.91, 240 - 288 1.02 0.94 0.89 0.83 0.80, two on every SM 1.13 1.04 1.00 0.92 0.89
+//   mLSTM       16 and 32: 1.00 0.95 0.88 0.81 0.78;  64: up to two on every SM 1.12 1.04 0.99 0.92 0.90, more 0.93 0.85 0.80 0.74 0.70
+// and of 64 channels: delta rule 1.0 - 1.2 of the time whatever the form; decay scan as with 128 (16), no better with 32 and 64.
 template <int MODE, int DP>
 int scan_block_columns(const mdb_scan_args& a, int64_t rows) {
   if (DP > 128 || (DP == 64 && MODE == kScanDelta)) return 0;
@@ -1158,10 +1163,20 @@ int scan_block_columns(const mdb_scan_args& a, int64_t rows) {
   if (ctas(64) > sms) return 0;
   const int cols = ctas(16) <= sms ? 16 : ctas(32) <= sms ? 32 : 64;
   if (MODE == kScanDecay && DP == 64 && cols != 16) return 0;
-  // tokens of a sequence on average
-  int least = 32;
-  if (MODE == kScanDelta && 4 * ctas(64) < 3 * sms) least = 64;
-  if (MODE == kScanMlstm && DP == 64 && cols != 16) least = 80;
+  const int per = scan_wide(a) ? 32 : 16;
+  const int64_t tokenwise = (a.vdim + (MODE == kScanMlstm ? 1 : 0) + per - 1) / per * heads;
+  const bool uneven = tokenwise * 5 >= 8 * sms && tokenwise < 2 * sms;      // most SMs have two CTAs, some one
+  int least = 32;                                       // tokens of a sequence on average
+  if (MODE == kScanMlstm) {
+    if (cols == 64 && tokenwise <= 2 * sms) least = 56;
+    if (cols != 16 && DP == 64) least = 80;
+  } else if (cols == 64) {
+    least = uneven ? 32 : MODE == kScanDelta && tokenwise >= 2 * sms ? 80 : 64;
+  } else if (MODE == kScanDelta) {
+    least = cols == 16 ? 64 : uneven ? 96 : 256;
+  } else if (cols == 32 && !uneven) {
+    least = 48;
+  }
   return rows >= static_cast<int64_t>(least) * a.bs ? cols : 0;
 }
 
@@ -1176,9 +1191,7 @@ int launch_scan_dim(const mdb_scan_args& a, int64_t rows, cudaStream_t st) {
       if (cols == 64) return launch_scan_blocks<MODE, DP, 64, 4>(a, st);
     }
   }
-  // blocks of 32 columns while they fill the SMs, narrower ones (more re-reads of k, q and g) below that
-  const int64_t wide = static_cast<int64_t>((a.vdim + 31) / 32) * a.heads * a.bs;
-  return wide >= 148 ? launch_scan_prompt<MODE, DP, 32>(a, st) : launch_scan_prompt<MODE, DP, 16>(a, st);
+  return scan_wide(a) ? launch_scan_prompt<MODE, DP, 32>(a, st) : launch_scan_prompt<MODE, DP, 16>(a, st);
 }
 
 template <int MODE>
