@@ -580,6 +580,8 @@ int mdb_scan(const mdb_scan_args* args, mdb_stream_t stream);
  * sequences, with heads of up to 128 channels, are scanned in blocks of 16 tokens.  The sums of a row are rounded in the order of
  * the form that is taken. */
 int mdb_scan_rows(const mdb_scan_args* args, int64_t rows, mdb_stream_t stream);
+/* The same, told the longest portion too (since version 103; 0: the portions are taken to be about as long as one another). */
+int mdb_scan_portions(const mdb_scan_args* args, int64_t rows, int64_t longest, mdb_stream_t stream);
 
 /* The decay scan over prompt portions in chunks of 64 tokens on the tensor cores: bf16 rows of ldq / ldk elements with head
  * g of q and k at column g * dim (dim a multiple of 8, missing channels up to dim_pad count as zeros) and rows of ldv elements

@@ -144,6 +144,7 @@ SIGNATURES = {
     "mdb_mlstm_prep": (_i, [C.POINTER(MlstmPrepArgs), _p]),
     "mdb_scan": (_i, [C.POINTER(ScanArgs), _p]),
     "mdb_scan_rows": (_i, [C.POINTER(ScanArgs), _i64, _p]),
+    "mdb_scan_portions": (_i, [C.POINTER(ScanArgs), _i64, _i64, _p]),
     "mdb_chunk_scan_supported": (_i, [_i, _i]),
     "mdb_chunk_scan": (_i, [C.POINTER(ChunkScanArgs), _p]),
     "mdb_moe_route": (_i, [C.POINTER(MoeRouteArgs), _p]),

@@ -444,7 +444,7 @@ const char* mdb_strerror(int code) {
   }
 }
 
-int mdb_version(void) { return 102; }
+int mdb_version(void) { return 103; }
 
 int mdb_set_trace(void* buffer, int64_t bytes) {
   TraceBuf t;

@@ -1156,13 +1156,18 @@ bool scan_wide(const mdb_scan_args& a) { return static_cast<int64_t>((a.vdim + 3
 //   mLSTM       16 and 32: 1.00 0.95 0.88 0.81 0.78;  64: up to two on every SM 1.12 1.04 0.99 0.92 0.90, more 0.93 0.85 0.80 0.74 0.70
 // and of 64 channels: delta rule 1.0 - 1.2 of the time whatever the form; decay scan as with 128 (16), no better with 32 and 64.
 template <int MODE, int DP>
-int scan_block_columns(const mdb_scan_args& a, int64_t rows) {
+int scan_block_columns(const mdb_scan_args& a, int64_t rows, int64_t longest) {
   if (DP > 128 || (DP == 64 && MODE == kScanDelta)) return 0;
   const int64_t heads = static_cast<int64_t>(a.heads) * a.bs, sms = at_sm_count();
   auto ctas = [&](int cols) { return (a.vdim + cols - 1) / cols * heads; };
   if (ctas(64) > sms) return 0;
   const int cols = ctas(16) <= sms ? 16 : ctas(32) <= sms ? 32 : 64;
   if (MODE == kScanDecay && DP == 64 && cols != 16) return 0;
+  // The columns fit the whole batch, but a portion much longer than the others is soon alone: a CTA of 64 columns then takes longer for a
+  // token than the form token by token does on an empty chip (seven portions of one token and one of 260, 16 heads of 64
+  // columns: delta rule 70 and 88 us, decay scan 50 and 55; the mLSTM 57 and 55).  Not where the rows would do for 4/5 of as many portions of that
+  // length as 64 columns are for.
+  if (longest > 0 && cols == 64 && MODE != kScanMlstm && (a.vdim + 31) / 32 * a.heads * rows * 5 <= sms * longest * 4) return 0;
   const int per = scan_wide(a) ? 32 : 16;
   const int64_t tokenwise = (a.vdim + (MODE == kScanMlstm ? 1 : 0) + per - 1) / per * heads;
   const bool uneven = tokenwise * 5 >= 8 * sms && tokenwise < 2 * sms;      // most SMs have two CTAs, some one
@@ -1181,9 +1186,9 @@ int scan_block_columns(const mdb_scan_args& a, int64_t rows) {
 }
 
 template <int MODE, int DP>
-int launch_scan_dim(const mdb_scan_args& a, int64_t rows, cudaStream_t st) {
+int launch_scan_dim(const mdb_scan_args& a, int64_t rows, int64_t longest, cudaStream_t st) {
   if (a.fused) return a.dtype == MDB_F32 ? launch_scan_token<float, MODE, DP / 32>(a, st) : launch_scan_token<bf16, MODE, DP / 32>(a, st);
-  const int cols = scan_block_columns<MODE, DP>(a, rows);
+  const int cols = scan_block_columns<MODE, DP>(a, rows, longest);
   if constexpr (DP == 128 || (DP == 64 && MODE != kScanDelta)) {
     if (cols == 16) return launch_scan_blocks<MODE, DP, 16, 2>(a, st);
     if constexpr (DP == 128 || MODE == kScanMlstm) {
@@ -1195,13 +1200,13 @@ int launch_scan_dim(const mdb_scan_args& a, int64_t rows, cudaStream_t st) {
 }
 
 template <int MODE>
-int launch_scan(const mdb_scan_args& a, int64_t rows, cudaStream_t st) {
+int launch_scan(const mdb_scan_args& a, int64_t rows, int64_t longest, cudaStream_t st) {
   switch (a.dim_pad) {
-    case 64: return launch_scan_dim<MODE, 64>(a, rows, st);
-    case 128: return launch_scan_dim<MODE, 128>(a, rows, st);
-    case 192: return launch_scan_dim<MODE, 192>(a, rows, st);
-    case 256: return launch_scan_dim<MODE, 256>(a, rows, st);
-    case 512: return launch_scan_dim<MODE, 512>(a, rows, st);
+    case 64: return launch_scan_dim<MODE, 64>(a, rows, longest, st);
+    case 128: return launch_scan_dim<MODE, 128>(a, rows, longest, st);
+    case 192: return launch_scan_dim<MODE, 192>(a, rows, longest, st);
+    case 256: return launch_scan_dim<MODE, 256>(a, rows, longest, st);
+    case 512: return launch_scan_dim<MODE, 512>(a, rows, longest, st);
     default: return MDB_ERR_UNSUPPORTED;
   }
 }
@@ -1345,10 +1350,12 @@ int mdb_mlstm_prep(const mdb_mlstm_prep_args* args, mdb_stream_t stream) {
                : mdb_launch(mlstm_prep_kernel<bf16, true, false>, grid, dim3(256), 0, st, a);
 }
 
-int mdb_scan(const mdb_scan_args* args, mdb_stream_t stream) { return mdb_scan_rows(args, 0, stream); }
+int mdb_scan(const mdb_scan_args* args, mdb_stream_t stream) { return mdb_scan_portions(args, 0, 0, stream); }
 
-int mdb_scan_rows(const mdb_scan_args* args, int64_t rows, mdb_stream_t stream) {
-  MDB_REQUIRE(args != nullptr && rows >= 0, MDB_ERR_ARG);
+int mdb_scan_rows(const mdb_scan_args* args, int64_t rows, mdb_stream_t stream) { return mdb_scan_portions(args, rows, 0, stream); }
+
+int mdb_scan_portions(const mdb_scan_args* args, int64_t rows, int64_t longest, mdb_stream_t stream) {
+  MDB_REQUIRE(args != nullptr && rows >= 0 && longest >= 0, MDB_ERR_ARG);
   const mdb_scan_args a = *args;
   MDB_REQUIRE(a.mode >= MDB_SCAN_DELTA && a.mode <= MDB_SCAN_DECAY, MDB_ERR_ARG);
   MDB_REQUIRE(a.bs >= 0 && a.heads > 0 && a.kv_heads > 0 && a.heads % a.kv_heads == 0 && a.dim > 0 && a.vdim > 0, MDB_ERR_ARG);
@@ -1368,8 +1375,8 @@ int mdb_scan_rows(const mdb_scan_args* args, int64_t rows, mdb_stream_t stream) 
               MDB_ERR_ALIGN);
   MDB_REQUIRE(a.heads <= 65535 && a.bs <= 65535, MDB_ERR_UNSUPPORTED);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (a.mode == MDB_SCAN_DECAY) return launch_scan<kScanDecay>(a, rows, st);
-  return a.mode == MDB_SCAN_DELTA ? launch_scan<kScanDelta>(a, rows, st) : launch_scan<kScanMlstm>(a, rows, st);
+  if (a.mode == MDB_SCAN_DECAY) return launch_scan<kScanDecay>(a, rows, longest, st);
+  return a.mode == MDB_SCAN_DELTA ? launch_scan<kScanDelta>(a, rows, longest, st) : launch_scan<kScanMlstm>(a, rows, longest, st);
 }
 
 }  // extern "C"

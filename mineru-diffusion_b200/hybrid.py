@@ -557,7 +557,7 @@ class HybridEngine:
                            b.max_q, o, skip=pw.get("skip"))
         else:
             ops.scan(ops.SCAN_DECAY, self.dtype, b.bs, heads, kvh, dim, vdim, *outs, st["s"], self._portions(b), out=o,
-                     skip=pw.get("skip"), one_token=one_token and ops.scan_fusable(dp, vdim))
+                     skip=pw.get("skip"), one_token=one_token and ops.scan_fusable(dp, vdim), max_q=b.max_q)
         leave()
 
     def _channel_delta(self, li: int, mx: ChannelDeltaSpec, lw: dict, h: torch.Tensor, b: StepBatch) -> ops.Rows:
@@ -586,7 +586,7 @@ class HybridEngine:
             scalars = self.buf("scan_scalars", m, heads, 4, dtype=f32)
             ops.channel_decay(raw, lw["a_log"], lw["dt_bias"], q, k, beta, self._portions(b), g, scalars, dim)
             o = self.buf("scan_o", m, heads, vdim, dtype=f32)
-            ops.scan(*common, g=g, scalars=scalars, out=o)
+            ops.scan(*common, g=g, scalars=scalars, out=o, max_q=b.max_q)
             ops.gated_norm(o, gate, lw["norm"], False, eps, y)
         return self._linear("mix_out", y, lw["o"])
 
@@ -609,7 +609,7 @@ class HybridEngine:
         else:
             o = self.buf("scan_o", m, heads, vdim, dtype=f32)
             den = self.buf("scan_den", m, heads, dtype=f32)
-            ops.scan(*args, out=o, den=den, mstate=st["m"])
+            ops.scan(*args, out=o, den=den, mstate=st["m"], max_q=b.max_q)
             ops.gated_norm(o, x.cols(g0), lw["norm"], True, eps, y, den=den)
         return self._linear("mix_out", y, lw["o"])
 

@@ -756,11 +756,12 @@ SCAN_DELTA, SCAN_MLSTM, SCAN_DECAY = 0, 1, 2
 def scan(mode: int, dtype: torch.dtype, bs: int, heads: int, kv_heads: int, dim: int, vdim: int, q, k, v, s0, s1, state,
          portions: tuple, eps: float = 0.0, g=None, scalars=None, mstate=None, den=None, out=None, raw_decay: Rows | None = None,
          a_log=None, dt_bias=None, gate: Rows | None = None, norm=None, per_head_norm: bool = False, y=None, skip=None,
-         one_token: bool = False) -> None:
+         one_token: bool = False, max_q: int = 0) -> None:
     """The recurrence over every sequence's portion; ``state`` [slots, heads, vdim (mLSTM: + 1), dim_pad] fp32.  With ``y``
     the fused one-token form runs (decay from ``raw_decay``, gated norm into ``y``), else ``out`` [m, heads, vdim] fp32
     (mLSTM: and ``den`` [m, heads]) is written.  Decay scan: s0 = decay, s1 = step, ``skip`` [heads] times v is added to the
-    read-out; ``one_token`` picks its one-token form."""
+    read-out; ``one_token`` picks its one-token form.  ``max_q`` = the longest portion, where the caller knows it (without it
+    they are taken to be about as long as one another); it bears on the form that is taken only."""
     _, cu_q, start, slot = portions
     a = _lib.ScanArgs(
         mode=mode, dtype=_DTYPES[dtype], fused=int(y is not None or one_token), bs=bs, heads=heads, kv_heads=kv_heads, dim=dim,
@@ -770,7 +771,7 @@ def scan(mode: int, dtype: torch.dtype, bs: int, heads: int, kv_heads: int, dim:
         out=_ptr(out), raw_decay=_rows_c(raw_decay), a_log=_ptr(a_log), dt_bias=_ptr(dt_bias), gate=_rows_c(gate),
         norm=_ptr(norm), norm_head_stride=vdim if per_head_norm else 0, y=_ptr(y), ldy=0 if y is None else _rows(y, "y"),
         skip=_ptr(skip))
-    _lib.check(_lib.lib().mdb_scan_rows(a, q.shape[0], _stream()), "mdb_scan_rows")
+    _lib.check(_lib.lib().mdb_scan_portions(a, q.shape[0], max_q, _stream()), "mdb_scan_portions")
 
 
 def chunk_scan_supported(dim_pad: int, vdim: int) -> bool:

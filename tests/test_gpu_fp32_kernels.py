@@ -304,3 +304,45 @@ def test_fp32_product_of_few_rows(form, n, k):
     for m in (1, 9, 33, 64, 100):
         assert torch.equal(product(x[:m]), whole[:m]), m
     assert pkg._lib.device_status() == 0
+
+
+# Either side of where blocks begin (96 tokens for the delta rule with 32 columns a CTA, 64 with 16, 48 for the decay scan), and portions of very unequal
+# length, told and not told: the form may change, the recurrence does not.  2e-6: as above.
+@pytest.mark.parametrize("mode,H,DV,counts", [(ops.SCAN_DELTA, 16, 128, [95, 95]), (ops.SCAN_DELTA, 16, 128, [96, 97]), (ops.SCAN_DELTA, 3, 40, [63]),
+                                              (ops.SCAN_DELTA, 3, 40, [64, 66]), (ops.SCAN_DECAY, 16, 80, [47, 47]), (ops.SCAN_DECAY, 16, 80, [48, 50]),
+                                              (ops.SCAN_DELTA, 16, 64, [1] * 7 + [260]), (ops.SCAN_DECAY, 16, 64, [1] * 7 + [260])])
+def test_scan_where_blocks_begin(mode, H, DV, counts):
+    D, g = 128, gen(21)
+    m = sum(counts)
+    k = torch.nn.functional.normalize(torch.randn(m, H, D, generator=g), dim=-1)
+    q, v, beta = torch.randn(m, H, D, generator=g) * D ** -0.5, torch.randn(m, H, DV, generator=g), torch.rand(m, H, generator=g)
+    decay = torch.exp(-torch.exp(torch.randn(m, H, D, generator=g) - 1))
+    if mode == ops.SCAN_DECAY:
+        decay = decay[..., :1].expand(m, H, D)
+    before = decay.double() * k.double().roll(1, 0)
+    sc = torch.stack([(k.double() * q.double()).sum(-1), (before * k.double()).sum(-1), (before * q.double()).sum(-1), beta.double()], -1).float().to(DEV)
+    p, got = _portions(counts, [0] * len(counts), list(range(len(counts)))), []
+    for longest in (0, max(counts)):
+        o, state = torch.full((m, H, DV), 9.0, device=DEV), torch.full((len(counts), H, DV, D), 5.0, device=DEV)
+        common = (mode, F32, len(counts), H, H, D, DV, q.to(DEV), k.to(DEV), v.to(DEV))
+        if mode == ops.SCAN_DELTA:
+            ops.scan(*common, None, None, state, p, g=decay.to(DEV), scalars=sc, out=o, max_q=longest)
+        else:
+            ops.scan(*common, decay[..., 0].contiguous().to(DEV), beta.to(DEV), state, p, out=o, max_q=longest)
+        at = 0
+        for n in counts:
+            r = slice(at, at + n)
+            at += n
+            qq, kk, vv, dd, bb = (t[r].double() for t in (q, k, v, decay, beta))
+            if mode == ops.SCAN_DELTA:
+                ref = orc.delta_scan(qq, kk, vv, dd, bb)
+            else:
+                S, ref = torch.zeros(H, DV, D, dtype=F64), []
+                for t in range(n):
+                    S = dd[t, :, 0][:, None, None] * S + bb[t][:, None, None] * vv[t][:, :, None] * kk[t][:, None]
+                    ref.append(torch.einsum("hvd,hd->hv", S, qq[t]))
+                ref = torch.stack(ref)
+            assert rel(o[r], ref) < 2e-6, (longest, n)
+        got.append(o)
+    assert torch.equal(*got) == (len(counts) < 8)      # the two forms round in their own order
+    assert pkg._lib.device_status() == 0
