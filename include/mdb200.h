@@ -336,7 +336,8 @@ int mdb_lmhead_tp_slots(int m, int cols);
 
 /* ---- decoders with an fp32 residual: recurrent mixers, latent attention, experts ----
  *
- * Activations are MDB_BF16 or MDB_F32 (argument `dtype`); in the fp32 form every product keeps fp32's 24 bits.  Argument
+ * Activations are MDB_BF16 or MDB_F32 (argument `dtype`); in the fp32 form every product of two numbers keeps
+ * fp32's 24 bits (mdb_gemm from k = 768 on: of numbers from 2^-122 on, in sums of sizes below the largest number).  Argument
  * blocks are host structs read during the call.  A "portion" is the run of tokens a sequence brings to a step:
  * rows [cu_q[s], cu_q[s + 1]) of the step, the first of them at position start[s] of the sequence.  state_slot[s]
  * is the sequence's slot in the state pools (-1: padding entry, skipped); a sequence at position 0 starts from a

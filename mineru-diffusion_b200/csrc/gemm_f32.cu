@@ -243,9 +243,13 @@ static int gemm_f32_dispatch(const mdb_gemm_args& a, cudaStream_t st) {
 static int gemm_f32_launch(const mdb_gemm_args& a, cudaStream_t st) {
   if (a.k % 16 != 0) return MDB_ERR_UNSUPPORTED;
   if ((static_cast<int64_t>(a.m) + 63) / 64 > 65535 || a.heads > 65535) return MDB_ERR_UNSUPPORTED;
-  // Above this k on the tensor cores, by k alone, so that a row's bits do not depend on how many rows there are.  Their form takes 6 to 9
-  // us for the smallest product: at k 512, 16 rows x 2048 columns lose by it (5.2 -> 7.0 us) and 500 rows gain; at k 1024 all but
-  // the narrowest gain, and its error, not k's root but level, is the smaller one.
+  // From this k on on the tensor cores, by k alone, so that a row's bits do not depend on how many rows there are.  us on FMAs and there,
+  // weights out of HBM, 1 / 8 / 16 / 500 rows:
+  //   k 512,  n 64   4.1 4.7 / 4.3 4.9 / 4.4 4.7 / 6.5 5.4       n 1024  4.5 5.5 / 4.5 5.6 / 4.7 5.7 / 18 11
+  //   k 640,  n 1024 5.6 6.4 / 5.5 6.5 / 5.7 6.5 / 22 12         n 4352  8.1 8.0 / 8.7 8.4 / 8.9 8.6 / 76 32
+  //   k 768,  n 64   5.6 5.4 / 5.8 5.4 / 6.1 5.4 / 9.3 6.2       n 1024  6.2 6.4 / 6.5 6.6 / 6.8 6.6 / 25 14
+  //   k 1024, n 1024 7.7 7.1 / 7.9 7.2 / 8.5 7.3 / 33 18         n 4352  12.0 10.2 / 12.7 10.6 / 13.1 10.8 / 117 45
+  // What loses at 768 is a few rows of 1600 to 2048 columns whose weights are in L2 (6.0 6.3 / 6.6 6.7 / 6.6 6.7).
   if (a.k >= 768) return gemm_f32_tc_launch(a, st);
   return a.act == MDB_ACT_RELU_GLU ? gemm_f32_dispatch<true>(a, st) : gemm_f32_dispatch<false>(a, st);
 }

@@ -29,7 +29,8 @@
 // products (116 KB).  500 rows, n x k 4352 x 1024, 45 us with eight products and with six; with six 32 without the loads, 35 with a
 // third of the parts' stores, 41 without splitting.  On FMAs it took 117; 1024 x 3072: 92 -> 35; 1024 x 1024: 33 -> 18.
 // Few rows: a chunk's latency, so the weight rows of a tile are as few as still run all at once, and rows of x that are not there are
-// not turned round (8 rows, 1024 x 1024, weights out of HBM: 9.4 us with 128 weight rows, 7.2 with 32; FMAs 7.9).  Not faster: two chunks
+// not turned round (8 rows, 1024 x 1024, weights out of HBM: 9.4 us with 128 weight rows, 7.2 with 32; FMAs 7.9).  Registers, 128 a
+// thread with 13 warps and 72 where two CTAs share an SM: 64 rows of x spill 16 bytes, tiles of 32 weight rows 40.  Not faster: two chunks
 // ahead in registers (9.4 against 8.6 out of L2), weights asked into L2 in front of the dependency wait (8.7 against 7.5).
 #include "mdb_common.cuh"
 

@@ -148,9 +148,10 @@ def test_scan_in_blocks_keeps_the_future_out():
     assert bool(torch.isfinite(o[:21]).all()) and not bool(torch.isfinite(o[21:T]).any()) and float(o[T:].abs().max()) == 0
 
 
-# From k = 768 on the products run on the tensor cores: tiles of 128 weight rows (64 with GLU) x 32 or 64 rows, chunks of 64 k, one to four
-# CTAs for a tile's k.  Sums of 64 products are cut off four times (2^-23 of a sum that is 1/16 of the whole in its square and
-# less) and added up in fp32: 2e-7 by measurement; 4e-7 leaves room for the activation, which doubles it.
+# From k = 768 on the products run on the tensor cores: tiles of 128, 64 or 32 weight rows (half of them up rows with GLU) x 32 or 64 rows, chunks
+# of 64 k, one to four CTAs for a tile's k.  Sums of 64 products are cut off four times (2^-23 of a sum that is 1/16 of the whole in its
+# square and less) and added up in fp32: 1e-7 by measurement; 4e-7 leaves room for the activation, which doubles it.  (Norms of dense
+# rows; outputs one by one, rows of few numbers and sums of one sign: test_fp32_product_output_by_output.)
 @pytest.mark.parametrize("m,n,k", [(1, 4, 768), (31, 132, 784), (33, 1000, 1040), (64, 260, 1552), (65, 4100, 768), (500, 1028, 3072), (1030, 2300, 816)])
 @pytest.mark.parametrize("act", [ops.ACT_NONE, ops.ACT_RELU2, ops.ACT_RELU_GLU, ops.ACT_SILU])
 def test_fp32_product_on_tensor_cores(m, n, k, act):
