@@ -19,10 +19,12 @@ _BF16 = torch.bfloat16
 _device, _raw_stream = (getattr(torch._C, name, None) for name in ("_cuda_getDevice", "_cuda_getCurrentRawStream"))
 
 
-def _stream() -> int:
-    if _device is None or _raw_stream is None:      # a torch without CUDA, or without these two
+if _device is None or _raw_stream is None:      # a torch without CUDA, or without these two
+    def _stream() -> int:
         return torch.cuda.current_stream().cuda_stream
-    return _raw_stream(_device())
+else:
+    def _stream() -> int:
+        return _raw_stream(_device())
 
 
 def _ptr(t: torch.Tensor | None) -> int | None:
