@@ -1140,21 +1140,20 @@ int launch_scan_prompt(const mdb_scan_args& a, cudaStream_t st) {
   return mdb_launch(kernel, dim3((columns + COLS - 1) / COLS, a.heads, a.bs), dim3(threads), smem, st, a);
 }
 
-// Columns per CTA of a prompt's scan token by token: 32 while they fill the SMs, fewer (more re-reads of k, q and g) below that
-bool scan_wide(const mdb_scan_args& a) { return static_cast<int64_t>((a.vdim + 31) / 32) * a.heads * a.bs >= 148; }
-
 // Columns per CTA of the scan in blocks of 16 tokens, 0: token by token.
 //
 // The blocks shorten the chain of a sequence but leave an SM to one CTA, so they lose (by 5 to 55 %) once their CTAs no longer run all
 // at once; within that, 64 columns per CTA, or 32 or 16 where those still fit.  What is left is how many tokens make up for the start
-// and for a last block that is partly empty.  Time in blocks over the time token by token, heads of 128 channels, one token into a new block,
-// 33 / 49 / 65 / 97 / 129 tokens, with the number of CTAs that the form token by token has (it is slow where some SMs have one more):
-//   delta rule  16 columns a CTA 1.15 1.05 1.00 0.93 0.89;  32: 160 CTAs 1.26 1.18 1.13 1.08 1.04, 240 - 288 1.18 1.11 1.07 1.00 0.96;
-//               64: 160 - 192 1.13 1.02 0.97 0.91 0.88, 240 - 288 0.99 0.91 0.86 0.81 0.77, two on every SM 1.19 1.08 1.03 0.98 0.95
-//   decay scan  16: 0.90 0.82 0.78 0.72 0.70;  32: 160 - 216 1.11 1.00 0.95 0.88 0.85, 224 - 288 1.00 0.93 0.86 0.78 0.75;
-//               64: 160 - 224 1.12 1.05 0.99 0.93 0.91, 240 - 288 1.02 0.94 0.89 0.83 0.80, two on every SM 1.13 1.04 1.00 0.92 0.89
-//   mLSTM       16 and 32: 1.00 0.95 0.88 0.81 0.78;  64: up to two on every SM 1.12 1.04 0.99 0.92 0.90, more 0.93 0.85 0.80 0.74 0.70
-// and of 64 channels: delta rule 1.0 - 1.2 of the time whatever the form; decay scan as with 128 (16), no better with 32 and 64.
+// and for a last block that is partly empty.  Measured behind the kernel that prepares the scan, as it always is in a model: there the form token by
+// token is slower than one scan behind another (2 x 115 tokens of 12 heads of 128 columns, delta rule with its decays, 53 us, where the scan alone takes
+// 35 and in blocks 41 and 36), as its CTAs share SMs that the kernel before still holds, and the blocks' cannot.  Preparing kernel and scan in
+// blocks over token by token, heads of 128 channels, one token into a new block, 33 / 49 / 65 / 129 / 257 tokens:
+//   delta rule  16 columns a CTA 0.75 - 1.09, 0.68 - 1.01, 0.63 - 0.96, 0.55 - 0.87, 0.51 - 0.76;  32: 1.01 0.93 0.89 0.79 0.76;  64: 0.79 0.75 0.68 0.65 0.58
+//   decay scan  16 and 32: 0.90 0.82 0.78 0.71 0.66;  64: 0.80 0.71 0.66 0.59 0.55
+//   mLSTM       16 and 32: 1.05 0.97 0.90 0.80 0.73;  64: up to two CTAs token by token on every SM 1.10 1.04 0.99 0.91 0.86, more 0.93 0.86 0.81 0.73 0.69
+// (The decay scan's with the mLSTM's preparing kernel in front.)  One scan behind another, 33 / 65 / 129 tokens: delta rule 16 columns 1.15 1.00 0.89, 32
+// 1.18 - 1.37, 1.03 - 1.24, 0.95 - 1.13, 64 0.99 - 1.19, 0.82 - 1.03, 0.73 - 0.95; decay scan 32 and 64 1.00 - 1.13, 0.83 - 1.00, 0.73 - 0.91.
+// Heads of 64 channels: delta rule 1.0 - 1.2 of the time whatever the form; decay scan as with 128 (16), no better with 32 and 64.
 template <int MODE, int DP>
 int scan_block_columns(const mdb_scan_args& a, int64_t rows, int64_t longest) {
   if (DP > 128 || (DP == 64 && MODE == kScanDelta)) return 0;
@@ -1163,25 +1162,15 @@ int scan_block_columns(const mdb_scan_args& a, int64_t rows, int64_t longest) {
   if (ctas(64) > sms) return 0;
   const int cols = ctas(16) <= sms ? 16 : ctas(32) <= sms ? 32 : 64;
   if (MODE == kScanDecay && DP == 64 && cols != 16) return 0;
-  // The columns fit the whole batch, but a portion much longer than the others is soon alone: a CTA of 64 columns then takes longer for a
-  // token than the form token by token does on an empty chip (seven portions of one token and one of 260, 16 heads of 64
-  // columns: delta rule 70 and 88 us, decay scan 50 and 55; the mLSTM 57 and 55).  Not where the rows would do for 4/5 of as many portions of that
-  // length as 64 columns are for.
-  if (longest > 0 && cols == 64 && MODE != kScanMlstm && (a.vdim + 31) / 32 * a.heads * rows * 5 <= sms * longest * 4) return 0;
-  const int per = scan_wide(a) ? 32 : 16;
-  const int64_t tokenwise = (a.vdim + (MODE == kScanMlstm ? 1 : 0) + per - 1) / per * heads;
-  const bool uneven = tokenwise * 5 >= 8 * sms && tokenwise < 2 * sms;      // most SMs have two CTAs, some one
+  // The columns fit the whole batch, but a portion much longer than the others is soon alone, and with few heads a CTA of 64 columns takes longer
+  // for a token than the form token by token does on an empty chip: delta rule with its decays, fifteen portions of one token and one of 500, four
+  // heads of 80 columns 135 us token by token, 169 in blocks; seven and one of 260, 4 heads of 160 1.27 of the time.  Only while its CTAs of 16 columns
+  // would fill less than 3/10 of the SMs (16 heads of 64 columns, seven and one of 260: 101 and 92), and not for the decay scan (94 and 104, 88 and 57).
+  if (MODE == kScanDelta && longest > 0 && cols == 64 && (a.vdim + 15) / 16 * a.heads * rows * 10 <= sms * longest * 3) return 0;
   int least = 32;                                       // tokens of a sequence on average
-  if (MODE == kScanMlstm) {
-    if (cols == 64 && tokenwise <= 2 * sms) least = 56;
-    if (cols != 16 && DP == 64) least = 80;
-  } else if (cols == 64) {
-    least = uneven ? 32 : MODE == kScanDelta && tokenwise >= 2 * sms ? 80 : 64;
-  } else if (MODE == kScanDelta) {
-    least = cols == 16 ? 64 : uneven ? 96 : 256;
-  } else if (cols == 32 && !uneven) {
-    least = 48;
-  }
+  if (MODE == kScanDelta && 4 * ctas(64) < 3 * sms) least = 64;
+  if (MODE == kScanMlstm && cols == 64 && (a.vdim + 32) / 32 * heads <= 2 * sms) least = 56;
+  if (MODE == kScanMlstm && DP == 64 && cols != 16) least = 80;
   return rows >= static_cast<int64_t>(least) * a.bs ? cols : 0;
 }
 
@@ -1196,7 +1185,9 @@ int launch_scan_dim(const mdb_scan_args& a, int64_t rows, int64_t longest, cudaS
       if (cols == 64) return launch_scan_blocks<MODE, DP, 64, 4>(a, st);
     }
   }
-  return scan_wide(a) ? launch_scan_prompt<MODE, DP, 32>(a, st) : launch_scan_prompt<MODE, DP, 16>(a, st);
+  // blocks of 32 columns while they fill the SMs, narrower ones (more re-reads of k, q and g) below that
+  const int64_t wide = static_cast<int64_t>((a.vdim + 31) / 32) * a.heads * a.bs;
+  return wide >= 148 ? launch_scan_prompt<MODE, DP, 32>(a, st) : launch_scan_prompt<MODE, DP, 16>(a, st);
 }
 
 template <int MODE>
