@@ -88,10 +88,9 @@ __global__ void __launch_bounds__(kRouteWarps * 32) moe_route_kernel(const mdb_m
 // list; beyond that (KEEP 0) the ids are read twice.  With up to 64 experts (FEW) half a warp has one, lists its tiles and marks the rows
 // that stay empty; with more of them a thread has one, and all rows are marked before they are given out.
 // us, two walks and all rows marked, tiles listed by the scan / now:
-//   8 experts, two a token:    1 token 2.2 / 1.8, 512 2.9 / 2.2, 1365 3.7 / 3.1, 4096 5.6 / 5.3
-//   64 experts, six a token:   1 token 2.8 / 2.3, 128 3.5 / 3.4, 512 5.1 / 4.7, 2048 11.2 / 11.0, 4096 19.8 / 18.7
+//   8 experts, two a token:    1 token 2.2 / 1.8, 512 2.9 / 2.2, 1365 3.7 / 3.1, 4096 5.6 / 5.2
+//   64 experts, six a token:   1 token 2.8 / 2.3, 128 3.5 / 3.4, 512 5.1 / 4.7, 2048 11.2 / 10.2, 4096 19.8 / 18.7
 //   256 experts, eight a token: 1 token 4.4 / 3.0, 128 7.4 / 5.4, 512 9.5 / 8.3, 2048 17.9 / 16.7
-// (More ids in registers: 2048 tokens of six of 64 experts 10.2 with 12, but with 24 for every number of ids 4.4 for one token.)
 constexpr int kPlanThreads = 1024, kPlanBatch = 8;
 template <int KEEP, bool FEW>
 __global__ void __launch_bounds__(kPlanThreads) moe_plan_kernel(const mdb_moe_plan_args a) {
@@ -288,9 +287,11 @@ int mdb_moe_plan(const mdb_moe_plan_args* args, mdb_stream_t stream) {
   MDB_REQUIRE(a.ids && a.slot && a.row_token && a.tile_expert && a.num_tiles, MDB_ERR_ARG);
   MDB_REQUIRE(a.experts <= 4096 && static_cast<int64_t>(a.m) * a.top < (1 << 30), MDB_ERR_UNSUPPORTED);
   const int each = (a.m * a.top + kPlanThreads - 1) / kPlanThreads;
-  const int keep = each < 1 || each > 4 ? 0 : each > 1 ? 4 : 1;
-  void (*const few)(mdb_moe_plan_args) = keep == 0 ? moe_plan_kernel<0, true> : keep == 1 ? moe_plan_kernel<1, true> : moe_plan_kernel<4, true>;
-  void (*const many)(mdb_moe_plan_args) = keep == 0 ? moe_plan_kernel<0, false> : keep == 1 ? moe_plan_kernel<1, false> : moe_plan_kernel<4, false>;
+  // ids in registers as far as they pay: up to 12 a thread with few experts (5 of them: 6.0 us with two walks, 5.5; 12: 11.0, 10.2; 24: 18.7,
+  // 18.2), up to four with many (8 of them: 10.7, 11.1).  An instance for more than there are costs 0.2 us an id.
+  void (*const few)(mdb_moe_plan_args) = each < 1 || each > 12 ? moe_plan_kernel<0, true> : each <= 1 ? moe_plan_kernel<1, true>
+                                         : each <= 4 ? moe_plan_kernel<4, true> : each <= 8 ? moe_plan_kernel<8, true> : moe_plan_kernel<12, true>;
+  void (*const many)(mdb_moe_plan_args) = each < 1 || each > 4 ? moe_plan_kernel<0, false> : each <= 1 ? moe_plan_kernel<1, false> : moe_plan_kernel<4, false>;
   void (*const kernel)(mdb_moe_plan_args) = a.experts <= 64 ? few : many;
   return mdb_launch(kernel, dim3(1), dim3(kPlanThreads), sizeof(int) * 2 * a.experts, static_cast<cudaStream_t>(stream), a);
 }
