@@ -423,7 +423,8 @@ static int gemm_f32_tc_run(const mdb_gemm_args& a, int ctas, cudaStream_t st) {
 // two and four (of a cluster of two the second CTA leaves two chains).  Clusters of four do not fill every SM: 33 run at once on 148.
 // Of 540 sizes (1 to 1000 rows, 64 to 8192 columns, k 768 to 3072) the form taken was within 8 % of the best of the twelve.
 struct FtForm { int rows, weights, chunk, rest[3]; };
-constexpr FtForm kFtForms[4] = {{64, 128, 108, {530, 900, 790}}, {32, 128, 87, {330, 560, 530}}, {32, 64, 70, {340, 460, 510}}, {32, 32, 58, {440, 540, 520}}};
+constexpr FtForm kFtForms[4] = {
+    {64, 128, 108, {530, 900, 790}}, {32, 128, 87, {390, 610, 530}}, {32, 64, 70, {390, 510, 510}}, {32, 32, 58, {440, 540, 520}}};
 template <bool GLU>
 static int gemm_f32_tc_dispatch(const mdb_gemm_args& a, cudaStream_t st) {
   const int chunks = (a.k + kFtK - 1) / kFtK;
