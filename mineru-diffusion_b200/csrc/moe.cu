@@ -194,8 +194,8 @@ __global__ void __launch_bounds__(kPlanThreads) moe_plan_kernel(const mdb_moe_pl
 }
 
 // Bound by memory and by a row's latencies, its place and its pieces; the next place is read meanwhile.  Few rows of up to 8 KB: a CTA per row, two
-// pieces of 16 bytes in flight per thread.  Many: a warp per row, or per eighth round of 512 bytes of it, all eight in flight, in steps that
-// shift a warp by 5/8 of a tile, as a tile's rows lie together and the rest of it is empty.
+// pieces of 16 bytes in flight per thread.  Many: a warp per row, or per 4 KB of it, in eight rounds of 512 bytes that are all in flight, and in
+// steps that shift a warp by 5/8 of a tile, as a tile's rows lie together and the rest of it is empty.
 // us, a CTA per row and a piece in flight per thread / now (a warp per row in steps of whole tiles beside them):
 //   rows of 4 KB:   2048 tokens of six of 64 experts 11.8 / 9.7 (9.7), 1000 6.2 / 5.8 (5.7), 300 of two of 8 2.0 / 2.1 (2.5)
 //   rows of 8 KB:   700 of eight of 160 11.2 / 10.5 (13.4), 700 of two of 8 3.8 / 3.6 (5.1)
